@@ -144,9 +144,6 @@ static void setup_one() {
 template <int MODE>
 static void setup_mode() { setup_one<MODE, 1>(); setup_one<MODE, 2>(); setup_one<MODE, 4>(); setup_one<MODE, 8>(); }
 
-template <int MODE>
-static int tc_smem_bytes() { return tc_smem_total(MODE); }
-
 extern "C" void coli_cuda_shutdown(void);
 
 static int decode_smem_bytes(int mode) {
@@ -196,8 +193,10 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<1>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         set_smem(k_moe_decode<SC_ROW>, decode_smem_bytes(SC_ROW)); set_smem(k_moe_decode<SC_H16>, decode_smem_bytes(SC_H16));
         set_smem(k_moe_decode<SC_F32>, decode_smem_bytes(SC_F32)); set_smem(k_moe_decode<SC_MX>, decode_smem_bytes(SC_MX));
-        set_smem(k_expert_gemm_tc<SC_ROW>, tc_smem_bytes<SC_ROW>()); set_smem(k_expert_gemm_tc<SC_H16>, tc_smem_bytes<SC_H16>());
-        set_smem(k_expert_gemm_tc<SC_MX>, tc_smem_bytes<SC_MX>());
+        set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
+        set_smem(k_expert_gemm_tc<SC_H16, 1>, tc_smem_total(SC_H16)); set_smem(k_expert_gemm_tc<SC_H16, 2>, tc_smem_total(SC_H16));
+        set_smem(k_expert_gemm_tc<SC_MX, 1>, tc_smem_total(SC_MX)); set_smem(k_expert_gemm_tc<SC_MX, 2>, tc_smem_total(SC_MX));
+        set_smem(k_tc_plan, 33 * ROUTE_MAX_E * (int)sizeof(int));
         if (!cuda_ok(cudaGetLastError(), "kernel attributes")) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
     }
     g_nctx = count;
@@ -337,8 +336,8 @@ static int scales_fit_half(const float *s, size_t n) {
 //   SC_ROW  integer codes, no shift
 //   SC_H16  scale * 2^shift puts the largest scale in [2^10, 2^11); every non-zero scale must
 //           lie within 2^-12 of the largest so that the hi/lo split keeps its low bits
-//   SC_MX   2^(e - 127 + 14 + shift) must be an fp16 power of two >= 2^-9 for every group
-//           that holds a non-zero code: shift = 128 - e_max, spread e_max - e <= 24
+//   SC_MX   2^(e - 127 + shift) must be an fp16 power of two <= 2^13 for every group that holds a
+//           non-zero code: shift = 140 - e_max, spread e_max - e <= TC_MX_SPREAD (down to 2^-11)
 static void tensor_tc_params(ColiCudaTensor *t, const void *weights, const void *scales) {
     t->tc_ok = 0; t->tc_shift = 0;
     if (!t->packed || (t->O % 128) || (t->I % 128)) return;
@@ -368,12 +367,12 @@ static void tensor_tc_params(ColiCudaTensor *t, const void *weights, const void 
         for (size_t i = 0; i < scount; i++) { if (e8[i] == 255) return; if (e8[i] > emax) emax = e8[i]; }
         const size_t rb = (size_t)t->I / 2;
         for (size_t i = 0; i < scount; i++) {
-            if (emax - (int)e8[i] <= 24) continue;
+            if (emax - (int)e8[i] <= TC_MX_SPREAD) continue;
             const size_t row = i / t->ng, g = i % t->ng;
             const uint8_t *c = q + row * rb + g * 16;
             for (int b = 0; b < 16; b++) if (c[b] & 0x77) return;   // a live group below the exact range
         }
-        t->tc_shift = 128 - emax; t->tc_ok = 1;
+        t->tc_shift = 140 - emax; t->tc_ok = 1;
     }
 }
 
@@ -419,8 +418,9 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
     const size_t pkbytes = nblk * ch;
     if (!reserve(c, &c->stage_w, wbytes) || (sbytes && !reserve(c, &c->stage_s, sbytes))) return 0;
     if (allocate) {
-        if (!cuda_ok(cudaMalloc((void **)&t->pk, pkbytes), "tensor allocation")) return 0;
-        t->physical_bytes = pkbytes;
+        // behind the tile streams: the tensor shift, for kernels that find the tensor by its address
+        if (!cuda_ok(cudaMalloc((void **)&t->pk, pkbytes + TC_TAIL_BYTES), "tensor allocation")) return 0;
+        t->physical_bytes = pkbytes + TC_TAIL_BYTES;
         if (mode == SC_ROW) {
             if (!cuda_ok(cudaMalloc((void **)&t->rowscale, (size_t)t->O * sizeof(float)), "scale allocation")) return 0;
             t->physical_bytes += (size_t)t->O * sizeof(float);
@@ -430,13 +430,15 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
     if (mode == SC_ROW) {
         if (!cuda_ok(cudaMemcpyAsync(t->rowscale, scales, (size_t)t->O * sizeof(float), cudaMemcpyHostToDevice, c->stream), "scale upload")) return 0;
     } else if (!cuda_ok(cudaMemcpyAsync(c->stage_s.p, scales, sbytes, cudaMemcpyHostToDevice, c->stream), "scale upload")) return 0;
+    if (!cuda_ok(cudaMemcpyAsync(t->pk + pkbytes, &t->tc_shift, sizeof(int), cudaMemcpyHostToDevice, c->stream), "tensor shift")) return 0;
     size_t words = nblk * 512;
     k_repack_codes<<<(unsigned)((words + 255) / 256), 256, 0, c->stream>>>(
         t->pk, static_cast<const uint8_t *>(c->stage_w.p), t->O, t->I, ch, t->fmt == 7);
     if (mode != SC_ROW) {
         size_t n = nblk * 128;
         k_repack_scales<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
-            t->pk, c->stage_s.p, t->O, t->I, ch, mode, t->gs > 0 ? t->gs : t->I, t->ng);
+            t->pk, c->stage_s.p, t->O, t->I, ch, mode, t->gs > 0 ? t->gs : t->I, t->ng,
+            mode == SC_MX && t->tc_ok ? 140 - t->tc_shift - TC_MX_SPREAD : 0);
     }
     if (!cuda_ok(cudaGetLastError(), "repack launch")) return 0;
     return cuda_ok(cudaStreamSynchronize(c->stream), "tensor upload sync");
@@ -812,155 +814,124 @@ static int group_shape_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
 // Tensor-core path of the expert group (gemm_tc.cuh): taken when some expert has
 // more rows than one streaming pass holds and every tensor qualifies.
 // ---------------------------------------------------------------------------
-// 0: never; 1: when it pays (below); 2: whenever the tensors and shapes allow it (tests).
-// A pass of the tensor-core kernel costs the same for 1 or 128 rows (the MMA is 128 rows
-// tall) while the streaming kernel's cost grows with the rows (it is bound by instruction
-// issue, one set of MMAs per 4 rows). Measured crossover on both benchmark shapes: a mean
-// of about 12 rows per expert (OLMoE shape: 3.2 vs 5.2 ms per 16 layers at 8 rows per
-// expert, 6.1 vs 5.2 ms at 16; DeepSeek-V3 shape: 8.1 vs 9.4 ms per 2 layers at 8, 18.8 vs
-// 10.2 ms at 16).
+// 0: never; 1: when it pays (tc_pays); 2: whenever the tensors and shapes allow it (tests).
 static int g_tc_enabled = 1;
 extern "C" void coli_cuda_set_tensor_core(int enabled) { g_tc_enabled = enabled < 0 ? 0 : enabled > 2 ? 2 : enabled; }
-#define TC_MIN_ROWS 13
-#define TC_MEAN_ROWS 12
+// The streaming kernel's cost grows with the rows (instruction issue: one set of MMAs per 4 rows and
+// block of weights), the tensor-core path's hardly does up to 30 rows per expert, but it has three launches
+// more. Measured: OLMoE shape (226 MB a layer), streaming / tensor cores: 2 rows per expert 106 / 156 us, 4 rows
+// 141 / 160, 8 rows 199 / 166, 31 rows 512 / 196; DeepSeek-V3 shape (6 GB): half a row 651 / 630, 2 rows
+// 1420 / 1255, 16 rows 9049 / 1848. So: from a mean of 6 rows per expert, or from half a GB of weights.
+static bool tc_pays(long rows, long experts, long D, long I) {
+    const double touched = (double)(rows < experts ? rows : experts) * 1.6 * (double)D * (double)I;
+    return rows >= 6 * experts || touched > 512e6;
+}
 
-template <int MODE>
-static void launch_tc_mode(DeviceCtx *c, const TcSeg *segs, const TcCtl *ctl, int ntask) {
-    int grid = ntask < c->sms ? ntask : c->sms;
+template <int MODE, int PHASE>
+static void launch_tc_one(DeviceCtx *c, const TcArgs &a) {
+    k_expert_gemm_tc<MODE, PHASE><<<c->sms, TC_THREADS, tc_smem_total(MODE), c->stream>>>(a);
+}
+static int launch_tc(DeviceCtx *c, int mode, int phase, const TcArgs &a) {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     kernel_event_pair(c, &e0, &e1);
     if (e0) cudaEventRecord(e0, c->stream);
-    k_expert_gemm_tc<MODE><<<grid, TC_THREADS, tc_smem_bytes<MODE>(), c->stream>>>(segs, ctl, c->status);
+    switch (mode * 2 + phase - 1) {
+    case SC_ROW * 2: launch_tc_one<SC_ROW, 1>(c, a); break;
+    case SC_ROW * 2 + 1: launch_tc_one<SC_ROW, 2>(c, a); break;
+    case SC_H16 * 2: launch_tc_one<SC_H16, 1>(c, a); break;
+    case SC_H16 * 2 + 1: launch_tc_one<SC_H16, 2>(c, a); break;
+    case SC_MX * 2: launch_tc_one<SC_MX, 1>(c, a); break;
+    case SC_MX * 2 + 1: launch_tc_one<SC_MX, 2>(c, a); break;
+    default: return 0;
+    }
     if (e1) cudaEventRecord(e1, c->stream);
     c->last_launches++;
+    return 1;
 }
 
-struct TcSegs {
-    std::vector<TcSeg> v[4];
-    int ntask[4] = {0, 0, 0, 0};
-};
-static void add_tc_seg(TcSegs *ts, const ColiCudaTensor *t, float *out, const __half *bq, const float *binv,
-                       const int *lo_flag, int nrows, int npad, int pos0, const int *rowdst = nullptr) {
-    TcSeg s;
-    std::memset(&s, 0, sizeof(s));
-    s.w = t->pk; s.rowscale = t->rowscale; s.bq = bq; s.binv = binv; s.lo_flag = lo_flag; s.out = out;
-    s.rowdst = rowdst;
-    s.nrows = nrows; s.npad = npad; s.pos0 = pos0;
-    s.O = t->O; s.nkb64 = t->I / TC_KB;
-    s.task0 = ts->ntask[t->mode];
-    s.shift = t->tc_shift;
-    s.out_scale = std::ldexp(1.0f, -t->tc_shift);
-    ts->ntask[t->mode] += (t->O + TC_FEAT - 1) / TC_FEAT;
-    ts->v[t->mode].push_back(s);
+// Device memory of a pass list with its tables, cut out of one block. `pass` comes first, then everything the
+// host may upload with it (grp_pass, rowsrc) and the rest.
+static size_t tc_list_layout(TcList *l, void *mem, int npass_cap, int ngrp_cap, int nrow_cap) {
+    uint8_t *p = static_cast<uint8_t *>(mem);
+    l->pass = reinterpret_cast<TcPass *>(p);
+    int *q = reinterpret_cast<int *>(l->pass + npass_cap);
+    l->npass = q; l->ngrp = q + 1; q += 4;
+    l->lo_x = q; q += npass_cap;
+    l->lo_h = q; q += npass_cap;
+    l->grp_pass = q; q += ngrp_cap;
+    l->rowsrc = nrow_cap ? q : nullptr; q += nrow_cap;
+    l->rowdst = nullptr;
+    return reinterpret_cast<uint8_t *>(q) - p;
 }
-static int run_tc_segs(DeviceCtx *c, TcSegs *ts, Buf *segbuf) {
-    size_t total = 0;
-    for (int m = 0; m < 4; m++) total += ts->v[m].size();
-    const size_t seg_bytes = total * sizeof(TcSeg), need = seg_bytes + 4 * sizeof(TcCtl);
-    if (!reserve(c, segbuf, need)) return 0;
-    std::vector<uint8_t> stage(need);   // pageable: captured by the copy call before it returns
-    uint8_t *hp = stage.data(), *dp = static_cast<uint8_t *>(segbuf->p);
-    size_t off = 0, seg_off[4];
-    TcCtl ctl[4];
-    for (int m = 0; m < 4; m++) {
-        seg_off[m] = off;
-        size_t b = ts->v[m].size() * sizeof(TcSeg);
-        if (b) std::memcpy(hp + off, ts->v[m].data(), b);
-        off += b;
-        ctl[m].nseg = (int)ts->v[m].size(); ctl[m].ntask = ts->ntask[m];
-    }
-    std::memcpy(hp + seg_bytes, ctl, sizeof(ctl));
-    if (!cuda_ok(cudaMemcpyAsync(dp, hp, need, cudaMemcpyHostToDevice, c->stream), "segment upload")) return 0;
-    for (int m = 0; m < 4; m++) {
-        if (ts->v[m].empty()) continue;
-        const TcSeg *sp = reinterpret_cast<const TcSeg *>(dp + seg_off[m]);
-        const TcCtl *cp = reinterpret_cast<const TcCtl *>(dp + seg_bytes) + m;
-        if (m == SC_ROW) launch_tc_mode<SC_ROW>(c, sp, cp, ts->ntask[m]);
-        else if (m == SC_H16) launch_tc_mode<SC_H16>(c, sp, cp, ts->ntask[m]);
-        else if (m == SC_MX) launch_tc_mode<SC_MX>(c, sp, cp, ts->ntask[m]);
-        else return 0;
-    }
+
+// The expert FFN over a pass list that is already on the device (built there by k_tc_plan, or
+// uploaded): rows x -> prepared tiles -> gate/up with the SwiGLU -> prepared tiles -> down -> y.
+//   npos_cap positions and ngrp_cap padded groups of 16 at most; x rows are bf16 when x_bf16.
+static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const void *x, int x_bf16, int npos_cap, int ngrp_cap,
+                  int D, int I, float *y) {
+    const size_t rows = (size_t)ngrp_cap * 16;
+    if (!reserve(c, &c->bq, rows * D * 2 * sizeof(__half)) || !reserve(c, &c->bs, (size_t)npos_cap * 2 * sizeof(float)) ||
+        !reserve(c, &c->pg, (size_t)npos_cap * I * sizeof(float)) || !reserve(c, &c->hq, rows * I * 2 * sizeof(__half))) return 0;
+    __half *xq = (__half *)c->bq.p, *hq = (__half *)c->hq.p;
+    float *xinv = (float *)c->bs.p, *hinv = xinv + npos_cap, *H = (float *)c->pg.p;
+    k_prep_tc<<<ngrp_cap * 8, TC_PREP_THREADS, 0, c->stream>>>(xq, xinv, l.lo_x, x, l.rowsrc, l.pass, l.grp_pass, l.ngrp, D, x_bf16);
+    TcArgs a;
+    a.pass = l.pass; a.npass = l.npass; a.status = c->status;
+    a.lo = l.lo_x; a.q = xq; a.qinv = xinv; a.rowdst = nullptr; a.out = H; a.K = D; a.O = I; a.ntile = I / 64;
+    if (!launch_tc(c, mode_gu, 1, a)) return 0;
+    k_prep_tc<<<ngrp_cap * 8, TC_PREP_THREADS, 0, c->stream>>>(hq, hinv, l.lo_h, H, nullptr, l.pass, l.grp_pass, l.ngrp, I, 0);
+    a.lo = l.lo_h; a.q = hq; a.qinv = hinv; a.rowdst = l.rowdst; a.out = y; a.K = I; a.O = D; a.ntile = D / 128;
+    if (!launch_tc(c, mode_d, 2, a)) return 0;
+    c->last_launches += 2;
     return cuda_ok(cudaGetLastError(), "tensor-core gemm launch");
 }
 
 static int group_tc_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                        ColiCudaTensor *const *downs, int count, int max_rows, int total) {
-    if (!g_tc_enabled || max_rows < TC_MIN_ROWS) return 0;
-    if (g_tc_enabled == 1 && (long)total < (long)TC_MEAN_ROWS * count) return 0;
+    if (!g_tc_enabled || max_rows < 2) return 0;
+    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->I, gates[0]->O)) return 0;
     for (int e = 0; e < count; e++)
-        if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok) return 0;
+        if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok || gates[e]->mode != gates[0]->mode ||
+            ups[e]->mode != gates[0]->mode || downs[e]->mode != downs[0]->mode) return 0;
     return 1;
 }
 
-// x_dev [total (or 1 when bcast), D] -> y_dev [total, D]; passes of up to 128 rows per expert.
-// y_dev must be 16-byte aligned (the accumulators are stored as float4).
-// rowsrc (host, optional): source row of x for every row of the call (a gather).
-// scatter_out: with rowsrc, the result of row r also goes to row rowsrc[r] of y_dev (the call
-// then works in place on a buffer whose rows are grouped differently: the expert-parallel layer).
+// x_dev [total (or 1 when bcast), D] -> y_dev [total, D].
+// rowmap (host, optional): row of x of every packed position (a gather), and the row of y its
+// result goes to (the expert-parallel layer works in place on differently grouped rows).
 // x_bf16: x_dev holds bf16 rows.
 static int group_device_tc(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                            ColiCudaTensor *const *downs, const int *rows, int count, int D, int I,
-                           int total, float *y_dev, const float *x_dev, int bcast, const int *rowsrc = nullptr,
-                           int scatter_out = 0, int x_bf16 = 0) {
-    // device tables: [rowsrc (total) | per pass: row0, npad, pos0, rows, lo flag of x, lo flag of h | per row group: pass, rg]
-    std::vector<int> pass_row0, pass_npad, pass_rows, pass_pos0, pass_expert, grp_pass, grp_rg;
-    int off = 0, padded = 0;
+                           int total, float *y_dev, const void *x_dev, int bcast, const int *rowmap = nullptr,
+                           int x_bf16 = 0) {
+    int npass = 0, ngrp = 0;
     for (int e = 0; e < count; e++) {
         const int re = rows ? rows[e] : 1;
-        for (int r0 = 0; r0 < re; r0 += TC_ROWS) {
-            const int nr = re - r0 < TC_ROWS ? re - r0 : TC_ROWS, npad = (nr + 15) & ~15;
-            const int p = (int)pass_row0.size();
-            pass_row0.push_back(padded); pass_npad.push_back(npad); pass_rows.push_back(nr);
-            pass_pos0.push_back(off + r0); pass_expert.push_back(e);
-            for (int g = 0; g < npad / 8; g++) { grp_pass.push_back(p); grp_rg.push_back(g); }
-            padded += npad;
+        npass += (re + TC_ROWS - 1) / TC_ROWS; ngrp += tc_pass_groups(re);
+    }
+    const int nmap = rowmap || bcast ? total : 0;
+    TcList dl, hl;
+    const size_t need = tc_list_layout(&dl, nullptr, npass, ngrp, nmap);
+    if (!reserve(c, &c->misc, need)) return 0;
+    std::vector<uint8_t> stage(need, 0);   // pageable: captured by the copy call before it returns
+    tc_list_layout(&hl, stage.data(), npass, ngrp, nmap);
+    tc_list_layout(&dl, c->misc.p, npass, ngrp, nmap);
+    int off = 0, p = 0, grp = 0;
+    for (int e = 0; e < count; e++) {
+        const int re = rows ? rows[e] : 1, rp = tc_pass_rows(re);
+        for (int r0 = 0; r0 < re; r0 += rp, p++) {
+            const int nr = re - r0 < rp ? re - r0 : rp, npad = (nr + 15) & ~15;
+            hl.pass[p] = TcPass{gates[e]->pk, ups[e]->pk, downs[e]->pk, gates[e]->rowscale, ups[e]->rowscale, downs[e]->rowscale,
+                                off + r0, nr, npad, grp * 16, gates[e]->tc_shift, ups[e]->tc_shift, downs[e]->tc_shift};
+            for (int i = 0; i < npad / 16; i++) hl.grp_pass[grp++] = p;
         }
         off += re;
     }
-    const int npass = (int)pass_row0.size(), ngrp = (int)grp_pass.size();
-    std::vector<int> meta((size_t)total + 6 * npass + 2 * ngrp, 0);
-    for (int r = 0; r < total; r++) meta[r] = rowsrc ? rowsrc[r] : bcast ? 0 : r;
-    int *mp = meta.data() + total;
-    for (int p = 0; p < npass; p++) {
-        mp[p] = pass_row0[p]; mp[npass + p] = pass_npad[p]; mp[2 * npass + p] = pass_pos0[p]; mp[3 * npass + p] = pass_rows[p];
-    }
-    int *mg = mp + 6 * npass;
-    for (int g = 0; g < ngrp; g++) { mg[g] = grp_pass[g]; mg[ngrp + g] = grp_rg[g]; }
-    if (!reserve(c, &c->misc, meta.size() * sizeof(int)) ||
-        !reserve(c, &c->bq, (size_t)padded * D * 2 * sizeof(__half)) ||
-        !reserve(c, &c->bs, (size_t)total * sizeof(float)) ||
-        !reserve(c, &c->pg, (size_t)total * I * sizeof(float)) ||
-        !reserve(c, &c->pu, (size_t)total * I * sizeof(float)) ||
-        !reserve(c, &c->hq, (size_t)padded * I * 2 * sizeof(__half)) ||
-        !reserve(c, &c->hs, (size_t)total * sizeof(float))) return 0;
-    if (!cuda_ok(cudaMemcpyAsync(c->misc.p, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream), "row table upload")) return 0;
-    int *d_meta = static_cast<int *>(c->misc.p);
-    const int *d_rowsrc = d_meta;
-    const int *d_pass_row0 = d_meta + total, *d_pass_npad = d_pass_row0 + npass, *d_pass_pos0 = d_pass_npad + npass,
-              *d_pass_rows = d_pass_pos0 + npass;
-    int *d_lo_x = d_meta + total + 4 * npass, *d_lo_h = d_lo_x + npass;
-    const int *d_grp_pass = d_meta + total + 6 * npass, *d_grp_rg = d_grp_pass + ngrp;
-    __half *bq = (__half *)c->bq.p, *hq = (__half *)c->hq.p;
-    float *binv = (float *)c->bs.p, *hinv = (float *)c->hs.p, *G = (float *)c->pg.p, *U = (float *)c->pu.p;
-    k_prep_umma<<<ngrp, 256, 0, c->stream>>>(bq, binv, x_dev, nullptr, d_rowsrc, d_grp_pass, d_grp_rg, d_pass_row0,
-                                             d_pass_npad, d_pass_pos0, d_pass_rows, d_lo_x, D, x_bf16);
-    c->last_launches++;
-    TcSegs t1, t2;
-    for (int p = 0; p < npass; p++) {
-        const int e = pass_expert[p];
-        const __half *bp = bq + (size_t)2 * D * pass_row0[p];
-        const __half *hp = hq + (size_t)2 * I * pass_row0[p];
-        add_tc_seg(&t1, gates[e], G, bp, binv + pass_pos0[p], d_lo_x + p, pass_rows[p], pass_npad[p], pass_pos0[p]);
-        add_tc_seg(&t1, ups[e], U, bp, binv + pass_pos0[p], d_lo_x + p, pass_rows[p], pass_npad[p], pass_pos0[p]);
-        add_tc_seg(&t2, downs[e], y_dev, hp, hinv + pass_pos0[p], d_lo_h + p, pass_rows[p], pass_npad[p], pass_pos0[p],
-                   scatter_out ? d_rowsrc : nullptr);
-    }
-    if (!run_tc_segs(c, &t1, &c->segs1)) return 0;
-    k_prep_umma<<<ngrp, 256, 0, c->stream>>>(hq, hinv, G, U, nullptr, d_grp_pass, d_grp_rg, d_pass_row0, d_pass_npad,
-                                             d_pass_pos0, d_pass_rows, d_lo_h, I, 0);
-    c->last_launches++;
-    if (!run_tc_segs(c, &t2, &c->segs2)) return 0;
-    return cuda_ok(cudaGetLastError(), "expert group launch");
+    *hl.npass = p; *hl.ngrp = grp;
+    if (rowmap) std::memcpy(hl.rowsrc, rowmap, (size_t)total * sizeof(int));   // (bcast: all zero)
+    if (!cuda_ok(cudaMemcpyAsync(c->misc.p, stage.data(), need, cudaMemcpyHostToDevice, c->stream), "pass list upload")) return 0;
+    dl.rowdst = rowmap ? dl.rowsrc : nullptr;
+    return tc_ffn(c, gates[0]->mode, downs[0]->mode, dl, x_dev, x_bf16, total, ngrp, D, I, y_dev);
 }
 
 static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
@@ -1502,8 +1473,8 @@ extern "C" int coli_cuda_ep_expert_group_dev(ColiCudaTensor *const *gates, ColiC
     int ok;
     if (all_packed && D % 128 == 0 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(y_dev) & 15) == 0 &&
         group_tc_ok(g.data(), u.data(), d.data(), (int)g.size(), max_rows, total)) {
-        ok = group_device_tc(c, g.data(), u.data(), d.data(), rows.data(), (int)g.size(), D, I, total, y_dev,
-                             static_cast<const float *>(x_dev), 0, rowmap.data(), 1, x_bf16);
+        ok = group_device_tc(c, g.data(), u.data(), d.data(), rows.data(), (int)g.size(), D, I, total, y_dev, x_dev, 0,
+                             rowmap.data(), x_bf16);
     } else {
         if (!reserve(c, &c->ep_ws, ((size_t)n) * sizeof(int)) || !reserve(c, &c->ep_x, (size_t)n * D * sizeof(float)) ||
             !reserve(c, &c->ep_y, (size_t)n * D * sizeof(float))) return 0;

@@ -13,48 +13,53 @@
 //
 // A matrix W[O, I] (O output rows, I = contraction length) is cut into tiles
 // of 32 output rows; a tile is cut along I into blocks of 128 columns. One
-// block is stored as one contiguous chunk
-//     [2048 B of 4-bit codes][scale bytes]
+// block is stored as one contiguous chunk of two halves of 16 rows each,
+//     [1024 B of 4-bit codes][scale bytes] [1024 B of 4-bit codes][scale bytes]
 // and the chunks of a tile follow each other in ascending column order, so a
 // tile's whole contraction is one linear stream (bulk-copyable without a
-// tensor map) and any column range of it is contiguous as well.
+// tensor map), any column range of it is contiguous, and so is one half of a
+// block (kernels that work on 16 rows copy just that).
 //
-// Inside the 2048-byte code part the order is the register order of the
+// Inside the 1024 code bytes of a half the order is the register order of the
 // m16n8k16 tensor-core A fragment, so a lane's 128-bit shared-memory load
 // yields finished fragments: with lane = g*4+t (g = 0..7, t = 0..3), slot
-// j = sub*2+h (sub = 16-row half of the tile, h = row g or g+8) sits at byte
-// j*512 + lane*16 and holds four 32-bit words, one per 32-column group. Word
-// (j, lane, grp) carries row sub*16+h*8+g, columns grp*32 + 8t + {0..7}, as
-// eight 4-bit fields in the order {0,2,4,6,1,3,5,7} (field f at bits 4f..4f+3),
-// which lets two mask operations split a word into the (k, k+1) half2 pairs
-// the fragment wants. (A group-major order with 32-bit loads and a rolled loop
-// over the groups was measured slower: the kernels are bound by the integer
-// pipe, so fewer, wider loads win over a smaller instruction footprint.)
-//   int4 (fmt 2, 4): a field is the stored offset-binary nibble (value+8).
-//   MXFP4 (fmt 7):   the four (k,k+1) pairs A,B,C,D of a word are re-encoded so
-//                    that each decodes with shifts and masks straight into
-//                    fp16 bit patterns: per 16-bit half, magnitude bits
-//                    (e1 e0 m) at 11..9 / 8..6 / 5..3 / 2..0 and sign bits at
-//                    15 / 12 / 13 / 14 for A/B/C/D. An fp16 with those three
-//                    bits in its exponent/mantissa top is e2m1 * 2^-14.
+// h (row g or g+8 of the half) sits at byte h*512 + lane*16 and holds four
+// 32-bit words, one per 32-column group. Word (h, lane, grp) carries row
+// h*8+g, columns grp*32 + 8t + {0..7}, as eight 4-bit fields:
+//   int4 (fmt 2, 4): the stored offset-binary nibbles (value+8) in the order
+//                    {0,2,4,6,1,3,5,7} (field f at bits 4f..4f+3), which lets
+//                    two mask operations split a word into the (k, k+1) half2
+//                    pairs the fragment wants.
+//   MXFP4 (fmt 7):   the container's bytes (columns 2b and 2b+1 in byte b): one
+//                    e2m1x2 -> f16x2 conversion per pair (12 issue cycles per word with
+//                    its multiply, against 18 for shifts and masks that place the fields).
 //
-// Scale part, by mode (always four 32-column slots per block; a group size of
-// 64 or 128 repeats its scale):
+// Scale part of a half, by mode (always four 32-column slots per block; a group
+// size of 64 or 128 repeats its scale), in the order [g][pair][h][i] for column
+// group grp = 2*pair + i:
 //   SC_ROW   nothing (one f32 per output row lives in a separate array)
-//   SC_H16   fp16 [sub][g][h][grp]  (256 B)  int4 scales that are exact in fp16
-//   SC_F32   f32  [sub][g][h][grp]  (512 B)  any other int4 scale
-//   SC_MX    u8   [sub][g][h][grp]  (128 B)  ue8m0 exponents
+//   SC_H16   fp16 (128 B)  int4 scales that are exact in fp16
+//   SC_F32   f32  (256 B)  any other int4 scale
+//   SC_MX    u8   (64 B)   ue8m0 exponents; of a tensor that qualifies for the
+//                          tensor-core path, groups without a non-zero code hold an
+//                          exponent of its fp16 range instead of their own
 // ---------------------------------------------------------------------------
 enum ScaleMode { SC_ROW = 0, SC_H16 = 1, SC_F32 = 2, SC_MX = 3 };
 
 #define TILE_ROWS 32
 #define BLOCK_K 128
 #define CODE_BYTES 2048
+#define TC_MX_SPREAD 24         // widest exponent spread of an MXFP4 tensor the tensor-core path carries exactly
+#define TC_TAIL_BYTES 16          // behind a packed tensor's tile streams: its tensor-core shift (int)
 
 __host__ __device__ inline int scale_bytes_of(int mode) {
     return mode == SC_H16 ? 256 : mode == SC_F32 ? 512 : mode == SC_MX ? 128 : 0;
 }
 __host__ __device__ inline int chunk_bytes_of(int mode) { return CODE_BYTES + scale_bytes_of(mode); }
+// one half of a chunk: 16 rows, 1024 B of codes and their scales
+__host__ __device__ constexpr int half_bytes_of(int mode) {
+    return 1024 + (mode == SC_H16 ? 128 : mode == SC_F32 ? 256 : mode == SC_MX ? 64 : 0);
+}
 
 struct ColiCudaTensor {
     int fmt, I, O, device, gs, ng;

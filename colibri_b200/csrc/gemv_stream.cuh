@@ -13,7 +13,7 @@
 //  * tasks = (segment, 32-row tile, slice of the contraction); task t goes to
 //    CTA t % grid, so every SM gets the same number of tasks (+-1);
 //  * a chunk is consumed with four 128-bit shared loads per lane that are
-//    already tensor-core A fragments after a mask/sub (int4) or shift/mask
+//    already tensor-core A fragments after a mask/sub (int4) or conversion
 //    (MXFP4) decode to exact fp16 integers; activations arrive as an fp16
 //    (hi, lo) pair per value, hi+lo carrying 22 significant bits, laid out as
 //    B fragments, so one m16n8k16 MMA column pair = one row of x with
@@ -99,11 +99,13 @@ __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_c
 template <int MODE>
 __device__ __forceinline__ void decode_word(uint32_t q, uint32_t (&v)[4]) {
     if (MODE == SC_MX) {
-        // e2m1 fields pre-positioned at upload; result is value * 2^-14 in fp16.
-        v[0] = q & 0x8E008E00u;
-        v[1] = (q << 3) & 0x8E008E00u;
-        v[2] = ((q << 6) & 0x0E000E00u) | ((q << 2) & 0x80008000u);
-        v[3] = ((q << 9) & 0x0E000E00u) | ((q << 1) & 0x80008000u);
+        asm("{\n\t.reg .b8 a, b, c, d;\n\t"
+            "mov.b32 {a, b, c, d}, %4;\n\t"
+            "cvt.rn.f16x2.e2m1x2 %0, a;\n\t"
+            "cvt.rn.f16x2.e2m1x2 %1, b;\n\t"
+            "cvt.rn.f16x2.e2m1x2 %2, c;\n\t"
+            "cvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(q));
     } else {
         // offset-binary nibble n -> fp16 (n-8), exactly: 0x6400|n is 1024+n.
         const uint32_t MAGIC = 0x64006400u;
@@ -128,31 +130,30 @@ __device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) {
 // the group's scales. loadB(grp, cs) returns the B fragments of a group.
 // GS: the activations carry one scale per 32-column group instead of one per block
 // (ixg[grp], the same for every column set); it is folded into the group flush.
-// NS: 16-row halves present at `st` (2: a whole chunk; 1: one half, its 1024 bytes of
-// codes followed by its half of the scales; bacc[.][1] is then left untouched).
+// NS: 16-row halves present at `st` (2: a whole chunk; 1: one half; bacc[.][1] is then left untouched).
 template <int MODE, int NC, bool GS = false, int NS = 2, class LoadB>
 __device__ __forceinline__ void block_mma(uint32_t st, int lane, int g, LoadB loadB, float (&bacc)[NC][2][4],
                                           const float *ixg = nullptr) {
-    constexpr int SC0 = NS * 1024;      // offset of the scale part
+    constexpr int HS = half_bytes_of(MODE);
     uint4 w[4];
 #pragma unroll
-    for (int j = 0; j < 2 * NS; j++) w[j] = lds128(st + j * 512 + lane * 16);
-    // scales of rows g (h=0) and g+8 (h=1) of both 16-row halves
+    for (int j = 0; j < 2 * NS; j++) w[j] = lds128(st + (j >> 1) * HS + (j & 1) * 512 + lane * 16);
+    // scales of rows g (h=0) and g+8 (h=1) of both 16-row halves, [pair][h][i] for group 2*pair + i
     uint4 sc16[2];
     uint4 sc32[2][2];
     uint2 sc8[2];
     if (MODE == SC_H16) {
 #pragma unroll
-        for (int s = 0; s < NS; s++) sc16[s] = lds128(st + SC0 + (s * 8 + g) * 16);
+        for (int s = 0; s < NS; s++) sc16[s] = lds128(st + s * HS + 1024 + g * 16);
     } else if (MODE == SC_F32) {
 #pragma unroll
         for (int s = 0; s < NS; s++) {
-            sc32[s][0] = lds128(st + SC0 + (s * 8 + g) * 32);
-            sc32[s][1] = lds128(st + SC0 + (s * 8 + g) * 32 + 16);
+            sc32[s][0] = lds128(st + s * HS + 1024 + g * 32);
+            sc32[s][1] = lds128(st + s * HS + 1024 + g * 32 + 16);
         }
     } else if (MODE == SC_MX) {
 #pragma unroll
-        for (int s = 0; s < NS; s++) sc8[s] = lds64(st + SC0 + (s * 8 + g) * 8);
+        for (int s = 0; s < NS; s++) sc8[s] = lds64(st + s * HS + 1024 + g * 8);
     }
 #pragma unroll
     for (int cs = 0; cs < NC; cs++)
@@ -172,17 +173,18 @@ __device__ __forceinline__ void block_mma(uint32_t st, int lane, int g, LoadB lo
             decode_word<MODE>(word_of(w[s * 2 + 1], grp), a_hi);   // row g+8
             float s0 = 1.f, s1 = 1.f;
             if (MODE == SC_H16) {
-                uint32_t p0w = grp < 2 ? sc16[s].x : sc16[s].y;
-                uint32_t p1w = grp < 2 ? sc16[s].z : sc16[s].w;
+                uint32_t p0w = grp < 2 ? sc16[s].x : sc16[s].z;
+                uint32_t p1w = grp < 2 ? sc16[s].y : sc16[s].w;
                 __half2 h0 = u32_as_h2(p0w), h1 = u32_as_h2(p1w);
                 s0 = (grp & 1) ? __high2float(h0) : __low2float(h0);
                 s1 = (grp & 1) ? __high2float(h1) : __low2float(h1);
             } else if (MODE == SC_F32) {
-                s0 = __uint_as_float(word_of(sc32[s][0], grp));
-                s1 = __uint_as_float(word_of(sc32[s][1], grp));
+                s0 = __uint_as_float(word_of(sc32[s][grp >> 1], grp & 1));
+                s1 = __uint_as_float(word_of(sc32[s][grp >> 1], 2 + (grp & 1)));
             } else if (MODE == SC_MX) {
-                s0 = __uint_as_float(((sc8[s].x >> (8 * grp)) & 0xFFu) << 23);
-                s1 = __uint_as_float(((sc8[s].y >> (8 * grp)) & 0xFFu) << 23);
+                const uint32_t e4 = grp < 2 ? sc8[s].x : sc8[s].y;
+                s0 = __uint_as_float(((e4 >> (8 * (grp & 1))) & 0xFFu) << 23);
+                s1 = __uint_as_float(((e4 >> (16 + 8 * (grp & 1))) & 0xFFu) << 23);
             }
             if (GS) { s0 *= ixg[grp]; s1 *= ixg[grp]; }
 #pragma unroll
@@ -347,7 +349,6 @@ k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
         }
         if (failed) break;
         // ---- write this task's partial sums --------------------------------
-        const float mx_fix = (MODE == SC_MX) ? 16384.f : 1.f;   // fp16 fields carry e2m1 * 2^-14
 #pragma unroll
         for (int cs = 0; cs < NC; cs++) {
             int r = cs * 4 + t;
@@ -355,8 +356,8 @@ k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
 #pragma unroll
                 for (int s = 0; s < 2; s++) {
                     int o = tile * TILE_ROWS + s * 16 + g;
-                    float v0 = (R[cs][s][0] + R[cs][s][1]) * mx_fix;
-                    float v1 = (R[cs][s][2] + R[cs][s][3]) * mx_fix;
+                    float v0 = R[cs][s][0] + R[cs][s][1];
+                    float v1 = R[cs][s][2] + R[cs][s][3];
                     if (MODE == SC_ROW) { v0 *= sg.rowscale[o]; v1 *= sg.rowscale[o + 8]; }
                     float *dst = sg.out + ((size_t)kpart * npos + sg.pos0 + r) * sg.O + o;
                     dst[0] = v0;

@@ -10,14 +10,6 @@
 // Upload-time repack: raw row-major nibbles [O, I/2] -> tile streams.
 // One thread per output 32-bit word.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t mx_field(uint32_t code, int slot, int half) {
-    // code = e2m1 nibble (bit3 sign, bits2..0 = e1 e0 m); slot 0..3 = pair A..D
-    const int mag_pos[4] = {9, 6, 3, 0};
-    const int sgn_pos[4] = {15, 12, 13, 14};
-    uint32_t v = ((code & 7u) << mag_pos[slot]) | (((code >> 3) & 1u) << sgn_pos[slot]);
-    return v << (16 * half);
-}
-
 __global__ void k_repack_codes(uint8_t *__restrict__ pk, const uint8_t *__restrict__ raw, int O,
                                int I, int chunk_bytes, int is_mx) {
     const int nkb = I / BLOCK_K, ntiles = O / TILE_ROWS;
@@ -34,26 +26,27 @@ __global__ void k_repack_codes(uint8_t *__restrict__ pk, const uint8_t *__restri
     int row = tile * TILE_ROWS + (j >> 1) * 16 + (j & 1) * 8 + g;
     int k0 = kb * BLOCK_K + grp * 32 + t * 8;
     const uint8_t *src = raw + (size_t)row * (I / 2) + k0 / 2;
-    uint32_t c[8];
-#pragma unroll
-    for (int b = 0; b < 4; b++) { c[2 * b] = src[b] & 15u; c[2 * b + 1] = src[b] >> 4; }
     uint32_t word = 0;
     if (is_mx) {
-        // pairs A..D = (k0,k1) (k2,k3) (k4,k5) (k6,k7); first of a pair in the low half
 #pragma unroll
-        for (int p = 0; p < 4; p++) word |= mx_field(c[2 * p], p, 0) | mx_field(c[2 * p + 1], p, 1);
+        for (int b = 0; b < 4; b++) word |= (uint32_t)src[b] << (8 * b);
     } else {
+        uint32_t c[8];
+#pragma unroll
+        for (int b = 0; b < 4; b++) { c[2 * b] = src[b] & 15u; c[2 * b + 1] = src[b] >> 4; }
         const int order[8] = {0, 2, 4, 6, 1, 3, 5, 7};
 #pragma unroll
         for (int f = 0; f < 8; f++) word |= c[order[f]] << (4 * f);
     }
-    uint32_t *dst = reinterpret_cast<uint32_t *>(pk + blk * (size_t)chunk_bytes + j * 512 + lane * 16 + grp * 4);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(pk + blk * (size_t)chunk_bytes + (j >> 1) * (chunk_bytes / 2) + (j & 1) * 512 +
+                                                 lane * 16 + grp * 4);
     *dst = word;
 }
 
-// Scales -> per-chunk scale part. One thread per (block, sub, g, h, grp).
+// Scales -> per-chunk scale part. One thread per (block, sub, g, h, grp). MXFP4: exponents below e_min
+// (groups without a non-zero code, see tensor_tc_params) are stored as e_min.
 __global__ void k_repack_scales(uint8_t *__restrict__ pk, const void *__restrict__ raw_s, int O, int I,
-                                int chunk_bytes, int mode, int gs, int ng) {
+                                int chunk_bytes, int mode, int gs, int ng, int e_min) {
     const int nkb = I / BLOCK_K, ntiles = O / TILE_ROWS;
     size_t total = (size_t)ntiles * nkb * 128;
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,10 +56,11 @@ __global__ void k_repack_scales(uint8_t *__restrict__ pk, const void *__restrict
     int kb = blk % nkb, tile = blk / nkb;
     int row = tile * TILE_ROWS + sub * 16 + h * 8 + g;
     int k = kb * BLOCK_K + grp * 32;
-    uint8_t *sp = pk + blk * (size_t)chunk_bytes + CODE_BYTES;
-    int slot = ((sub * 8 + g) * 2 + h) * 4 + grp;
+    uint8_t *sp = pk + blk * (size_t)chunk_bytes + sub * (chunk_bytes / 2) + 1024;
+    int slot = ((g * 2 + (grp >> 1)) * 2 + h) * 2 + (grp & 1);
     if (mode == SC_MX) {
-        sp[slot] = static_cast<const uint8_t *>(raw_s)[(size_t)row * ng + k / 32];
+        const int e = static_cast<const uint8_t *>(raw_s)[(size_t)row * ng + k / 32];
+        sp[slot] = (uint8_t)(e > e_min ? e : e_min);
     } else {
         float s = static_cast<const float *>(raw_s)[(size_t)row * ng + k / gs];
         if (mode == SC_H16) reinterpret_cast<__half *>(sp)[slot] = __float2half_rn(s);

@@ -429,15 +429,14 @@ struct DecPhase {
 struct DecIt {
     int live, u, kb, mat, p;         // live 0: nothing left; p: pass (local down phase only)
     const uint8_t *base0, *base1;    // block 0 of the current tile: gate / up, or down / unused
-                                     // (local down phase: codes / scales of the 16-row half)
+                                     // (local down phase: the 16-row half / unused)
 };
 
 template <int CH>
 __device__ __forceinline__ void dec_it_unit(DecIt &it, const DecPhase &ph, const DecShared *sh) {
     if (ph.local) {
         const uint8_t *tile0 = sh->pass[it.p].wd + (size_t)(it.u >> 1) * ph.nkb * CH;
-        it.base0 = tile0 + (it.u & 1) * 1024;
-        it.base1 = tile0 + CODE_BYTES + (it.u & 1) * ((CH - CODE_BYTES) / 2);
+        it.base0 = tile0 + (it.u & 1) * (CH / 2);
         return;
     }
     const int pass = dec_div(it.u, ph.mg_nt), tile = it.u - pass * ph.nt;
@@ -493,11 +492,8 @@ __device__ __forceinline__ void dec_issue_one(WarpRing &wr, DecIt &it, const Dec
     if (lane == 0) {
         const uint32_t bar = wr.bars + wr.pi * 8, dst = wr.ring + wr.pi * wr.sb;
         if (ph.local) {
-            // one 16-row half: 1024 bytes of codes, then its half of the scales
-            constexpr int SCH = (CH - CODE_BYTES) / 2;
-            mbar_expect_tx(bar, 1024 + SCH);
-            bulk_g2s(dst, it.base0 + (size_t)it.kb * CH, 1024, bar);
-            if (SCH) bulk_g2s(dst + 1024, it.base1 + (size_t)it.kb * CH, SCH, bar);
+            mbar_expect_tx(bar, CH / 2);        // one 16-row half
+            bulk_g2s(dst, it.base0 + (size_t)it.kb * CH, CH / 2, bar);
         } else {
             mbar_expect_tx(bar, CH);
             bulk_g2s(dst, (it.mat ? it.base1 : it.base0) + (size_t)it.kb * CH, CH, bar);
@@ -972,7 +968,6 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
     }
     DEC_PROBE(a, 2);
     if (fast1) route_tail();     // beside the stream; the weights are first needed by the final combine
-    const float mx_fix = (MODE == SC_MX) ? 16384.f : 1.f;   // fp16 fields carry e2m1 * 2^-14
 
     // ---- gate / up -> SwiGLU activations ------------------------------------------------
     {
@@ -1021,8 +1016,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                     if (tid == 0 && wr.consumed == 1) DEC_PROBE_T(a, 3);      // first block of the stream consumed
                     dec_issue_one<CH, NST>(wr, it, ph1, sh, lane);
                 }
-                pb[mat] = make_float4((R[0][0] + R[0][1]) * mx_fix, (R[0][2] + R[0][3]) * mx_fix,
-                                      (R[1][0] + R[1][1]) * mx_fix, (R[1][2] + R[1][3]) * mx_fix);
+                pb[mat] = make_float4((R[0][0] + R[0][1]), (R[0][2] + R[0][3]),
+                                      (R[1][0] + R[1][1]), (R[1][2] + R[1][3]));
             }
             bar_sync_named(1 + ph1.gidx, ph1.wpk * 32);
             // Four warps of the group (a different four every unit) add the per-warp sums in
@@ -1153,8 +1148,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                 // rows g and g+8 of the 16-row half for token row t
                 if (svalid) {
                     float *dst = pp + ((size_t)(ps.pos0 + t) * ph2.wpk + ph2.wl) * 16 + g;
-                    dst[0] = (R[0] + R[1]) * mx_fix;
-                    dst[8] = (R[2] + R[3]) * mx_fix;
+                    dst[0] = (R[0] + R[1]);
+                    dst[8] = (R[2] + R[3]);
                 }
             }
             if (tid == 0) DEC_PROBE_T(a, 7);
@@ -1226,8 +1221,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                 dec_issue_one<CH, NST>(wr, it, ph2, sh, lane);
             }
             float4 *pb = reinterpret_cast<float4 *>(part + (ucount & 1) * DEC_PART_BYTES) + (warp * 32 + lane) * 2;
-            pb[0] = make_float4((R[0][0] + R[0][1]) * mx_fix, (R[0][2] + R[0][3]) * mx_fix,
-                                (R[1][0] + R[1][1]) * mx_fix, (R[1][2] + R[1][3]) * mx_fix);
+            pb[0] = make_float4((R[0][0] + R[0][1]), (R[0][2] + R[0][3]),
+                                (R[1][0] + R[1][1]), (R[1][2] + R[1][3]));
             bar_sync_named(1 + ph2.gidx, ph2.wpk * 32);
             const int lw = (ph2.wl + 4 * (nrot - (ucount & (nrot - 1)))) & (ph2.wpk - 1);
             if (lw < 4) {

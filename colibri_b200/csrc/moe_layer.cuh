@@ -19,7 +19,6 @@ struct ColiCudaMoeLayer {
     ColiCudaTensor **h_gates, **h_ups, **h_downs;
     ColiCudaTensor *h_shared[3];
     int tc_ok;                               // every tensor of the layer qualifies for the tensor-core path
-    int *host_route;                         // pinned: idx [max_rows*K] + keff [max_rows]
 };
 
 static int layer_mode_of(const ColiCudaTensor *t) { return t && t->packed ? t->mode : -1; }
@@ -78,7 +77,6 @@ extern "C" int coli_cuda_moe_layer_create(ColiCudaMoeLayer **layer, const ColiCu
         L->h_shared[0] = d->shared_gate; L->h_shared[1] = d->shared_up; L->h_shared[2] = d->shared_down;
         L->tc_ok &= d->shared_gate->tc_ok && d->shared_up->tc_ok && d->shared_down->tc_ok;
     }
-    if (ok) ok = cuda_ok(cudaMallocHost((void **)&L->host_route, ((size_t)max_rows * d->K + max_rows) * sizeof(int)), "pinned allocation");
     if (!ok) { coli_cuda_moe_layer_free(L); return 0; }
     const void *const *tp = static_cast<const void *const *>(L->table_mem);
     L->tab.gate_pk = reinterpret_cast<const uint8_t *const *>(tp);
@@ -107,7 +105,6 @@ extern "C" void coli_cuda_moe_layer_free(ColiCudaMoeLayer *L) {
         if (L->router_bias) cudaFree(L->router_bias);
         if (L->table_mem) cudaFree(L->table_mem);
         if (L->host_io) cudaFreeHost(L->host_io);
-        if (L->host_route) cudaFreeHost(L->host_route);
         (void)cudaGetLastError();
     }
     delete[] L->h_gates; delete[] L->h_ups; delete[] L->h_downs;
@@ -159,42 +156,35 @@ static LayerPlan layer_plan(const ColiCudaMoeLayer *L, const DeviceCtx *c, int M
     return p;
 }
 
-// Prefill-sized calls on the tensor cores: the routing result comes back to the host
-// (one synchronisation per call), rows are grouped per expert in ascending expert order
-// (row order kept inside an expert), the grouped GEMM runs with the row gather, and the
-// combine adds in each row's selection order, shared expert last.
-#define TC_LAYER_MIN_ROWS 32
+// Calls with more rows than the fused kernel takes, on the tensor cores (gemm_tc.cuh): plan (rows
+// grouped per expert), prepared rows, the two grouped GEMMs and the combine, all on the device and
+// without the host. The combine adds in each row's selection order, shared expert last.
+#define TC_LAYER_MIN_ROWS 9
 static int layer_run_tc(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const float *x_dev, int M,
                         const int *idx_dev, const float *w_dev, const int *keff_dev) {
     const RouteRule &r = L->rule;
-    int *h_idx = L->host_route, *h_keff = L->host_route + (size_t)M * r.K;
-    if (!cuda_ok(cudaMemcpyAsync(h_idx, idx_dev, (size_t)M * r.K * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "routing download") ||
-        !cuda_ok(cudaMemcpyAsync(h_keff, keff_dev, (size_t)M * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "routing download") ||
-        !cuda_ok(cudaStreamSynchronize(c->stream), "routing download")) return 0;
-    std::vector<int> cnt(r.E, 0), start(r.E + 1, 0);
-    for (int s = 0; s < M; s++) for (int kk = 0; kk < h_keff[s]; kk++) cnt[h_idx[s * r.K + kk]]++;
-    for (int e = 0; e < r.E; e++) start[e + 1] = start[e] + cnt[e];
-    const int routed = start[r.E], npos = routed + (L->has_shared ? M : 0);
-    std::vector<int> pos_scal((size_t)M * r.K + 4, 0), rowsrc(npos), fill(start.begin(), start.end() - 1);
-    for (int s = 0; s < M; s++)
-        for (int kk = 0; kk < h_keff[s]; kk++) {
-            int pos = fill[h_idx[s * r.K + kk]]++;
-            pos_scal[(size_t)s * r.K + kk] = pos; rowsrc[pos] = s;
-        }
-    for (int s = 0; s < M && L->has_shared; s++) rowsrc[routed + s] = s;
-    pos_scal[(size_t)M * r.K + 1] = npos; pos_scal[(size_t)M * r.K + 2] = routed;
-    std::vector<ColiCudaTensor *> g, u, d;
-    std::vector<int> rows;
-    for (int e = 0; e < r.E; e++) if (cnt[e]) { g.push_back(L->h_gates[e]); u.push_back(L->h_ups[e]); d.push_back(L->h_downs[e]); rows.push_back(cnt[e]); }
-    if (L->has_shared) { g.push_back(L->h_shared[0]); u.push_back(L->h_shared[1]); d.push_back(L->h_shared[2]); rows.push_back(M); }
-    if (!reserve(c, &L->pos_of, pos_scal.size() * sizeof(int)) || !reserve(c, &L->pd, (size_t)npos * r.D * sizeof(float))) return 0;
-    if (!cuda_ok(cudaMemcpyAsync(L->pos_of.p, pos_scal.data(), pos_scal.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream), "position table upload")) return 0;
-    if (npos > 0 && !group_device_tc(c, g.data(), u.data(), d.data(), rows.data(), (int)rows.size(), r.D, r.I, npos,
-                                     (float *)L->pd.p, x_dev, 0, rowsrc.data())) return 0;
-    const int *scal = (const int *)L->pos_of.p + (size_t)M * r.K;
+    const int sh = L->has_shared, npos_cap = M * r.K + (sh ? M : 0);
+    const int nexp = r.E < M * r.K ? r.E : M * r.K, nshp = sh ? (M + TC_ROWS - 1) / TC_ROWS : 0;
+    const int npass_cap = nexp + M * r.K / TC_ROWS + nshp;
+    const int ngrp_cap = npos_cap / 16 + npass_cap + 1;
+    TcList l;
+    const size_t need = tc_list_layout(&l, nullptr, npass_cap, ngrp_cap, npos_cap);
+    if (!reserve(c, &L->seg1, need) || !reserve(c, &L->pd, (size_t)npos_cap * r.D * sizeof(float))) return 0;
+    tc_list_layout(&l, L->seg1.p, npass_cap, ngrp_cap, npos_cap);
+    int *scal = (int *)L->scal.p;      // [1] npos [2] shared_pos0
+    TcPlanTables t;
+    t.gate_pk = L->tab.gate_pk; t.up_pk = L->tab.up_pk; t.down_pk = L->tab.down_pk;
+    t.gate_rs = L->tab.gate_rs; t.up_rs = L->tab.up_rs; t.down_rs = L->tab.down_rs;
+    t.sh_gate_pk = L->tab.sh_gate_pk; t.sh_up_pk = L->tab.sh_up_pk; t.sh_down_pk = L->tab.sh_down_pk;
+    t.sh_gate_rs = L->tab.sh_gate_rs; t.sh_up_rs = L->tab.sh_up_rs; t.sh_down_rs = L->tab.sh_down_rs;
+    const size_t nblk = (size_t)(r.D / TILE_ROWS) * (r.I / BLOCK_K);
+    t.gu_tail = nblk * chunk_bytes_of(L->mode_gu); t.d_tail = nblk * chunk_bytes_of(L->mode_d);
+    k_tc_plan<<<1, 1024, 33 * r.E * sizeof(int), c->stream>>>(l, scal + 1, scal + 2, (int *)L->pos_of.p, idx_dev, keff_dev, M, r.K, r.E, t);
+    c->last_launches++;
+    if (!tc_ffn(c, L->mode_gu, L->mode_d, l, x_dev, 0, npos_cap, ngrp_cap, r.D, r.I, (float *)L->pd.p)) return 0;
     size_t n4 = (size_t)M * r.D / 4;
     k_combine<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(out_dev, (const float *)L->pd.p, (const int *)L->pos_of.p, w_dev,
-                                                                keff_dev, scal + 1, M, r.K, r.D, 1, L->has_shared ? scal + 2 : nullptr);
+                                                                keff_dev, scal + 1, M, r.K, r.D, 1, sh ? scal + 2 : nullptr);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "layer launch");
 }
@@ -207,9 +197,8 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     const RouteRule &r = L->rule;
     const LayerPlan p = layer_plan(L, c, M);
     const int nkb1 = r.D / BLOCK_K, nkb2 = r.I / BLOCK_K;
-    // worth it from a mean of TC_MEAN_ROWS rows per routed expert (see group_tc_ok)
     bool use_tc = !route_only && !uniq_dev && L->tc_ok && M >= TC_LAYER_MIN_ROWS &&
-                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && (long)M * r.K >= (long)TC_MEAN_ROWS * r.E));
+                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, r.D, r.I)));
     if (use_tc) {
         // coli_cuda_tensor_update may have refreshed a tensor with scales the tensor-core
         // path cannot carry exactly since the layer was created: look again (E flags)

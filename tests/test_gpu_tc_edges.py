@@ -1,0 +1,63 @@
+"""Grouped tensor-core GEMM at the edges of its tiles: row counts around the 16-row padding
+and the 64-row pass, contractions that fill a partial sum of four 128-column blocks and ones that
+end inside it, rows with and without fp16 lo terms in one pass, and a layer whose plan is made on
+the device. CPU oracle, max relative error 1e-3."""
+import numpy as np
+import pytest
+
+from colibri_b200 import workloads as W
+from colibri_b200.backend import MoeLayer
+from tests.test_gpu_grouped import rand_qt
+from tests.util import max_rel_err, upload_qt
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fmt,gs", [(4, 32), (2, 0), (7, 0)])
+@pytest.mark.parametrize("D,I", [(128, 128), (512, 128), (640, 384), (1152, 256)])
+@pytest.mark.parametrize("rows", [[2, 1], [15, 16, 17], [63, 64, 65], [128, 129, 193]])
+def test_tile_edges(be, oracle, fmt, gs, D, I, rows):
+    rng = np.random.default_rng(D + I + sum(rows) + fmt)
+    experts = [(rand_qt(rng, I, D, fmt, gs, half=True), rand_qt(rng, I, D, fmt, gs, half=True),
+                rand_qt(rng, D, I, fmt, gs, half=True)) for _ in rows]
+    total = sum(rows)
+    x = ((rng.random((total, D)) - 0.5) * 2).astype(np.float32)
+    x[::3] = W.bf16_round(x[::3])                        # rows without lo terms among rows with them
+    hs = [[upload_qt(be, t) for t in e] for e in experts]
+    try:
+        be.set_tensor_core(2)
+        ok, y = be.run_expert_group([h[0] for h in hs], [h[1] for h in hs], [h[2] for h in hs], rows, x, D)
+    finally:
+        be.set_tensor_core(1)
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
+    assert ok and be.kernel_status(0) == 0
+    off = 0
+    for e, r in zip(experts, rows):
+        assert max_rel_err(y[off:off + r], oracle.expert_mlp(x[off:off + r], *e)) <= 1e-3
+        off += r
+
+
+@pytest.mark.parametrize("E,K,M", [(5, 5, 9), (64, 8, 9), (33, 3, 200), (3, 2, 700)])
+def test_device_plan(be, E, K, M):
+    """The plan kernel's grouping against the multi-kernel path on the same routing."""
+    cfg = dict(D=256, I=128, E=E, K=K, gating=0, norm_topk=0, shared=True, fmt=4, gs=32)
+    L = W.HostLayerWeights(cfg, 3)
+    up = lambda t: upload_qt(be, t)
+    g, u, d = ([up(t) for t in side] for side in (L.gate, L.up, L.down))
+    sh = tuple(up(t) for t in L.shared)
+    lay = MoeLayer(be, 256, 128, E, K, g, u, d, 0, 0, shared=sh, max_rows=M)
+    x, lg = W.activations(M, 256, 1), W.router_logits(M, E, 2, zipf=1.1)
+    outs = []
+    try:
+        for mode in (2, 0):
+            be.set_tensor_core(mode)
+            outs.append(lay(x, lg))
+    finally:
+        be.set_tensor_core(1)
+        lay.free()
+        for t in g + u + d + list(sh):
+            be.tensor_free(t)
+    assert np.array_equal(outs[0][1], outs[1][1])
+    assert max_rel_err(outs[0][0], outs[1][0]) <= 1e-3 and be.kernel_status(0) == 0
