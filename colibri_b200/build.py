@@ -26,6 +26,7 @@ FLAGS = [
 
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")) +
+                  glob.glob(os.path.join(CSRC, "*.h")) +
                   glob.glob(os.path.join(ROOT, "include", "*.h")))
 
 

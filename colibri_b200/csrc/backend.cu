@@ -16,11 +16,13 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.h"
 #include "gemv_stream.cuh"
 #include "kernels_misc.cuh"
 #include "router.cuh"
 #include "moe_decode.cuh"
 #include "gemm_tc.cuh"
+#include "dense_mma.cuh"
 #include "ep_kernels.cuh"
 
 // ---------------------------------------------------------------------------
@@ -42,8 +44,13 @@ struct DeviceCtx {
     Buf x, y, bq, bs, pg, pu, hq, hs, pd, segs1, segs2, ctl, gbuf, ubuf, misc;
     Buf pipe[27];
     Buf ep_ws, ep_x, ep_y;                    // expert-parallel layer: plan tables, permuted rows (streaming-kernel path)
-    float *host_x = nullptr, *host_y = nullptr;
+    float *host_x = nullptr, *host_y = nullptr;   // pinned rows of the grouped call (result valid until the next issue)
     size_t host_x_cap = 0, host_y_cap = 0;
+    float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the other host-buffer calls
+    size_t io_x_cap = 0, io_y_cap = 0;
+    UploadRing up = {};                       // pinned pieces of large uploads
+    uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
+    uint32_t *check_host = nullptr;
     int group_pending = 0;
     int *status = nullptr;                    // pinned host int the kernels store into (kstat_set): sticky kernel status
     unsigned int *dec_sync = nullptr;         // fused decode kernel: the grid barriers' arrival counter
@@ -67,6 +74,7 @@ static int g_timing = 0;
 static std::atomic<long> g_gpu_calls{0};
 static thread_local int g_cur_dev = -1;
 static int g_fp8_lut_ready = 0;           // the fmt 8 decode table has been handed over (coli_cuda_fp8_set_lut)
+static int g_fp8_standard = 0;            // ... and is E4M3's own, NaN codes included
 
 static int cuda_ok(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return 1;
@@ -182,6 +190,8 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
             !cuda_ok(cudaHostAlloc((void **)&c->status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "status") ||
             !cuda_ok(cudaMalloc((void **)&c->dec_sync, DEC_SYNC_WORDS * sizeof(unsigned int)), "grid barrier") ||
             !cuda_ok(cudaMemset(c->dec_sync, 0, DEC_SYNC_WORDS * sizeof(unsigned int)), "grid barrier") ||
+            !cuda_ok(cudaMalloc((void **)&c->check, 4 * sizeof(uint32_t)), "scale check") ||
+            !cuda_ok(cudaMallocHost((void **)&c->check_host, 4 * sizeof(uint32_t)), "scale check") ||
             !cuda_ok(cudaMalloc((void **)&c->exp_tab_dev, sizeof(tab)), "exp table") ||
             !cuda_ok(cudaMemcpy(c->exp_tab_dev, tab, sizeof(tab), cudaMemcpyHostToDevice), "exp table") ||
             !cuda_ok(cudaMemcpyToSymbol(c_exp2_tab, tab, sizeof(tab)), "exp table")) {
@@ -190,7 +200,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         *c->status = 0;
         setup_mode<SC_ROW>(); setup_mode<SC_H16>(); setup_mode<SC_F32>(); setup_mode<SC_MX>();
         set_smem(k_router_logits, ROUTER_TILE_SMEM);
-        set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<1>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
+        set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         set_smem(k_moe_decode<SC_ROW>, decode_smem_bytes(SC_ROW)); set_smem(k_moe_decode<SC_H16>, decode_smem_bytes(SC_H16));
         set_smem(k_moe_decode<SC_F32>, decode_smem_bytes(SC_F32)); set_smem(k_moe_decode<SC_MX>, decode_smem_bytes(SC_MX));
         set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
@@ -218,8 +228,13 @@ extern "C" void coli_cuda_shutdown(void) {
         for (int s = 0; s < 27; s++) free_buf(&c->pipe[s]);
         if (c->host_x) cudaFreeHost(c->host_x);
         if (c->host_y) cudaFreeHost(c->host_y);
+        if (c->io_x) cudaFreeHost(c->io_x);
+        if (c->io_y) cudaFreeHost(c->io_y);
         if (c->status) cudaFreeHost(c->status);
         if (c->dec_sync) cudaFree(c->dec_sync);
+        if (c->check) cudaFree(c->check);
+        if (c->check_host) cudaFreeHost(c->check_host);
+        upload_ring_free(&c->up);
         if (c->exp_tab_dev) cudaFree(c->exp_tab_dev);
         if (c->ev0) cudaEventDestroy(c->ev0);
         if (c->ev1) cudaEventDestroy(c->ev1);
@@ -293,6 +308,13 @@ extern "C" int coli_cuda_fp8_set_lut(const float *lut) {
         if (!cuda_ok(cudaGetSymbolAddress(&p, d_e4m3_lut), "e4m3 table address")) return 0;
         g_ctx[i].e4m3_lut_dev = static_cast<const float *>(p);
     }
+    g_fp8_standard = 1;
+    for (int i = 0; i < 256; i++) {
+        const int e = (i >> 3) & 15, m = i & 7;
+        float v = e ? std::ldexp(1.f + m / 8.f, e - 7) : std::ldexp(m / 8.f, -6);
+        if (i & 128) v = -v;
+        if ((i & 127) == 127 ? !std::isnan(lut[i]) : lut[i] != v) g_fp8_standard = 0;
+    }
     g_fp8_lut_ready = 1;
     return 1;
 }
@@ -323,36 +345,23 @@ extern "C" int coli_cuda_kernel_status(int device) {
 // ---------------------------------------------------------------------------
 // Tensors
 // ---------------------------------------------------------------------------
-static int scales_fit_half(const float *s, size_t n) {
-    for (size_t i = 0; i < n; i++) {
-        float v = s[i];
-        if (__half2float(__float2half(v)) != v) return 0;
-    }
-    return 1;
-}
-
-// Decides whether the tensor-core path can carry this tensor exactly and with which
-// power-of-two pre-multiplier (gemm_tc.cuh):
+// Decides from the scale facts that k_check_scales / k_check_mx left (kernels_misc.cuh) whether the
+// tensor-core path can carry this tensor exactly and with which power-of-two pre-multiplier (gemm_tc.cuh):
 //   SC_ROW  integer codes, no shift
 //   SC_H16  scale * 2^shift puts the largest scale in [2^10, 2^11); every non-zero scale must
 //           lie within 2^-12 of the largest so that the hi/lo split keeps its low bits
 //   SC_MX   2^(e - 127 + shift) must be an fp16 power of two <= 2^13 for every group that holds a
 //           non-zero code: shift = 140 - e_max, spread e_max - e <= TC_MX_SPREAD (down to 2^-11)
-static void tensor_tc_params(ColiCudaTensor *t, const void *weights, const void *scales) {
+static void tensor_tc_params(ColiCudaTensor *t, const uint32_t *f) {
     t->tc_ok = 0; t->tc_shift = 0;
     if (!t->packed || (t->O % 128) || (t->I % 128)) return;
-    const size_t scount = (size_t)t->O * (size_t)t->ng;
     if (t->mode == SC_ROW) { t->tc_ok = 1; return; }
     if (t->mode == SC_H16) {
-        const float *s = static_cast<const float *>(scales);
-        float smax = 0.f, smin = 0.f;
-        for (size_t i = 0; i < scount; i++) {
-            float a = std::fabs(s[i]);
-            if (!(a <= 65504.f)) return;          // inf / nan
-            if (a > smax) smax = a;
-            if (a > 0.f && (smin == 0.f || a < smin)) smin = a;
-        }
-        if (smax == 0.f) { t->tc_ok = 1; return; }
+        float smax, smin;
+        const uint32_t lo = 0x7FFFFFFFu - f[2];
+        std::memcpy(&smax, &f[1], 4); std::memcpy(&smin, &lo, 4);
+        if (f[3]) return;                             // inf / nan / beyond fp16
+        if (f[1] == 0) { t->tc_ok = 1; return; }
         if (smin < smax * (1.0f / 4096.0f)) return;
         int ex; std::frexp(smax, &ex);             // smax = m * 2^ex, m in [0.5, 1)
         int shift = 11 - ex;                       // smax * 2^shift in [2^10, 2^11)
@@ -361,17 +370,8 @@ static void tensor_tc_params(ColiCudaTensor *t, const void *weights, const void 
         return;
     }
     if (t->mode == SC_MX) {
-        const uint8_t *e8 = static_cast<const uint8_t *>(scales);
-        const uint8_t *q = static_cast<const uint8_t *>(weights);
-        int emax = 0;
-        for (size_t i = 0; i < scount; i++) { if (e8[i] == 255) return; if (e8[i] > emax) emax = e8[i]; }
-        const size_t rb = (size_t)t->I / 2;
-        for (size_t i = 0; i < scount; i++) {
-            if (emax - (int)e8[i] <= TC_MX_SPREAD) continue;
-            const size_t row = i / t->ng, g = i % t->ng;
-            const uint8_t *c = q + row * rb + g * 16;
-            for (int b = 0; b < 16; b++) if (c[b] & 0x77) return;   // a live group below the exact range
-        }
+        const int emax = (int)f[0], emin = f[1] ? 255 - (int)f[1] : emax;      // emin over groups with a non-zero code
+        if (f[2] || emax - emin > TC_MX_SPREAD) return;
         t->tc_shift = 140 - emax; t->tc_ok = 1;
     }
 }
@@ -395,28 +395,45 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
     const size_t sbytes = t->fmt == 7 ? scount : scount * sizeof(float);
     if (!t->packed) {
         if (allocate) {
-            if (!cuda_ok(cudaMalloc(&t->raw_w, wbytes), "tensor allocation")) return 0;
+            // 16 spare bytes: the matmul reads whole words of rows that start anywhere
+            if (!cuda_ok(cudaMalloc(&t->raw_w, wbytes + 16), "tensor allocation")) return 0;
             if (sbytes && !cuda_ok(cudaMalloc(&t->raw_s, sbytes), "scale allocation")) return 0;
             t->physical_bytes = wbytes + sbytes;
         }
-        if (!cuda_ok(cudaMemcpyAsync(t->raw_w, weights, wbytes, cudaMemcpyHostToDevice, c->stream), "tensor upload")) return 0;
-        if (sbytes && !cuda_ok(cudaMemcpyAsync(t->raw_s, scales, sbytes, cudaMemcpyHostToDevice, c->stream), "scale upload")) return 0;
+        if (!cuda_ok(upload_staged(&c->up, t->raw_w, weights, wbytes, c->stream), "tensor upload")) return 0;
+        if (sbytes && !cuda_ok(upload_staged(&c->up, t->raw_s, scales, sbytes, c->stream), "scale upload")) return 0;
         return cuda_ok(cudaStreamSynchronize(c->stream), "tensor upload sync");
     }
+    if (!reserve(c, &c->stage_w, wbytes) || (sbytes && !reserve(c, &c->stage_s, sbytes))) return 0;
+    // Scales first: what the storage class depends on is found on the device while the codes travel.
+    // Nothing of an existing tensor is overwritten before its new scales have been accepted.
+    if (!cuda_ok(upload_staged(&c->up, c->stage_s.p, scales, sbytes, c->stream), "scale upload")) return 0;
+    if (t->fmt == 4) {
+        cudaMemsetAsync(c->check, 0, 4 * sizeof(uint32_t), c->stream);
+        k_check_scales<<<(unsigned)((scount + 1023) / 1024), 256, 0, c->stream>>>(c->check, static_cast<const float *>(c->stage_s.p), scount);
+        cudaMemcpyAsync(c->check_host, c->check, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+        cudaEventRecord(c->ev_done, c->stream);
+    }
+    if (!cuda_ok(upload_staged(&c->up, c->stage_w.p, weights, wbytes, c->stream), "tensor upload")) return 0;
+    if (t->fmt == 7) {
+        cudaMemsetAsync(c->check, 0, 4 * sizeof(uint32_t), c->stream);
+        k_check_mx<<<(unsigned)((scount + 255) / 256), 256, 0, c->stream>>>(c->check, static_cast<const uint8_t *>(c->stage_w.p),
+                                                                            static_cast<const uint8_t *>(c->stage_s.p), scount);
+        cudaMemcpyAsync(c->check_host, c->check, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+        cudaEventRecord(c->ev_done, c->stream);
+    }
+    if (t->fmt != 2 && !cuda_ok(cudaEventSynchronize(c->ev_done), "scale check")) return 0;
     int mode = t->mode;
     if (allocate) {
-        mode = t->fmt == 2 ? SC_ROW : t->fmt == 7 ? SC_MX
-             : scales_fit_half(static_cast<const float *>(scales), scount) ? SC_H16 : SC_F32;
+        mode = t->fmt == 2 ? SC_ROW : t->fmt == 7 ? SC_MX : c->check_host[0] == 0 ? SC_H16 : SC_F32;
         t->mode = mode;
-    } else if (t->fmt == 4 && mode == SC_H16 &&
-               !scales_fit_half(static_cast<const float *>(scales), scount)) {
+    } else if (t->fmt == 4 && mode == SC_H16 && c->check_host[0]) {
         return 0;   // the refreshed scales no longer fit the storage chosen at upload
     }
-    tensor_tc_params(t, weights, scales);
+    tensor_tc_params(t, c->check_host);
     const int ch = chunk_bytes_of(mode);
     const size_t nblk = (size_t)(t->O / TILE_ROWS) * (t->I / BLOCK_K);
     const size_t pkbytes = nblk * ch;
-    if (!reserve(c, &c->stage_w, wbytes) || (sbytes && !reserve(c, &c->stage_s, sbytes))) return 0;
     if (allocate) {
         // behind the tile streams: the tensor shift, for kernels that find the tensor by its address
         if (!cuda_ok(cudaMalloc((void **)&t->pk, pkbytes + TC_TAIL_BYTES), "tensor allocation")) return 0;
@@ -426,15 +443,12 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
             t->physical_bytes += (size_t)t->O * sizeof(float);
         }
     }
-    if (!cuda_ok(cudaMemcpyAsync(c->stage_w.p, weights, wbytes, cudaMemcpyHostToDevice, c->stream), "tensor upload")) return 0;
-    if (mode == SC_ROW) {
-        if (!cuda_ok(cudaMemcpyAsync(t->rowscale, scales, (size_t)t->O * sizeof(float), cudaMemcpyHostToDevice, c->stream), "scale upload")) return 0;
-    } else if (!cuda_ok(cudaMemcpyAsync(c->stage_s.p, scales, sbytes, cudaMemcpyHostToDevice, c->stream), "scale upload")) return 0;
-    if (!cuda_ok(cudaMemcpyAsync(t->pk + pkbytes, &t->tc_shift, sizeof(int), cudaMemcpyHostToDevice, c->stream), "tensor shift")) return 0;
     size_t words = nblk * 512;
     k_repack_codes<<<(unsigned)((words + 255) / 256), 256, 0, c->stream>>>(
-        t->pk, static_cast<const uint8_t *>(c->stage_w.p), t->O, t->I, ch, t->fmt == 7);
-    if (mode != SC_ROW) {
+        t->pk, static_cast<const uint8_t *>(c->stage_w.p), t->O, t->I, ch, t->fmt == 7, t->tc_shift);
+    if (mode == SC_ROW) {
+        if (!cuda_ok(cudaMemcpyAsync(t->rowscale, c->stage_s.p, (size_t)t->O * sizeof(float), cudaMemcpyDeviceToDevice, c->stream), "scale upload")) return 0;
+    } else {
         size_t n = nblk * 128;
         k_repack_scales<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
             t->pk, c->stage_s.p, t->O, t->I, ch, mode, t->gs > 0 ? t->gs : t->I, t->ng,
@@ -708,14 +722,45 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
     return cuda_ok(cudaGetLastError(), "linear launch");
 }
 
+template <int FMT, bool AL16>
+static void launch_dense(DeviceCtx *c, const ColiCudaTensor *t, float *y, int S, const __half *bq, const float *bs) {
+    const int nc = S <= 4 ? 1 : S <= 8 ? 2 : 4;
+    const dim3 grid((unsigned)((t->O + 31) / 32), (unsigned)((S + 4 * nc - 1) / (4 * nc)));
+    const uint8_t *w = static_cast<const uint8_t *>(t->raw_w);
+    const size_t rb = row_bytes(t->fmt, t->I);
+    const int gs = t->gs > 0 ? t->gs : t->I;
+    if (nc == 1) k_dense_mma<FMT, 1, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    else if (nc == 2) k_dense_mma<FMT, 2, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    else k_dense_mma<FMT, 4, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+}
+
 static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {
+    // Quantised rows take the tensor-core kernel; scale groups must hold whole 32-column groups, and FP8
+    // tables other than E4M3's own have no conversion instruction.
+    const bool whole = t->fmt != 4 || t->ng == 1 || t->gs % 32 == 0;
+    if (t->fmt != 0 && whole && (t->fmt != 8 || g_fp8_standard)) {
+        const int nkb = (t->I + 127) / 128;
+        if (!reserve(c, &c->bq, (size_t)S * nkb * 256 * sizeof(__half)) || !reserve(c, &c->bs, (size_t)S * nkb * sizeof(float))) return 0;
+        __half *bq = (__half *)c->bq.p;
+        float *bs = (float *)c->bs.p;
+        k_prep_dense<<<(S * nkb * 32 + 255) / 256, 256, 0, c->stream>>>(bq, bs, x_dev, S, t->I, t->fmt);
+        switch (t->fmt) {
+        case 1: if (t->I % 16 == 0) launch_dense<1, true>(c, t, y_dev, S, bq, bs); else launch_dense<1, false>(c, t, y_dev, S, bq, bs); break;
+        case 8: if (t->I % 16 == 0) launch_dense<8, true>(c, t, y_dev, S, bq, bs); else launch_dense<8, false>(c, t, y_dev, S, bq, bs); break;
+        case 2: launch_dense<2, false>(c, t, y_dev, S, bq, bs); break;
+        case 3: launch_dense<3, false>(c, t, y_dev, S, bq, bs); break;
+        case 4: launch_dense<4, false>(c, t, y_dev, S, bq, bs); break;
+        default: launch_dense<7, false>(c, t, y_dev, S, bq, bs); break;
+        }
+        c->last_launches += 2;
+        return cuda_ok(cudaGetLastError(), "matmul launch");
+    }
     // rows that start 16-byte aligned take the streaming kernel (128-bit loads)
-    const bool dense = (t->fmt == 0 && t->I % 4 == 0) || ((t->fmt == 1 || t->fmt == 8) && t->I % 16 == 0);
+    const bool dense = (t->fmt == 0 && t->I % 4 == 0) || (t->fmt == 8 && t->I % 16 == 0);
     if (dense && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0 && (reinterpret_cast<uintptr_t>(t->raw_w) & 15) == 0) {
         dim3 grid((unsigned)((t->O + 31) / 32), (unsigned)((S + 7) / 8));
         const float *sc = static_cast<const float *>(t->raw_s);
         if (t->fmt == 0) k_dense_gemv<0><<<grid, 256, DENSE_GEMV_SMEM, c->stream>>>(y_dev, x_dev, t->raw_w, sc, nullptr, S, t->I, t->O);
-        else if (t->fmt == 1) k_dense_gemv<1><<<grid, 256, DENSE_GEMV_SMEM, c->stream>>>(y_dev, x_dev, t->raw_w, sc, nullptr, S, t->I, t->O);
         else k_dense_gemv<8><<<grid, 256, DENSE_GEMV_SMEM, c->stream>>>(y_dev, x_dev, t->raw_w, sc, c->e4m3_lut_dev, S, t->I, t->O);
         c->last_launches++;
         return cuda_ok(cudaGetLastError(), "matmul launch");
@@ -744,6 +789,30 @@ static int check_status(DeviceCtx *c) {
     return 1;
 }
 
+// Host rows of a blocking call. Everything passes through pinned memory (a copy out of the cache and a DMA
+// are faster than the driver's pageable path, 21 us against 27 at 300 KB), and small rows are not copied to the
+// device at all: the kernel that reads them once, or stores the result, addresses the pinned buffer.
+#define IO_DIRECT_BYTES (64u << 10)
+// -> where the kernels find x, or NULL. read_once: the first kernel reads every element once (not every CTA all of them).
+static const float *io_in(DeviceCtx *c, const float *x, size_t bytes, bool read_once) {
+    if (!reserve_pinned(&c->io_x, &c->io_x_cap, bytes)) return nullptr;
+    CopyPool::get().copy(c->io_x, x, bytes);
+    if (read_once && bytes <= IO_DIRECT_BYTES) return c->io_x;
+    if (!reserve(c, &c->x, bytes) || !cuda_ok(cudaMemcpyAsync(c->x.p, c->io_x, bytes, cudaMemcpyHostToDevice, c->stream), "input upload")) return nullptr;
+    return (const float *)c->x.p;
+}
+static float *io_out(DeviceCtx *c, size_t bytes) {
+    if (!reserve_pinned(&c->io_y, &c->io_y_cap, bytes)) return nullptr;
+    if (bytes <= IO_DIRECT_BYTES) return c->io_y;
+    return reserve(c, &c->y, bytes) ? (float *)c->y.p : nullptr;
+}
+static int io_finish(DeviceCtx *c, float *y, const float *y_dev, size_t bytes) {
+    if (y_dev != c->io_y && !cuda_ok(cudaMemcpyAsync(c->io_y, y_dev, bytes, cudaMemcpyDeviceToHost, c->stream), "output download")) return 0;
+    if (!check_status(c)) return 0;
+    CopyPool::get().copy(y, c->io_y, bytes);
+    return 1;
+}
+
 extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *x, const void *weights,
                                 const float *scales, int fmt, int S, int I, int O, int device, int gs) {
     if (fault_injected()) return 0;
@@ -755,14 +824,15 @@ extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *
     DeviceCtx *c = find_ctx(t->device);
     if (!select_ctx(c)) return 0;
     size_t xb = (size_t)S * I * sizeof(float), yb = (size_t)S * O * sizeof(float);
-    if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, yb)) return 0;
-    if (!cuda_ok(cudaMemcpyAsync(c->x.p, x, xb, cudaMemcpyHostToDevice, c->stream), "input upload")) return 0;
+    const float *xd = io_in(c, x, xb, t->packed || t->fmt != 0);
+    float *yd = io_out(c, yb);
+    if (!xd || !yd) return 0;
     timing_begin(c);
-    if (!linear_any(c, t, (float *)c->y.p, (const float *)c->x.p, S)) return 0;
+    if (!linear_any(c, t, yd, xd, S)) return 0;
     timing_end(c);
-    if (!check_status(c)) return 0;
+    if (!io_finish(c, y, yd, yb)) return 0;
     timing_collect(c);
-    return cuda_ok(cudaMemcpy(y, c->y.p, yb, cudaMemcpyDeviceToHost), "output download");
+    return 1;
 }
 
 extern "C" int coli_cuda_matmul_mxfp4(float *y, const float *x, const unsigned char *q4,
@@ -1031,7 +1101,7 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         profile = 0; break;
     }
     if (profile) cudaEventRecord(ev[0], c->stream);
-    std::memcpy(c->host_x, x, xb);
+    CopyPool::get().copy(c->host_x, x, xb);
     if (!cuda_ok(cudaMemcpyAsync(c->x.p, c->host_x, xb, cudaMemcpyHostToDevice, c->stream), "expert group input upload")) return 0;
     if (profile) cudaEventRecord(ev[1], c->stream);
     timing_begin(c);
@@ -1049,7 +1119,7 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
     }
     if (!check_status(c)) return 0;
     timing_collect(c);
-    std::memcpy(y, c->host_y, xb);
+    CopyPool::get().copy(y, c->host_y, xb);
     if (profile) {
         float a = 0, b = 0, d = 0;
         cudaEventElapsedTime(&a, ev[0], ev[1]); cudaEventElapsedTime(&b, ev[1], ev[2]); cudaEventElapsedTime(&d, ev[2], ev[3]);
@@ -1092,14 +1162,15 @@ extern "C" int coli_cuda_expert_mlp(ColiCudaTensor *gate, ColiCudaTensor *up, Co
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
     size_t xb = (size_t)S * D * sizeof(float);
-    if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, xb)) return 0;
-    if (!cuda_ok(cudaMemcpyAsync(c->x.p, x, xb, cudaMemcpyHostToDevice, c->stream), "expert input upload")) return 0;
+    const float *xd = io_in(c, x, xb, all_packed);
+    float *yd = io_out(c, xb);
+    if (!xd || !yd) return 0;
     timing_begin(c);
-    if (!group_device(c, g, u, d, rows, 1, D, I, total, max_rows, all_packed, (float *)c->y.p, (const float *)c->x.p, nullptr)) return 0;
+    if (!group_device(c, g, u, d, rows, 1, D, I, total, max_rows, all_packed, yd, xd, nullptr)) return 0;
     timing_end(c);
-    if (!check_status(c)) return 0;
+    if (!io_finish(c, y, yd, xb)) return 0;
     timing_collect(c);
-    return cuda_ok(cudaMemcpy(y, c->y.p, xb, cudaMemcpyDeviceToHost), "expert output download");
+    return 1;
 }
 // The reference's W4A16 tensor-core shared-expert call (c/backend_cuda.cu:1457-1484)
 // is the same function with per-row int4 tensors required.

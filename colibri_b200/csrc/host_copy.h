@@ -1,0 +1,105 @@
+// Host side of large transfers: pageable caller memory goes through pinned buffers, copied by a few
+// threads while the previous piece is on the bus.
+//
+// Measured on a 16-thread host: a 25 MB upload from pageable memory takes the driver 1.19 ms
+// (21 GB/s); one thread copies 18 GB/s, four copy 60 GB/s, and the bus takes 47 GB/s from pinned
+// memory. Below a few hundred KB a single copy into a pinned buffer (51 GB/s out of the cache) and
+// one DMA beat the driver's path too (21 us against 27 us at 300 KB).
+#pragma once
+#include <condition_variable>
+#include <cstring>
+#include <mutex>
+#include <thread>
+
+// Three helper threads, started on first use and kept until the process ends. One job at a time;
+// a caller that finds them busy copies alone, so any number of threads may copy at once.
+class CopyPool {
+public:
+    static CopyPool &get() {
+        static CopyPool *p = new CopyPool();        // never destroyed: the helpers may outlive static teardown
+        return *p;
+    }
+    void copy(void *dst, const void *src, size_t bytes) {
+        if (bytes < MIN_SPLIT || !owner_.try_lock()) { std::memcpy(dst, src, bytes); return; }
+        {
+            std::lock_guard<std::mutex> l(m_);
+            if (!started_) {
+                for (int i = 0; i < HELPERS; i++) std::thread([this, i] { work(i); }).detach();
+                started_ = true;
+            }
+            dst_ = static_cast<char *>(dst); src_ = static_cast<const char *>(src); bytes_ = bytes;
+            left_ = HELPERS;
+            job_++;
+        }
+        cv_.notify_all();
+        part(HELPERS);
+        std::unique_lock<std::mutex> l(m_);
+        done_.wait(l, [this] { return left_ == 0; });
+        l.unlock();
+        owner_.unlock();
+    }
+
+private:
+    static constexpr int HELPERS = 3;
+    static constexpr size_t MIN_SPLIT = 1 << 19;
+    void part(int i) {
+        const size_t step = (bytes_ / (HELPERS + 1) + 63) & ~(size_t)63, a = step * i;
+        if (a < bytes_) std::memcpy(dst_ + a, src_ + a, i == HELPERS || bytes_ - a < step ? bytes_ - a : step);
+    }
+    void work(int i) {
+        unsigned long seen = 0;
+        for (;;) {
+            {
+                std::unique_lock<std::mutex> l(m_);
+                cv_.wait(l, [&] { return job_ != seen; });
+                seen = job_;
+            }
+            part(i);
+            std::lock_guard<std::mutex> l(m_);
+            if (--left_ == 0) done_.notify_one();
+        }
+    }
+    std::mutex owner_, m_;
+    std::condition_variable cv_, done_;
+    bool started_ = false;
+    unsigned long job_ = 0;
+    int left_ = 0;
+    char *dst_ = nullptr;
+    const char *src_ = nullptr;
+    size_t bytes_ = 0;
+};
+
+// Pinned pieces of one device's uploads, each with the event of the last copy out of it.
+struct UploadRing {
+    static constexpr int N = 4;
+    static constexpr size_t PIECE = 2u << 20;
+    char *buf[N];
+    cudaEvent_t ev[N];
+    bool busy[N];
+    int next;
+};
+static void upload_ring_free(UploadRing *r) {
+    for (int i = 0; i < UploadRing::N; i++) {
+        if (r->ev[i]) cudaEventDestroy(r->ev[i]);
+        if (r->buf[i]) cudaFreeHost(r->buf[i]);
+    }
+    std::memset(r, 0, sizeof(*r));
+}
+// src (any host memory) -> dst (device) on `stream`. The source has been read when the call returns.
+static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    if (bytes <= (64u << 10)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);   // the driver's inline path
+    for (size_t off = 0; off < bytes; off += UploadRing::PIECE) {
+        const size_t n = bytes - off < UploadRing::PIECE ? bytes - off : UploadRing::PIECE;
+        const int i = r->next;
+        r->next = (i + 1) % UploadRing::N;
+        cudaError_t e;
+        if (!r->buf[i] && ((e = cudaMallocHost(reinterpret_cast<void **>(&r->buf[i]), UploadRing::PIECE)) != cudaSuccess ||
+                           (e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming)) != cudaSuccess)) return e;
+        if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;
+        CopyPool::get().copy(r->buf[i], static_cast<const char *>(src) + off, n);
+        if ((e = cudaMemcpyAsync(static_cast<char *>(dst) + off, r->buf[i], n, cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
+            (e = cudaEventRecord(r->ev[i], stream)) != cudaSuccess) return e;
+        r->busy[i] = true;
+    }
+    return cudaSuccess;
+}

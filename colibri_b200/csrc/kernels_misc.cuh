@@ -10,12 +10,59 @@
 // Upload-time repack: raw row-major nibbles [O, I/2] -> tile streams.
 // One thread per output 32-bit word.
 // ---------------------------------------------------------------------------
+// Facts about a tensor's scales that decide its storage and whether the tensor-core path can carry it;
+// the words start at zero and only grow. Bound by HBM, a few us per tensor (one pass on a host thread: 2 ms
+// for the 459 000 scales of a 7168 x 2048 matrix in groups of 32).
+// f32 scales: [0] some value is not exact in fp16, [1] largest |s| (bits), [2] 0x7FFFFFFF - smallest
+// non-zero |s| (bits), [3] some |s| is not at most 65504.
+__global__ void __launch_bounds__(256) k_check_scales(uint32_t *__restrict__ out, const float *__restrict__ s, size_t n) {
+    uint32_t inexact = 0, mx = 0, mn = 0, wild = 0;
+    for (int j = 0; j < 4; j++) {
+        const size_t i = (size_t)blockIdx.x * 1024 + j * 256 + threadIdx.x;
+        if (i < n) {
+            const float v = s[i], a = fabsf(v);
+            inexact |= !(__half2float(__float2half_rn(v)) == v);
+            wild |= !(a <= 65504.f);
+            const uint32_t b = __float_as_uint(a);
+            mx = max(mx, b);
+            if (b) mn = max(mn, 0x7FFFFFFFu - b);
+        }
+    }
+    inexact = __reduce_or_sync(0xffffffffu, inexact); wild = __reduce_or_sync(0xffffffffu, wild);
+    mx = __reduce_max_sync(0xffffffffu, mx); mn = __reduce_max_sync(0xffffffffu, mn);
+    if ((threadIdx.x & 31) == 0) {
+        if (inexact) out[0] = 1;
+        if (wild) out[3] = 1;
+        atomicMax(&out[1], mx); atomicMax(&out[2], mn);
+    }
+}
+// ue8m0 exponents with their 16 code bytes per group: [0] largest exponent, [1] 255 - smallest exponent of a
+// group with a non-zero code, [2] some exponent is 255 (NaN).
+__global__ void __launch_bounds__(256) k_check_mx(uint32_t *__restrict__ out, const uint8_t *__restrict__ codes,
+                                                  const uint8_t *__restrict__ e8, size_t n) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    uint32_t mx = 0, mn = 0, nan = 0;
+    if (i < n) {
+        const uint32_t e = e8[i];
+        const uint4 c = reinterpret_cast<const uint4 *>(codes)[i];
+        mx = e; nan = e == 255;
+        if ((c.x | c.y | c.z | c.w) & 0x77777777u) mn = 255 - e;
+    }
+    nan = __reduce_or_sync(0xffffffffu, nan);
+    mx = __reduce_max_sync(0xffffffffu, mx); mn = __reduce_max_sync(0xffffffffu, mn);
+    if ((threadIdx.x & 31) == 0) {
+        if (nan) out[2] = 1;
+        atomicMax(&out[0], mx); atomicMax(&out[1], mn);
+    }
+}
+
 __global__ void k_repack_codes(uint8_t *__restrict__ pk, const uint8_t *__restrict__ raw, int O,
-                               int I, int chunk_bytes, int is_mx) {
+                               int I, int chunk_bytes, int is_mx, int tc_shift) {
     const int nkb = I / BLOCK_K, ntiles = O / TILE_ROWS;
     size_t total = (size_t)ntiles * nkb * 512;   // words
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
+    if (idx == 0) *reinterpret_cast<int *>(pk + (size_t)ntiles * nkb * chunk_bytes) = tc_shift;
     int grp = idx & 3;
     int lane = (idx >> 2) & 31;
     int j = (idx >> 7) & 3;
@@ -294,10 +341,9 @@ __global__ void k_generic_matmul(float *__restrict__ y, const float *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Streaming GEMV for row-major tensors that the packed layout does not cover and whose
-// rows are 16-byte aligned: fmt 0 (f32, e.g. a vocabulary head), fmt 1 (int8 with a scale
-// per row) and fmt 8 (FP8 E4M3 bytes with one f32 scale per 128x128 block, the decode
-// table in `lut`). Bound by HBM: every weight byte is read once with 128-bit loads.
+// Streaming GEMV for row-major tensors whose rows are 16-byte aligned: fmt 0 (f32, e.g. a
+// vocabulary head) and fmt 8 (FP8 bytes with one f32 scale per 128x128 block) with a decode
+// table other than E4M3's own. Bound by HBM: every weight byte is read once with 128-bit loads.
 //   y[s*O + o] = sum_i x[s,i] * w[o,i]
 // One warp owns 4 output rows and up to 8 rows of x (blockIdx.y selects the group of 8);
 // the CTA stages 1024 columns of those x rows in shared memory per round (two buffers, filled
@@ -380,12 +426,12 @@ __global__ void __launch_bounds__(256, FMT == 0 ? 3 : 2) k_dense_gemv(float *__r
                     float wd[4][16];
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
-                        const float bs = (FMT == 8 && o0 + r < O) ? sc[(size_t)((o0 + r) >> 7) * nblk + (col >> 7)] : 1.f;
+                        const float bs = o0 + r < O ? sc[(size_t)((o0 + r) >> 7) * nblk + (col >> 7)] : 1.f;
                         const uint32_t wds[4] = {cur[r].x, cur[r].y, cur[r].z, cur[r].w};
 #pragma unroll
                         for (int b = 0; b < 16; b++) {
                             const uint32_t byte = (wds[b >> 2] >> (8 * (b & 3))) & 0xFFu;
-                            wd[r][b] = FMT == 8 ? s_lut[byte] * bs : (float)(int)(int8_t)byte;
+                            wd[r][b] = s_lut[byte] * bs;
                         }
                     }
 #pragma unroll
@@ -419,7 +465,7 @@ __global__ void __launch_bounds__(256, FMT == 0 ? 3 : 2) k_dense_gemv(float *__r
 #pragma unroll
             for (int off = 16; off; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
             if (lane == 0 && q < ns && o0 + r < O)
-                y[(size_t)(s0 + q) * O + o0 + r] = FMT == 1 ? a * sc[o0 + r] : a;
+                y[(size_t)(s0 + q) * O + o0 + r] = a;
         }
 }
 
