@@ -23,6 +23,7 @@
 #include "moe_decode.cuh"
 #include "gemm_tc.cuh"
 #include "dense_mma.cuh"
+#include "gemv_rows.cuh"
 #include "ep_kernels.cuh"
 
 // ---------------------------------------------------------------------------
@@ -159,6 +160,12 @@ static int decode_smem_bytes(int mode) {
            2 * DEC_PART_BYTES + dec_act_bytes(mode);
 }
 
+template <int MODE>
+static void setup_decode() {
+    set_smem(k_moe_decode<MODE, false>, decode_smem_bytes(MODE)); set_smem(k_moe_decode<MODE, true>, decode_smem_bytes(MODE));
+    set_smem(k_gemv_rows<MODE, 1>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096); set_smem(k_gemv_rows<MODE, 2>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096);
+}
+
 extern "C" int coli_cuda_init(const int *devices, int count) {
     if (!devices || count < 1 || count > COLI_CUDA_MAX_DEVICES) return 0;
     if (g_nctx) coli_cuda_shutdown();
@@ -201,8 +208,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         setup_mode<SC_ROW>(); setup_mode<SC_H16>(); setup_mode<SC_F32>(); setup_mode<SC_MX>();
         set_smem(k_router_logits, ROUTER_TILE_SMEM);
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
-        set_smem(k_moe_decode<SC_ROW>, decode_smem_bytes(SC_ROW)); set_smem(k_moe_decode<SC_H16>, decode_smem_bytes(SC_H16));
-        set_smem(k_moe_decode<SC_F32>, decode_smem_bytes(SC_F32)); set_smem(k_moe_decode<SC_MX>, decode_smem_bytes(SC_MX));
+        setup_decode<SC_ROW>(); setup_decode<SC_H16>(); setup_decode<SC_F32>(); setup_decode<SC_MX>();
         set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
         set_smem(k_expert_gemm_tc<SC_H16, 1>, tc_smem_total(SC_H16)); set_smem(k_expert_gemm_tc<SC_H16, 2>, tc_smem_total(SC_H16));
         set_smem(k_expert_gemm_tc<SC_MX, 1>, tc_smem_total(SC_MX)); set_smem(k_expert_gemm_tc<SC_MX, 2>, tc_smem_total(SC_MX));
@@ -696,9 +702,30 @@ static int run_host_segs(DeviceCtx *c, HostSegs *hs, Buf *segbuf, int ctl_slot, 
     return cuda_ok(cudaGetLastError(), "gemv launch");
 }
 
+// Rows the one-launch kernel takes: up to 8, and up to 96 KB of split activations beside its weight ring.
+template <int MODE, int NC>
+static void launch_rows(DeviceCtx *c, const ColiCudaTensor *t, float *y, const float *x, int S) {
+    k_gemv_rows<MODE, NC><<<t->O / 16, ROWS_WARPS * 32, rows_smem(MODE, S, t->I), c->stream>>>(y, x, t->pk, t->rowscale, S, t->I, t->O,
+                                                                                              c->status);
+}
+
 // y_dev[S,O] = x_dev[S,I] @ W^T for a packed tensor, all on c->stream.
 static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {
     const int nkb = t->I / BLOCK_K;
+    if (S <= 8 && S * t->I <= ROWS_MAX_X && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0) {
+        switch (t->mode * 2 + (S > 4)) {
+        case SC_ROW * 2: launch_rows<SC_ROW, 1>(c, t, y_dev, x_dev, S); break;
+        case SC_ROW * 2 + 1: launch_rows<SC_ROW, 2>(c, t, y_dev, x_dev, S); break;
+        case SC_H16 * 2: launch_rows<SC_H16, 1>(c, t, y_dev, x_dev, S); break;
+        case SC_H16 * 2 + 1: launch_rows<SC_H16, 2>(c, t, y_dev, x_dev, S); break;
+        case SC_F32 * 2: launch_rows<SC_F32, 1>(c, t, y_dev, x_dev, S); break;
+        case SC_F32 * 2 + 1: launch_rows<SC_F32, 2>(c, t, y_dev, x_dev, S); break;
+        case SC_MX * 2: launch_rows<SC_MX, 1>(c, t, y_dev, x_dev, S); break;
+        default: launch_rows<SC_MX, 2>(c, t, y_dev, x_dev, S); break;
+        }
+        c->last_launches++;
+        return cuda_ok(cudaGetLastError(), "linear launch");
+    }
     const int nc = pick_nc(S), rpp = 4 * nc;
     const int npass = (S + rpp - 1) / rpp;
     const int nkpart = pick_nkpart(nkb, (long)npass * (t->O / TILE_ROWS), c->sms);
@@ -824,7 +851,7 @@ extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *
     DeviceCtx *c = find_ctx(t->device);
     if (!select_ctx(c)) return 0;
     size_t xb = (size_t)S * I * sizeof(float), yb = (size_t)S * O * sizeof(float);
-    const float *xd = io_in(c, x, xb, t->packed || t->fmt != 0);
+    const float *xd = io_in(c, x, xb, t->packed ? S > 8 : t->fmt != 0);
     float *yd = io_out(c, yb);
     if (!xd || !yd) return 0;
     timing_begin(c);
@@ -1004,6 +1031,133 @@ static int group_device_tc(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaT
     return tc_ffn(c, gates[0]->mode, downs[0]->mode, dl, x_dev, x_bf16, total, ngrp, D, I, y_dev);
 }
 
+static int g_fused_decode = 3;
+extern "C" void coli_cuda_set_fused_decode(int enabled) { g_fused_decode = enabled; }
+#ifdef COLI_DECODE_PROBE
+// Development builds only (-DCOLI_DECODE_PROBE): phase timestamps of the fused kernel.
+static unsigned long long *g_decode_probe = nullptr;
+extern "C" void coli_cuda_set_decode_probe(void *dev_buffer) { g_decode_probe = static_cast<unsigned long long *>(dev_buffer); }
+#endif
+
+// Warps that share one unit of a phase of the fused decode kernel (4, 8 or 16): the count
+// that wastes the fewest warp slots on the phase's nkb blocks, ties going to 8 for the
+// gate/up phase (few units per CTA) and to 4 for the down phase (many). A function of the
+// shape only: the order of every sum in the kernel follows from it.
+static int dec_pick_wpk(int nkb, int phase) {
+    const int pref[2][3] = {{8, 16, 4}, {4, 8, 16}};
+    int best = 0, bw = 1 << 30;
+    for (int i = 0; i < 3; i++) {
+        const int w = pref[phase - 1][i];
+        const int waste = (nkb + w - 1) / w * w - nkb;
+        if (waste < bw) { bw = waste; best = w; }
+    }
+    return best;
+}
+
+// Launches the fused decode kernel; a carries the problem (rule, x, out, M and, for a layer, tables, logits and
+// routing outputs), preset the pass list of a call whose routing the host knows. npos: packed rows at most.
+static int launch_decode(DeviceCtx *c, int mode, DecodeArgs &a, const DecPreset *preset, int npos, Buf *xq, Buf *xs, Buf *hq,
+                         Buf *hs, Buf *pd) {
+    const int D = a.rule.D, I = a.rule.I, nkb1 = D / BLOCK_K, nkb2 = I / BLOCK_K;
+    const size_t act_cap = (size_t)dec_act_bytes(mode);
+    a.act_smem = (size_t)a.M * nkb1 * 516 <= act_cap;
+    // Down phase with a local combine (a CTA owns 16 output rows over every pass): when every
+    // pass row's activations fit one CTA's shared memory and D/16 slices spread well over the SMs.
+    const long units2 = D / 16, waves2 = (units2 + c->sms - 1) / c->sms;
+    a.wpk1 = dec_pick_wpk(nkb1, 1); a.wpk2 = dec_pick_wpk(nkb2, 2);
+    a.local2 = (size_t)npos * ((size_t)I * 4 + (size_t)nkb2 * 16 + 64) <= act_cap && units2 * 100 >= 85 * waves2 * c->sms &&
+               (size_t)npos * a.wpk2 * 64 <= (size_t)2 * DEC_PART_BYTES;
+    if (!reserve(c, hq, (size_t)npos * I * 2 * sizeof(__half)) || !reserve(c, hs, (size_t)npos * (I / 32) * sizeof(float)) ||
+        !reserve(c, pd, (size_t)npos * D * sizeof(float))) return 0;
+    if (!a.act_smem) {
+        // x does not fit the kernel's shared memory: split it once here, the kernel reads the fragments
+        if (!reserve(c, xq, (size_t)a.M * D * 2 * sizeof(__half)) || !reserve(c, xs, (size_t)a.M * nkb1 * sizeof(float))) return 0;
+        k_prep_rows<<<(a.M * nkb1 * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)xq->p, (float *)xs->p, a.x, nullptr, a.M, D);
+        c->last_launches++;
+    }
+    a.xq = (const __half *)xq->p; a.xs = (const float *)xs->p;
+    a.hq = (__half *)hq->p; a.hs = (float *)hs->p; a.Y = (float *)pd->p;
+    a.sync = c->dec_sync; a.exp_tab = c->exp_tab_dev; a.status = c->status;
+    a.mg_grid = dec_magic((unsigned int)c->sms); a.mg_nt1 = dec_magic((unsigned int)(I / TILE_ROWS));
+    a.mg_nt2 = dec_magic((unsigned int)(D / TILE_ROWS));
+#ifdef COLI_DECODE_PROBE
+    a.probe = g_decode_probe;
+#endif
+    DecRouted routed;
+    void *args[] = {&a, preset ? const_cast<DecPreset *>(preset) : static_cast<void *>(&routed)};
+    static const void *const fns[4][2] = {
+        {(const void *)k_moe_decode<SC_ROW, false>, (const void *)k_moe_decode<SC_ROW, true>},
+        {(const void *)k_moe_decode<SC_H16, false>, (const void *)k_moe_decode<SC_H16, true>},
+        {(const void *)k_moe_decode<SC_F32, false>, (const void *)k_moe_decode<SC_F32, true>},
+        {(const void *)k_moe_decode<SC_MX, false>, (const void *)k_moe_decode<SC_MX, true>}};
+    const void *fn = fns[mode][preset != nullptr];
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    kernel_event_pair(c, &e0, &e1);
+    if (e0) cudaEventRecord(e0, c->stream);
+    // 1: cooperative launch (co-residency of the grid guaranteed by the driver).
+    // 2: plain launch (the grid is one CTA per SM, so it still fits the device).
+    // 3: plain launch with programmatic stream serialisation: the next layer's CTAs are
+    //    scheduled as this grid's CTAs exit and wait at griddepcontrol.wait, which hides
+    //    most of the launch latency between back-to-back layer calls.
+    cudaError_t err;
+    const size_t smem = (size_t)decode_smem_bytes(mode);
+    if (g_fused_decode == 3) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c->sms); cfg.blockDim = dim3(DEC_WARPS * 32);
+        cfg.dynamicSmemBytes = smem; cfg.stream = c->stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        err = cudaLaunchKernelExC(&cfg, fn, args);
+    } else if (g_fused_decode == 2) {
+        err = cudaLaunchKernel(fn, dim3(c->sms), dim3(DEC_WARPS * 32), args, smem, c->stream);
+    } else {
+        err = cudaLaunchCooperativeKernel(fn, dim3(c->sms), dim3(DEC_WARPS * 32), args, smem, c->stream);
+    }
+    if (e1) cudaEventRecord(e1, c->stream);
+    c->last_launches++;
+    return cuda_ok(err, "fused decode launch");
+}
+// What the fused kernel takes, apart from its row and expert counts.
+static bool decode_shape_ok(const DeviceCtx *c, int D, int I, const void *out) {
+    return g_fused_decode && D % BLOCK_K == 0 && I % BLOCK_K == 0 && I <= DEC_MAX_I && c->sms >= DEC_MAX_PASS && c->sms <= 256 &&
+           (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+}
+
+// A grouped call of at most 8 rows (or one row through up to 16 experts, weighted and added) as one launch of
+// the fused decode kernel. -> 1 done, 0 failed, -1 not this kernel's. Against split + descriptors + two GEMVs +
+// SwiGLU + reduction (six stream operations) it takes 41 us instead of 95 for 8 experts of a 6144 x 2048 layer.
+//   rows: per expert (y gets one row per packed row), or NULL: x is one row, y = sum_i weights[i] * expert_i(x)
+static int group_decode(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTensor *const *ups, ColiCudaTensor *const *downs,
+                        const int *rows, const float *weights, int count, int D, int I, int total, float *y, const float *x) {
+    if ((rows && total > DEC_MAX_M) || !decode_shape_ok(c, D, I, y) || (reinterpret_cast<uintptr_t>(x) & 15)) return -1;
+    const int mode = gates[0]->mode;
+    DecPreset p;
+    std::memset(&p, 0, sizeof(p));
+    int off = 0;
+    for (int e = 0; e < count; e++) {
+        if (gates[e]->mode != mode || ups[e]->mode != mode || downs[e]->mode != mode) return -1;
+        const int re = rows ? rows[e] : 1;
+        for (int r0 = 0; r0 < re; r0 += 4) {
+            if (p.npass == DEC_PRESET_MAX) return -1;
+            auto &ps = p.pass[p.npass++];
+            ps.wg = gates[e]->pk; ps.wu = ups[e]->pk; ps.wd = downs[e]->pk;
+            ps.rg = gates[e]->rowscale; ps.ru = ups[e]->rowscale; ps.rd = downs[e]->rowscale;
+            ps.nrows = re - r0 < 4 ? re - r0 : 4; ps.pos0 = off + r0;
+            for (int i = 0; i < ps.nrows; i++) ps.rowid[i] = (unsigned char)(rows ? off + r0 + i : 0);
+        }
+        off += re;
+    }
+    p.npos = off;
+    for (int i = 0; i < off; i++) { p.w[i] = weights ? weights[i] : 1.f; p.pos[i] = (unsigned char)i; }
+    DecodeArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.rule.D = D; a.rule.I = I; a.rule.K = rows ? 1 : off; a.rule.gating = 1;
+    a.M = rows ? off : 1; a.x = x; a.out = y;
+    return launch_decode(c, mode, a, &p, off, &c->bq, &c->bs, &c->hq, &c->hs, &c->pd);
+}
+
 static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                         ColiCudaTensor *const *downs, const int *rows, int count, int D, int I,
                         int total, int max_rows, int all_packed, float *y_dev, const float *x_dev,
@@ -1012,6 +1166,10 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
         group_tc_ok(gates, ups, downs, count, max_rows, total))
         return group_device_tc(c, gates, ups, downs, rows, count, D, I, total, y_dev, x_dev, bcast_src != nullptr);
     if (all_packed) {
+        if (!bcast_src && rows) {
+            const int r = group_decode(c, gates, ups, downs, rows, nullptr, count, D, I, total, y_dev, x_dev);
+            if (r >= 0) return r;
+        }
         const int nc = pick_nc(max_rows), rpp = 4 * nc;
         long npass = 0;
         for (int e = 0; e < count; e++) npass += ((rows ? rows[e] : 1) + rpp - 1) / rpp;
@@ -1162,7 +1320,7 @@ extern "C" int coli_cuda_expert_mlp(ColiCudaTensor *gate, ColiCudaTensor *up, Co
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
     size_t xb = (size_t)S * D * sizeof(float);
-    const float *xd = io_in(c, x, xb, all_packed);
+    const float *xd = io_in(c, x, xb, all_packed && S > DEC_MAX_M);
     float *yd = io_out(c, xb);
     if (!xd || !yd) return 0;
     timing_begin(c);
@@ -1372,6 +1530,11 @@ extern "C" int coli_cuda_expert_group_resident_issue(ColiCudaTensor *const *gate
     if (!all_packed && any_packed) return 0;
     DeviceCtx *c = find_ctx(device), *home = find_ctx(home_device);
     if (!home || !select_ctx(c)) return 0;
+    if (device == home_device && all_packed) {
+        const int r = group_decode(c, gates, ups, downs, nullptr, weights, count, D, I, total, partial_slot_dev, x_src_dev);
+        if (r == 0) return 0;
+        if (r > 0) return cuda_ok(cudaEventRecord(c->ev_done, c->stream), "resident event record");
+    }
     // fixed capacities (64 experts) so that a re-issue never reallocates under queued work
     if (!reserve(c, &c->x, (size_t)64 * D * sizeof(float)) || !reserve(c, &c->y, (size_t)64 * D * sizeof(float)) ||
         !reserve(c, &c->misc, (size_t)(D + 64) * sizeof(float) + 4096)) return 0;

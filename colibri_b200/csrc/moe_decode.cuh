@@ -105,6 +105,18 @@ struct DecodeArgs {
 #endif
 };
 
+// A call whose experts, rows and weights the host knows (the engine's grouped and resident calls): the
+// routing is skipped and the pass list comes with the launch. Entry i = s*K + kk of row s adds w[i] times
+// packed row pos[i]; every row has K entries.
+#define DEC_PRESET_MAX 16
+struct DecPreset {
+    int npass, npos;
+    struct { const uint8_t *wg, *wu, *wd; const float *rg, *ru, *rd; int nrows, pos0; unsigned char rowid[4]; } pass[DEC_PRESET_MAX];
+    float w[DEC_PRESET_MAX];
+    unsigned char pos[DEC_PRESET_MAX];
+};
+struct DecRouted {};              // the layer's call: routing in the kernel
+
 struct DecShared {
     int idx[DEC_MAX_M * DEC_MAX_K];
     float w[DEC_MAX_M * DEC_MAX_K];
@@ -533,8 +545,11 @@ __device__ __forceinline__ void dec_part_src(int r, int mrow, int &src_lane, int
     el = (r >> 4) * 2 + ((r >> 3) & 1);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) {
+template <bool PRESET> struct DecExtra { typedef DecRouted type; };
+template <> struct DecExtra<true> { typedef DecPreset type; };
+
+template <int MODE, bool PRESET>
+__global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, typename DecExtra<PRESET>::type preset) {
     constexpr int CH = CODE_BYTES + (MODE == SC_H16 ? 256 : MODE == SC_F32 ? 512 : MODE == SC_MX ? 128 : 0);
     constexpr int NST = DEC_NST;
     constexpr int nst = NST;
@@ -711,7 +726,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
     // is expert number kk of the union, pass kk, packed row kk. The ranking threads then write the
     // pass list themselves and the weight stream starts one barrier later; the weights' tail
     // (normalisation, scale) runs in warp 0 beside it and is first needed by the final combine.
-    const bool fast1 = M == 1 && !any_bad && !(r.gating == 1 && r.topp > 0.f && r.topp < 1.f);
+    const bool fast1 = !PRESET && M == 1 && !any_bad && !(r.gating == 1 && r.topp > 0.f && r.topp < 1.f);
     // The engine's tail on the K selected weights (top-p cut, normalisation, scale): one warp per row.
     auto route_tail = [&]() {
         if (warp < M) {
@@ -823,12 +838,24 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
             sh->npass = npass; sh->npos = spos; sh->nu = K;
         }
         __syncthreads();
-        if (!fast1) route_tail();
-        if (!fast1) __syncthreads();
+        if (!PRESET && !fast1) route_tail();
+        if (!PRESET && !fast1) __syncthreads();
     }
     DEC_PROBE(a, 10);
     // ---- union, packed row order and pass list -----------------------------------------
-    if (fast1) {
+    if constexpr (PRESET) {
+        if (tid < preset.npass) {
+            DecPass &ps = sh->pass[tid];
+            ps.e = tid; ps.nrows = preset.pass[tid].nrows; ps.pos0 = preset.pass[tid].pos0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) ps.rowid[i] = preset.pass[tid].rowid[i];
+            ps.wg = preset.pass[tid].wg; ps.wu = preset.pass[tid].wu; ps.wd = preset.pass[tid].wd;
+        }
+        if (tid < M * K) { sh->w[tid] = preset.w[tid]; sh->pos_of[tid] = preset.pos[tid]; }
+        if (tid < M) sh->keff[tid] = K;
+        if (tid == 0) { sh->npass = preset.npass; sh->npos = sh->shared_pos0 = preset.npos; }
+        __syncthreads();
+    } else if (fast1) {
         // written by the ranking threads
     } else if (M == 1 && sh->rowflag[0] == 0) {
         // one row without NaN candidates: its selections are distinct experts, so entry kk is
@@ -922,7 +949,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
         }
         __syncthreads();
     }
-    if (!fast1) {
+    if (!PRESET && !fast1) {
 #pragma unroll 1
         for (int p = tid; p < sh->npass; p += blockDim.x) {
             DecPass &ps = sh->pass[p];
@@ -931,7 +958,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
         }
         __syncthreads();
     }
-    if (blockIdx.x == 0 && !fast1) {
+    if (!PRESET && blockIdx.x == 0 && !fast1) {
 #pragma unroll 1
         for (int i = tid; i < M * K; i += blockDim.x) {
             if (a.idx_out) a.idx_out[i] = sh->idx[i];
@@ -941,6 +968,15 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
     }
     DEC_PROBE(a, 1);   // routing and tables done
     const int npass = sh->npass;
+    // per-row scales of a pass's tensors (SC_ROW): which 0 gate, 1 up, 2 down
+    auto row_scales = [&](const DecPass &ps, int which) -> const float * {
+        if constexpr (PRESET)
+            return which == 0 ? preset.pass[ps.e].rg : which == 1 ? preset.pass[ps.e].ru : preset.pass[ps.e].rd;
+        else
+            return which == 0 ? (ps.e >= 0 ? a.tab.gate_rs[ps.e] : a.tab.sh_gate_rs)
+                 : which == 1 ? (ps.e >= 0 ? a.tab.up_rs[ps.e] : a.tab.sh_up_rs)
+                              : (ps.e >= 0 ? a.tab.down_rs[ps.e] : a.tab.sh_down_rs);
+    };
 
     DecPhase ph1, ph2;
     ph1.which = 1; ph1.nt = nt1; ph1.nkb = nkb1; ph1.wpk = a.wpk1; ph1.wsh = 31 - __clz(a.wpk1);
@@ -1033,8 +1069,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                 for (int w = 0; w < ph1.wpk; w++) { gs += pbase[w * 256]; us += pbase[w * 256 + 4]; }
                 if (MODE == SC_ROW) {
                     const int o = tile * TILE_ROWS + lane;
-                    gs *= (ps.e >= 0 ? a.tab.gate_rs[ps.e] : a.tab.sh_gate_rs)[o];
-                    us *= (ps.e >= 0 ? a.tab.up_rs[ps.e] : a.tab.sh_up_rs)[o];
+                    gs *= row_scales(ps, 0)[o];
+                    us *= row_scales(ps, 1)[o];
                 }
                 const float h = mrow < nrows ? (gs / (1.0f + expf(-gs))) * us : 0.f;
                 const float m = warp_max(fabsf(h));
@@ -1165,7 +1201,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                     float y = 0.f;
 #pragma unroll 4
                     for (int w = 0; w < ph2.wpk; w++) y += src[w * 16];
-                    if (MODE == SC_ROW) y *= (ps.e >= 0 ? a.tab.down_rs[ps.e] : a.tab.sh_down_rs)[u * 16 + rr];
+                    if (MODE == SC_ROW) y *= row_scales(ps, 2)[u * 16 + rr];
                     ybuf[pos * 16 + rr] = y;
                 }
             }
@@ -1234,7 +1270,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a) 
                 float y = 0.f;
                 for (int w = 0; w < ph2.wpk; w++) y += pbase[w * 256];
                 const int o = tile * TILE_ROWS + lane;
-                if (MODE == SC_ROW) y *= (ps.e >= 0 ? a.tab.down_rs[ps.e] : a.tab.sh_down_rs)[o];
+                if (MODE == SC_ROW) y *= row_scales(ps, 2)[o];
                 if (mrow < nrows) a.Y[(size_t)(ps.pos0 + mrow) * D + o] = y;
             }
         }

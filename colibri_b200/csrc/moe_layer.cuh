@@ -111,29 +111,6 @@ extern "C" void coli_cuda_moe_layer_free(ColiCudaMoeLayer *L) {
     delete L;
 }
 
-static int g_fused_decode = 3;
-extern "C" void coli_cuda_set_fused_decode(int enabled) { g_fused_decode = enabled; }
-#ifdef COLI_DECODE_PROBE
-// Development builds only (-DCOLI_DECODE_PROBE): phase timestamps of the fused kernel.
-static unsigned long long *g_decode_probe = nullptr;
-extern "C" void coli_cuda_set_decode_probe(void *dev_buffer) { g_decode_probe = static_cast<unsigned long long *>(dev_buffer); }
-#endif
-
-// Warps that share one unit of a phase of the fused decode kernel (4, 8 or 16): the count
-// that wastes the fewest warp slots on the phase's nkb blocks, ties going to 8 for the
-// gate/up phase (few units per CTA) and to 4 for the down phase (many). A function of the
-// shape only: the order of every sum in the kernel follows from it.
-static int dec_pick_wpk(int nkb, int phase) {
-    const int pref[2][3] = {{8, 16, 4}, {4, 8, 16}};
-    int best = 0, bw = 1 << 30;
-    for (int i = 0; i < 3; i++) {
-        const int w = pref[phase - 1][i];
-        const int waste = (nkb + w - 1) / w * w - nkb;
-        if (waste < bw) { bw = waste; best = w; }
-    }
-    return best;
-}
-
 struct LayerPlan {
     int nc, rpp, nkp1, nkp2, seg_cap, npos_cap;
 };
@@ -233,69 +210,13 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
         M * r.K + 2 <= DEC_MAX_PASS && c->sms >= DEC_MAX_PASS && c->sms <= 256 &&
         (reinterpret_cast<uintptr_t>(out_dev) & 15) == 0) {
         // one kernel for the whole layer (moe_decode.cuh)
-        const size_t act_cap = (size_t)dec_act_bytes(L->mode_gu);
-        const int act_smem = (size_t)M * nkb1 * 516 <= act_cap;
-        // Down phase with a local combine (a CTA owns 16 output rows over every pass): when every
-        // pass row's activations fit one CTA's shared memory and D/16 slices spread well over the SMs.
-        const long units2 = r.D / 16, waves2 = (units2 + c->sms - 1) / c->sms;
-        const int local2 = (size_t)p.npos_cap * ((size_t)r.I * 4 + (size_t)nkb2 * 16 + 64) <= act_cap &&
-                           units2 * 100 >= 85 * waves2 * c->sms &&
-                           (size_t)p.npos_cap * dec_pick_wpk(nkb2, 2) * 64 <= (size_t)2 * DEC_PART_BYTES;
-        if (!reserve(c, &L->hq, (size_t)p.npos_cap * r.I * 2 * sizeof(__half)) ||
-            !reserve(c, &L->hs, (size_t)p.npos_cap * (r.I / 32) * sizeof(float)) ||
-            !reserve(c, &L->pd, (size_t)p.npos_cap * r.D * sizeof(float))) return 0;
-        if (!act_smem) {
-            // x does not fit the kernel's shared memory: split it once here, the kernel reads the fragments
-            k_prep_rows<<<(M * nkb1 * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)L->xq.p, (float *)L->xs.p, x_dev, nullptr, M, r.D);
-            c->last_launches++;
-        }
         DecodeArgs a;
         std::memset(&a, 0, sizeof(a));
         a.rule = r; a.tab = L->tab;
         a.x = x_dev; a.logits = lg; a.router_bias = L->router_bias;
         a.out = out_dev; a.idx_out = idx_dev; a.w_out = w_dev; a.keff_out = keff_dev;
-        a.xq = (const __half *)L->xq.p; a.xs = (const float *)L->xs.p;
-        a.hq = (__half *)L->hq.p; a.hs = (float *)L->hs.p; a.Y = (float *)L->pd.p;
-        a.sync = c->dec_sync; a.exp_tab = c->exp_tab_dev; a.status = c->status;
-        a.M = M; a.act_smem = act_smem;
-        a.wpk1 = dec_pick_wpk(nkb1, 1); a.wpk2 = dec_pick_wpk(nkb2, 2); a.local2 = local2;
-        a.mg_grid = dec_magic((unsigned int)c->sms); a.mg_nt1 = dec_magic((unsigned int)(r.I / TILE_ROWS));
-        a.mg_nt2 = dec_magic((unsigned int)(r.D / TILE_ROWS));
-#ifdef COLI_DECODE_PROBE
-        a.probe = g_decode_probe;
-#endif
-        void *args[] = {&a};
-        const void *fn = L->mode_gu == SC_ROW ? (const void *)k_moe_decode<SC_ROW>
-                       : L->mode_gu == SC_H16 ? (const void *)k_moe_decode<SC_H16>
-                       : L->mode_gu == SC_F32 ? (const void *)k_moe_decode<SC_F32>
-                                              : (const void *)k_moe_decode<SC_MX>;
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        kernel_event_pair(c, &e0, &e1);
-        if (e0) cudaEventRecord(e0, c->stream);
-        // 1: cooperative launch (co-residency of the grid guaranteed by the driver).
-        // 2: plain launch (the grid is one CTA per SM, so it still fits the device).
-        // 3: plain launch with programmatic stream serialisation: the next layer's CTAs are
-        //    scheduled as this grid's CTAs exit and wait at griddepcontrol.wait, which hides
-        //    most of the launch latency between back-to-back layer calls.
-        cudaError_t err;
-        if (g_fused_decode == 3) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(c->sms); cfg.blockDim = dim3(DEC_WARPS * 32);
-            cfg.dynamicSmemBytes = (size_t)decode_smem_bytes(L->mode_gu); cfg.stream = c->stream;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = at; cfg.numAttrs = 1;
-            err = cudaLaunchKernelExC(&cfg, fn, args);
-        } else if (g_fused_decode == 2) {
-            err = cudaLaunchKernel(fn, dim3(c->sms), dim3(DEC_WARPS * 32), args, (size_t)decode_smem_bytes(L->mode_gu), c->stream);
-        } else {
-            err = cudaLaunchCooperativeKernel(fn, dim3(c->sms), dim3(DEC_WARPS * 32), args,
-                                              (size_t)decode_smem_bytes(L->mode_gu), c->stream);
-        }
-        if (e1) cudaEventRecord(e1, c->stream);
-        c->last_launches++;
-        return cuda_ok(err, "fused decode launch");
+        a.M = M;
+        return launch_decode(c, L->mode_gu, a, nullptr, p.npos_cap, &L->xq, &L->xs, &L->hq, &L->hs, &L->pd);
     }
     {
         const int warps = 4;
