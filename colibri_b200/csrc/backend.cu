@@ -206,7 +206,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         }
         *c->status = 0;
         setup_mode<SC_ROW>(); setup_mode<SC_H16>(); setup_mode<SC_F32>(); setup_mode<SC_MX>();
-        set_smem(k_router_logits, ROUTER_TILE_SMEM);
+        set_smem(k_router_logits<16>, router_smem(16)); set_smem(k_router_logits<64>, router_smem(64));
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         setup_decode<SC_ROW>(); setup_decode<SC_H16>(); setup_decode<SC_F32>(); setup_decode<SC_MX>();
         set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
@@ -1424,7 +1424,7 @@ extern "C" int coli_cuda_pipe_rmsnorm_s(int device, float *y_dev, const float *x
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (S < 1 || D < 1 || xstride < D || ystride < D || !select_ctx(c)) return 0;
-    k_rmsnorm<<<S, 256, 0, c->stream>>>(y_dev, x_dev, w_dev, D, eps, xstride, ystride);
+    k_rmsnorm<<<S, RMSNORM_THREADS, 0, c->stream>>>(y_dev, x_dev, w_dev, D, eps, xstride, ystride);
     return cuda_ok(cudaGetLastError(), "pipe rmsnorm");
 }
 extern "C" int coli_cuda_pipe_rmsnorm(int device, float *y_dev, const float *x_dev, const float *w_dev,
@@ -1494,29 +1494,31 @@ extern "C" int coli_cuda_pipe_sync(int device) {
     return cuda_ok(cudaDeviceSynchronize(), "pipe sync");
 }
 
+// Few outputs per CTA while that fills no more than two waves of SMs with chains; then 64, which share x and
+// weight tiles better.
+static void launch_router(DeviceCtx *c, float *logits, const float *x, const float *w, int M, int D, int E) {
+    const int n = M * E;
+    if (n <= 16 * 4 * c->sms) k_router_logits<16><<<(n + 15) / 16, ROUTER_THREADS, router_smem(16), c->stream>>>(logits, x, w, M, D, E);
+    else k_router_logits<64><<<(n + 63) / 64, ROUTER_THREADS, router_smem(64), c->stream>>>(logits, x, w, M, D, E);
+}
+
 extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void *rw_dev, const void *rb_dev,
                                      int D, int E, int Ksel, float topp, int norm_topk, float routed_scale,
                                      int *idx_host, float *w_host, int *keff_host) {
     DeviceCtx *c = find_ctx(device);
     if (!x_dev || !rw_dev || !rb_dev || D < 1 || E < 1 || E > ROUTE_MAX_E || Ksel < 1 || Ksel > ROUTE_MAX_K ||
         Ksel > E || !idx_host || !w_host || !keff_host || !select_ctx(c)) return 0;
-    size_t need = (size_t)E * 4 + (size_t)Ksel * 8 + 16;
-    if (!reserve(c, &c->misc, need)) return 0;
-    float *logits = (float *)c->misc.p;
-    int *idx = (int *)(logits + E);
-    float *w = (float *)(idx + Ksel);
-    int *keff = (int *)(w + Ksel);
+    // the selection goes straight to pinned memory: idx [Ksel] | w [Ksel] | keff
+    if (!reserve(c, &c->misc, (size_t)E * 4) || !reserve_pinned(&c->io_y, &c->io_y_cap, (size_t)Ksel * 8 + 4)) return 0;
+    float *logits = (float *)c->misc.p, *w = c->io_y + Ksel;
+    int *idx = (int *)c->io_y, *keff = (int *)(w + Ksel);
     RouteRule rule{D, 0, E, Ksel, 1, norm_topk, routed_scale, topp};
-    k_router_logits<<<(E + 63) / 64, ROUTER_THREADS, ROUTER_TILE_SMEM, c->stream>>>(logits, x_dev, (const float *)rw_dev, 1, D, E);
-    size_t sm = (size_t)(2 * E + 2 * ROUTE_MAX_K) * sizeof(float);
-    k_route_topk<<<1, 32, sm, c->stream>>>(logits, (const float *)rb_dev, rule, 1, idx, w, keff);
-    if (!cuda_ok(cudaGetLastError(), "pipe router launch")) return 0;
-    std::vector<char> buf((size_t)Ksel * 8 + 4);
-    if (!cuda_ok(cudaMemcpyAsync(buf.data(), idx, buf.size(), cudaMemcpyDeviceToHost, c->stream), "pipe router readback") ||
-        !cuda_ok(cudaStreamSynchronize(c->stream), "pipe router sync")) return 0;
-    std::memcpy(idx_host, buf.data(), (size_t)Ksel * 4);
-    std::memcpy(w_host, buf.data() + (size_t)Ksel * 4, (size_t)Ksel * 4);
-    std::memcpy(keff_host, buf.data() + (size_t)Ksel * 8, 4);
+    launch_router(c, logits, x_dev, (const float *)rw_dev, 1, D, E);
+    k_route_topk<<<1, ROUTE_THREADS, route_smem(E), c->stream>>>(logits, (const float *)rb_dev, rule, 1, idx, w, keff);
+    if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !cuda_ok(cudaStreamSynchronize(c->stream), "pipe router sync")) return 0;
+    std::memcpy(idx_host, idx, (size_t)Ksel * 4);
+    std::memcpy(w_host, w, (size_t)Ksel * 4);
+    std::memcpy(keff_host, keff, 4);
     return 1;
 }
 

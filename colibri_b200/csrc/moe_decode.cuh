@@ -208,106 +208,16 @@ __device__ __forceinline__ void grid_barrier(unsigned int *sync, int *s_failed, 
     }
 }
 
-// One row of routing by one warp, outputs in shared memory. `tab` is the 2^(i/32)
-// table of expf_exact.h (shared memory here, so that 32 lanes with 32 different
-// indices do not serialise on the constant cache).
-//
 // Selection: the engine makes K passes of "largest untaken by strict '>', lowest
 // index wins ties". When every candidate is an ordinary number above -1e30 that is
 // the same as ranking: rank(e) = #{e' : c[e'] > c[e] or (c[e'] == c[e] and e' < e)},
-// and slot kk holds the element of rank kk. Each lane ranks its own elements against
-// all E values (independent shared-memory reads, no cross-lane traffic). Rows with a
-// NaN or a value <= -1e30 take the pass-by-pass form, which also reproduces the
-// engine's "nothing found -> expert kk" degradation.
-__device__ __forceinline__ void route_row_warp(const float *z, const float *bias, const RouteRule &rule,
-                                               float *score, float *choice, int *idx, float *wk,
-                                               int *keff, int lane, const uint64_t *tab) {
-    const int E = rule.E, K = rule.K;
-    if (rule.gating == 0) {
-        float m = -1e30f;
-        for (int e = lane; e < E; e += 32) { float v = z[e]; if (v > m) m = v; }
-#pragma unroll
-        for (int off = 16; off; off >>= 1) { float o = __shfl_xor_sync(0xffffffffu, m, off); if (o > m) m = o; }
-        for (int e = lane; e < E; e += 32) score[e] = coli_expf_exact(__fsub_rn(z[e], m), tab);
-        __syncwarp();
-        float tot = 0.f;
-        if (lane == 0) {     // the engine's serial ascending sum; loads batched four at a time
-            int e = 0;
-            const bool al = (reinterpret_cast<uintptr_t>(score) & 15) == 0;   // else scalar adds, same order
-            for (; al && e + 4 <= E; e += 4) {
-                float4 v = *reinterpret_cast<const float4 *>(score + e);
-                tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, v.x), v.y), v.z), v.w);
-            }
-            for (; e < E; e++) tot = __fadd_rn(tot, score[e]);
-        }
-        tot = __shfl_sync(0xffffffffu, tot, 0);
-        for (int e = lane; e < E; e += 32) { float p = __fdiv_rn(score[e], tot); score[e] = p; choice[e] = p; }
-    } else {
-        for (int e = lane; e < E; e += 32) {
-            float sg = __fdiv_rn(1.f, __fadd_rn(1.f, coli_expf_exact(-z[e], tab)));
-            score[e] = sg;
-            choice[e] = bias ? __fadd_rn(sg, bias[e]) : sg;
-        }
-    }
-    __syncwarp();
-    bool odd = false;
-    for (int e = lane; e < E; e += 32) { float c = choice[e]; odd |= !(c > -1e30f); }
-    if (!__any_sync(0xffffffffu, odd)) {
-        for (int e = lane; e < E; e += 32) {
-            const float c = choice[e];
-            int rank = 0;
-            for (int o = 0; o < E; o++) { float v = choice[o]; rank += (v > c) || (v == c && o < e); }
-            if (rank < K) { idx[rank] = e; wk[rank] = score[e]; }
-        }
-        __syncwarp();
-    } else {
-        for (int kk = 0; kk < K; kk++) {
-            int best = -1;
-            float bv = -1e30f;
-            for (int e = lane; e < E; e += 32) { float c = choice[e]; if (c > bv) { bv = c; best = e; } }
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-                float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-                int ob = __shfl_xor_sync(0xffffffffu, best, off);
-                bool take = ob >= 0 && (best < 0 || ov > bv || (ov == bv && ob < best));
-                if (take) { bv = ov; best = ob; }
-            }
-            if (best < 0) best = kk < E ? kk : 0;
-            if (lane == 0) { idx[kk] = best; wk[kk] = score[best]; choice[best] = __uint_as_float(0x7fc00000u); }
-            __syncwarp();
-        }
-    }
-    if (lane == 0) {
-        int Ke = K;
-        if (rule.gating == 1 && rule.topp > 0.f && rule.topp < 1.f) {
-            for (int a = 1; a < K; a++) {
-                int ii = idx[a]; float ww = wk[a]; int b = a - 1;
-                while (b >= 0 && wk[b] < ww) { wk[b + 1] = wk[b]; idx[b + 1] = idx[b]; b--; }
-                wk[b + 1] = ww; idx[b + 1] = ii;
-            }
-            float tot = 1e-20f;
-            for (int kk = 0; kk < K; kk++) tot = __fadd_rn(tot, wk[kk]);
-            float cum = 0.f;
-            for (int kk = 0; kk < K; kk++) {
-                cum = __fadd_rn(cum, wk[kk]);
-                if (cum >= __fmul_rn(rule.topp, tot)) { Ke = kk + 1; break; }
-            }
-        }
-        if (rule.norm_topk) {
-            float sm = 0.f;
-            for (int kk = 0; kk < Ke; kk++) sm = __fadd_rn(sm, wk[kk]);
-            if (rule.gating == 1) sm = __fadd_rn(sm, 1e-20f);
-            for (int kk = 0; kk < Ke; kk++) wk[kk] = __fdiv_rn(wk[kk], sm);
-        }
-        if (rule.gating == 1) for (int kk = 0; kk < Ke; kk++) wk[kk] = __fmul_rn(wk[kk], rule.routed_scale);
-        *keff = Ke;
-    }
-    __syncwarp();
-}
-
+// and slot kk holds the element of rank kk. Rows with a NaN or a value <= -1e30 take the
+// pass-by-pass form, which also reproduces the engine's "nothing found -> expert kk" degradation.
+//
 // CTA-parallel routing of M rows (all threads of the CTA). score/choice: [M*E] floats
-// of scratch; outputs idx/wk [M*K], keff [M] in shared memory. Same arithmetic, element
-// for element, as route_row_warp.
+// of scratch; outputs idx/wk [M*K], keff [M] in shared memory. `tab` is the 2^(i/32) table of
+// expf_exact.h (shared memory, so that 32 lanes with 32 different indices do not serialise on the
+// constant cache).
 __device__ __noinline__ void route_rows_cta(const float *logits, const float *bias, const RouteRule &rule,
                                                int M, float *score, float *choice, float *rowtmp,
                                                int *rowflag, int *idx, float *wk, int *keff,
@@ -663,7 +573,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 
     // ---- routing, redundantly in every CTA -------------------------------------------
     // Scores: softmax rows by one warp each (the serial denominator is the long pole),
-    // sigmoid scores by all threads. Same arithmetic, element for element, as route_row_warp.
+    // sigmoid scores by all threads. Same arithmetic, element for element, as route_rows_cta.
     bool bad = false;
     if (r.gating == 0) {
         if (warp < M) {
@@ -786,7 +696,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         route_rows_cta(a.logits, a.router_bias, sh->rule, M, score, choice, sh->rowtmp, sh->rowflag, sh->idx, sh->w,
                        sh->keff, reinterpret_cast<const uint64_t *>(sh->exp_tab));
     } else {
-        // Selection by ranking (see route_row_warp): slot kk holds the element of rank kk. Four
+        // Selection by ranking (see route_rows_cta): slot kk holds the element of rank kk. Four
         // neighbouring lanes share an element: each counts over a quarter of the candidates.
         {
             const int q = tid & 3;
@@ -1313,31 +1223,29 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     }
 }
 
-// Stand-alone routing kernel of the multi-kernel path: one warp per row, E <= 1024,
-// K <= 64; the same routing function as the fused kernel.
-__global__ void k_route_topk(const float *__restrict__ logits, const float *__restrict__ bias,
-                             RouteRule rule, int M, int *__restrict__ idx_out,
-                             float *__restrict__ w_out, int *__restrict__ keff_out) {
-    extern __shared__ float sm_route[];
+// Stand-alone routing kernel of the multi-kernel path: one CTA per row (one warp per row took 49 us for
+// 2048 rows of 256 scores), E <= 1024, K <= 64; the same routing function as the fused kernel. Dynamic shared
+// memory: 2 * E floats.
+#define ROUTE_THREADS 128
+__global__ void __launch_bounds__(ROUTE_THREADS) k_route_topk(const float *__restrict__ logits, const float *__restrict__ bias,
+                                                              RouteRule rule, int M, int *__restrict__ idx_out,
+                                                              float *__restrict__ w_out, int *__restrict__ keff_out) {
+    extern __shared__ __align__(16) float sm_route[];
     __shared__ unsigned long long s_tab[32];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int E = rule.E, K = rule.K;
-    if (threadIdx.x < 32) s_tab[threadIdx.x] = c_exp2_tab[threadIdx.x];
+    __shared__ RouteRule s_rule;
+    __shared__ float s_tmp[2 * DEC_MAX_M], s_wk[ROUTE_MAX_K];
+    __shared__ int s_flag[DEC_MAX_M], s_idx[ROUTE_MAX_K], s_keff[1];
+    const int s = blockIdx.x, tid = threadIdx.x, E = rule.E, K = rule.K;
+    if (tid < 32) s_tab[tid] = c_exp2_tab[tid];
+    if (tid == 0) s_rule = rule;
     __syncthreads();
-    float *score = sm_route + (size_t)warp * (2 * E + 2 * ROUTE_MAX_K);
-    float *choice = score + E;
-    int *idx = reinterpret_cast<int *>(choice + E);
-    float *wk = reinterpret_cast<float *>(idx + ROUTE_MAX_K);
-    __shared__ int s_keff[32];
-    int s = blockIdx.x * warps + warp;
-    if (s >= M) return;
-    route_row_warp(logits + (size_t)s * E, bias, rule, score, choice, idx, wk, &s_keff[warp], lane,
+    // E rounded up to 4: the second array starts 16-byte aligned too
+    route_rows_cta(logits + (size_t)s * E, bias, s_rule, 1, sm_route, sm_route + ((E + 3) & ~3), s_tmp, s_flag, s_idx, s_wk, s_keff,
                    reinterpret_cast<const uint64_t *>(s_tab));
-    if (lane == 0) {
-        for (int kk = 0; kk < K; kk++) {
-            idx_out[(size_t)s * K + kk] = idx[kk];
-            w_out[(size_t)s * K + kk] = wk[kk];
-        }
-        keff_out[s] = s_keff[warp];
+    for (int kk = tid; kk < K; kk += ROUTE_THREADS) {
+        idx_out[(size_t)s * K + kk] = s_idx[kk];
+        w_out[(size_t)s * K + kk] = s_wk[kk];
     }
+    if (tid == 0) keff_out[s] = s_keff[0];
 }
+static inline size_t route_smem(int E) { return (size_t)2 * ((E + 3) & ~3) * sizeof(float); }

@@ -200,8 +200,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     const float *lg = logits_dev;
     if (!lg) {
         if (!L->router_w) return 0;
-        int n = M * r.E;
-        k_router_logits<<<(n + 63) / 64, ROUTER_THREADS, ROUTER_TILE_SMEM, c->stream>>>((float *)L->logits.p, x_dev, L->router_w, M, r.D, r.E);
+        launch_router(c, (float *)L->logits.p, x_dev, L->router_w, M, r.D, r.E);
         c->last_launches++;
         lg = (const float *)L->logits.p;
     }
@@ -218,12 +217,8 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
         a.M = M;
         return launch_decode(c, L->mode_gu, a, nullptr, p.npos_cap, &L->xq, &L->xs, &L->hq, &L->hs, &L->pd);
     }
-    {
-        const int warps = 4;
-        size_t sm = (size_t)warps * (2 * r.E + 2 * ROUTE_MAX_K) * sizeof(float);
-        k_route_topk<<<(M + warps - 1) / warps, warps * 32, sm, c->stream>>>(lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
-        c->last_launches++;
-    }
+    k_route_topk<<<M, ROUTE_THREADS, route_smem(r.E), c->stream>>>(lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
+    c->last_launches++;
     if (use_tc)
         return layer_run_tc(L, c, out_dev, x_dev, M, idx_dev, w_dev, keff_dev);
     int *scal = (int *)L->scal.p;   // [0]=nu [1]=npos [2]=shared_pos0
@@ -355,9 +350,7 @@ extern "C" int coli_cuda_route_topk_dev(int device, const float *logits_dev, con
     if (!logits_dev || !idx_dev || !w_dev || !keff_dev || M < 1 || E < 1 || E > ROUTE_MAX_E || K < 1 ||
         K > ROUTE_MAX_K || K > E || !select_ctx(c)) return 0;
     RouteRule r{0, 0, E, K, gating, norm_topk, routed_scale, topp};
-    const int warps = 4;
-    size_t sm = (size_t)warps * (2 * E + 2 * ROUTE_MAX_K) * sizeof(float);
-    k_route_topk<<<(M + warps - 1) / warps, warps * 32, sm, c->stream>>>(logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
+    k_route_topk<<<M, ROUTE_THREADS, route_smem(E), c->stream>>>(logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "route launch");
 }

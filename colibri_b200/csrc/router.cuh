@@ -25,29 +25,29 @@ __device__ __forceinline__ float expf_host_exact(float x) { return coli_expf_exa
 
 // logits[s*E+e] = sum_i x[s,i]*W[e,i], ascending i, multiply and add rounded separately
 // (the engine's order, so the sum is one dependent chain of D additions per output: about
-// 4 cycles each, which is the floor). One thread per (s,e), 64 outputs per CTA. The operands
-// are brought in by the CTA together: per 64-column tile, row r of the tile is the 64 floats
-// of output r's weight row (and of its x row), copied asynchronously with coalesced accesses
-// into a ring of ROUTER_STAGES shared-memory tiles (row stride 68 floats, so that rows start
-// 16-byte aligned and the 128-bit reads of threads walking different rows do not collide);
-// the copies run ROUTER_STAGES - 1 tiles ahead of the arithmetic, which hides the memory
-// latency behind the chain (one tile ahead left the kernel waiting for memory: 300 us for
-// 8 x 256 outputs of 7168 terms).
-// The CTA has ROUTER_THREADS threads: all of them issue copies, the first 64 own the outputs.
-// Launch: ROUTER_THREADS threads, ROUTER_TILE_SMEM bytes of dynamic shared memory.
-#define ROUTER_THREADS 256
+// 4 cycles each, which is the floor: 13 us at D = 6144). One thread per (s,e), OUT outputs per CTA: few,
+// because an SM takes in about 50 B per cycle and 64 weight rows at once were slower than their chains.
+// Per 64-column tile, row r of the tile is the 64 floats of output r's weight row (and of its x row),
+// brought in by the copy warps with asynchronous copies, ROUTER_STAGES - 1 tiles ahead (row stride 68
+// floats: rows start 16-byte aligned and the 128-bit reads of 8 threads walking different rows do not
+// collide). The products of tile t are formed while the additions of tile t-1 run: the loads and
+// multiplications fill the chain's gaps. Measured at 256 outputs of 6144 terms: 89 us with 64 outputs
+// per CTA and products before additions.
+// Launch: ROUTER_THREADS threads, router_smem(OUT) bytes of dynamic shared memory.
+#define ROUTER_THREADS 128
 #define ROUTER_TILE 64
 #define ROUTER_LD 68
-#define ROUTER_STAGES 6
-#define ROUTER_TILE_SMEM (ROUTER_STAGES * 2 * 64 * ROUTER_LD * 4)
+#define ROUTER_STAGES 8
+__host__ __device__ constexpr int router_smem(int out) { return ROUTER_STAGES * 2 * out * ROUTER_LD * 4; }
+template <int OUT>
 __global__ void __launch_bounds__(ROUTER_THREADS) k_router_logits(float *__restrict__ logits, const float *__restrict__ x,
-                                                      const float *__restrict__ W, int M, int D, int E) {
-    extern __shared__ __align__(16) float rt[];         // [stage][w | x][64][68]
-    __shared__ const float *s_wrow[64], *s_xrow[64];
-    constexpr int LD = ROUTER_LD, NS = ROUTER_STAGES, NW = ROUTER_THREADS / 32;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int i0 = blockIdx.x * 64, n = M * E;
-    const int nrow = min(64, n - i0);
+                                                                  const float *__restrict__ W, int M, int D, int E) {
+    extern __shared__ __align__(16) float rt[];         // [stage][w | x][OUT][68]
+    __shared__ const float *s_wrow[OUT], *s_xrow[OUT];
+    constexpr int LD = ROUTER_LD, NS = ROUTER_STAGES, CW = (OUT + 31) / 32, NC = ROUTER_THREADS - CW * 32;
+    const int tid = threadIdx.x, ctid = tid - CW * 32;
+    const int i0 = blockIdx.x * OUT, n = M * E;
+    const int nrow = min(OUT, n - i0);
     const bool al16 = (D & 3) == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
     if (tid < nrow) {
         const int i = i0 + tid, s = i / E, e = i - s * E;
@@ -56,77 +56,74 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router_logits(float *__restr
     }
     __syncthreads();
     // when all outputs of the CTA belong to one row of x, that row is staged once (tile row 0)
-    const bool one_x = nrow > 0 && s_xrow[0] == s_xrow[nrow - 1];
-    const int ntile = (D + ROUTER_TILE - 1) / ROUTER_TILE;
-    auto fetch = [&](int tile) {
+    const bool one_x = s_xrow[0] == s_xrow[nrow - 1];
+    const int ntile = (D + ROUTER_TILE - 1) / ROUTER_TILE, xrows = one_x ? 1 : nrow;
+    auto fetch = [&](int tile) {                        // copy warps only
         if (tile < ntile) {
             const int c0 = tile * ROUTER_TILE, buf = tile % NS;
-            float *wt = rt + (size_t)buf * 2 * 64 * LD, *xt = wt + 64 * LD;
+            float *wt = rt + (size_t)buf * 2 * OUT * LD, *xt = wt + OUT * LD;
             const int width = min(ROUTER_TILE, D - c0);
             if (al16) {
-                // half a warp per row: 16 pieces of 16 bytes
-                const int j = (lane & 15) * 4;
-                for (int r = warp * 2 + (lane >> 4); r < nrow; r += 2 * NW) {
+                for (int i = ctid; i < (nrow + xrows) * 16; i += NC) {         // 16 pieces of 16 bytes per row
+                    const int r = i >> 4, j = (i & 15) * 4;
                     if (j < width) {
-                        const uint32_t dw = (uint32_t)__cvta_generic_to_shared(wt + r * LD + j);
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dw), "l"(s_wrow[r] + c0 + j) : "memory");
-                        if (!one_x || r == 0) {
-                            const uint32_t dx = (uint32_t)__cvta_generic_to_shared(xt + r * LD + j);
-                            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(s_xrow[r] + c0 + j) : "memory");
-                        }
+                        const float *src = (r < nrow ? s_wrow[r] : s_xrow[r - nrow]) + c0 + j;
+                        float *dst = r < nrow ? wt + r * LD + j : xt + (r - nrow) * LD + j;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
                     }
                 }
             } else {
-                for (int r = warp; r < nrow; r += NW)
-                    for (int j = lane; j < width; j += 32) {
-                        const uint32_t dw = (uint32_t)__cvta_generic_to_shared(wt + r * LD + j);
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dw), "l"(s_wrow[r] + c0 + j) : "memory");
-                        if (!one_x || r == 0) {
-                            const uint32_t dx = (uint32_t)__cvta_generic_to_shared(xt + r * LD + j);
-                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dx), "l"(s_xrow[r] + c0 + j) : "memory");
-                        }
+                for (int i = ctid; i < (nrow + xrows) * ROUTER_TILE; i += NC) {
+                    const int r = i / ROUTER_TILE, j = i % ROUTER_TILE;
+                    if (j < width) {
+                        const float *src = (r < nrow ? s_wrow[r] : s_xrow[r - nrow]) + c0 + j;
+                        float *dst = r < nrow ? wt + r * LD + j : xt + (r - nrow) * LD + j;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
                     }
+                }
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");      // one group per tile, also when it is empty
     };
+    const int row = tid & (OUT - 1);                    // (lanes beyond OUT repeat a row)
     float a = 0.f;
-    for (int t = 0; t < NS - 1; t++) fetch(t);
+    float4 p[ROUTER_TILE / 4];                          // products of the tile before
+#pragma unroll
+    for (int q = 0; q < ROUTER_TILE / 4; q++) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&]() {
+#pragma unroll
+        for (int q = 0; q < ROUTER_TILE / 4; q++) {
+            a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
+            a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
+        }
+    };
+    if (ctid >= 0) for (int t = 0; t < NS - 1; t++) fetch(t);
     for (int t = 0; t < ntile; t++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");     // tile t has landed (this thread's copies)
+        if (ctid >= 0) asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");     // tile t has landed (this thread's copies)
         __syncthreads();                // ... and everybody's; the buffer of tile t-1 is no longer read
-        fetch(t + NS - 1);              // into the buffer tile t-1 used
-        const int c0 = t * ROUTER_TILE;
-        const float *wt = rt + (size_t)(t % NS) * 2 * 64 * LD + tid * LD;
-        const float *xt = rt + (size_t)(t % NS) * 2 * 64 * LD + 64 * LD + (one_x ? 0 : tid) * LD;
-        const int width = min(ROUTER_TILE, D - c0);
-        if (tid >= 64) continue;        // copy-only warps
+        if (ctid >= 0) { fetch(t + NS - 1); continue; }            // into the buffer tile t-1 used
+        const float *wt = rt + (size_t)(t % NS) * 2 * OUT * LD + row * LD;
+        const float *xt = rt + (size_t)(t % NS) * 2 * OUT * LD + OUT * LD + (one_x ? 0 : row) * LD;
+        const int width = min(ROUTER_TILE, D - t * ROUTER_TILE);
         if (width == ROUTER_TILE) {
-            // all of the tile's operands first (independent loads, products off the chain), then
-            // the 64 additions back to back
-            float4 wv[ROUTER_TILE / 4], xv[ROUTER_TILE / 4];
+            float4 nx[ROUTER_TILE / 4];
 #pragma unroll
             for (int q = 0; q < ROUTER_TILE / 4; q++) {
-                wv[q] = reinterpret_cast<const float4 *>(wt)[q];
-                xv[q] = reinterpret_cast<const float4 *>(xt)[q];
+                const float4 wv = reinterpret_cast<const float4 *>(wt)[q], xv = reinterpret_cast<const float4 *>(xt)[q];
+                nx[q] = make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w));
             }
+            if (t) add();               // (before the first tile there is nothing to add: a sum of -0 stays -0)
 #pragma unroll
-            for (int q = 0; q < ROUTER_TILE / 4; q++) {
-                wv[q].x = __fmul_rn(xv[q].x, wv[q].x); wv[q].y = __fmul_rn(xv[q].y, wv[q].y);
-                wv[q].z = __fmul_rn(xv[q].z, wv[q].z); wv[q].w = __fmul_rn(xv[q].w, wv[q].w);
-            }
-#pragma unroll
-            for (int q = 0; q < ROUTER_TILE / 4; q++) {
-                a = __fadd_rn(a, wv[q].x);
-                a = __fadd_rn(a, wv[q].y);
-                a = __fadd_rn(a, wv[q].z);
-                a = __fadd_rn(a, wv[q].w);
-            }
-        } else {
+            for (int q = 0; q < ROUTER_TILE / 4; q++) p[q] = nx[q];
+        } else {                        // a ragged last tile
+            if (t) add();
             for (int j = 0; j < width; j++) a = __fadd_rn(a, __fmul_rn(xt[j], wt[j]));
         }
     }
-    if (tid < nrow) logits[i0 + tid] = a;
+    if (tid < nrow) {
+        if (D % ROUTER_TILE == 0) add();
+        logits[i0 + tid] = a;
+    }
 }
 
 #define ROUTE_MAX_E 1024
