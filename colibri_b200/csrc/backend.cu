@@ -206,7 +206,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         }
         *c->status = 0;
         setup_mode<SC_ROW>(); setup_mode<SC_H16>(); setup_mode<SC_F32>(); setup_mode<SC_MX>();
-        set_smem(k_router_logits<16>, router_smem(16)); set_smem(k_router_logits<64>, router_smem(64));
+        set_smem(k_router_logits<16, 256>, router_smem(16, 256)); set_smem(k_router_logits<64, 64>, router_smem(64, 64));
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         setup_decode<SC_ROW>(); setup_decode<SC_H16>(); setup_decode<SC_F32>(); setup_decode<SC_MX>();
         set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
@@ -1408,16 +1408,17 @@ extern "C" int coli_cuda_pipe_copy_async(int device, void *dst, const void *src,
     return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice,
                                    stream ? static_cast<cudaStream_t>(stream) : c->stream), "pipe copy");
 }
+// Both run on the legacy stream, which waits for, and is waited for by, the backend's stream and every other
+// blocking stream of the device. An upload returns when the source has been read, a download when dst is filled.
 extern "C" int coli_cuda_pipe_upload(int device, void *dst, const void *src, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
-    return cuda_ok(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), "pipe upload");
+    return cuda_ok(upload_staged(&c->up, dst, src, bytes, cudaStreamLegacy), "pipe upload");
 }
 extern "C" int coli_cuda_pipe_download(int device, const void *src, void *dst, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
-    if (!cuda_ok(cudaStreamSynchronize(c->stream), "pipe download sync")) return 0;
-    return cuda_ok(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "pipe download");
+    return cuda_ok(download_staged(&c->up, dst, src, bytes, cudaStreamLegacy), "pipe download");
 }
 extern "C" int coli_cuda_pipe_rmsnorm_s(int device, float *y_dev, const float *x_dev, const float *w_dev,
                                         int S, int D, float eps, int xstride, int ystride) {
@@ -1494,12 +1495,16 @@ extern "C" int coli_cuda_pipe_sync(int device) {
     return cuda_ok(cudaDeviceSynchronize(), "pipe sync");
 }
 
-// Few outputs per CTA while that fills no more than two waves of SMs with chains; then 64, which share x and
-// weight tiles better.
 static void launch_router(DeviceCtx *c, float *logits, const float *x, const float *w, int M, int D, int E) {
     const int n = M * E;
-    if (n <= 16 * 4 * c->sms) k_router_logits<16><<<(n + 15) / 16, ROUTER_THREADS, router_smem(16), c->stream>>>(logits, x, w, M, D, E);
-    else k_router_logits<64><<<(n + 63) / 64, ROUTER_THREADS, router_smem(64), c->stream>>>(logits, x, w, M, D, E);
+    const bool aligned = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+    // up to two waves of CTAs: few outputs each, for the shortest chain time; beyond: more chains per SM
+    if (aligned && n <= 16 * 2 * c->sms)
+        k_router_logits<16, 256><<<(n + 15) / 16, 64, router_smem(16, 256), c->stream>>>(logits, x, w, M, D, E, c->status);
+    else if (aligned)
+        k_router_logits<64, 64><<<(n + 63) / 64, 96, router_smem(64, 64), c->stream>>>(logits, x, w, M, D, E, c->status);
+    else
+        k_router_logits_any<<<(n + 63) / 64, 64, 0, c->stream>>>(logits, x, w, M, D, E);
 }
 
 extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void *rw_dev, const void *rb_dev,
@@ -1609,7 +1614,7 @@ extern "C" int coli_cuda_expert_group_dev(ColiCudaTensor *const *gates, ColiCuda
 extern "C" int coli_cuda_pipe_argmax(int device, int *idx_dev, const float *x_dev, int S, int N) {
     DeviceCtx *c = find_ctx(device);
     if (!idx_dev || !x_dev || S < 1 || N < 1 || !select_ctx(c)) return 0;
-    k_argmax_rows<<<S, 1024, 0, c->stream>>>(idx_dev, x_dev, N);
+    k_argmax_rows<<<S * ARGMAX_CLUSTER, 1024, 0, c->stream>>>(idx_dev, x_dev, N);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "argmax launch");
 }

@@ -103,3 +103,34 @@ static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size
     }
     return cudaSuccess;
 }
+
+// src (device) -> dst (any host memory), after all work the stream waits for; done when the call returns. Pieces
+// of 1 MB leave the device while earlier ones are copied out of the pinned buffers (the driver's pageable
+// path moves 4 MB in 244 us, the bus in 84).
+static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    constexpr size_t STEP = 1u << 20;
+    cudaError_t e;
+    size_t out = 0;                             // pieces out: copied to dst
+    const size_t np = (bytes + STEP - 1) / STEP;
+    const int first = r->next;
+    for (size_t in = 0; out < np;) {
+        if (in < np && in - out < UploadRing::N) {
+            const int i = (first + (int)(in % UploadRing::N)) % UploadRing::N;
+            if (!r->buf[i] && ((e = cudaMallocHost(reinterpret_cast<void **>(&r->buf[i]), UploadRing::PIECE)) != cudaSuccess ||
+                               (e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming)) != cudaSuccess)) return e;
+            if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;      // an upload's copy out of it
+            const size_t n = bytes - in * STEP < STEP ? bytes - in * STEP : STEP;
+            if ((e = cudaMemcpyAsync(r->buf[i], static_cast<const char *>(src) + in * STEP, n, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+                (e = cudaEventRecord(r->ev[i], stream)) != cudaSuccess) return e;
+            r->busy[i] = false;
+            in++;
+            continue;
+        }
+        const int i = (first + (int)(out % UploadRing::N)) % UploadRing::N;
+        if ((e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;
+        const size_t n = bytes - out * STEP < STEP ? bytes - out * STEP : STEP;
+        CopyPool::get().copy(static_cast<char *>(dst) + out * STEP, r->buf[i], n);
+        out++;
+    }
+    return cudaSuccess;
+}

@@ -576,37 +576,52 @@ __global__ void k_sum_slots(float *dst, const float *slots, int n, int D) {
 // Row-wise argmax with the engine's scan semantics (c/olmoe.c:966-967, c/colibri.c greedy
 // pick): best = 0, then every i with x[i] > x[best] in ascending order, i.e. the first index
 // of the largest value, NaNs never winning; a NaN in x[0] keeps the answer at 0.
-__global__ void k_argmax_rows(int *__restrict__ out, const float *__restrict__ x, int N) {
-    const float *row = x + (size_t)blockIdx.x * N;
+// A row is shared by a cluster of ARGMAX_CLUSTER CTAs whose answers meet in the first one's shared memory: one CTA
+// per row took 35 us for 8 rows of 129280, waiting for its own loads.
+#define ARGMAX_CLUSTER 8
+__device__ __forceinline__ void argmax_take(float &bv, int &bi, float v, int i) {
+    if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
+}
+__global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k_argmax_rows(int *__restrict__ out, const float *__restrict__ x,
+                                                                                             int N) {
+    const int part = blockIdx.x % ARGMAX_CLUSTER, r = blockIdx.x / ARGMAX_CLUSTER, tid = threadIdx.x;
+    const float *row = x + (size_t)r * N;
     __shared__ float sv[32];
     __shared__ int si[32];
+    __shared__ float cv[ARGMAX_CLUSTER];
+    __shared__ int ci[ARGMAX_CLUSTER];
+    const int per = (N + ARGMAX_CLUSTER - 1) / ARGMAX_CLUSTER, i0 = part * per, i1 = min(N, i0 + per);
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        float v = row[i];
-        if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
-    }
-#pragma unroll
-    for (int off = 16; off; off >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = bv; si[threadIdx.x >> 5] = bi; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        bv = threadIdx.x < nw ? sv[threadIdx.x] : -INFINITY;
-        bi = threadIdx.x < nw ? si[threadIdx.x] : 0x7fffffff;
+#pragma unroll 4
+    for (int i = i0 + tid; i < i1; i += 1024) argmax_take(bv, bi, row[i], i);
+    auto warp_best = [&]() {
 #pragma unroll
         for (int off = 16; off; off >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+            argmax_take(bv, bi, ov, oi);
         }
-        if (threadIdx.x == 0) {
-            const float first = row[0];
-            out[blockIdx.x] = (first != first || bi == 0x7fffffff) ? 0 : bi;
+    };
+    warp_best();
+    if ((tid & 31) == 0) { sv[tid >> 5] = bv; si[tid >> 5] = bi; }
+    __syncthreads();
+    if (tid < 32) {
+        bv = sv[tid]; bi = si[tid];
+        warp_best();
+        if (tid == 0) {
+            uint32_t dv, di;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dv) : "r"((uint32_t)__cvta_generic_to_shared(cv + part)), "r"(0));
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(di) : "r"((uint32_t)__cvta_generic_to_shared(ci + part)), "r"(0));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dv), "f"(bv) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(di), "r"(bi) : "memory");
         }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (part == 0 && tid == 0) {
+        bv = -INFINITY; bi = 0x7fffffff;
+        for (int i = 0; i < ARGMAX_CLUSTER; i++) argmax_take(bv, bi, cv[i], ci[i]);
+        const float first = row[0];
+        out[r] = (first != first || bi == 0x7fffffff) ? 0 : bi;
     }
 }

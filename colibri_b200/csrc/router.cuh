@@ -16,6 +16,7 @@
 //    sum) are formed serially, divisions are IEEE.
 #pragma once
 #include "common.cuh"
+#include "gemv_stream.cuh"
 #include "expf_exact.h"
 
 // 2^(i/32) table in the "bits minus (i<<47)" form the scheme wants; filled at init.
@@ -25,105 +26,109 @@ __device__ __forceinline__ float expf_host_exact(float x) { return coli_expf_exa
 
 // logits[s*E+e] = sum_i x[s,i]*W[e,i], ascending i, multiply and add rounded separately
 // (the engine's order, so the sum is one dependent chain of D additions per output: about
-// 4 cycles each, which is the floor: 13 us at D = 6144). One thread per (s,e), OUT outputs per CTA: few,
+// 4 cycles each, which is the floor: 13 us at D = 6144). One thread per (s,e), 16 outputs per CTA: few,
 // because an SM takes in about 50 B per cycle and 64 weight rows at once were slower than their chains.
-// Per 64-column tile, row r of the tile is the 64 floats of output r's weight row (and of its x row),
-// brought in by the copy warps with asynchronous copies, ROUTER_STAGES - 1 tiles ahead (row stride 68
-// floats: rows start 16-byte aligned and the 128-bit reads of 8 threads walking different rows do not
-// collide). The products of tile t are formed while the additions of tile t-1 run: the loads and
+// A stage of the ring is 256 columns of the CTA's weight rows and of its x row(s) (row stride 260 floats:
+// rows start 16-byte aligned and the 128-bit reads of 8 threads walking different rows do not collide).
+// The products of 64 columns are formed while the additions of the 64 before run: the loads and
 // multiplications fill the chain's gaps. Measured at 256 outputs of 6144 terms: 89 us with 64 outputs
-// per CTA and products before additions.
-// Launch: ROUTER_THREADS threads, router_smem(OUT) bytes of dynamic shared memory.
-#define ROUTER_THREADS 128
-#define ROUTER_TILE 64
-#define ROUTER_LD 68
-#define ROUTER_STAGES 8
-__host__ __device__ constexpr int router_smem(int out) { return ROUTER_STAGES * 2 * out * ROUTER_LD * 4; }
-template <int OUT>
-__global__ void __launch_bounds__(ROUTER_THREADS) k_router_logits(float *__restrict__ logits, const float *__restrict__ x,
-                                                                  const float *__restrict__ W, int M, int D, int E) {
-    extern __shared__ __align__(16) float rt[];         // [stage][w | x][OUT][68]
-    __shared__ const float *s_wrow[OUT], *s_xrow[OUT];
-    constexpr int LD = ROUTER_LD, NS = ROUTER_STAGES, CW = (OUT + 31) / 32, NC = ROUTER_THREADS - CW * 32;
-    const int tid = threadIdx.x, ctid = tid - CW * 32;
-    const int i0 = blockIdx.x * OUT, n = M * E;
-    const int nrow = min(OUT, n - i0);
-    const bool al16 = (D & 3) == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
-    if (tid < nrow) {
-        const int i = i0 + tid, s = i / E, e = i - s * E;
-        s_wrow[tid] = W + (size_t)e * D;
-        s_xrow[tid] = x + (size_t)s * D;
+// per CTA, products before additions and CTA barriers between tiles of 64; 39 us with 16 outputs, the barriers left.
+// Two forms: k_router_logits, one copy warp with bulk copies of 256 columns per row and an mbarrier per stage
+// (rows that start 16-byte aligned), and k_router_logits_any, plain loads, for the rest.
+#define ROUTER_STAGES 6
+__host__ __device__ constexpr int router_smem(int out, int tile) { return ROUTER_STAGES * 2 * out * (tile + 4) * 4; }
+template <int OUT, int TILE>
+__global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(float *__restrict__ logits, const float *__restrict__ x,
+                                                                             const float *__restrict__ W, int M, int D, int E,
+                                                                             int *status) {
+    extern __shared__ __align__(16) float rt[];         // [stage][w | x][OUT][TILE + 4]
+    __shared__ __align__(8) unsigned long long s_full[ROUTER_STAGES], s_empty[ROUTER_STAGES];
+    constexpr int LD = TILE + 4, NS = ROUTER_STAGES, CW = (OUT + 31) / 32;
+    const int tid = threadIdx.x, lane = tid & 31, i0 = blockIdx.x * OUT, nrow = min(OUT, M * E - i0);
+    // when all outputs of the CTA belong to one row of x, that row is staged once (tile row 0)
+    const bool one_x = i0 / E == (i0 + nrow - 1) / E;
+    const int ntile = (D + TILE - 1) / TILE;
+    if (tid == 0) {
+        for (int i = 0; i < NS; i++) { mbar_init(smem_u32(s_full + i), 1); mbar_init(smem_u32(s_empty + i), CW); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // when all outputs of the CTA belong to one row of x, that row is staged once (tile row 0)
-    const bool one_x = s_xrow[0] == s_xrow[nrow - 1];
-    const int ntile = (D + ROUTER_TILE - 1) / ROUTER_TILE, xrows = one_x ? 1 : nrow;
-    auto fetch = [&](int tile) {                        // copy warps only
-        if (tile < ntile) {
-            const int c0 = tile * ROUTER_TILE, buf = tile % NS;
-            float *wt = rt + (size_t)buf * 2 * OUT * LD, *xt = wt + OUT * LD;
-            const int width = min(ROUTER_TILE, D - c0);
-            if (al16) {
-                for (int i = ctid; i < (nrow + xrows) * 16; i += NC) {         // 16 pieces of 16 bytes per row
-                    const int r = i >> 4, j = (i & 15) * 4;
-                    if (j < width) {
-                        const float *src = (r < nrow ? s_wrow[r] : s_xrow[r - nrow]) + c0 + j;
-                        float *dst = r < nrow ? wt + r * LD + j : xt + (r - nrow) * LD + j;
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-                    }
-                }
-            } else {
-                for (int i = ctid; i < (nrow + xrows) * ROUTER_TILE; i += NC) {
-                    const int r = i / ROUTER_TILE, j = i % ROUTER_TILE;
-                    if (j < width) {
-                        const float *src = (r < nrow ? s_wrow[r] : s_xrow[r - nrow]) + c0 + j;
-                        float *dst = r < nrow ? wt + r * LD + j : xt + (r - nrow) * LD + j;
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-                    }
-                }
+    if (tid >= CW * 32) {
+        // copies: row j of the weights, or of x
+        const int rows = nrow + (one_x ? 1 : nrow);
+        for (int t = 0; t < ntile; t++) {
+            const int st = t % NS, width = min(TILE, D - t * TILE);
+            const uint32_t bar = smem_u32(s_full + st);
+            if (t >= NS && !mbar_wait_bounded(smem_u32(s_empty + st), (t / NS + 1) & 1)) break;
+            if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * width * 4);
+            __syncwarp();
+            for (int j = lane; j < rows; j += 32) {
+                const bool is_x = j >= nrow;
+                const int r = is_x ? j - nrow : j, i = i0 + r, s = i / E;
+                const float *src = (is_x ? x + (size_t)s * D : W + (size_t)(i - s * E) * D) + (size_t)t * TILE;
+                bulk_g2s(smem_u32(rt + ((size_t)(st * 2 + is_x) * OUT + r) * LD), src, width * 4, bar);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");      // one group per tile, also when it is empty
-    };
+        return;
+    }
     const int row = tid & (OUT - 1);                    // (lanes beyond OUT repeat a row)
     float a = 0.f;
-    float4 p[ROUTER_TILE / 4];                          // products of the tile before
+    float4 p[16];                                       // products of the 64 columns before
 #pragma unroll
-    for (int q = 0; q < ROUTER_TILE / 4; q++) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto add = [&]() {
-#pragma unroll
-        for (int q = 0; q < ROUTER_TILE / 4; q++) {
-            a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
-            a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
-        }
-    };
-    if (ctid >= 0) for (int t = 0; t < NS - 1; t++) fetch(t);
+    for (int q = 0; q < 16; q++) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool ok = true;
     for (int t = 0; t < ntile; t++) {
-        if (ctid >= 0) asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");     // tile t has landed (this thread's copies)
-        __syncthreads();                // ... and everybody's; the buffer of tile t-1 is no longer read
-        if (ctid >= 0) { fetch(t + NS - 1); continue; }            // into the buffer tile t-1 used
-        const float *wt = rt + (size_t)(t % NS) * 2 * OUT * LD + row * LD;
-        const float *xt = rt + (size_t)(t % NS) * 2 * OUT * LD + OUT * LD + (one_x ? 0 : row) * LD;
-        const int width = min(ROUTER_TILE, D - t * ROUTER_TILE);
-        if (width == ROUTER_TILE) {
-            float4 nx[ROUTER_TILE / 4];
+        const int st = t % NS, width = min(TILE, D - t * TILE);
+        if (!mbar_wait_bounded(smem_u32(s_full + st), (t / NS) & 1)) ok = false;
+        const float4 *wt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2) * OUT + row) * LD);
+        const float4 *xt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2 + 1) * OUT + (one_x ? 0 : row)) * LD);
+        for (int c = 0; c < width; c += 64, wt += 16, xt += 16) {
+            const int n4 = min(16, (width - c) >> 2);
+            // (the first round adds the zeros p starts with: the engine's sum starts from zero too)
+            if (n4 == 16) {
 #pragma unroll
-            for (int q = 0; q < ROUTER_TILE / 4; q++) {
-                const float4 wv = reinterpret_cast<const float4 *>(wt)[q], xv = reinterpret_cast<const float4 *>(xt)[q];
-                nx[q] = make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w));
+                for (int q = 0; q < 16; q++) {
+                    const float4 wv = wt[q], xv = xt[q], old = p[q];
+                    p[q] = make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w));
+                    a = __fadd_rn(a, old.x); a = __fadd_rn(a, old.y);
+                    a = __fadd_rn(a, old.z); a = __fadd_rn(a, old.w);
+                }
+            } else {                                    // the ragged end: nothing stays pending
+#pragma unroll
+                for (int q = 0; q < 16; q++) {
+                    a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
+                    a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
+                    p[q] = make_float4(-0.f, -0.f, -0.f, -0.f);
+                }
+                for (int q = 0; q < n4; q++) {
+                    const float4 wv = wt[q], xv = xt[q];
+                    a = __fadd_rn(a, __fmul_rn(xv.x, wv.x)); a = __fadd_rn(a, __fmul_rn(xv.y, wv.y));
+                    a = __fadd_rn(a, __fmul_rn(xv.z, wv.z)); a = __fadd_rn(a, __fmul_rn(xv.w, wv.w));
+                }
             }
-            if (t) add();               // (before the first tile there is nothing to add: a sum of -0 stays -0)
-#pragma unroll
-            for (int q = 0; q < ROUTER_TILE / 4; q++) p[q] = nx[q];
-        } else {                        // a ragged last tile
-            if (t) add();
-            for (int j = 0; j < width; j++) a = __fadd_rn(a, __fmul_rn(xt[j], wt[j]));
         }
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(s_empty + st)) : "memory");
     }
-    if (tid < nrow) {
-        if (D % ROUTER_TILE == 0) add();
-        logits[i0 + tid] = a;
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+        a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
+        a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
     }
+    if (tid < nrow) logits[i0 + tid] = a;
+    if (!ok && lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
+}
+// One thread per output, operands straight from memory.
+__global__ void k_router_logits_any(float *__restrict__ logits, const float *__restrict__ x, const float *__restrict__ W, int M, int D,
+                                    int E) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M * E) return;
+    const int s = i / E;
+    const float *xr = x + (size_t)s * D, *wr = W + (size_t)(i - s * E) * D;
+    float a = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < D; k++) a = __fadd_rn(a, __fmul_rn(xr[k], wr[k]));
+    logits[i] = a;
 }
 
 #define ROUTE_MAX_E 1024
