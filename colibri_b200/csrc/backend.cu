@@ -156,7 +156,7 @@ static void setup_mode() { setup_one<MODE, 1>(); setup_one<MODE, 2>(); setup_one
 extern "C" void coli_cuda_shutdown(void);
 
 static int decode_smem_bytes(int mode) {
-    return DEC_WARPS * DEC_NST * chunk_bytes_of(mode) + 1024 + (int)((sizeof(DecShared) + 127) & ~127) +
+    return DEC_WARPS * DEC_NST * chunk_bytes_of(mode) + DEC_BAR_BYTES + (int)((sizeof(DecShared) + 127) & ~127) +
            2 * DEC_PART_BYTES + dec_act_bytes(mode);
 }
 

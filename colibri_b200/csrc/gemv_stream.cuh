@@ -62,6 +62,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     }
     return true;
 }
+// 1 in one lane of the (converged) warp: what it guards is issued with uniform operands.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
+}
 // 1-D bulk copy global -> this CTA's shared memory, completion counted in bytes on `bar`.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile(
@@ -90,6 +96,15 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The first MMA of a sum: the zeros are an operand constant, not four registers set for it.
+__device__ __forceinline__ void mma_f16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                              uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
@@ -156,12 +171,6 @@ __device__ __forceinline__ void block_mma(uint32_t st, int lane, int g, LoadB lo
         for (int s = 0; s < NS; s++) sc8[s] = lds64(st + s * HS + 1024 + g * 8);
     }
 #pragma unroll
-    for (int cs = 0; cs < NC; cs++)
-#pragma unroll
-        for (int s = 0; s < NS; s++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) bacc[cs][s][i] = 0.f;
-#pragma unroll
     for (int grp = 0; grp < 4; grp++) {
         uint4 b[NC];
 #pragma unroll
@@ -189,12 +198,15 @@ __device__ __forceinline__ void block_mma(uint32_t st, int lane, int g, LoadB lo
             if (GS) { s0 *= ixg[grp]; s1 *= ixg[grp]; }
 #pragma unroll
             for (int cs = 0; cs < NC; cs++) {
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_f16(c, a_lo[0], a_hi[0], a_lo[1], a_hi[1], b[cs].x, b[cs].y);
+                float c[4];
+                mma_f16_first(c, a_lo[0], a_hi[0], a_lo[1], a_hi[1], b[cs].x, b[cs].y);
                 mma_f16(c, a_lo[2], a_hi[2], a_lo[3], a_hi[3], b[cs].z, b[cs].w);
                 if (MODE == SC_ROW && !GS) {
-                    bacc[cs][s][0] += c[0]; bacc[cs][s][1] += c[1];
-                    bacc[cs][s][2] += c[2]; bacc[cs][s][3] += c[3];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) bacc[cs][s][i] = grp ? bacc[cs][s][i] + c[i] : c[i];
+                } else if (grp == 0) {
+                    bacc[cs][s][0] = c[0] * s0; bacc[cs][s][1] = c[1] * s0;
+                    bacc[cs][s][2] = c[2] * s1; bacc[cs][s][3] = c[3] * s1;
                 } else {
                     bacc[cs][s][0] = fmaf(c[0], s0, bacc[cs][s][0]);
                     bacc[cs][s][1] = fmaf(c[1], s0, bacc[cs][s][1]);

@@ -75,6 +75,7 @@ __host__ __device__ constexpr int dec_act_bytes(int mode) { return mode == SC_F3
 #define DEC_PART_BYTES 16384     // one buffer of per-warp partial sums: 16 warps x 32 lanes x 2 float4
 #define DEC_MAX_I 2048           // two passes x 4 rows x I x 4 bytes must fit the activation region
 #define DEC_SYNC_WORDS 16
+#define DEC_BAR_BYTES 1280       // the warps' ring barriers and one more
 
 struct DecPass {
     int e;            // expert id, or -1 for the shared expert
@@ -345,46 +346,42 @@ struct DecPhase {
     unsigned long long mg_nt;
     int u0, u1, first_u, wl, gidx;
     int local, npass; // local: units are 16-row halves of the output, every group walks passes gidx, gidx + ng, ...
+    int cnt;          // blocks of one tile that are this warp's
 };
 
-// Position of a warp's copy stream inside one phase.
+// Position of a warp's copy stream inside one phase: the next block, and how many of the tile are left
+// after it. Walking on is an addition; the rest happens once per tile.
 struct DecIt {
-    int live, u, kb, mat, p;         // live 0: nothing left; p: pass (local down phase only)
-    const uint8_t *base0, *base1;    // block 0 of the current tile: gate / up, or down / unused
-                                     // (local down phase: the 16-row half / unused)
+    int live, left, u, mat, p;       // live 0: nothing left; p: pass (local down phase only)
+    const uint8_t *ptr;
 };
 
 template <int CH>
 __device__ __forceinline__ void dec_it_unit(DecIt &it, const DecPhase &ph, const DecShared *sh) {
+    it.left = ph.cnt;
     if (ph.local) {
-        const uint8_t *tile0 = sh->pass[it.p].wd + (size_t)(it.u >> 1) * ph.nkb * CH;
-        it.base0 = tile0 + (it.u & 1) * (CH / 2);
+        it.ptr = sh->pass[it.p].wd + ((size_t)(it.u >> 1) * ph.nkb + ph.wl) * CH + (it.u & 1) * (CH / 2);
         return;
     }
     const int pass = dec_div(it.u, ph.mg_nt), tile = it.u - pass * ph.nt;
     const DecPass &ps = sh->pass[pass];
-    const size_t off = (size_t)tile * ph.nkb * CH;
-    if (ph.which == 1) { it.base0 = ps.wg + off; it.base1 = ps.wu + off; }
-    else { it.base0 = ps.wd + off; it.base1 = nullptr; }
+    it.ptr = (ph.which == 1 ? (it.mat ? ps.wu : ps.wg) : ps.wd) + ((size_t)tile * ph.nkb + ph.wl) * CH;
 }
 template <int CH>
 __device__ __forceinline__ void dec_it_start(DecIt &it, const DecPhase &ph, const DecShared *sh) {
-    it.live = ph.first_u < ph.u1 && ph.wl < ph.nkb && (!ph.local || ph.gidx < ph.npass);
-    it.u = ph.first_u; it.kb = ph.wl; it.mat = 0; it.p = ph.gidx;
-    it.base0 = nullptr; it.base1 = nullptr;
+    it.live = ph.first_u < ph.u1 && ph.cnt > 0 && (!ph.local || ph.gidx < ph.npass);
+    it.u = ph.first_u; it.mat = 0; it.p = ph.gidx; it.left = 0; it.ptr = nullptr;
     if (it.live) dec_it_unit<CH>(it, ph, sh);
 }
 template <int CH>
 __device__ __forceinline__ void dec_it_next(DecIt &it, const DecPhase &ph, const DecShared *sh) {
-    it.kb += ph.wpk;
-    if (it.kb < ph.nkb) return;
-    it.kb = ph.wl;
+    it.ptr += ph.wpk * CH;
+    if (--it.left > 0) return;
     if (ph.local) {
         it.p += ph.ng;
         if (it.p >= ph.npass) { it.p = ph.gidx; it.u += 1; }
     } else if (ph.which == 1 && it.mat == 0) {
         it.mat = 1;
-        return;
     } else {
         it.mat = 0;
         it.u += ph.ng;
@@ -392,34 +389,30 @@ __device__ __forceinline__ void dec_it_next(DecIt &it, const DecPhase &ph, const
     if (it.u < ph.u1) dec_it_unit<CH>(it, ph, sh); else it.live = 0;
 }
 
-// Ring state of one warp across the phases of the kernel: `nst` slots of `sb` bytes, one
-// mbarrier per slot (six exist per warp). A barrier's phase parity lives in `parbits`, so the
-// slot geometry can change between the phases (3 whole chunks, or 6 half-chunks for the local
-// down phase) without re-initialising anything, as long as nothing is in flight at the switch.
+// Ring state of one warp: `nst` slots of `sb` bytes with an mbarrier each, walked in turn by the copies (p) and
+// the consumer (c). The two phases of the kernel have rings of different geometry in the same memory and
+// barriers of their own; nothing is in flight at the switch.
 struct WarpRing {
     uint32_t ring, bars;
     int issued, consumed;     // totals (issued - consumed = copies in flight)
     int pi, ci;               // slot the next copy goes to / the next wait looks at
     int nst, sb;
-    uint32_t parbits;
+    uint32_t par;             // parity the consumer waits with, flips when it wraps
     bool ok;                  // false once a wait has expired: later waits are skipped
+    __device__ __forceinline__ void start(uint32_t r, uint32_t b, int n, int bytes) {
+        ring = r; bars = b; nst = n; sb = bytes; issued = consumed = pi = ci = 0; par = 0;
+    }
 };
-#define DEC_BARS_PER_WARP 6
+#define DEC_BARS_PER_WARP (DEC_NST + 2 * DEC_NST)      // gate/up ring, then a down ring of up to twice the slots
 
-template <int CH, int NST>
-__device__ __forceinline__ void dec_issue_one(WarpRing &wr, DecIt &it, const DecPhase &ph, const DecShared *sh,
-                                              int lane) {
+// Requests the stream's next block (the caller has a free slot).
+template <int CH>
+__device__ __forceinline__ void dec_issue_one(WarpRing &wr, DecIt &it, const DecPhase &ph, const DecShared *sh, uint32_t el) {
     if (!it.live) return;
-    if (wr.issued - wr.consumed >= wr.nst) return;
-    if (lane == 0) {
-        const uint32_t bar = wr.bars + wr.pi * 8, dst = wr.ring + wr.pi * wr.sb;
-        if (ph.local) {
-            mbar_expect_tx(bar, CH / 2);        // one 16-row half
-            bulk_g2s(dst, it.base0 + (size_t)it.kb * CH, CH / 2, bar);
-        } else {
-            mbar_expect_tx(bar, CH);
-            bulk_g2s(dst, (it.mat ? it.base1 : it.base0) + (size_t)it.kb * CH, CH, bar);
-        }
+    if (el) {
+        const uint32_t bar = wr.bars + wr.pi * 8, bytes = ph.local ? CH / 2 : CH;       // local: one 16-row half
+        mbar_expect_tx(bar, bytes);
+        bulk_g2s(wr.ring + wr.pi * wr.sb, it.ptr, bytes, bar);
     }
     wr.issued++;
     if (++wr.pi == wr.nst) wr.pi = 0;
@@ -427,17 +420,14 @@ __device__ __forceinline__ void dec_issue_one(WarpRing &wr, DecIt &it, const Dec
 }
 
 // Waits for the oldest outstanding chunk of the ring; returns its shared-memory address.
-template <int CH, int NST>
 __device__ __forceinline__ uint32_t dec_wait_chunk(WarpRing &wr) {
-    const int slot = wr.ci;
-    if (wr.ok && !mbar_wait_bounded(wr.bars + slot * 8, (wr.parbits >> slot) & 1u)) wr.ok = false;
-    return wr.ring + slot * wr.sb;
+    if (wr.ok && !mbar_wait_bounded(wr.bars + wr.ci * 8, wr.par)) wr.ok = false;
+    return wr.ring + wr.ci * wr.sb;
 }
 // after the chunk has been read: its slot is free again
 __device__ __forceinline__ void dec_release_chunk(WarpRing &wr) {
-    wr.parbits ^= 1u << wr.ci;
     wr.consumed++;
-    if (++wr.ci == wr.nst) wr.ci = 0;
+    if (++wr.ci == wr.nst) { wr.ci = 0; wr.par ^= 1; }
 }
 
 // This CTA's contiguous share [t0, t1) of n units: sizes differ by at most one.
@@ -465,9 +455,9 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     constexpr int nst = NST;
     const uint32_t ring_bytes = (uint32_t)DEC_WARPS * nst * CH;
     extern __shared__ __align__(128) uint8_t smem[];
-    // layout: rings | mbarriers (1024 B) | DecShared | partial sums (2 buffers; the routing
+    // layout: rings | mbarriers (DEC_BAR_BYTES) | DecShared | partial sums (2 buffers; the routing
     // scratch and tables live here first) | activation region
-    DecShared *sh = reinterpret_cast<DecShared *>(smem + ring_bytes + 1024);
+    DecShared *sh = reinterpret_cast<DecShared *>(smem + ring_bytes + DEC_BAR_BYTES);
     uint8_t *part = reinterpret_cast<uint8_t *>(sh) + ((sizeof(DecShared) + 127) & ~127);
     uint8_t *act = part + 2 * DEC_PART_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
@@ -476,9 +466,9 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     const int E = r.E, K = r.K, M = a.M, D = r.D, I = r.I;
     const int nkb1 = D / BLOCK_K, nkb2 = I / BLOCK_K, nt1 = I / TILE_ROWS, nt2 = D / TILE_ROWS;
     WarpRing wr;
-    wr.ring = smem_u32(smem) + warp * (nst * CH);
-    wr.bars = smem_u32(smem) + ring_bytes + warp * DEC_BARS_PER_WARP * 8;
-    wr.issued = 0; wr.consumed = 0; wr.pi = 0; wr.ci = 0; wr.nst = nst; wr.sb = CH; wr.parbits = 0; wr.ok = true;
+    wr.ok = true;
+    wr.start(smem_u32(smem) + warp * (nst * CH), smem_u32(smem) + ring_bytes + warp * DEC_BARS_PER_WARP * 8, nst, CH);
+    const uint32_t el = elect_one();
     // routing scratch inside the partial-sum buffers (dead before the first partial sum is written)
     float *score = reinterpret_cast<float *>(part);                     // [M*E]  (<= 8 KB)
     float *choice = reinterpret_cast<float *>(part + 8192);             // [M*E]
@@ -894,10 +884,12 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     dec_cta_range(npass * nt1, a.mg_grid, ph1.u0, ph1.u1);
     ph1.gidx = warp >> ph1.wsh; ph1.wl = warp & (a.wpk1 - 1); ph1.first_u = ph1.u0 + ph1.gidx;
     ph1.local = 0; ph1.npass = npass;
+    ph1.cnt = ph1.wl < nkb1 ? (nkb1 - ph1.wl + ph1.wpk - 1) >> ph1.wsh : 0;
     ph2.which = 2; ph2.nt = nt2; ph2.nkb = nkb2; ph2.wpk = a.wpk2; ph2.wsh = 31 - __clz(a.wpk2);
     ph2.ng = DEC_WARPS >> ph2.wsh; ph2.mg_nt = a.mg_nt2;
     ph2.local = a.local2; ph2.npass = npass;
     ph2.gidx = warp >> ph2.wsh; ph2.wl = warp & (a.wpk2 - 1);
+    ph2.cnt = ph2.wl < nkb2 ? (nkb2 - ph2.wl + ph2.wpk - 1) >> ph2.wsh : 0;
     if (a.local2) { dec_cta_range(2 * nt2, a.mg_grid, ph2.u0, ph2.u1); ph2.first_u = ph2.u0; }
     else { dec_cta_range(npass * nt2, a.mg_grid, ph2.u0, ph2.u1); ph2.first_u = ph2.u0 + ph2.gidx; }
 
@@ -909,7 +901,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     dec_it_start<CH>(it, ph1, sh);
 #pragma unroll 1
     for (int s = 0; s < nst; s++) {
-        dec_issue_one<CH, NST>(wr, it, ph1, sh, lane);
+        dec_issue_one<CH>(wr, it, ph1, sh, el);
         if (s + 1 < nst) __syncthreads();
     }
     DEC_PROBE(a, 2);
@@ -950,7 +942,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                     for (int grp = 0; grp < 4; grp++)
                         bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                    const uint32_t st = dec_wait_chunk<CH, NST>(wr);
+                    const uint32_t st = dec_wait_chunk(wr);
                     float bacc[1][2][4];
                     block_mma<MODE, 1>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc);
 #pragma unroll
@@ -960,7 +952,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
                     dec_release_chunk(wr);
                     __syncwarp();
                     if (tid == 0 && wr.consumed == 1) DEC_PROBE_T(a, 3);      // first block of the stream consumed
-                    dec_issue_one<CH, NST>(wr, it, ph1, sh, lane);
+                    dec_issue_one<CH>(wr, it, ph1, sh, el);
                 }
                 pb[mat] = make_float4((R[0][0] + R[0][1]), (R[0][2] + R[0][3]),
                                       (R[1][0] + R[1][1]), (R[1][2] + R[1][3]));
@@ -1001,11 +993,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     // Every gate/up block of this warp has landed and been read, so nothing is in flight: the
     // down stream starts now, ahead of the barrier (its weights do not depend on the other
     // CTAs). For the local combine the ring becomes six slots of half a chunk.
-    if (a.local2) { wr.nst = min(2 * nst, DEC_BARS_PER_WARP); wr.sb = CH / 2; }
-    wr.pi = 0; wr.ci = 0; wr.issued = 0; wr.consumed = 0;
+    wr.start(wr.ring, wr.bars + nst * 8, a.local2 ? 2 * nst : nst, a.local2 ? CH / 2 : CH);
     dec_it_start<CH>(it, ph2, sh);
 #pragma unroll 1
-    for (int s = 0; s < wr.nst; s++) dec_issue_one<CH, NST>(wr, it, ph2, sh, lane);
+    for (int s = 0; s < wr.nst; s++) dec_issue_one<CH>(wr, it, ph2, sh, el);
     DEC_PROBE(a, 4);   // gate/up consumed (the ring already holds the first down blocks)
     grid_barrier(a.sync, &sh->failed, bar_target);
     DEC_PROBE(a, 5);
@@ -1081,7 +1072,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                     for (int grp = 0; grp < 4; grp++)
                         bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                    const uint32_t st = dec_wait_chunk<CH, NST>(wr);
+                    const uint32_t st = dec_wait_chunk(wr);
                     if (tid == 0 && p == ph2.gidx && kb == ph2.wl) DEC_PROBE_T(a, 11);   // first down block has landed
                     float bacc[1][2][4];
                     block_mma<MODE, 1, true, 1>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc, ixg);
@@ -1089,7 +1080,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
                     for (int i = 0; i < 4; i++) R[i] += bacc[0][0][i];
                     dec_release_chunk(wr);
                     __syncwarp();
-                    dec_issue_one<CH, NST>(wr, it, ph2, sh, lane);
+                    dec_issue_one<CH>(wr, it, ph2, sh, el);
                 }
                 // rows g and g+8 of the 16-row half for token row t
                 if (svalid) {
@@ -1155,7 +1146,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                 for (int grp = 0; grp < 4; grp++)
                     bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                const uint32_t st = dec_wait_chunk<CH, NST>(wr);
+                const uint32_t st = dec_wait_chunk(wr);
                 float bacc[1][2][4];
                 block_mma<MODE, 1, true>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc, ixg);
 #pragma unroll
@@ -1164,7 +1155,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
                     for (int i = 0; i < 4; i++) R[s][i] += bacc[0][s][i];
                 dec_release_chunk(wr);
                 __syncwarp();
-                dec_issue_one<CH, NST>(wr, it, ph2, sh, lane);
+                dec_issue_one<CH>(wr, it, ph2, sh, el);
             }
             float4 *pb = reinterpret_cast<float4 *>(part + (ucount & 1) * DEC_PART_BYTES) + (warp * 32 + lane) * 2;
             pb[0] = make_float4((R[0][0] + R[0][1]), (R[0][2] + R[0][3]),
@@ -1216,9 +1207,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         if (tid == 0) kstat_set(a.status, sh->failed == 2 ? KSTAT_MBAR_TIMEOUT : KSTAT_GRID_TIMEOUT);
         // drain copies still in flight before the shared memory goes away (bounded)
         for (int i = wr.consumed; i < wr.issued; i++) {
-            if (!mbar_wait_bounded(wr.bars + wr.ci * 8, (wr.parbits >> wr.ci) & 1u)) break;
-            wr.parbits ^= 1u << wr.ci;
-            if (++wr.ci == wr.nst) wr.ci = 0;
+            if (!mbar_wait_bounded(wr.bars + wr.ci * 8, wr.par)) break;
+            if (++wr.ci == wr.nst) { wr.ci = 0; wr.par ^= 1; }
         }
     }
 }
