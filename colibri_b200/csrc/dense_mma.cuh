@@ -81,12 +81,12 @@ __device__ __forceinline__ void dense_f8x4(uint32_t q, uint32_t (&v)[2]) {
 __device__ __forceinline__ void dense_i4x8(uint32_t q, uint32_t (&v)[4]) {       // pairs (j, j + 4)
     const __half2 k1032 = __floats2half2_rn(1032.f, 1032.f);
 #pragma unroll
-    for (int j = 0; j < 4; j++) v[j] = h2_as_u32(__hsub2(u32_as_h2(((q >> (4 * j)) & 0x000F000Fu) | 0x64006400u), k1032));
+    for (int j = 0; j < 4; j++) v[j] = h2_as_u32(__hsub2(u32_as_h2(((q >> (4 * j)) & 0x000F000Fu) | c_magic_1024), k1032));
 }
 __device__ __forceinline__ void dense_i2x16(uint32_t q, uint32_t (&v)[8]) {      // pairs (j, j + 8)
     const __half2 k1026 = __floats2half2_rn(1026.f, 1026.f);
 #pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = h2_as_u32(__hsub2(u32_as_h2(((q >> (2 * j)) & 0x00030003u) | 0x64006400u), k1026));
+    for (int j = 0; j < 8; j++) v[j] = h2_as_u32(__hsub2(u32_as_h2(((q >> (2 * j)) & 0x00030003u) | c_magic_1024), k1026));
 }
 
 template <int FMT, int NC, bool AL16>
