@@ -8,6 +8,7 @@
 #include "../../include/coli_cuda_b200.h"
 
 #include <cstdio>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
@@ -50,6 +51,7 @@ struct DeviceCtx {
     float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the other host-buffer calls
     size_t io_x_cap = 0, io_y_cap = 0;
     UploadRing up = {};                       // pinned pieces of large uploads
+    IoPieces io = {};                         // events of the pieces of a call's result
     uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
     uint32_t *check_host = nullptr;
     int group_pending = 0;
@@ -143,7 +145,7 @@ static void set_smem(K kern, int bytes) {
 }
 
 // launch geometry of the streaming GEMV per column-set count
-template <int NC> struct GemvCfg { static constexpr int WARPS = NC <= 2 ? 16 : 8; static constexpr int NST = NC <= 2 ? 4 : 6; };
+template <int NC> struct GemvCfg { static constexpr int WARPS = NC <= 2 ? 16 : 8; static constexpr int NST = NC <= 2 ? 3 : 6; };
 
 template <int MODE, int NC>
 static void setup_one() {
@@ -151,7 +153,7 @@ static void setup_one() {
     set_smem(k_gemv_stream<MODE, NC, W, N>, W * N * (chunk_bytes_of(MODE) + 8));
 }
 template <int MODE>
-static void setup_mode() { setup_one<MODE, 1>(); setup_one<MODE, 2>(); setup_one<MODE, 4>(); setup_one<MODE, 8>(); }
+static void setup_mode() { setup_one<MODE, 2>(); setup_one<MODE, 4>(); setup_one<MODE, 8>(); }
 
 extern "C" void coli_cuda_shutdown(void);
 
@@ -241,6 +243,7 @@ extern "C" void coli_cuda_shutdown(void) {
         if (c->check) cudaFree(c->check);
         if (c->check_host) cudaFreeHost(c->check_host);
         upload_ring_free(&c->up);
+        c->io.free();
         if (c->exp_tab_dev) cudaFree(c->exp_tab_dev);
         if (c->ev0) cudaEventDestroy(c->ev0);
         if (c->ev1) cudaEventDestroy(c->ev1);
@@ -558,7 +561,6 @@ template <int MODE>
 static void launch_mode(DeviceCtx *c, int nc, const GemvSeg *segs, const GemvCtl *ctl,
                         const __half *bq, const float *bs) {
     switch (nc) {
-    case 1: launch_one<MODE, 1>(c, segs, ctl, bq, bs); break;
     case 2: launch_one<MODE, 2>(c, segs, ctl, bq, bs); break;
     case 4: launch_one<MODE, 4>(c, segs, ctl, bq, bs); break;
     default: launch_one<MODE, 8>(c, segs, ctl, bq, bs); break;
@@ -612,21 +614,22 @@ extern "C" int coli_cuda_kernel_events(int device, float *total_ms, int *launche
     return 1;
 }
 
-// column sets (4 rows each) per pass for a given largest row count
-static int pick_nc(int max_rows) { return max_rows <= 4 ? 1 : max_rows <= 8 ? 2 : max_rows <= 16 ? 4 : 8; }
+// column sets (4 rows each) per pass at most, for a given largest row count
+static int pick_nc(int max_rows) { return max_rows <= 8 ? 2 : max_rows <= 16 ? 4 : 8; }
 
-// Split of the contraction: enough tasks that every SM gets a few dozen, at
-// least two blocks per task so that the copy pipeline stays primed, and a
-// divisor of the block count.
+// Split of the contraction into k slices, a divisor of the block count: every warp of the grid works through
+// its share of the tasks, so the time goes with the rounds that takes times a task's blocks, plus about two
+// blocks' worth per task for starting it and storing its sums. At least two blocks per task.
 static int pick_nkpart(int nkb, long base_tasks, int sms) {
-    long want = ((long)sms * 13 + base_tasks - 1) / (base_tasks > 0 ? base_tasks : 1);
-    int cap = nkb >= 2 ? nkb / 2 : 1;
-    if (want > cap) want = cap;
-    if (want < 1) want = 1;
-    int k = (int)want;
-    while (k < nkb && nkb % k) k++;
-    if (k > cap) { k = cap; while (k > 1 && nkb % k) k--; }
-    return k;
+    const long warps = (long)sms * 16;      // (8 with more than 8 rows a pass: the rounds only double)
+    int best = 1;
+    long best_cost = LONG_MAX;
+    for (int k = 1; k == 1 || k <= nkb / 2; k++) {
+        if (nkb % k) continue;
+        const long cost = (base_tasks * k + warps - 1) / warps * (nkb / k + 2);
+        if (cost < best_cost) { best_cost = cost; best = k; }
+    }
+    return best;
 }
 
 static void timing_begin(DeviceCtx *c) {
@@ -802,8 +805,8 @@ static int linear_any(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const
     return t->packed ? linear_packed(c, t, y_dev, x_dev, S) : linear_raw(c, t, y_dev, x_dev, S);
 }
 
-static int check_status(DeviceCtx *c) {
-    if (!cuda_ok(cudaStreamSynchronize(c->stream), "synchronize")) return 0;
+// after the call's kernels are done
+static int kernels_ok(DeviceCtx *c) {
     const int v = *reinterpret_cast<volatile int *>(c->status);
     if (v) {
         std::fprintf(stderr, "[CUDA] kernel wait guard expired (status %d)\n", v);
@@ -815,17 +818,34 @@ static int check_status(DeviceCtx *c) {
     }
     return 1;
 }
+static int check_status(DeviceCtx *c) {
+    return cuda_ok(cudaStreamSynchronize(c->stream), "synchronize") && kernels_ok(c);
+}
 
 // Host rows of a blocking call. Everything passes through pinned memory (a copy out of the cache and a DMA
 // are faster than the driver's pageable path, 21 us against 27 at 300 KB), and small rows are not copied to the
 // device at all: the kernel that reads them once, or stores the result, addresses the pinned buffer.
 #define IO_DIRECT_BYTES (64u << 10)
+// A few rows out of pinned memory into device memory by a kernel: the kernel behind it starts 5 us earlier than
+// behind a copy command, whose completion the stream has to be told by another engine. n4: float4s.
+static int pull_rows(DeviceCtx *c, void *dst, const void *pinned, size_t bytes) {
+    const int n4 = (int)(bytes / 16);
+    k_pull<<<(n4 + 255) / 256, 256, 0, c->stream>>>(static_cast<float4 *>(dst), static_cast<const float4 *>(pinned), n4);
+    return cuda_ok(cudaGetLastError(), "input upload");
+}
 // -> where the kernels find x, or NULL. read_once: the first kernel reads every element once (not every CTA all of them).
 static const float *io_in(DeviceCtx *c, const float *x, size_t bytes, bool read_once) {
     if (!reserve_pinned(&c->io_x, &c->io_x_cap, bytes)) return nullptr;
-    CopyPool::get().copy(c->io_x, x, bytes);
-    if (read_once && bytes <= IO_DIRECT_BYTES) return c->io_x;
-    if (!reserve(c, &c->x, bytes) || !cuda_ok(cudaMemcpyAsync(c->x.p, c->io_x, bytes, cudaMemcpyHostToDevice, c->stream), "input upload")) return nullptr;
+    if (read_once && bytes <= IO_DIRECT_BYTES) {
+        std::memcpy(c->io_x, x, bytes);
+        return c->io_x;
+    }
+    if (!reserve(c, &c->x, bytes)) return nullptr;
+    if (bytes <= IO_DIRECT_BYTES && bytes % 16 == 0) {
+        std::memcpy(c->io_x, x, bytes);
+        return pull_rows(c, c->x.p, c->io_x, bytes) ? (const float *)c->x.p : nullptr;
+    }
+    if (!cuda_ok(IoPieces::in(c->x.p, c->io_x, x, bytes, c->stream), "input upload")) return nullptr;
     return (const float *)c->x.p;
 }
 static float *io_out(DeviceCtx *c, size_t bytes) {
@@ -834,10 +854,13 @@ static float *io_out(DeviceCtx *c, size_t bytes) {
     return reserve(c, &c->y, bytes) ? (float *)c->y.p : nullptr;
 }
 static int io_finish(DeviceCtx *c, float *y, const float *y_dev, size_t bytes) {
-    if (y_dev != c->io_y && !cuda_ok(cudaMemcpyAsync(c->io_y, y_dev, bytes, cudaMemcpyDeviceToHost, c->stream), "output download")) return 0;
-    if (!check_status(c)) return 0;
-    CopyPool::get().copy(y, c->io_y, bytes);
-    return 1;
+    if (y_dev == c->io_y) {
+        if (!check_status(c)) return 0;
+        std::memcpy(y, c->io_y, bytes);
+        return 1;
+    }
+    return cuda_ok(c->io.out_start(c->io_y, y_dev, bytes, c->stream), "output download") &&
+           c->io.out_finish(y, c->io_y, bytes, [c] { return kernels_ok(c) != 0; });
 }
 
 extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *x, const void *weights,
@@ -914,15 +937,12 @@ static int group_shape_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
 // 0: never; 1: when it pays (tc_pays); 2: whenever the tensors and shapes allow it (tests).
 static int g_tc_enabled = 1;
 extern "C" void coli_cuda_set_tensor_core(int enabled) { g_tc_enabled = enabled < 0 ? 0 : enabled > 2 ? 2 : enabled; }
-// The streaming kernel's cost grows with the rows (instruction issue: one set of MMAs per 4 rows and
-// block of weights), the tensor-core path's hardly does up to 30 rows per expert, but it has three launches
-// more. Measured: OLMoE shape (226 MB a layer), streaming / tensor cores: 2 rows per expert 106 / 156 us, 4 rows
-// 141 / 160, 8 rows 199 / 166, 31 rows 512 / 196; DeepSeek-V3 shape (6 GB): half a row 651 / 630, 2 rows
-// 1420 / 1255, 16 rows 9049 / 1848. So: from a mean of 6 rows per expert, or from half a GB of weights.
-static bool tc_pays(long rows, long experts, long D, long I) {
-    const double touched = (double)(rows < experts ? rows : experts) * 1.6 * (double)D * (double)I;
-    return rows >= 6 * experts || touched > 512e6;
-}
+// The streaming kernel's cost grows with the rows (one set of MMAs per 4 rows and block of weights), the tensor-core
+// path's hardly does up to 30 rows per expert, but it starts higher, most of all where a weight takes two fp16
+// terms. Measured, streaming / tensor cores, at a mean of R rows per expert: per-row int4, OLMoE shape R = 2: 101 /
+// 105 us, 4: 129 / 109; MXFP4, DeepSeek-V3 shape R = 1: 841 / 940, 2: 1297 / 1200; grouped int4, OLMoE shape
+// R = 6: 154 / 160, 8: 167 / 161, 12: 255 / 166, DeepSeek-V3 shape R = 2: 1407 / 2390, 4: 2160 / 2797.
+static bool tc_pays(long rows, long experts, int mode) { return rows >= (mode == SC_H16 ? 7 : 2) * experts; }
 
 template <int MODE, int PHASE>
 static void launch_tc_one(DeviceCtx *c, const TcArgs &a) {
@@ -986,7 +1006,7 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
 static int group_tc_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                        ColiCudaTensor *const *downs, int count, int max_rows, int total) {
     if (!g_tc_enabled || max_rows < 2) return 0;
-    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->I, gates[0]->O)) return 0;
+    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode)) return 0;
     for (int e = 0; e < count; e++)
         if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok || gates[e]->mode != gates[0]->mode ||
             ups[e]->mode != gates[0]->mode || downs[e]->mode != downs[0]->mode) return 0;
@@ -1170,9 +1190,12 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
             const int r = group_decode(c, gates, ups, downs, rows, nullptr, count, D, I, total, y_dev, x_dev);
             if (r >= 0) return r;
         }
-        const int nc = pick_nc(max_rows), rpp = 4 * nc;
-        long npass = 0;
-        for (int e = 0; e < count; e++) npass += ((rows ? rows[e] : 1) + rpp - 1) / rpp;
+        int nc = pick_nc(max_rows);
+        auto passes = [&](int per) { long n = 0; for (int e = 0; e < count; e++) n += ((rows ? rows[e] : 1) + per - 1) / per; return n; };
+        // a few experts above 8 rows: two passes for these cost less than the slower code for 16 rows costs all of them
+        while (nc > 2 && 4 * passes(2 * nc) <= 5 * (long)count) nc >>= 1;
+        const int rpp = 4 * nc;
+        const long npass = passes(rpp);
         const int nkb1 = D / BLOCK_K, nkb2 = I / BLOCK_K;
         const int nkp1 = pick_nkpart(nkb1, 2 * npass * (I / TILE_ROWS), c->sms);
         const int nkp2 = pick_nkpart(nkb2, npass * (D / TILE_ROWS), c->sms);
@@ -1259,15 +1282,14 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         profile = 0; break;
     }
     if (profile) cudaEventRecord(ev[0], c->stream);
-    CopyPool::get().copy(c->host_x, x, xb);
-    if (!cuda_ok(cudaMemcpyAsync(c->x.p, c->host_x, xb, cudaMemcpyHostToDevice, c->stream), "expert group input upload")) return 0;
+    if (!cuda_ok(IoPieces::in(c->x.p, c->host_x, x, xb, c->stream), "expert group input upload")) return 0;
     if (profile) cudaEventRecord(ev[1], c->stream);
     timing_begin(c);
     if (!group_device(c, gates, ups, downs, rows, count, D, I, total, max_rows, all_packed,
                       (float *)c->y.p, (const float *)c->x.p, nullptr)) return 0;
     timing_end(c);
     if (profile) cudaEventRecord(ev[2], c->stream);
-    if (!cuda_ok(cudaMemcpyAsync(c->host_y, c->y.p, xb, cudaMemcpyDeviceToHost, c->stream), "expert group output download")) return 0;
+    if (!cuda_ok(c->io.out_start(c->host_y, c->y.p, xb, c->stream), "expert group output download")) return 0;
     if (profile) cudaEventRecord(ev[3], c->stream);
     if (async_issue) {
         c->group_pending = 1;
@@ -1275,9 +1297,9 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         if (profile) for (int i = 0; i < 4; i++) cudaEventDestroy(ev[i]);
         return 1;
     }
-    if (!check_status(c)) return 0;
+    if (!c->io.out_finish(y, c->host_y, xb, [c] { return kernels_ok(c) != 0; })) return 0;
+    if (profile && !cuda_ok(cudaStreamSynchronize(c->stream), "synchronize")) return 0;
     timing_collect(c);
-    CopyPool::get().copy(y, c->host_y, xb);
     if (profile) {
         float a = 0, b = 0, d = 0;
         cudaEventElapsedTime(&a, ev[0], ev[1]); cudaEventElapsedTime(&b, ev[1], ev[2]); cudaEventElapsedTime(&d, ev[2], ev[3]);
@@ -1796,11 +1818,12 @@ extern "C" int coli_cuda_pipe_gemm_noalloc(ColiCudaTensor *t, float *y_dev, cons
     }
     const int nkb = t->I / BLOCK_K;
     const int nc = pick_nc(S);
-    const int nkpart = pick_nkpart(nkb, (long)(t->O / TILE_ROWS), c->sms);
     const size_t bs_bytes = (size_t)S * nkb * sizeof(float);
     const size_t bq_bytes = (size_t)S * t->I * 2 * sizeof(__half);
-    const size_t pd_bytes = (size_t)nkpart * S * t->O * sizeof(float);
-    const size_t need = NOALLOC_HEADER_BYTES + NOALLOC_SCALE_BYTES + bq_bytes + pd_bytes;
+    auto scratch = [&](int k) { return NOALLOC_HEADER_BYTES + NOALLOC_SCALE_BYTES + bq_bytes + (size_t)k * S * t->O * sizeof(float); };
+    int nkpart = pick_nkpart(nkb, (long)(t->O / TILE_ROWS), c->sms);
+    while (nkpart > 1 && (nkb % nkpart || scratch(nkpart) > NOALLOC_SCRATCH_BYTES)) nkpart--;     // the partial sums have to fit
+    const size_t need = scratch(nkpart);
     if (bs_bytes > NOALLOC_SCALE_BYTES || need > NOALLOC_SCRATCH_BYTES) {
         std::fprintf(stderr, "[CUDA] pipe_gemm_noalloc: S=%d I=%d O=%d needs %zu bytes of scratch, the fixed "
                              "array holds %u\n", S, t->I, t->O, need, NOALLOC_SCRATCH_BYTES);

@@ -10,8 +10,8 @@
 //    stages; lane 0 keeps NST bulk async copies (cp.async.bulk, completion on
 //    an mbarrier) in flight, so each SM has WARPS*NST chunks outstanding
 //    without holding registers for them;
-//  * tasks = (segment, 32-row tile, slice of the contraction); task t goes to
-//    CTA t % grid, so every SM gets the same number of tasks (+-1);
+//  * tasks = (segment, 32-row tile, slice of the contraction), dealt out to the
+//    CTAs in groups of four neighbours, which read the same activations;
 //  * a chunk is consumed with four 128-bit shared loads per lane that are
 //    already tensor-core A fragments after a mask/sub (int4) or conversion
 //    (MXFP4) decode to exact fp16 integers; activations arrive as an fp16
@@ -251,16 +251,99 @@ __device__ __forceinline__ void task_setup(TaskPos &p, const GemvSeg *segs, int 
     p.ptr = s.w + ((size_t)tile * s.nkb + p.kb) * CH;
 }
 
+// Column sets of a pass: the smallest of 1, 2, 4, 8 that holds its rows. A launch is compiled for the largest
+// that its passes need and branches per task: decoding a block costs about 200 instructions whatever the
+// rows, every column set 45 to 60 more, so a pass of three rows beside one of eight runs as what it is.
+template <int MODE, int NC, class Issue>
+__device__ __forceinline__ bool gemv_task(const GemvSeg &sg, int kb0, int kb1, int tile, int kpart, int npos, const __half *__restrict__ bq,
+                                          const float *__restrict__ bscale, int lane, uint32_t ring, uint32_t bars, int nst, int &ci,
+                                          uint32_t &par, int &consumed, Issue issue_one) {
+    constexpr int HS = half_bytes_of(MODE), CH = 2 * HS;
+    // more than 16 rows: the two 16-row halves of a block in turn, for the registers that their sums take
+    constexpr int NS = NC >= 8 ? 1 : 2;
+    const int g = lane >> 2, t = lane & 3;
+    const int nrows = sg.nrows, nkb = sg.nkb;
+    // B operand: lane (g,t) supplies column g of each 8-column set: row
+    // cs*4 + g/2, half (hi/lo) g&1, its 8 k values 8t..8t+7 of every group. Columns without a row repeat the
+    // pass's first row; what they sum up is not stored.
+    const __half *bptr[NC];
+    const float *sptr[NC];   // block scale of the row whose results this lane holds (row cs*4+t)
+#pragma unroll
+    for (int cs = 0; cs < NC; cs++) {
+        const int r = cs * 4 + (g >> 1), rt = cs * 4 + t;
+        bptr[cs] = bq + (size_t)sg.rowid[r < nrows ? r : 0] * nkb * 256 + (g & 1) * 32 + t * 8;
+        sptr[cs] = bscale + (size_t)sg.rowid[rt < nrows ? rt : 0] * nkb;
+    }
+    float R[NC][2][4];
+#pragma unroll
+    for (int cs = 0; cs < NC; cs++)
+#pragma unroll
+        for (int s = 0; s < 2; s++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) R[cs][s][i] = 0.f;
+#pragma unroll 1
+    for (int kb = kb0; kb < kb1; kb++) {
+        const uint32_t st = ring + ci * CH;
+        float ixs[NC];
+#pragma unroll
+        for (int cs = 0; cs < NC; cs++) ixs[cs] = __ldg(sptr[cs] + kb);
+        uint4 bpre[4];       // one column set: its fragments do not depend on the chunk, so they are fetched before waiting for it
+        if (NC == 1) {
+#pragma unroll
+            for (int grp = 0; grp < 4; grp++) bpre[grp] = ldg_nc128(bptr[0] + (size_t)kb * 256 + grp * 64);
+        }
+        if (!mbar_wait_bounded(bars + ci * 8, par)) return false;
+#pragma unroll
+        for (int h = 0; h < 2; h += NS) {
+            float bacc[NC][2][4];
+            block_mma<MODE, NC, false, NS>(st + h * HS, lane, g,
+                                           [&](int grp, int cs) { return NC == 1 ? bpre[grp] : ldg_nc128(bptr[cs] + (size_t)kb * 256 + grp * 64); },
+                                           bacc);
+#pragma unroll
+            for (int cs = 0; cs < NC; cs++)
+#pragma unroll
+                for (int s = 0; s < NS; s++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) R[cs][h + s][i] = fmaf(bacc[cs][s][i], ixs[cs], R[cs][h + s][i]);
+        }
+        consumed++;
+        if (++ci == nst) { ci = 0; par ^= 1; }
+        __syncwarp();
+        issue_one();   // refill the stage just drained
+    }
+    // ---- write this task's partial sums --------------------------------
+#pragma unroll
+    for (int cs = 0; cs < NC; cs++) {
+        const int r = cs * 4 + t;
+        if (r < nrows) {
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+                const int o = tile * TILE_ROWS + s * 16 + g;
+                float v0 = R[cs][s][0] + R[cs][s][1];
+                float v1 = R[cs][s][2] + R[cs][s][3];
+                if (MODE == SC_ROW) { v0 *= sg.rowscale[o]; v1 *= sg.rowscale[o + 8]; }
+                float *dst = sg.out + ((size_t)kpart * npos + sg.pos0 + r) * sg.O + o;
+                dst[0] = v0;
+                dst[8] = v1;
+            }
+        }
+    }
+    return true;
+}
+
+// Neighbouring tasks (tiles of one pass and slice, which read the same activations) of a CTA.
+#define GEMV_TASK_GROUP 4
+
 template <int MODE, int NC, int WARPS, int NST>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
               const __half *__restrict__ bq, const float *__restrict__ bscale, int *status) {
-    constexpr int CH = CODE_BYTES + (MODE == SC_H16 ? 256 : MODE == SC_F32 ? 512 : MODE == SC_MX ? 128 : 0);
+    constexpr int CH = 2 * half_bytes_of(MODE);
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, t = lane & 3;
     const uint32_t ring = smem_u32(smem) + warp * (NST * CH);
     const uint32_t bars = smem_u32(smem) + WARPS * NST * CH + warp * NST * 8;
+    const uint32_t el = elect_one();
 
     if (lane == 0) {
         for (int s = 0; s < NST; s++) mbar_init(bars + s * 8, 1);
@@ -270,22 +353,24 @@ k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
 
     const int nseg = ctl->nseg, ntask = ctl->ntask, npos = ctl->npos, tps = ctl->tasks_per_seg;
     const int P = gridDim.x * WARPS;
-    const int p0 = warp * gridDim.x + blockIdx.x;   // task t -> CTA t % grid: equal task counts per SM
+    // groups of tasks go to the CTAs in turn, so every SM gets the same number of tasks (+- a group)
+    const int p0 = ((warp / GEMV_TASK_GROUP) * gridDim.x + blockIdx.x) * GEMV_TASK_GROUP + warp % GEMV_TASK_GROUP;
 
     // ---- producer side: keep NST chunks in flight --------------------------
     TaskPos prod;
     prod.task = p0;
     int dummy_a, dummy_b, dummy_c;
     if (prod.task < ntask) task_setup<CH>(prod, segs, nseg, tps, dummy_a, dummy_b, dummy_c);
-    int issued = 0;
+    int issued = 0, pi = 0;
     auto issue_one = [&]() {
         if (prod.task >= ntask) return;
-        if (lane == 0) {
-            uint32_t bar = bars + (issued % NST) * 8;
+        if (el) {
+            const uint32_t bar = bars + pi * 8;
             mbar_expect_tx(bar, CH);
-            bulk_g2s(ring + (issued % NST) * CH, prod.ptr, CH, bar);
+            bulk_g2s(ring + pi * CH, prod.ptr, CH, bar);
         }
         issued++;
+        if (++pi == NST) pi = 0;
         prod.kb++;
         prod.ptr += CH;
         if (prod.kb == prod.kb_end) {
@@ -298,96 +383,28 @@ k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
     // ---- consumer side ------------------------------------------------------
     TaskPos cons;
     cons.task = p0;
-    int consumed = 0;
-    bool failed = false;
-    while (cons.task < ntask) {
+    int consumed = 0, ci = 0;
+    uint32_t par = 0;
+    bool ok = true;
+    while (ok && cons.task < ntask) {
         int seg_i, tile, kpart;
         task_setup<CH>(cons, segs, nseg, tps, seg_i, tile, kpart);
         const GemvSeg &sg = segs[seg_i];
-        const int nrows = sg.nrows, nkb = sg.nkb;
-        // B operand: lane (g,t) supplies column g of each 8-column set: row
-        // cs*4 + g/2, half (hi/lo) g&1, its 8 k values 8t..8t+7 of every group.
-        const __half *bptr[NC];
-        bool bvalid[NC];
-        const float *sptr[NC];   // block scale of the row whose results this lane holds (row cs*4+t)
-        bool svalid[NC];
-#pragma unroll
-        for (int cs = 0; cs < NC; cs++) {
-            int r = cs * 4 + (g >> 1);
-            bvalid[cs] = r < nrows;
-            int rid = bvalid[cs] ? sg.rowid[r] : 0;
-            bptr[cs] = bq + (size_t)rid * nkb * 256 + (g & 1) * 32 + t * 8;
-            int rt = cs * 4 + t;
-            svalid[cs] = rt < nrows;
-            int rids = svalid[cs] ? sg.rowid[rt] : 0;
-            sptr[cs] = bscale + (size_t)rids * nkb;
-        }
-        float R[NC][2][4];
-#pragma unroll
-        for (int cs = 0; cs < NC; cs++)
-#pragma unroll
-            for (int s = 0; s < 2; s++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) R[cs][s][i] = 0.f;
-
-        for (int kb = cons.kb; kb < cons.kb_end; kb++) {
-            const int stage = consumed % NST;
-            const uint32_t st = ring + stage * CH;
-            float ixs[NC];
-#pragma unroll
-            for (int cs = 0; cs < NC; cs++) ixs[cs] = svalid[cs] ? __ldg(sptr[cs] + kb) : 0.f;
-            float bacc[NC][2][4];
-            if (NC == 1) {
-                // the B fragments do not depend on the chunk: fetch them before waiting for it
-                uint4 bpre[4];
-#pragma unroll
-                for (int grp = 0; grp < 4; grp++)
-                    bpre[grp] = bvalid[0] ? ldg_nc128(bptr[0] + (size_t)kb * 256 + grp * 64) : make_uint4(0, 0, 0, 0);
-                if (!mbar_wait_bounded(bars + stage * 8, (consumed / NST) & 1)) { failed = true; break; }
-                block_mma<MODE, NC>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc);
-            } else {
-                if (!mbar_wait_bounded(bars + stage * 8, (consumed / NST) & 1)) { failed = true; break; }
-                block_mma<MODE, NC>(st, lane, g,
-                                    [&](int grp, int cs) {
-                                        return bvalid[cs] ? ldg_nc128(bptr[cs] + (size_t)kb * 256 + grp * 64)
-                                                          : make_uint4(0, 0, 0, 0);
-                                    },
-                                    bacc);
-            }
-#pragma unroll
-            for (int cs = 0; cs < NC; cs++)
-#pragma unroll
-                for (int s = 0; s < 2; s++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) R[cs][s][i] = fmaf(bacc[cs][s][i], ixs[cs], R[cs][s][i]);
-            consumed++;
-            __syncwarp();
-            issue_one();   // refill the stage just drained
-        }
-        if (failed) break;
-        // ---- write this task's partial sums --------------------------------
-#pragma unroll
-        for (int cs = 0; cs < NC; cs++) {
-            int r = cs * 4 + t;
-            if (r < nrows) {
-#pragma unroll
-                for (int s = 0; s < 2; s++) {
-                    int o = tile * TILE_ROWS + s * 16 + g;
-                    float v0 = R[cs][s][0] + R[cs][s][1];
-                    float v1 = R[cs][s][2] + R[cs][s][3];
-                    if (MODE == SC_ROW) { v0 *= sg.rowscale[o]; v1 *= sg.rowscale[o + 8]; }
-                    float *dst = sg.out + ((size_t)kpart * npos + sg.pos0 + r) * sg.O + o;
-                    dst[0] = v0;
-                    dst[8] = v1;
-                }
-            }
-        }
+        const int nrows = sg.nrows;
+#define GEMV_TASK(N) ok = gemv_task<MODE, N>(sg, cons.kb, cons.kb_end, tile, kpart, npos, bq, bscale, lane, ring, bars, NST, ci, par, consumed, issue_one)
+        if (nrows <= 4) GEMV_TASK(1);
+        else if (NC == 2 || nrows <= 8) GEMV_TASK(2);
+        else if (NC == 4 || nrows <= 16) GEMV_TASK(NC < 4 ? 2 : 4);
+        else GEMV_TASK(NC);
+#undef GEMV_TASK
         cons.task += P;
     }
-    if (failed) {
+    if (!ok) {
         if (lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
         // drain whatever is still in flight before leaving (bounded)
-        for (int i = consumed; i < issued; i++)
-            if (!mbar_wait_bounded(bars + (i % NST) * 8, (i / NST) & 1)) break;
+        for (int i = consumed; i < issued; i++) {
+            if (!mbar_wait_bounded(bars + ci * 8, par)) break;
+            if (++ci == NST) { ci = 0; par ^= 1; }
+        }
     }
 }

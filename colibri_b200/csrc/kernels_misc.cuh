@@ -495,6 +495,13 @@ __global__ void k_rope_rows(float *v, const int *pos, int pos_base, int stride, 
 // ---------------------------------------------------------------------------
 // Elementwise / row primitives of the resident pipeline.
 // ---------------------------------------------------------------------------
+// Rows from pinned host memory to device memory.
+__global__ void k_pull(float4 *__restrict__ dst, const float4 *__restrict__ src, int n4) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n4) dst[i] = src[i];
+}
+
 __global__ void k_silu_mul(float *g, const float *u, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { float v = g[i]; g[i] = (v / (1.0f + expf(-v))) * u[i]; }

@@ -175,7 +175,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     const LayerPlan p = layer_plan(L, c, M);
     const int nkb1 = r.D / BLOCK_K, nkb2 = r.I / BLOCK_K;
     bool use_tc = !route_only && !uniq_dev && L->tc_ok && M >= TC_LAYER_MIN_ROWS &&
-                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, r.D, r.I)));
+                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, L->mode_gu)));
     if (use_tc) {
         // coli_cuda_tensor_update may have refreshed a tensor with scales the tensor-core
         // path cannot carry exactly since the layer was created: look again (E flags)
@@ -299,9 +299,17 @@ extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float 
         L->host_io_cap = need;
     }
     uint8_t *hp = reinterpret_cast<uint8_t *>(L->host_io);
-    std::memcpy(hp, x, xb);
-    if (lb) std::memcpy(hp + xb, logits, lb);
-    if (!cuda_ok(cudaMemcpyAsync(L->x.p, hp, xb + lb, cudaMemcpyHostToDevice, c->stream), "layer input upload")) return 0;
+    if (xb + lb <= IO_DIRECT_BYTES && (xb + lb) % 16 == 0) {
+        std::memcpy(hp, x, xb);
+        if (lb) std::memcpy(hp + xb, logits, lb);
+        if (!pull_rows(c, L->x.p, hp, xb + lb)) return 0;
+    } else {
+        if (lb) {
+            std::memcpy(hp + xb, logits, lb);
+            if (!cuda_ok(cudaMemcpyAsync(static_cast<uint8_t *>(L->x.p) + xb, hp + xb, lb, cudaMemcpyHostToDevice, c->stream), "layer input upload")) return 0;
+        }
+        if (!cuda_ok(IoPieces::in(L->x.p, hp, x, xb, c->stream), "layer input upload")) return 0;
+    }
     const float *x_dev = (const float *)L->x.p;
     const float *lg_dev = lb ? reinterpret_cast<const float *>(static_cast<uint8_t *>(L->x.p) + xb) : nullptr;
     uint8_t *ho = hp + xb + lb;
@@ -322,16 +330,20 @@ extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float 
         if (!layer_run(L, c, (float *)L->out.p, x_dev, lg_dev, M, (int *)L->idx.p, (float *)L->w.p, (int *)L->keff.p,
                        0, nullptr, nullptr)) return 0;
         timing_end(c);
-        if (!cuda_ok(cudaMemcpyAsync(ho, L->out.p, xb, cudaMemcpyDeviceToHost, c->stream), "layer output download")) return 0;
         if (want_route) {
             cudaMemcpyAsync(ho + xb, L->idx.p, kb, cudaMemcpyDeviceToHost, c->stream);
             cudaMemcpyAsync(ho + xb + kb, L->w.p, kb, cudaMemcpyDeviceToHost, c->stream);
             cudaMemcpyAsync(ho + xb + 2 * kb, L->keff.p, (size_t)M * 4, cudaMemcpyDeviceToHost, c->stream);
         }
+        if (!cuda_ok(c->io.out_start(ho, L->out.p, xb, c->stream), "layer output download")) return 0;
     }
-    if (!check_status(c)) return 0;
+    if (direct) {
+        if (!check_status(c)) return 0;
+        std::memcpy(out, ho, xb);
+    } else if (!c->io.out_finish(out, ho, xb, [c] { return kernels_ok(c) != 0; })) {
+        return 0;
+    }
     timing_collect(c);
-    std::memcpy(out, ho, xb);
     if (want_route) {
         if (idx_out) std::memcpy(idx_out, ho + xb, kb);
         if (w_out) std::memcpy(w_out, ho + xb + kb, kb);
