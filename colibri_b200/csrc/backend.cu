@@ -14,6 +14,7 @@
 #include <cmath>
 #include <atomic>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -50,6 +51,7 @@ struct DeviceCtx {
     size_t host_x_cap = 0, host_y_cap = 0;
     float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the other host-buffer calls
     size_t io_x_cap = 0, io_y_cap = 0;
+    bool chain = false;                       // the last thing this call put on the stream is a kernel
     UploadRing up = {};                       // pinned pieces of large uploads
     IoPieces io = {};                         // events of the pieces of a call's result
     uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
@@ -91,6 +93,7 @@ static DeviceCtx *find_ctx(int device) {
 }
 static int select_ctx(DeviceCtx *c) {
     if (!c) return 0;
+    c->chain = false;
     if (g_cur_dev == c->device) return 1;
     if (!cuda_ok(cudaSetDevice(c->device), "select device")) return 0;
     g_cur_dev = c->device;
@@ -138,6 +141,23 @@ static size_t row_bytes(int fmt, int I) {
 // Lifecycle
 // ---------------------------------------------------------------------------
 static void fill_exp2_table(uint64_t *tab) { coli_expf_fill_table(tab); }
+
+// Launch of a kernel of the call's chain. Behind another kernel of the same call (c->chain) it does not wait for
+// that one's end on the queue: its CTAs are placed while the other drains and wait in pdl_enter, which saves 2 to 4 us
+// per launch in a chain of short kernels. A call's first kernel, and one behind a copy, is launched in the ordinary
+// way, and what a chained kernel reads of its predecessors it reads by ordinary loads (not ld.global.nc, whose
+// lines may be older than the wait).
+template <class... P, class... A>
+static void launch_pdl(DeviceCtx *c, void (*kern)(P...), dim3 grid, unsigned block, size_t smem, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = c->chain ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);      // (an error stays for cudaGetLastError)
+    c->chain = true;
+}
 
 template <typename K>
 static void set_smem(K kern, int bytes) {
@@ -555,7 +575,7 @@ static void launch_one(DeviceCtx *c, const GemvSeg *segs, const GemvCtl *ctl, co
                        const float *bs) {
     constexpr int W = GemvCfg<NC>::WARPS, N = GemvCfg<NC>::NST;
     size_t smem = (size_t)W * N * (chunk_bytes_of(MODE) + 8);
-    k_gemv_stream<MODE, NC, W, N><<<c->sms, W * 32, smem, c->stream>>>(segs, ctl, bq, bs, c->status);
+    launch_pdl(c, k_gemv_stream<MODE, NC, W, N>, c->sms, W * 32, smem, segs, ctl, bq, bs, c->status);
 }
 template <int MODE>
 static void launch_mode(DeviceCtx *c, int nc, const GemvSeg *segs, const GemvCtl *ctl,
@@ -585,6 +605,7 @@ static void launch_gemv(DeviceCtx *c, int mode, int nc, const GemvSeg *segs, con
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     kernel_event_pair(c, &e0, &e1);
     if (e0) cudaEventRecord(e0, c->stream);
+    if (e0) c->chain = false;
     switch (mode) {
     case SC_ROW: launch_mode<SC_ROW>(c, nc, segs, ctl, bq, bs); break;
     case SC_H16: launch_mode<SC_H16>(c, nc, segs, ctl, bq, bs); break;
@@ -669,46 +690,51 @@ static void add_seg(HostSegs *hs, const ColiCudaTensor *t, float *out, const int
     hs->v[t->mode].push_back(s);
 }
 
-// Uploads the host-built segment lists and launches one GEMV per scale mode present.
-static int run_host_segs(DeviceCtx *c, HostSegs *hs, Buf *segbuf, int ctl_slot, int nc, int npos,
-                         const __half *bq, const float *bs) {
-    size_t total = 0;
-    for (int m = 0; m < 4; m++) total += hs->v[m].size();
-    size_t seg_bytes = total * sizeof(GemvSeg);
-    size_t need = seg_bytes + 4 * sizeof(GemvCtl);
-    if (!reserve(c, segbuf, need)) return 0;
+// Segment lists of a call on the device: uploaded in one copy before its kernels.
+struct SegLists {
+    const GemvSeg *seg[2][4];
+    const GemvCtl *ctl[2][4];
+};
+static int upload_segs(DeviceCtx *c, SegLists *sl, const HostSegs *const *hs, int n, Buf *buf, int npos) {
+    size_t need = 0;
+    for (int k = 0; k < n; k++) for (int m = 0; m < 4; m++) need += hs[k]->v[m].size() * sizeof(GemvSeg) + sizeof(GemvCtl);
+    if (!reserve(c, buf, need)) return 0;
     // Pageable staging: cudaMemcpyAsync from pageable memory returns once the
     // source has been captured, so the vector can die with this call even
     // though the stream has not run yet.
     std::vector<uint8_t> stage(need);
-    uint8_t *hp = stage.data();
-    (void)ctl_slot;
-    uint8_t *dp = static_cast<uint8_t *>(segbuf->p);
+    const uint8_t *dp = static_cast<const uint8_t *>(buf->p);
     size_t off = 0;
-    GemvCtl ctl[4];
-    size_t seg_off[4];
-    for (int m = 0; m < 4; m++) {
-        seg_off[m] = off;
-        size_t b = hs->v[m].size() * sizeof(GemvSeg);
-        if (b) std::memcpy(hp + off, hs->v[m].data(), b);
-        off += b;
-        ctl[m].nseg = (int)hs->v[m].size(); ctl[m].ntask = hs->ntask[m]; ctl[m].npos = npos;
-        ctl[m].tasks_per_seg = hs->uniform[m] > 0 ? hs->uniform[m] : 0;
-    }
-    std::memcpy(hp + seg_bytes, ctl, sizeof(ctl));
-    if (!cuda_ok(cudaMemcpyAsync(dp, hp, need, cudaMemcpyHostToDevice, c->stream), "segment upload")) return 0;
-    for (int m = 0; m < 4; m++) {
-        if (hs->v[m].empty()) continue;
-        launch_gemv(c, m, nc, reinterpret_cast<const GemvSeg *>(dp + seg_off[m]),
-                    reinterpret_cast<const GemvCtl *>(dp + seg_bytes) + m, bq, bs);
-    }
+    for (int k = 0; k < n; k++)
+        for (int m = 0; m < 4; m++) {
+            const std::vector<GemvSeg> &v = hs[k]->v[m];
+            if (!v.empty()) std::memcpy(stage.data() + off, v.data(), v.size() * sizeof(GemvSeg));
+            sl->seg[k][m] = v.empty() ? nullptr : reinterpret_cast<const GemvSeg *>(dp + off);
+            off += v.size() * sizeof(GemvSeg);
+        }
+    for (int k = 0; k < n; k++)
+        for (int m = 0; m < 4; m++) {
+            GemvCtl ctl;
+            ctl.nseg = (int)hs[k]->v[m].size(); ctl.ntask = hs[k]->ntask[m]; ctl.npos = npos;
+            ctl.tasks_per_seg = hs[k]->uniform[m] > 0 ? hs[k]->uniform[m] : 0;
+            std::memcpy(stage.data() + off, &ctl, sizeof(ctl));
+            sl->ctl[k][m] = reinterpret_cast<const GemvCtl *>(dp + off);
+            off += sizeof(ctl);
+        }
+    c->chain = false;
+    return cuda_ok(cudaMemcpyAsync(buf->p, stage.data(), need, cudaMemcpyHostToDevice, c->stream), "segment upload");
+}
+// One GEMV launch per scale mode present in list k.
+static int run_segs(DeviceCtx *c, const SegLists &sl, int k, int nc, const __half *bq, const float *bs) {
+    for (int m = 0; m < 4; m++)
+        if (sl.seg[k][m]) launch_gemv(c, m, nc, sl.seg[k][m], sl.ctl[k][m], bq, bs);
     return cuda_ok(cudaGetLastError(), "gemv launch");
 }
 
 // Rows the one-launch kernel takes: up to 8, and up to 96 KB of split activations beside its weight ring.
 template <int MODE, int NC>
 static void launch_rows(DeviceCtx *c, const ColiCudaTensor *t, float *y, const float *x, int S) {
-    k_gemv_rows<MODE, NC><<<t->O / 16, ROWS_WARPS * 32, rows_smem(MODE, S, t->I), c->stream>>>(y, x, t->pk, t->rowscale, S, t->I, t->O,
+    launch_pdl(c, k_gemv_rows<MODE, NC>, t->O / 16, ROWS_WARPS * 32, rows_smem(MODE, S, t->I), y, x, t->pk, t->rowscale, S, t->I, t->O,
                                                                                               c->status);
 }
 
@@ -735,9 +761,6 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
     if (!reserve(c, &c->bq, (size_t)S * t->I * 2 * sizeof(__half)) ||
         !reserve(c, &c->bs, (size_t)S * nkb * sizeof(float)) ||
         !reserve(c, &c->pd, (size_t)nkpart * S * t->O * sizeof(float))) return 0;
-    int nw = S * nkb;
-    k_prep_rows<<<(nw * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, S, t->I);
-    c->last_launches++;
     HostSegs hs;
     int rowid[SEG_MAX_ROWS];
     for (int p = 0; p < npass; p++) {
@@ -745,9 +768,15 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
         for (int r = 0; r < nr; r++) rowid[r] = r0 + r;
         add_seg(&hs, t, (float *)c->pd.p, rowid, nr, r0, nkpart);
     }
-    if (!run_host_segs(c, &hs, &c->segs2, 1, nc, S, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
+    SegLists sl;
+    const HostSegs *lists[1] = {&hs};
+    if (!upload_segs(c, &sl, lists, 1, &c->segs2, S)) return 0;
+    int nw = S * nkb;
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, S, t->I);
+    c->last_launches++;
+    if (!run_segs(c, sl, 0, nc, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
     size_t n4 = (size_t)S * t->O / 4;
-    k_reduce_parts<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(y_dev, (const float *)c->pd.p, S, t->O, nkpart);
+    launch_pdl(c, k_reduce_parts, (unsigned)((n4 + 255) / 256), 256, 0, y_dev, (const float *)c->pd.p, S, t->O, nkpart);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "linear launch");
 }
@@ -759,9 +788,9 @@ static void launch_dense(DeviceCtx *c, const ColiCudaTensor *t, float *y, int S,
     const uint8_t *w = static_cast<const uint8_t *>(t->raw_w);
     const size_t rb = row_bytes(t->fmt, t->I);
     const int gs = t->gs > 0 ? t->gs : t->I;
-    if (nc == 1) k_dense_mma<FMT, 1, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
-    else if (nc == 2) k_dense_mma<FMT, 2, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
-    else k_dense_mma<FMT, 4, AL16><<<grid, DENSE_WARPS * 32, 0, c->stream>>>(y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    if (nc == 1) launch_pdl(c, k_dense_mma<FMT, 1, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    else if (nc == 2) launch_pdl(c, k_dense_mma<FMT, 2, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    else launch_pdl(c, k_dense_mma<FMT, 4, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
 }
 
 static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {
@@ -773,7 +802,7 @@ static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const
         if (!reserve(c, &c->bq, (size_t)S * nkb * 256 * sizeof(__half)) || !reserve(c, &c->bs, (size_t)S * nkb * sizeof(float))) return 0;
         __half *bq = (__half *)c->bq.p;
         float *bs = (float *)c->bs.p;
-        k_prep_dense<<<(S * nkb * 32 + 255) / 256, 256, 0, c->stream>>>(bq, bs, x_dev, S, t->I, t->fmt);
+        launch_pdl(c, k_prep_dense, (S * nkb * 32 + 255) / 256, 256, 0, bq, bs, x_dev, S, t->I, t->fmt);
         switch (t->fmt) {
         case 1: if (t->I % 16 == 0) launch_dense<1, true>(c, t, y_dev, S, bq, bs); else launch_dense<1, false>(c, t, y_dev, S, bq, bs); break;
         case 8: if (t->I % 16 == 0) launch_dense<8, true>(c, t, y_dev, S, bq, bs); else launch_dense<8, false>(c, t, y_dev, S, bq, bs); break;
@@ -790,13 +819,13 @@ static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const
     if (dense && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0 && (reinterpret_cast<uintptr_t>(t->raw_w) & 15) == 0) {
         dim3 grid((unsigned)((t->O + 31) / 32), (unsigned)((S + 7) / 8));
         const float *sc = static_cast<const float *>(t->raw_s);
-        if (t->fmt == 0) k_dense_gemv<0><<<grid, 256, DENSE_GEMV_SMEM, c->stream>>>(y_dev, x_dev, t->raw_w, sc, nullptr, S, t->I, t->O);
-        else k_dense_gemv<8><<<grid, 256, DENSE_GEMV_SMEM, c->stream>>>(y_dev, x_dev, t->raw_w, sc, c->e4m3_lut_dev, S, t->I, t->O);
+        if (t->fmt == 0) launch_pdl(c, k_dense_gemv<0>, grid, 256, DENSE_GEMV_SMEM, y_dev, x_dev, t->raw_w, sc, nullptr, S, t->I, t->O);
+        else launch_pdl(c, k_dense_gemv<8>, grid, 256, DENSE_GEMV_SMEM, y_dev, x_dev, t->raw_w, sc, c->e4m3_lut_dev, S, t->I, t->O);
         c->last_launches++;
         return cuda_ok(cudaGetLastError(), "matmul launch");
     }
     dim3 grid((unsigned)((t->O + 7) / 8), (unsigned)((S + 7) / 8));
-    k_generic_matmul<<<grid, 256, 0, c->stream>>>(y_dev, x_dev, t->raw_w, t->raw_s, t->fmt, S, t->I, t->O,
+    launch_pdl(c, k_generic_matmul, grid, 256, 0, y_dev, x_dev, t->raw_w, t->raw_s, t->fmt, S, t->I, t->O,
                                                   t->gs > 0 ? t->gs : t->I, t->ng);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "matmul launch");
@@ -830,7 +859,7 @@ static int check_status(DeviceCtx *c) {
 // behind a copy command, whose completion the stream has to be told by another engine. n4: float4s.
 static int pull_rows(DeviceCtx *c, void *dst, const void *pinned, size_t bytes) {
     const int n4 = (int)(bytes / 16);
-    k_pull<<<(n4 + 255) / 256, 256, 0, c->stream>>>(static_cast<float4 *>(dst), static_cast<const float4 *>(pinned), n4);
+    launch_pdl(c, k_pull, (n4 + 255) / 256, 256, 0, static_cast<float4 *>(dst), static_cast<const float4 *>(pinned), n4);
     return cuda_ok(cudaGetLastError(), "input upload");
 }
 // -> where the kernels find x, or NULL. read_once: the first kernel reads every element once (not every CTA all of them).
@@ -946,12 +975,13 @@ static bool tc_pays(long rows, long experts, int mode) { return rows >= (mode ==
 
 template <int MODE, int PHASE>
 static void launch_tc_one(DeviceCtx *c, const TcArgs &a) {
-    k_expert_gemm_tc<MODE, PHASE><<<c->sms, TC_THREADS, tc_smem_total(MODE), c->stream>>>(a);
+    launch_pdl(c, k_expert_gemm_tc<MODE, PHASE>, c->sms, TC_THREADS, tc_smem_total(MODE), a);
 }
 static int launch_tc(DeviceCtx *c, int mode, int phase, const TcArgs &a) {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     kernel_event_pair(c, &e0, &e1);
     if (e0) cudaEventRecord(e0, c->stream);
+    if (e0) c->chain = false;
     switch (mode * 2 + phase - 1) {
     case SC_ROW * 2: launch_tc_one<SC_ROW, 1>(c, a); break;
     case SC_ROW * 2 + 1: launch_tc_one<SC_ROW, 2>(c, a); break;
@@ -991,12 +1021,12 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
         !reserve(c, &c->pg, (size_t)npos_cap * I * sizeof(float)) || !reserve(c, &c->hq, rows * I * 2 * sizeof(__half))) return 0;
     __half *xq = (__half *)c->bq.p, *hq = (__half *)c->hq.p;
     float *xinv = (float *)c->bs.p, *hinv = xinv + npos_cap, *H = (float *)c->pg.p;
-    k_prep_tc<<<ngrp_cap * 8, TC_PREP_THREADS, 0, c->stream>>>(xq, xinv, l.lo_x, x, l.rowsrc, l.pass, l.grp_pass, l.ngrp, D, x_bf16);
+    launch_pdl(c, k_prep_tc, ngrp_cap * 8, TC_PREP_THREADS, 0, xq, xinv, l.lo_x, x, l.rowsrc, l.pass, l.grp_pass, l.ngrp, D, x_bf16);
     TcArgs a;
     a.pass = l.pass; a.npass = l.npass; a.status = c->status;
     a.lo = l.lo_x; a.q = xq; a.qinv = xinv; a.rowdst = nullptr; a.out = H; a.K = D; a.O = I; a.ntile = I / 64;
     if (!launch_tc(c, mode_gu, 1, a)) return 0;
-    k_prep_tc<<<ngrp_cap * 8, TC_PREP_THREADS, 0, c->stream>>>(hq, hinv, l.lo_h, H, nullptr, l.pass, l.grp_pass, l.ngrp, I, 0);
+    launch_pdl(c, k_prep_tc, ngrp_cap * 8, TC_PREP_THREADS, 0, hq, hinv, l.lo_h, H, nullptr, l.pass, l.grp_pass, l.ngrp, I, 0);
     a.lo = l.lo_h; a.q = hq; a.qinv = hinv; a.rowdst = l.rowdst; a.out = y; a.K = I; a.O = D; a.ntile = D / 128;
     if (!launch_tc(c, mode_d, 2, a)) return 0;
     c->last_launches += 2;
@@ -1046,6 +1076,7 @@ static int group_device_tc(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaT
     }
     *hl.npass = p; *hl.ngrp = grp;
     if (rowmap) std::memcpy(hl.rowsrc, rowmap, (size_t)total * sizeof(int));   // (bcast: all zero)
+    c->chain = false;
     if (!cuda_ok(cudaMemcpyAsync(c->misc.p, stage.data(), need, cudaMemcpyHostToDevice, c->stream), "pass list upload")) return 0;
     dl.rowdst = rowmap ? dl.rowsrc : nullptr;
     return tc_ffn(c, gates[0]->mode, downs[0]->mode, dl, x_dev, x_bf16, total, ngrp, D, I, y_dev);
@@ -1092,7 +1123,7 @@ static int launch_decode(DeviceCtx *c, int mode, DecodeArgs &a, const DecPreset 
     if (!a.act_smem) {
         // x does not fit the kernel's shared memory: split it once here, the kernel reads the fragments
         if (!reserve(c, xq, (size_t)a.M * D * 2 * sizeof(__half)) || !reserve(c, xs, (size_t)a.M * nkb1 * sizeof(float))) return 0;
-        k_prep_rows<<<(a.M * nkb1 * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)xq->p, (float *)xs->p, a.x, nullptr, a.M, D);
+        launch_pdl(c, k_prep_rows, (a.M * nkb1 * 32 + 255) / 256, 256, 0, (__half *)xq->p, (float *)xs->p, a.x, nullptr, a.M, D);
         c->last_launches++;
     }
     a.xq = (const __half *)xq->p; a.xs = (const float *)xs->p;
@@ -1136,6 +1167,7 @@ static int launch_decode(DeviceCtx *c, int mode, DecodeArgs &a, const DecPreset 
         err = cudaLaunchCooperativeKernel(fn, dim3(c->sms), dim3(DEC_WARPS * 32), args, smem, c->stream);
     }
     if (e1) cudaEventRecord(e1, c->stream);
+    c->chain = !e1;
     c->last_launches++;
     return cuda_ok(err, "fused decode launch");
 }
@@ -1207,9 +1239,6 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
             !reserve(c, &c->hq, (size_t)total * I * 2 * sizeof(__half)) ||
             !reserve(c, &c->hs, (size_t)total * nkb2 * sizeof(float)) ||
             !reserve(c, &c->pd, (size_t)nkp2 * total * D * sizeof(float))) return 0;
-        int nw = nxrows * nkb1;
-        k_prep_rows<<<(nw * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, nxrows, D);
-        c->last_launches++;
         HostSegs h1, h2;
         int rowid[SEG_MAX_ROWS], posid[SEG_MAX_ROWS], off = 0;
         for (int e = 0; e < count; e++) {
@@ -1223,15 +1252,21 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
             }
             off += re;
         }
-        if (!run_host_segs(c, &h1, &c->segs1, 0, nc, total, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
+        SegLists sl;
+        const HostSegs *lists[2] = {&h1, &h2};
+        if (!upload_segs(c, &sl, lists, 2, &c->segs1, total)) return 0;
+        int nw = nxrows * nkb1;
+        launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, nxrows, D);
+        c->last_launches++;
+        if (!run_segs(c, sl, 0, nc, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
         int nw2 = total * nkb2;
-        k_swiglu_prep<<<(nw2 * 32 + 255) / 256, 256, 0, c->stream>>>(
+        launch_pdl(c, k_swiglu_prep, (nw2 * 32 + 255) / 256, 256, 0, 
             (__half *)c->hq.p, (float *)c->hs.p, (const float *)c->pg.p, (const float *)c->pu.p, nullptr,
             total, I, nkp1, nullptr);
         c->last_launches++;
-        if (!run_host_segs(c, &h2, &c->segs2, 1, nc, total, (const __half *)c->hq.p, (const float *)c->hs.p)) return 0;
+        if (!run_segs(c, sl, 1, nc, (const __half *)c->hq.p, (const float *)c->hs.p)) return 0;
         size_t n4 = (size_t)total * D / 4;
-        k_reduce_parts<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(y_dev, (const float *)c->pd.p, total, D, nkp2);
+        launch_pdl(c, k_reduce_parts, (unsigned)((n4 + 255) / 256), 256, 0, y_dev, (const float *)c->pd.p, total, D, nkp2);
         c->last_launches++;
         return cuda_ok(cudaGetLastError(), "expert group launch");
     }
@@ -1247,7 +1282,7 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
         if (!linear_raw(c, gates[e], (float *)c->gbuf.p, xe, rs) ||
             !linear_raw(c, ups[e], (float *)c->ubuf.p, xe, rs)) return 0;
         size_t n = (size_t)rs * I;
-        k_silu_mul<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>((float *)c->gbuf.p, (const float *)c->ubuf.p, n);
+        launch_pdl(c, k_silu_mul, (unsigned)((n + 255) / 256), 256, 0, (float *)c->gbuf.p, (const float *)c->ubuf.p, n);
         c->last_launches++;
         if (!linear_raw(c, downs[e], y_dev + (size_t)off * D, (const float *)c->gbuf.p, rs)) return 0;
         off += re;
@@ -1447,7 +1482,7 @@ extern "C" int coli_cuda_pipe_rmsnorm_s(int device, float *y_dev, const float *x
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (S < 1 || D < 1 || xstride < D || ystride < D || !select_ctx(c)) return 0;
-    k_rmsnorm<<<S, RMSNORM_THREADS, 0, c->stream>>>(y_dev, x_dev, w_dev, D, eps, xstride, ystride);
+    launch_pdl(c, k_rmsnorm, S, RMSNORM_THREADS, 0, y_dev, x_dev, w_dev, D, eps, xstride, ystride);
     return cuda_ok(cudaGetLastError(), "pipe rmsnorm");
 }
 extern "C" int coli_cuda_pipe_rmsnorm(int device, float *y_dev, const float *x_dev, const float *w_dev,
@@ -1458,7 +1493,7 @@ extern "C" int coli_cuda_pipe_silu_mul(int device, float *gate_dev, const float 
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!n || !select_ctx(c)) return 0;
-    k_silu_mul<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(gate_dev, up_dev, n);
+    launch_pdl(c, k_silu_mul, (unsigned)((n + 255) / 256), 256, 0, gate_dev, up_dev, n);
     return cuda_ok(cudaGetLastError(), "pipe silu mul");
 }
 extern "C" int coli_cuda_pipe_rope(int device, float *v_dev, const int *pos_dev, int rows, int stride, int offset,
@@ -1466,7 +1501,7 @@ extern "C" int coli_cuda_pipe_rope(int device, float *v_dev, const int *pos_dev,
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!v_dev || !pos_dev || rows < 1 || R < 2 || R > 256 || heads < 1 || !select_ctx(c)) return 0;
-    k_rope_rows<<<rows, 128, 0, c->stream>>>(v_dev, pos_dev, 0, stride, offset, R, heads, theta);
+    launch_pdl(c, k_rope_rows, rows, 128, 0, v_dev, pos_dev, 0, stride, offset, R, heads, theta);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "pipe rope");
 }
@@ -1475,7 +1510,7 @@ extern "C" int coli_cuda_pipe_rope_base(int device, float *v_dev, int pos_base, 
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!v_dev || rows < 1 || R < 2 || R > 256 || heads < 1 || !select_ctx(c)) return 0;
-    k_rope_rows<<<rows, 128, 0, c->stream>>>(v_dev, nullptr, pos_base, stride, offset, R, heads, theta);
+    launch_pdl(c, k_rope_rows, rows, 128, 0, v_dev, nullptr, pos_base, stride, offset, R, heads, theta);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "pipe rope");
 }
@@ -1483,7 +1518,7 @@ extern "C" int coli_cuda_pipe_add(int device, float *x_dev, const float *t_dev, 
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!n || !select_ctx(c)) return 0;
-    k_add<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(x_dev, t_dev, n);
+    launch_pdl(c, k_add, (unsigned)((n + 255) / 256), 256, 0, x_dev, t_dev, n);
     return cuda_ok(cudaGetLastError(), "pipe add");
 }
 extern "C" int coli_cuda_pipe_rows_add(int device, float *x_dev, const float *partial_dev,
@@ -1491,7 +1526,7 @@ extern "C" int coli_cuda_pipe_rows_add(int device, float *x_dev, const float *pa
     if (fault_injected()) return 0;
     DeviceCtx *c = find_ctx(device);
     if (nrows < 1 || D < 1 || !select_ctx(c)) return 0;
-    k_rows_add<<<nrows, 256, 0, c->stream>>>(x_dev, partial_dev, rows_dev, D);
+    launch_pdl(c, k_rows_add, nrows, 256, 0, x_dev, partial_dev, rows_dev, D);
     return cuda_ok(cudaGetLastError(), "pipe rows add");
 }
 extern "C" int coli_cuda_pipe_copy2d(int device, float *dst, int dpitch, const float *src, int spitch,
@@ -1522,11 +1557,11 @@ static void launch_router(DeviceCtx *c, float *logits, const float *x, const flo
     const bool aligned = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
     // up to two waves of CTAs: few outputs each, for the shortest chain time; beyond: more chains per SM
     if (aligned && n <= 16 * 2 * c->sms)
-        k_router_logits<16, 256><<<(n + 15) / 16, 64, router_smem(16, 256), c->stream>>>(logits, x, w, M, D, E, c->status);
+        launch_pdl(c, k_router_logits<16, 256>, (n + 15) / 16, 64, router_smem(16, 256), logits, x, w, M, D, E, c->status);
     else if (aligned)
-        k_router_logits<64, 64><<<(n + 63) / 64, 96, router_smem(64, 64), c->stream>>>(logits, x, w, M, D, E, c->status);
+        launch_pdl(c, k_router_logits<64, 64>, (n + 63) / 64, 96, router_smem(64, 64), logits, x, w, M, D, E, c->status);
     else
-        k_router_logits_any<<<(n + 63) / 64, 64, 0, c->stream>>>(logits, x, w, M, D, E);
+        launch_pdl(c, k_router_logits_any, (n + 63) / 64, 64, 0, logits, x, w, M, D, E);
 }
 
 extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void *rw_dev, const void *rb_dev,
@@ -1541,7 +1576,7 @@ extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void 
     int *idx = (int *)c->io_y, *keff = (int *)(w + Ksel);
     RouteRule rule{D, 0, E, Ksel, 1, norm_topk, routed_scale, topp};
     launch_router(c, logits, x_dev, (const float *)rw_dev, 1, D, E);
-    k_route_topk<<<1, ROUTE_THREADS, route_smem(E), c->stream>>>(logits, (const float *)rb_dev, rule, 1, idx, w, keff);
+    launch_pdl(c, k_route_topk, 1, ROUTE_THREADS, route_smem(E), logits, (const float *)rb_dev, rule, 1, idx, w, keff);
     if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !cuda_ok(cudaStreamSynchronize(c->stream), "pipe router sync")) return 0;
     std::memcpy(idx_host, idx, (size_t)Ksel * 4);
     std::memcpy(w_host, w, (size_t)Ksel * 4);
@@ -1568,6 +1603,7 @@ extern "C" int coli_cuda_expert_group_resident_issue(ColiCudaTensor *const *gate
     if (!reserve(c, &c->x, (size_t)64 * D * sizeof(float)) || !reserve(c, &c->y, (size_t)64 * D * sizeof(float)) ||
         !reserve(c, &c->misc, (size_t)(D + 64) * sizeof(float) + 4096)) return 0;
     float *partial_local = (float *)c->misc.p, *w_dev = partial_local + D;
+    c->chain = false;
     if (!cuda_ok(cudaMemcpyAsync(w_dev, weights, (size_t)count * sizeof(float), cudaMemcpyHostToDevice, c->stream), "resident group weights")) return 0;
     cudaError_t e = device == home_device
         ? cudaMemcpyAsync(c->x.p, x_src_dev, (size_t)D * sizeof(float), cudaMemcpyDeviceToDevice, c->stream)
@@ -1576,7 +1612,7 @@ extern "C" int coli_cuda_expert_group_resident_issue(ColiCudaTensor *const *gate
     int one = 1;
     if (!group_device(c, gates, ups, downs, nullptr, count, D, I, total, 1, all_packed, (float *)c->y.p,
                       (const float *)c->x.p, &one)) return 0;
-    k_weighted_sum_rows<<<48, 256, 0, c->stream>>>(partial_local, (const float *)c->y.p, w_dev, count, D);
+    launch_pdl(c, k_weighted_sum_rows, 48, 256, 0, partial_local, (const float *)c->y.p, w_dev, count, D);
     e = device == home_device
         ? cudaMemcpyAsync(partial_slot_dev, partial_local, (size_t)D * sizeof(float), cudaMemcpyDeviceToDevice, c->stream)
         : cudaMemcpyPeerAsync(partial_slot_dev, home_device, partial_local, device, (size_t)D * sizeof(float), c->stream);
@@ -1594,7 +1630,7 @@ extern "C" int coli_cuda_expert_group_resident_take(int home_device, const int *
         if (!src) return 0;
         if (!cuda_ok(cudaStreamWaitEvent(home->stream, src->ev_done, 0), "resident take wait")) return 0;
     }
-    k_sum_slots<<<48, 256, 0, home->stream>>>(acc_dev, slots_dev, n_issued, D);
+    launch_pdl(home, k_sum_slots, 48, 256, 0, acc_dev, slots_dev, n_issued, D);
     return cuda_ok(cudaGetLastError(), "resident take reduce");
 }
 
@@ -1636,7 +1672,7 @@ extern "C" int coli_cuda_expert_group_dev(ColiCudaTensor *const *gates, ColiCuda
 extern "C" int coli_cuda_pipe_argmax(int device, int *idx_dev, const float *x_dev, int S, int N) {
     DeviceCtx *c = find_ctx(device);
     if (!idx_dev || !x_dev || S < 1 || N < 1 || !select_ctx(c)) return 0;
-    k_argmax_rows<<<S * ARGMAX_CLUSTER, 1024, 0, c->stream>>>(idx_dev, x_dev, N);
+    launch_pdl(c, k_argmax_rows, S * ARGMAX_CLUSTER, 1024, 0, idx_dev, x_dev, N);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "argmax launch");
 }
@@ -1652,7 +1688,7 @@ extern "C" int coli_cuda_moe_combine_dev(int device, float *out_dev, const float
     if (!out_dev || !entry_of_dev || !w_dev || !keff_dev || M < 1 || K < 1 || D < 4 || D % 4 || !select_ctx(c)) return 0;
     if ((reinterpret_cast<uintptr_t>(out_dev) | reinterpret_cast<uintptr_t>(y_dev) | reinterpret_cast<uintptr_t>(shared_dev)) & 15) return 0;
     size_t n4 = (size_t)M * D / 4;
-    k_combine_rows<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(out_dev, y_dev, entry_of_dev, w_dev, keff_dev,
+    launch_pdl(c, k_combine_rows, (unsigned)((n4 + 255) / 256), 256, 0, out_dev, y_dev, entry_of_dev, w_dev, keff_dev,
                                                                      shared_dev, M, K, D);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "combine launch");
@@ -1684,14 +1720,15 @@ extern "C" int coli_cuda_ep_plan_dev(int device, const float *x_dev, int m, int 
         !inexact_dev || m < 1 || K < 1 || K > 31 || E < 1 || G < 1 || slots < 1 || D < 4 || D % 4 || !select_ctx(c)) return 0;
     if (!reserve(c, &c->ep_ws, ((size_t)nb + 1 + (size_t)m * K) * sizeof(int))) return 0;
     int *off = static_cast<int *>(c->ep_ws.p), *row_of = off + nb + 1;
+    c->chain = false;
     if (!cuda_ok(cudaMemsetAsync(counts_dev, 0, (size_t)nb * sizeof(int), c->stream), "ep plan") ||
         !cuda_ok(cudaMemsetAsync(entry_of_dev, 0xFF, (size_t)m * K * sizeof(int), c->stream), "ep plan")) return 0;
     const int n = m * K;
-    k_ep_count<<<(n + 255) / 256, 256, 0, c->stream>>>(counts_dev, idx_dev, keff_dev, dest_dev, slot_dev, m, K, slots);
-    k_ep_offsets<<<1, 256, 0, c->stream>>>(off, counts_dev, nb);
-    k_ep_place<<<(E + 7) / 8, 256, 0, c->stream>>>(entry_of_dev, row_of, off, idx_dev, keff_dev, dest_dev, slot_dev, m, K, E, slots);
-    if (payload_bf16) k_ep_gather<true><<<n, 256, 0, c->stream>>>(send_dev, x_dev, row_of, off + nb, D, inexact_dev);
-    else k_ep_gather<false><<<n, 256, 0, c->stream>>>(send_dev, x_dev, row_of, off + nb, D, inexact_dev);
+    launch_pdl(c, k_ep_count, (n + 255) / 256, 256, 0, counts_dev, idx_dev, keff_dev, dest_dev, slot_dev, m, K, slots);
+    launch_pdl(c, k_ep_offsets, 1, 256, 0, off, counts_dev, nb);
+    launch_pdl(c, k_ep_place, (E + 7) / 8, 256, 0, entry_of_dev, row_of, off, idx_dev, keff_dev, dest_dev, slot_dev, m, K, E, slots);
+    if (payload_bf16) launch_pdl(c, k_ep_gather<true>, n, 256, 0, send_dev, x_dev, row_of, off + nb, D, inexact_dev);
+    else launch_pdl(c, k_ep_gather<false>, n, 256, 0, send_dev, x_dev, row_of, off + nb, D, inexact_dev);
     c->last_launches += 4;
     return cuda_ok(cudaGetLastError(), "ep plan launch");
 }
@@ -1742,14 +1779,15 @@ extern "C" int coli_cuda_ep_expert_group_dev(ColiCudaTensor *const *gates, ColiC
         if (!reserve(c, &c->ep_ws, ((size_t)n) * sizeof(int)) || !reserve(c, &c->ep_x, (size_t)n * D * sizeof(float)) ||
             !reserve(c, &c->ep_y, (size_t)n * D * sizeof(float))) return 0;
         int *map_dev = static_cast<int *>(c->ep_ws.p);
+        c->chain = false;
         if (!cuda_ok(cudaMemcpyAsync(map_dev, rowmap.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->stream), "ep row map")) return 0;
-        if (x_bf16) k_ep_permute<true, false><<<n, 256, 0, c->stream>>>((float *)c->ep_x.p, x_dev, map_dev, n, D);
-        else k_ep_permute<false, false><<<n, 256, 0, c->stream>>>((float *)c->ep_x.p, x_dev, map_dev, n, D);
+        if (x_bf16) launch_pdl(c, k_ep_permute<true, false>, n, 256, 0, (float *)c->ep_x.p, x_dev, map_dev, n, D);
+        else launch_pdl(c, k_ep_permute<false, false>, n, 256, 0, (float *)c->ep_x.p, x_dev, map_dev, n, D);
         c->last_launches++;
         ok = group_device(c, g.data(), u.data(), d.data(), rows.data(), (int)g.size(), D, I, total, max_rows, all_packed,
                           (float *)c->ep_y.p, (const float *)c->ep_x.p, nullptr);
         if (ok) {
-            k_ep_permute<false, true><<<n, 256, 0, c->stream>>>(y_dev, c->ep_y.p, map_dev, n, D);
+            launch_pdl(c, k_ep_permute<false, true>, n, 256, 0, y_dev, c->ep_y.p, map_dev, n, D);
             c->last_launches++;
             ok = cuda_ok(cudaGetLastError(), "ep permute launch");
         }
@@ -1768,7 +1806,7 @@ extern "C" int coli_cuda_ep_combine_dev(int device, float *out_dev, const float 
     if (!out_dev || !y_dev || !entry_of_dev || !w_dev || !keff_dev || m < 1 || K < 1 || D < 4 || D % 4 || !select_ctx(c)) return 0;
     if ((reinterpret_cast<uintptr_t>(out_dev) | reinterpret_cast<uintptr_t>(y_dev) | reinterpret_cast<uintptr_t>(shared_dev)) & 15) return 0;
     const size_t n4 = (size_t)m * D / 4;
-    k_ep_combine<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(out_dev, y_dev, entry_of_dev, w_dev, keff_dev,
+    launch_pdl(c, k_ep_combine, (unsigned)((n4 + 255) / 256), 256, 0, out_dev, y_dev, entry_of_dev, w_dev, keff_dev,
                                                                    shared_dev, m, K, D);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "ep combine launch");
@@ -1851,10 +1889,11 @@ extern "C" int coli_cuda_pipe_gemm_noalloc(ColiCudaTensor *t, float *y_dev, cons
     hs.seg.O = t->O; hs.seg.ntiles = t->O / TILE_ROWS; hs.seg.nkb = nkb;
     hs.seg.nkpart = nkpart; hs.seg.kb_per_part = nkb / nkpart; hs.seg.task0 = 0;
     hc.nseg = 1; hc.ntask = hs.seg.ntiles * nkpart; hc.npos = S; hc.tasks_per_seg = hc.ntask;
+    c->chain = false;
     if (!cuda_ok(cudaMemcpyAsync(seg_dev, &hs.seg, sizeof(GemvSeg), cudaMemcpyHostToDevice, c->stream), "noalloc segment") ||
         !cuda_ok(cudaMemcpyAsync(ctl_dev, &hc, sizeof(GemvCtl), cudaMemcpyHostToDevice, c->stream), "noalloc control")) return 0;
     const int nw = S * nkb;
-    k_prep_rows<<<(nw * 32 + 255) / 256, 256, 0, c->stream>>>(bq_dev, bs_dev, x_dev, nullptr, S, t->I);
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, bq_dev, bs_dev, x_dev, nullptr, S, t->I);
     switch (t->mode) {
     case SC_ROW: launch_mode<SC_ROW>(c, nc, seg_dev, ctl_dev, bq_dev, bs_dev); break;
     case SC_H16: launch_mode<SC_H16>(c, nc, seg_dev, ctl_dev, bq_dev, bs_dev); break;
@@ -1862,7 +1901,7 @@ extern "C" int coli_cuda_pipe_gemm_noalloc(ColiCudaTensor *t, float *y_dev, cons
     default: launch_mode<SC_MX>(c, nc, seg_dev, ctl_dev, bq_dev, bs_dev); break;
     }
     const size_t n4 = (size_t)S * t->O / 4;
-    k_reduce_parts<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(y_dev, pd_dev, S, t->O, nkpart);
+    launch_pdl(c, k_reduce_parts, (unsigned)((n4 + 255) / 256), 256, 0, y_dev, pd_dev, S, t->O, nkpart);
     c->last_launches += 3;
     return cuda_ok(cudaGetLastError(), "pipe_gemm_noalloc launch");
 }

@@ -97,6 +97,14 @@ struct GemvCtl {
     int tasks_per_seg;   // > 0 when every segment has this many tasks (then seg = task / tasks_per_seg)
 };
 
+// First statement of every kernel launched by launch_pdl: lets the stream's next kernel take its place on the SMs as
+// soon as this one's CTAs all have theirs, and waits until the kernel before has finished and its writes are
+// visible. Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #define KSTAT_MBAR_TIMEOUT 1
 
 // The status word lives in pinned host memory that the device addresses directly, so the

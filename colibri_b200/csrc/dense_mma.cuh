@@ -39,7 +39,8 @@ __device__ __forceinline__ int dense_pos(int fmt, int k) {
 __host__ __device__ constexpr int dense_lo_off(int fmt) { return dense_run16(fmt) ? 64 : 32; }
 
 // One warp per (row, block): power-of-two scale, hi and lo parts; columns beyond I are zero.
-__global__ void k_prep_dense(__half *__restrict__ bq, float *__restrict__ bscale, const float *__restrict__ x, int S, int I, int fmt) {
+__global__ void k_prep_dense(__half *__restrict__ bq, float *__restrict__ bscale, const float *x, int S, int I, int fmt) {
+    pdl_enter();
     const int nkb = (I + 127) / 128, wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (wid >= S * nkb) return;
     const int row = wid / nkb, kb = wid - row * nkb;
@@ -90,10 +91,11 @@ __device__ __forceinline__ void dense_i2x16(uint32_t q, uint32_t (&v)[8]) {     
 }
 
 template <int FMT, int NC, bool AL16>
-__global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restrict__ y, const __half *__restrict__ bq,
-                                                                const float *__restrict__ bscale, const uint8_t *__restrict__ w,
-                                                                const void *__restrict__ sc, int S, int I, int O, size_t rowb,
+__global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restrict__ y, const __half *bq,
+                                                                const float *bscale, const uint8_t *__restrict__ w,
+                                                                const void *sc, int S, int I, int O, size_t rowb,
                                                                 int gs, int ng) {
+    pdl_enter();
     constexpr bool RUN16 = dense_run16(FMT);
     constexpr int VPW = (FMT == 1 || FMT == 8) ? 4 : FMT == 3 ? 16 : 8;      // values per 32-bit word
     __shared__ float2 s_part[DENSE_WARPS][NC][2][32];
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
         }
         float ixs[NC];
 #pragma unroll
-        for (int cs = 0; cs < NC; cs++) ixs[cs] = __ldg(sp[cs] + kb);
+        for (int cs = 0; cs < NC; cs++) ixs[cs] = sp[cs][kb];
         float bacc[NC][2][4];
 #pragma unroll
         for (int cs = 0; cs < NC; cs++)
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b0 = ldg_nc128(bp[cs] + (size_t)kb * 256 + c * 128), b1 = ldg_nc128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
+                    const uint4 b0 = ldg128(bp[cs] + (size_t)kb * 256 + c * 128), b1 = ldg128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         mma_f16(bacc[cs][m], v[2 * m][0], v[2 * m + 1][0], v[2 * m][1], v[2 * m + 1][1], b0.x, b0.y);
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b = ldg_nc128(bp[cs] + (size_t)kb * 256 + c * 64);
+                    const uint4 b = ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         float acc[4] = {0.f, 0.f, 0.f, 0.f};

@@ -13,8 +13,9 @@
 #include <cuda_bf16.h>
 
 // cnt[dest[e]*slots + slot[e]] += 1 for every live entry (row, kk < keff[row]).
-__global__ void k_ep_count(int *__restrict__ cnt, const int *__restrict__ idx, const int *__restrict__ keff,
-                           const int *__restrict__ dest, const int *__restrict__ slot, int m, int K, int slots) {
+__global__ void k_ep_count(int *__restrict__ cnt, const int *idx, const int *keff,
+                           const int *dest, const int *slot, int m, int K, int slots) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m * K) return;
     const int s = i / K, kk = i - s * K;
@@ -24,7 +25,8 @@ __global__ void k_ep_count(int *__restrict__ cnt, const int *__restrict__ idx, c
 }
 
 // One block: exclusive prefix sum of the nb bucket counts -> off[nb], total -> off[nb].
-__global__ void k_ep_offsets(int *__restrict__ off, const int *__restrict__ cnt, int nb) {
+__global__ void k_ep_offsets(int *__restrict__ off, const int *cnt, int nb) {
+    pdl_enter();
     __shared__ int part[1024];
     const int tid = threadIdx.x, nth = blockDim.x;
     const int per = (nb + nth - 1) / nth, b0 = tid * per, b1 = min(nb, b0 + per);
@@ -46,10 +48,11 @@ __global__ void k_ep_offsets(int *__restrict__ off, const int *__restrict__ cnt,
 // get consecutive positions of e's bucket in row order (a row that selects e twice keeps
 // its kk order). entry_of[row*K+kk] = position in the send buffer; row_of[position] = row.
 // entry_of must hold -1 everywhere beforehand (dead entries keep it).
-__global__ void k_ep_place(int *__restrict__ entry_of, int *__restrict__ row_of, const int *__restrict__ off,
-                           const int *__restrict__ idx, const int *__restrict__ keff,
-                           const int *__restrict__ dest, const int *__restrict__ slot, int m, int K, int E,
+__global__ void k_ep_place(int *__restrict__ entry_of, int *__restrict__ row_of, const int *off,
+                           const int *idx, const int *keff,
+                           const int *dest, const int *slot, int m, int K, int E,
                            int slots) {
+    pdl_enter();
     const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (e >= E) return;
     int run = off[dest[e] * slots + slot[e]];
@@ -81,8 +84,9 @@ __global__ void k_ep_place(int *__restrict__ entry_of, int *__restrict__ row_of,
 // values are exact in bf16; any value that is not raises *inexact) or as f32.
 // Launched for the largest possible count; blocks beyond *total leave.
 template <bool BF16>
-__global__ void k_ep_gather(void *__restrict__ send, const float *__restrict__ x, const int *__restrict__ row_of,
-                            const int *__restrict__ total, int D, int *__restrict__ inexact) {
+__global__ void k_ep_gather(void *__restrict__ send, const float *x, const int *row_of,
+                            const int *total, int D, int *__restrict__ inexact) {
+    pdl_enter();
     const int p = blockIdx.x;
     if (p >= *total) return;
     const float4 *src = reinterpret_cast<const float4 *>(x + (size_t)row_of[p] * D);
@@ -103,8 +107,9 @@ __global__ void k_ep_gather(void *__restrict__ send, const float *__restrict__ x
 
 // dst[map[p]] = src[p] (FORWARD) or dst[p] = src[map[p]] (gather), rows of D floats; src may be bf16.
 template <bool SRC_BF16, bool SCATTER>
-__global__ void k_ep_permute(float *__restrict__ dst, const void *__restrict__ src, const int *__restrict__ map,
+__global__ void k_ep_permute(float *__restrict__ dst, const void *src, const int *map,
                              int n, int D) {
+    pdl_enter();
     const int p = blockIdx.x;
     if (p >= n) return;
     const int q = map[p];
@@ -124,9 +129,10 @@ __global__ void k_ep_permute(float *__restrict__ dst, const void *__restrict__ s
 
 // out[s] = sum_{kk < keff[s]} w[s,kk] * y[entry_of[s,kk]]  (+ shared[s]): the row's selection
 // order, shared expert last; the same arithmetic as the single-GPU layer's combine.
-__global__ void k_ep_combine(float *__restrict__ out, const float *__restrict__ y, const int *__restrict__ entry_of,
-                             const float *__restrict__ wts, const int *__restrict__ keff,
-                             const float *__restrict__ shared, int m, int K, int D) {
+__global__ void k_ep_combine(float *__restrict__ out, const float *y, const int *entry_of,
+                             const float *wts, const int *keff,
+                             const float *shared, int m, int K, int D) {
+    pdl_enter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int dq = D / 4;
     if (i >= (size_t)m * dq) return;

@@ -20,10 +20,17 @@ __host__ __device__ constexpr int rows_smem(int mode, int S, int I) {
 }
 
 template <int MODE, int NC>
-__global__ void __launch_bounds__(ROWS_WARPS * 32) k_gemv_rows(float *__restrict__ y, const float *__restrict__ x,
-                                                               const uint8_t *__restrict__ w, const float *__restrict__ rowscale,
+__global__ void __launch_bounds__(ROWS_WARPS * 32) k_gemv_rows(float *__restrict__ y, const float *x,
+                                                               const uint8_t *__restrict__ w, const float *rowscale,
                                                                int S, int I, int O, int *status) {
     constexpr int HS = half_bytes_of(MODE);
+    // While the kernel before drains: ask for this CTA's weights to be brought into L2 (no value is read yet).
+    if (threadIdx.x < 32) {
+        const uint8_t *base = w + (size_t)(blockIdx.x >> 1) * (I / BLOCK_K) * 2 * HS + (blockIdx.x & 1) * HS;
+        for (int kb = threadIdx.x; kb < I / BLOCK_K; kb += 32)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + (size_t)kb * 2 * HS), "r"(HS) : "memory");
+    }
+    pdl_enter();
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nkb = I / BLOCK_K;
     const uint32_t ring = smem_u32(smem) + warp * ROWS_NST * HS;

@@ -85,9 +85,9 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ uint4 ldg_nc128(const void *p) {
+__device__ __forceinline__ uint4 ldg128(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
@@ -255,8 +255,8 @@ __device__ __forceinline__ void task_setup(TaskPos &p, const GemvSeg *segs, int 
 // that its passes need and branches per task: decoding a block costs about 200 instructions whatever the
 // rows, every column set 45 to 60 more, so a pass of three rows beside one of eight runs as what it is.
 template <int MODE, int NC, class Issue>
-__device__ __forceinline__ bool gemv_task(const GemvSeg &sg, int kb0, int kb1, int tile, int kpart, int npos, const __half *__restrict__ bq,
-                                          const float *__restrict__ bscale, int lane, uint32_t ring, uint32_t bars, int nst, int &ci,
+__device__ __forceinline__ bool gemv_task(const GemvSeg &sg, int kb0, int kb1, int tile, int kpart, int npos, const __half *bq,
+                                          const float *bscale, int lane, uint32_t ring, uint32_t bars, int nst, int &ci,
                                           uint32_t &par, int &consumed, Issue issue_one) {
     constexpr int HS = half_bytes_of(MODE), CH = 2 * HS;
     // more than 16 rows: the two 16-row halves of a block in turn, for the registers that their sums take
@@ -286,18 +286,18 @@ __device__ __forceinline__ bool gemv_task(const GemvSeg &sg, int kb0, int kb1, i
         const uint32_t st = ring + ci * CH;
         float ixs[NC];
 #pragma unroll
-        for (int cs = 0; cs < NC; cs++) ixs[cs] = __ldg(sptr[cs] + kb);
+        for (int cs = 0; cs < NC; cs++) ixs[cs] = sptr[cs][kb];
         uint4 bpre[4];       // one column set: its fragments do not depend on the chunk, so they are fetched before waiting for it
         if (NC == 1) {
 #pragma unroll
-            for (int grp = 0; grp < 4; grp++) bpre[grp] = ldg_nc128(bptr[0] + (size_t)kb * 256 + grp * 64);
+            for (int grp = 0; grp < 4; grp++) bpre[grp] = ldg128(bptr[0] + (size_t)kb * 256 + grp * 64);
         }
         if (!mbar_wait_bounded(bars + ci * 8, par)) return false;
 #pragma unroll
         for (int h = 0; h < 2; h += NS) {
             float bacc[NC][2][4];
             block_mma<MODE, NC, false, NS>(st + h * HS, lane, g,
-                                           [&](int grp, int cs) { return NC == 1 ? bpre[grp] : ldg_nc128(bptr[cs] + (size_t)kb * 256 + grp * 64); },
+                                           [&](int grp, int cs) { return NC == 1 ? bpre[grp] : ldg128(bptr[cs] + (size_t)kb * 256 + grp * 64); },
                                            bacc);
 #pragma unroll
             for (int cs = 0; cs < NC; cs++)
@@ -336,8 +336,9 @@ __device__ __forceinline__ bool gemv_task(const GemvSeg &sg, int kb0, int kb1, i
 
 template <int MODE, int NC, int WARPS, int NST>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-k_gemv_stream(const GemvSeg *__restrict__ segs, const GemvCtl *__restrict__ ctl,
-              const __half *__restrict__ bq, const float *__restrict__ bscale, int *status) {
+k_gemv_stream(const GemvSeg *segs, const GemvCtl *ctl,
+              const __half *bq, const float *bscale, int *status) {
+    pdl_enter();
     constexpr int CH = 2 * half_bytes_of(MODE);
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

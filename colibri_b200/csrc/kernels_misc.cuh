@@ -161,8 +161,9 @@ __device__ __forceinline__ float warp_max(float m) {
 }
 
 __global__ void k_prep_rows(__half *__restrict__ bq, float *__restrict__ bscale,
-                            const float *__restrict__ x, const int *__restrict__ src_row, int nrows,
+                            const float *x, const int *src_row, int nrows,
                             int K) {
+    pdl_enter();
     const int nkb = K / BLOCK_K;
     int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (wid >= nrows * nkb) return;
@@ -180,9 +181,10 @@ __global__ void k_prep_rows(__half *__restrict__ bq, float *__restrict__ bscale,
 //   g = sum_kp pg[(kp*npos+pos)*I + o] (ascending kp), same for u;
 //   h = g/(1+exp(-g)) * u
 __global__ void k_swiglu_prep(__half *__restrict__ hq, float *__restrict__ hscale,
-                              const float *__restrict__ pg, const float *__restrict__ pu,
-                              const int *__restrict__ npos_p, int npos_cap, int I, int nkpart,
+                              const float *pg, const float *pu,
+                              const int *npos_p, int npos_cap, int I, int nkpart,
                               float *__restrict__ h_out) {
+    pdl_enter();
     const int npos = npos_p ? *npos_p : npos_cap;
     const int nkb = I / BLOCK_K;
     int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -209,8 +211,9 @@ __global__ void k_swiglu_prep(__half *__restrict__ hq, float *__restrict__ hscal
 }
 
 // y[pos, o] = sum_kp part[(kp*npos+pos)*O + o]  (ascending kp)
-__global__ void k_reduce_parts(float *__restrict__ y, const float *__restrict__ part, int npos, int O,
+__global__ void k_reduce_parts(float *__restrict__ y, const float *part, int npos, int O,
                                int nkpart) {
+    pdl_enter();
     size_t n = (size_t)npos * O / 4;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -225,10 +228,11 @@ __global__ void k_reduce_parts(float *__restrict__ y, const float *__restrict__ 
 // Weighted combine of a layer: for token s,
 //   out[s] = sum_{kk<keff[s]} w[s,kk] * Y[pos_of[s*K+kk]]  (+ Y[shared_pos0 + s])
 // with Y[pos] = sum_kp part[(kp*npos+pos)*D + d]; selection order, shared last.
-__global__ void k_combine(float *__restrict__ out, const float *__restrict__ part,
-                          const int *__restrict__ pos_of, const float *__restrict__ wts,
-                          const int *__restrict__ keff, const int *__restrict__ npos_p, int M, int K,
-                          int D, int nkpart, const int *__restrict__ shared_pos0_p) {
+__global__ void k_combine(float *__restrict__ out, const float *part,
+                          const int *pos_of, const float *wts,
+                          const int *keff, const int *npos_p, int M, int K,
+                          int D, int nkpart, const int *shared_pos0_p) {
+    pdl_enter();
     const int npos = *npos_p;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     int dq = D / 4;
@@ -261,10 +265,11 @@ __global__ void k_combine(float *__restrict__ out, const float *__restrict__ par
 // Weighted combine over separate buffers (expert-parallel layer): for row s,
 //   out[s] = sum_{kk<keff[s]} w[s,kk] * y[entry_of[s*K+kk]]  (+ shared[s]),
 // selection order, shared expert last. entry_of is 64-bit (a torch index tensor).
-__global__ void k_combine_rows(float *__restrict__ out, const float *__restrict__ y,
-                               const long long *__restrict__ entry_of, const float *__restrict__ wts,
-                               const long long *__restrict__ keff, const float *__restrict__ shared, int M,
+__global__ void k_combine_rows(float *__restrict__ out, const float *y,
+                               const long long *entry_of, const float *wts,
+                               const long long *keff, const float *shared, int M,
                                int K, int D) {
+    pdl_enter();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     int dq = D / 4;
     if (i >= (size_t)M * dq) return;
@@ -315,8 +320,9 @@ __device__ __forceinline__ float raw_weight(const void *w, const void *sc, int f
     return mag * __uint_as_float(sb << 23);
 }
 
-__global__ void k_generic_matmul(float *__restrict__ y, const float *__restrict__ x, const void *w,
+__global__ void k_generic_matmul(float *__restrict__ y, const float *x, const void *w,
                                  const void *sc, int fmt, int S, int I, int O, int gs, int ng) {
+    pdl_enter();
     int o = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     int s0 = blockIdx.y * 8;
@@ -356,9 +362,10 @@ __global__ void k_generic_matmul(float *__restrict__ y, const float *__restrict_
 #define DENSE_GEMV_CK 1024
 #define DENSE_GEMV_SMEM (2 * 8 * DENSE_GEMV_CK * 4)
 template <int FMT>
-__global__ void __launch_bounds__(256, FMT == 0 ? 3 : 2) k_dense_gemv(float *__restrict__ y, const float *__restrict__ x,
-                                                    const void *__restrict__ w, const float *__restrict__ sc,
-                                                    const float *__restrict__ lut, int S, int I, int O) {
+__global__ void __launch_bounds__(256, FMT == 0 ? 3 : 2) k_dense_gemv(float *__restrict__ y, const float *x,
+                                                    const void *__restrict__ w, const float *sc,
+                                                    const float *lut, int S, int I, int O) {
+    pdl_enter();
     constexpr int VPL = FMT == 0 ? 4 : 16;          // values in one 16-byte piece
     constexpr int CK = DENSE_GEMV_CK;               // columns of x staged per round
     constexpr int PIECES = CK / (32 * VPL);
@@ -475,6 +482,7 @@ __global__ void __launch_bounds__(256, FMT == 0 ? 3 : 2) k_dense_gemv(float *__r
 // input lands at (j, R/2 + j).
 __global__ void k_rope_rows(float *v, const int *pos, int pos_base, int stride, int offset, int R, int heads,
                             float theta) {
+    pdl_enter();
     float *p = v + (size_t)blockIdx.x * stride + offset;
     const int half = R / 2;
     const int ps = pos ? pos[blockIdx.x / heads] : pos_base + (int)(blockIdx.x / heads);
@@ -496,22 +504,25 @@ __global__ void k_rope_rows(float *v, const int *pos, int pos_base, int stride, 
 // Elementwise / row primitives of the resident pipeline.
 // ---------------------------------------------------------------------------
 // Rows from pinned host memory to device memory.
-__global__ void k_pull(float4 *__restrict__ dst, const float4 *__restrict__ src, int n4) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__global__ void k_pull(float4 *__restrict__ dst, const float4 *src, int n4) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n4) dst[i] = src[i];
 }
 
 __global__ void k_silu_mul(float *g, const float *u, size_t n) {
+    pdl_enter();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { float v = g[i]; g[i] = (v / (1.0f + expf(-v))) * u[i]; }
 }
 __global__ void k_add(float *x, const float *t, size_t n) {
+    pdl_enter();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] += t[i];
 }
 // Block b adds partial row b into x row rows[b]; target rows are distinct.
 __global__ void k_rows_add(float *x, const float *partial, const int *rows, int D) {
+    pdl_enter();
     float *xr = x + (size_t)rows[blockIdx.x] * D;
     const float *pr = partial + (size_t)blockIdx.x * D;
     for (int i = threadIdx.x; i < D; i += blockDim.x) xr[i] += pr[i];
@@ -523,6 +534,7 @@ __global__ void k_rows_add(float *x, const float *partial, const int *rows, int 
 #define RMSNORM_THREADS 1024
 __global__ void __launch_bounds__(RMSNORM_THREADS) k_rmsnorm(float *y, const float *x, const float *w, int D, float eps, int xstride,
                                                              int ystride) {
+    pdl_enter();
     const float *xr = x + (size_t)blockIdx.x * xstride;
     float *yr = y + (size_t)blockIdx.x * ystride;
     __shared__ double sh[32];
@@ -566,6 +578,7 @@ __global__ void __launch_bounds__(RMSNORM_THREADS) k_rmsnorm(float *y, const flo
 }
 // out[i] = sum_c w[c] * y[c*D+i] in call order (resident group accumulate)
 __global__ void k_weighted_sum_rows(float *out, const float *y, const float *w, int count, int D) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D; i += gridDim.x * blockDim.x) {
         float acc = 0.f;
         for (int c = 0; c < count; c++) acc += w[c] * y[(size_t)c * D + i];
@@ -573,6 +586,7 @@ __global__ void k_weighted_sum_rows(float *out, const float *y, const float *w, 
     }
 }
 __global__ void k_sum_slots(float *dst, const float *slots, int n, int D) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D; i += gridDim.x * blockDim.x) {
         float acc = 0.f;
         for (int s = 0; s < n; s++) acc += slots[(size_t)s * D + i];
@@ -589,8 +603,9 @@ __global__ void k_sum_slots(float *dst, const float *slots, int n, int D) {
 __device__ __forceinline__ void argmax_take(float &bv, int &bi, float v, int i) {
     if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
 }
-__global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k_argmax_rows(int *__restrict__ out, const float *__restrict__ x,
+__global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k_argmax_rows(int *__restrict__ out, const float *x,
                                                                                              int N) {
+    pdl_enter();
     const int part = blockIdx.x % ARGMAX_CLUSTER, r = blockIdx.x / ARGMAX_CLUSTER, tid = threadIdx.x;
     const float *row = x + (size_t)r * N;
     __shared__ float sv[32];

@@ -1217,9 +1217,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 // 2048 rows of 256 scores), E <= 1024, K <= 64; the same routing function as the fused kernel. Dynamic shared
 // memory: 2 * E floats.
 #define ROUTE_THREADS 128
-__global__ void __launch_bounds__(ROUTE_THREADS) k_route_topk(const float *__restrict__ logits, const float *__restrict__ bias,
+__global__ void __launch_bounds__(ROUTE_THREADS) k_route_topk(const float *logits, const float *bias,
                                                               RouteRule rule, int M, int *__restrict__ idx_out,
                                                               float *__restrict__ w_out, int *__restrict__ keff_out) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm_route[];
     __shared__ unsigned long long s_tab[32];
     __shared__ RouteRule s_rule;

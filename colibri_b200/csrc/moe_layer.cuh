@@ -156,11 +156,11 @@ static int layer_run_tc(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const
     t.sh_gate_rs = L->tab.sh_gate_rs; t.sh_up_rs = L->tab.sh_up_rs; t.sh_down_rs = L->tab.sh_down_rs;
     const size_t nblk = (size_t)(r.D / TILE_ROWS) * (r.I / BLOCK_K);
     t.gu_tail = nblk * chunk_bytes_of(L->mode_gu); t.d_tail = nblk * chunk_bytes_of(L->mode_d);
-    k_tc_plan<<<1, 1024, 33 * r.E * sizeof(int), c->stream>>>(l, scal + 1, scal + 2, (int *)L->pos_of.p, idx_dev, keff_dev, M, r.K, r.E, t);
+    launch_pdl(c, k_tc_plan, 1, 1024, 33 * r.E * sizeof(int), l, scal + 1, scal + 2, (int *)L->pos_of.p, idx_dev, keff_dev, M, r.K, r.E, t);
     c->last_launches++;
     if (!tc_ffn(c, L->mode_gu, L->mode_d, l, x_dev, 0, npos_cap, ngrp_cap, r.D, r.I, (float *)L->pd.p)) return 0;
     size_t n4 = (size_t)M * r.D / 4;
-    k_combine<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(out_dev, (const float *)L->pd.p, (const int *)L->pos_of.p, w_dev,
+    launch_pdl(c, k_combine, (unsigned)((n4 + 255) / 256), 256, 0, out_dev, (const float *)L->pd.p, (const int *)L->pos_of.p, w_dev,
                                                                 keff_dev, scal + 1, M, r.K, r.D, 1, sh ? scal + 2 : nullptr);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "layer launch");
@@ -217,7 +217,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
         a.M = M;
         return launch_decode(c, L->mode_gu, a, nullptr, p.npos_cap, &L->xq, &L->xs, &L->hq, &L->hs, &L->pd);
     }
-    k_route_topk<<<M, ROUTE_THREADS, route_smem(r.E), c->stream>>>(lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
+    launch_pdl(c, k_route_topk, M, ROUTE_THREADS, route_smem(r.E), lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
     c->last_launches++;
     if (use_tc)
         return layer_run_tc(L, c, out_dev, x_dev, M, idx_dev, w_dev, keff_dev);
@@ -228,22 +228,22 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     bo.pos_of = (int *)L->pos_of.p; bo.uniq = uniq_dev ? uniq_dev : (int *)L->uniq.p;
     bo.nu = nu_dev ? nu_dev : scal; bo.npos = scal + 1; bo.shared_pos0 = scal + 2;
     bo.partG = (float *)L->pg.p; bo.partU = (float *)L->pu.p; bo.partD = (float *)L->pd.p;
-    k_route_build<<<1, 1024, (size_t)5 * r.E * sizeof(int), c->stream>>>(idx_dev, keff_dev, M, r, L->tab, bo, p.rpp,
+    launch_pdl(c, k_route_build, 1, 1024, (size_t)5 * r.E * sizeof(int), idx_dev, keff_dev, M, r, L->tab, bo, p.rpp,
                                                                       p.nkp1, p.nkp2, p.seg_cap);
     c->last_launches++;
     if (route_only) return cuda_ok(cudaGetLastError(), "route launch");
     int nw = M * nkb1;
-    k_prep_rows<<<(nw * 32 + 255) / 256, 256, 0, c->stream>>>((__half *)L->xq.p, (float *)L->xs.p, x_dev, nullptr, M, r.D);
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)L->xq.p, (float *)L->xs.p, x_dev, nullptr, M, r.D);
     c->last_launches++;
     launch_gemv(c, L->mode_gu, p.nc, bo.seg1, bo.ctl1, (const __half *)L->xq.p, (const float *)L->xs.p);
     long nw2 = (long)p.npos_cap * nkb2;
-    k_swiglu_prep<<<(unsigned)((nw2 * 32 + 255) / 256), 256, 0, c->stream>>>(
+    launch_pdl(c, k_swiglu_prep, (unsigned)((nw2 * 32 + 255) / 256), 256, 0, 
         (__half *)L->hq.p, (float *)L->hs.p, (const float *)L->pg.p, (const float *)L->pu.p, scal + 1,
         p.npos_cap, r.I, p.nkp1, nullptr);
     c->last_launches++;
     launch_gemv(c, L->mode_d, p.nc, bo.seg2, bo.ctl2, (const __half *)L->hq.p, (const float *)L->hs.p);
     size_t n4 = (size_t)M * r.D / 4;
-    k_combine<<<(unsigned)((n4 + 255) / 256), 256, 0, c->stream>>>(
+    launch_pdl(c, k_combine, (unsigned)((n4 + 255) / 256), 256, 0, 
         out_dev, (const float *)L->pd.p, (const int *)L->pos_of.p, w_dev, keff_dev, scal + 1, M, r.K, r.D,
         p.nkp2, L->has_shared ? scal + 2 : nullptr);
     c->last_launches++;
@@ -362,7 +362,7 @@ extern "C" int coli_cuda_route_topk_dev(int device, const float *logits_dev, con
     if (!logits_dev || !idx_dev || !w_dev || !keff_dev || M < 1 || E < 1 || E > ROUTE_MAX_E || K < 1 ||
         K > ROUTE_MAX_K || K > E || !select_ctx(c)) return 0;
     RouteRule r{0, 0, E, K, gating, norm_topk, routed_scale, topp};
-    k_route_topk<<<M, ROUTE_THREADS, route_smem(E), c->stream>>>(logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
+    launch_pdl(c, k_route_topk, M, ROUTE_THREADS, route_smem(E), logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "route launch");
 }

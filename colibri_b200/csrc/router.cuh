@@ -38,9 +38,10 @@ __device__ __forceinline__ float expf_host_exact(float x) { return coli_expf_exa
 #define ROUTER_STAGES 6
 __host__ __device__ constexpr int router_smem(int out, int tile) { return ROUTER_STAGES * 2 * out * (tile + 4) * 4; }
 template <int OUT, int TILE>
-__global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(float *__restrict__ logits, const float *__restrict__ x,
+__global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(float *__restrict__ logits, const float *x,
                                                                              const float *__restrict__ W, int M, int D, int E,
                                                                              int *status) {
+    pdl_enter();
     extern __shared__ __align__(16) float rt[];         // [stage][w | x][OUT][TILE + 4]
     __shared__ __align__(8) unsigned long long s_full[ROUTER_STAGES], s_empty[ROUTER_STAGES];
     constexpr int LD = TILE + 4, NS = ROUTER_STAGES, CW = (OUT + 31) / 32;
@@ -119,8 +120,9 @@ __global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(flo
     if (!ok && lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
 }
 // One thread per output, operands straight from memory.
-__global__ void k_router_logits_any(float *__restrict__ logits, const float *__restrict__ x, const float *__restrict__ W, int M, int D,
+__global__ void k_router_logits_any(float *__restrict__ logits, const float *x, const float *__restrict__ W, int M, int D,
                                     int E) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M * E) return;
     const int s = i / E;
@@ -153,9 +155,10 @@ struct BuildOut {
 
 // One CTA. Builds the union, the packed row order (expert-major in union
 // order, rows of an expert in ascending token order) and the segment lists.
-__global__ void k_route_build(const int *__restrict__ idx, const int *__restrict__ keff, int M,
+__global__ void k_route_build(const int *idx, const int *keff, int M,
                               RouteRule rule, LayerTables tab, BuildOut out, int rpp, int nkpart1,
                               int nkpart2, int seg_cap) {
+    pdl_enter();
     extern __shared__ int sm_build[];
     const int E = rule.E, K = rule.K, D = rule.D, I = rule.I;
     int *first = sm_build, *cnt = first + E, *base = cnt + E, *uniq = base + E, *passbase = uniq + E;
