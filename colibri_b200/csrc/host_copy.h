@@ -6,13 +6,19 @@
 // memory. Below a few hundred KB a single copy into a pinned buffer (51 GB/s out of the cache) and
 // one DMA beat the driver's path too (21 us against 27 us at 300 KB).
 #pragma once
+#include <atomic>
+#include <chrono>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <thread>
 
 // Three helper threads, started on first use and kept until the process ends. One job at a time;
 // a caller that finds them busy copies alone, so any number of threads may copy at once.
+// A job is cut into pieces of 64 KB that the caller and whoever is awake take one after the other, so a copy never
+// waits for a sleeping helper (waking one takes about 50 us, as long as 1 MB takes to copy). Helpers look for
+// the next job for 200 us before they sleep: a call's result usually follows its input within that time.
 class CopyPool {
 public:
     static CopyPool &get() {
@@ -20,53 +26,84 @@ public:
         return *p;
     }
     void copy(void *dst, const void *src, size_t bytes) {
-        if (bytes < MIN_SPLIT || !owner_.try_lock()) { std::memcpy(dst, src, bytes); return; }
-        {
-            std::lock_guard<std::mutex> l(m_);
-            if (!started_) {
-                for (int i = 0; i < HELPERS; i++) std::thread([this, i] { work(i); }).detach();
-                started_ = true;
-            }
-            dst_ = static_cast<char *>(dst); src_ = static_cast<const char *>(src); bytes_ = bytes;
-            left_ = HELPERS;
-            job_++;
+        if (bytes < MIN_SPLIT || bytes > MAX_JOB || !owner_.try_lock()) {
+            if (bytes > MAX_JOB)
+                for (size_t off = 0; off < bytes; off += MAX_JOB)
+                    copy(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, bytes - off < MAX_JOB ? bytes - off : MAX_JOB);
+            else std::memcpy(dst, src, bytes);
+            return;
         }
-        cv_.notify_all();
-        part(HELPERS);
-        std::unique_lock<std::mutex> l(m_);
-        done_.wait(l, [this] { return left_ == 0; });
-        l.unlock();
+        const uint64_t n = (bytes + PIECE - 1) / PIECE;
+        dst_.store(static_cast<char *>(dst), std::memory_order_relaxed);
+        src_.store(static_cast<const char *>(src), std::memory_order_relaxed);
+        bytes_.store(bytes, std::memory_order_relaxed);
+        done_.store(0, std::memory_order_relaxed);
+        const uint64_t job = (++epoch_ << 32) | (n << 16);
+        ticket_.store(job, std::memory_order_seq_cst);
+        if (!started_) {
+            for (int i = 0; i < HELPERS; i++) std::thread([this] { work(); }).detach();
+            started_ = true;
+        }
+        if (asleep_.load(std::memory_order_seq_cst)) {
+            { std::lock_guard<std::mutex> l(m_); }
+            cv_.notify_all();
+        }
+        take();
+        while (done_.load(std::memory_order_acquire) < n) pause();       // pieces that helpers are in the middle of
         owner_.unlock();
     }
 
 private:
     static constexpr int HELPERS = 3;
-    static constexpr size_t MIN_SPLIT = 1 << 19;
-    void part(int i) {
-        const size_t step = (bytes_ / (HELPERS + 1) + 63) & ~(size_t)63, a = step * i;
-        if (a < bytes_) std::memcpy(dst_ + a, src_ + a, i == HELPERS || bytes_ - a < step ? bytes_ - a : step);
+    static constexpr size_t MIN_SPLIT = 1 << 18, PIECE = 1 << 16, MAX_JOB = (size_t)1 << 30;
+    static void pause() {
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
     }
-    void work(int i) {
-        unsigned long seen = 0;
+    // Copies pieces of the current job until none is left. ticket_: job number | pieces << 16 | next piece; the
+    // job's fields change only while its ticket has no piece left, so a piece won from a ticket belongs to what was read.
+    void take() {
+        uint64_t t = ticket_.load(std::memory_order_acquire);
         for (;;) {
-            {
-                std::unique_lock<std::mutex> l(m_);
-                cv_.wait(l, [&] { return job_ != seen; });
-                seen = job_;
-            }
-            part(i);
-            std::lock_guard<std::mutex> l(m_);
-            if (--left_ == 0) done_.notify_one();
+            const uint64_t n = (t >> 16) & 0xFFFF, i = t & 0xFFFF;
+            if (i >= n) return;
+            char *dst = dst_.load(std::memory_order_relaxed);
+            const char *src = src_.load(std::memory_order_relaxed);
+            const size_t bytes = bytes_.load(std::memory_order_relaxed);
+            if (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire)) continue;
+            const size_t a = i * PIECE;
+            std::memcpy(dst + a, src + a, bytes - a < PIECE ? bytes - a : PIECE);
+            done_.fetch_add(1, std::memory_order_release);
+            t = ticket_.load(std::memory_order_acquire);
+        }
+    }
+    bool open() const {
+        const uint64_t t = ticket_.load(std::memory_order_seq_cst);
+        return (t & 0xFFFF) < ((t >> 16) & 0xFFFF);
+    }
+    void work() {
+        for (;;) {
+            take();
+            const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+            while (!open() && std::chrono::steady_clock::now() < until)
+                for (int i = 0; i < 16; i++) pause();
+            if (open()) continue;
+            std::unique_lock<std::mutex> l(m_);
+            asleep_.fetch_add(1, std::memory_order_seq_cst);
+            cv_.wait(l, [this] { return open(); });
+            asleep_.fetch_sub(1, std::memory_order_seq_cst);
         }
     }
     std::mutex owner_, m_;
-    std::condition_variable cv_, done_;
+    std::condition_variable cv_;
     bool started_ = false;
-    unsigned long job_ = 0;
-    int left_ = 0;
-    char *dst_ = nullptr;
-    const char *src_ = nullptr;
-    size_t bytes_ = 0;
+    uint64_t epoch_ = 0;
+    std::atomic<uint64_t> ticket_{0}, done_{0};
+    std::atomic<size_t> bytes_{0};
+    std::atomic<char *> dst_{nullptr};
+    std::atomic<const char *> src_{nullptr};
+    std::atomic<int> asleep_{0};
 };
 
 // Pinned pieces of one device's uploads, each with the event of the last copy out of it.
@@ -136,25 +173,21 @@ static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, si
 }
 
 // Rows of a blocking call, between the caller's memory and a pinned buffer of the same size, in up to 16 pieces so
-// that the bus works on one while the next is copied. Pieces of 256 KB and more: a copy command costs the host 4 us. (Waking
-// the pool for a part of a megabyte costs more than it saves: a call with 1.5 MB each way took 100 us longer.)
+// that the bus works on one while the next is copied. Pieces of 512 KB and more: a copy command costs the host 4 us,
+// and four threads copy such a piece in about as long as the bus takes for it.
 struct IoPieces {
     static constexpr int N = 16;
     cudaEvent_t ev[N];
     static size_t piece(size_t bytes) {
         const size_t p = ((bytes + N - 1) / N + 4095) & ~(size_t)4095;
-        return p < (256u << 10) ? 256u << 10 : p;
-    }
-    static void copy(void *dst, const void *src, size_t n) {
-        if (n >= (1u << 20)) CopyPool::get().copy(dst, src, n);
-        else std::memcpy(dst, src, n);
+        return p < (512u << 10) ? 512u << 10 : p;
     }
     // src -> pinned -> dst; src has been read when the call returns
     static cudaError_t in(void *dst, void *pinned, const void *src, size_t bytes, cudaStream_t stream) {
         const size_t p = piece(bytes);
         for (size_t off = 0; off < bytes; off += p) {
             const size_t n = bytes - off < p ? bytes - off : p;
-            copy(static_cast<char *>(pinned) + off, static_cast<const char *>(src) + off, n);
+            CopyPool::get().copy(static_cast<char *>(pinned) + off, static_cast<const char *>(src) + off, n);
             const cudaError_t e = cudaMemcpyAsync(static_cast<char *>(dst) + off, static_cast<char *>(pinned) + off, n, cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) return e;
         }
@@ -180,7 +213,7 @@ struct IoPieces {
         int i = 0;
         for (size_t off = 0; off < bytes; off += p, i++) {
             if (cudaEventSynchronize(ev[i]) != cudaSuccess || (i == 0 && !ready())) return false;
-            copy(static_cast<char *>(dst) + off, static_cast<const char *>(pinned) + off, bytes - off < p ? bytes - off : p);
+            CopyPool::get().copy(static_cast<char *>(dst) + off, static_cast<const char *>(pinned) + off, bytes - off < p ? bytes - off : p);
         }
         return true;
     }
