@@ -1011,12 +1011,6 @@ static size_t tc_list_layout(TcList *l, void *mem, int npass_cap, int ngrp_cap, 
     return reinterpret_cast<uint8_t *>(q) - p;
 }
 
-static void launch_prep_tc(DeviceCtx *c, int ngrp_cap, __half *q, float *qinv, int *lo, const void *x, const int *rowsrc, const TcList &l,
-                           int K, int x_bf16) {
-    const int pieces = (K / 8 + TC_PREP_THREADS - 1) / TC_PREP_THREADS;
-    auto k = pieces <= 1 ? k_prep_tc<1> : pieces <= 2 ? k_prep_tc<2> : k_prep_tc<4>;
-    launch_pdl(c, k, ngrp_cap * 8, TC_PREP_THREADS, 0, q, qinv, lo, x, rowsrc, l.pass, l.grp_pass, l.ngrp, K, x_bf16);
-}
 // The expert FFN over a pass list that is already on the device (built there by k_tc_plan, or
 // uploaded): rows x -> prepared tiles -> gate/up with the SwiGLU -> prepared tiles -> down -> y.
 //   npos_cap positions and ngrp_cap padded groups of 16 at most; x rows are bf16 when x_bf16.
@@ -1027,12 +1021,12 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
         !reserve(c, &c->pg, (size_t)npos_cap * I * sizeof(float)) || !reserve(c, &c->hq, rows * I * 2 * sizeof(__half))) return 0;
     __half *xq = (__half *)c->bq.p, *hq = (__half *)c->hq.p;
     float *xinv = (float *)c->bs.p, *hinv = xinv + npos_cap, *H = (float *)c->pg.p;
-    launch_prep_tc(c, ngrp_cap, xq, xinv, l.lo_x, x, l.rowsrc, l, D, x_bf16);
+    launch_pdl(c, k_prep_tc, ngrp_cap * 8, TC_PREP_THREADS, 0, xq, xinv, l.lo_x, x, l.rowsrc, l.pass, l.grp_pass, l.ngrp, D, x_bf16);
     TcArgs a;
     a.pass = l.pass; a.npass = l.npass; a.status = c->status;
     a.lo = l.lo_x; a.q = xq; a.qinv = xinv; a.rowdst = nullptr; a.out = H; a.K = D; a.O = I; a.ntile = I / 64;
     if (!launch_tc(c, mode_gu, 1, a)) return 0;
-    launch_prep_tc(c, ngrp_cap, hq, hinv, l.lo_h, H, nullptr, l, I, 0);
+    launch_pdl(c, k_prep_tc, ngrp_cap * 8, TC_PREP_THREADS, 0, hq, hinv, l.lo_h, H, nullptr, l.pass, l.grp_pass, l.ngrp, I, 0);
     a.lo = l.lo_h; a.q = hq; a.qinv = hinv; a.rowdst = l.rowdst; a.out = y; a.K = I; a.O = D; a.ntile = D / 128;
     if (!launch_tc(c, mode_d, 2, a)) return 0;
     c->last_launches += 2;
@@ -1732,7 +1726,7 @@ extern "C" int coli_cuda_ep_plan_dev(int device, const float *x_dev, int m, int 
     const int n = m * K;
     launch_pdl(c, k_ep_count, (n + 255) / 256, 256, 0, counts_dev, idx_dev, keff_dev, dest_dev, slot_dev, m, K, slots);
     launch_pdl(c, k_ep_offsets, 1, 256, 0, off, counts_dev, nb);
-    launch_pdl(c, k_ep_place, (E + 7) / 8, 256, 0, entry_of_dev, row_of, off, idx_dev, keff_dev, dest_dev, slot_dev, m, K, E, slots);
+    launch_pdl(c, k_ep_place, E, EP_PLACE_WARPS * 32, 0, entry_of_dev, row_of, off, idx_dev, keff_dev, dest_dev, slot_dev, m, K, slots);
     if (payload_bf16) launch_pdl(c, k_ep_gather<true>, n, 256, 0, send_dev, x_dev, row_of, off + nb, D, inexact_dev);
     else launch_pdl(c, k_ep_gather<false>, n, 256, 0, send_dev, x_dev, row_of, off + nb, D, inexact_dev);
     c->last_launches += 4;
