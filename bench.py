@@ -55,7 +55,7 @@ sys.path.insert(0, ROOT)
 from colibri_b200 import workloads as W  # noqa: E402
 from colibri_b200.quant import QTensor  # noqa: E402
 
-TC_MEAN_ROWS = 12     # the backend's rule for prefill-sized layer calls: mean rows per expert
+TC_MEAN_ROWS = {4: 7, 2: 2, 7: 2}     # the backend's rule for layer calls of more than 8 rows: mean rows per expert by format
 ROUTED_SCALE = 2.5    # sigmoid-gated configurations (GLM / DeepSeek-V3 style)
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the fused decode kernel (one ncu
 # capture of configuration 2 at M=1); other workloads have no capture and report null
@@ -821,7 +821,7 @@ def run_gpu_arm(args):
         e2e_med = float(np.median(e2e_b))
         e2e = all_bytes * steps / (e2e_med * 1e-3) / 1e9
         fused = M <= 8
-        uses_tc = M >= 32 and (args.tc == 2 or (args.tc == 1 and M * K >= TC_MEAN_ROWS * E))
+        uses_tc = M > 8 and (args.tc == 2 or (args.tc == 1 and M * K >= TC_MEAN_ROWS.get(fmt, 1 << 30) * E))
         if fused:
             # one launch per layer call: the kernel's share of the timed step (launch gaps included)
             launch_us = ms_med / steps / L * 1e3

@@ -335,9 +335,10 @@ void coli_cuda_set_fused_decode(int enabled);
 /* Expert groups and layer calls with many rows per expert run on the tcgen05
  * tensor-core kernel when every tensor involved is int4 with per-row or fp16-exact
  * group scales, or MXFP4, and D and I are multiples of 128:
- *   1 (default)  when it pays: a mean of at least 12 rows per expert of the call
- *                (layer calls: M >= 32 and M*K >= 12*E), the measured crossover with
- *                the streaming kernel
+ *   1 (default)  when it pays, by the measured crossover with the streaming kernel: a mean
+ *                of at least 7 rows per expert of the call for int4 with group scales (two
+ *                fp16 terms per weight), 2 for MXFP4 and per-row int4; layer calls count M*K
+ *                rows over E experts, from 9 rows (fewer are the fused kernel's)
  *   2            whenever the tensors and shapes allow it (tests)
  *   0            never: the streaming kernel takes every size (A/B testing)
  * No counterpart in the reference. */

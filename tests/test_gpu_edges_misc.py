@@ -1,0 +1,71 @@
+"""Branches chosen by size or alignment: the router GEMV's three forms, the cluster-wide argmax at small and
+ragged widths, and transfers of one and several staged pieces."""
+import numpy as np
+import pytest
+
+import colibri_b200.workloads as W
+from colibri_b200.backend import MoeLayer
+from tests.test_gpu_router import free_layer, upload_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,M", [(8, 1), (33, 9), (64, 74), (64, 75), (200, 40)])      # 64 x 74: the last that fits two waves of 148 x 16
+def test_router_forms(be, E, M):
+    cfg = dict(W.CONFIGS["c2_small"], E=E, K=2, gating=1, norm_topk=1)
+    L = W.HostLayerWeights(cfg, 5 + E)
+    g, u, d, sh = upload_layer(be, L)
+    rw = np.random.default_rng(E).standard_normal((E, cfg["D"])).astype(np.float32)
+    lay = MoeLayer(be, cfg["D"], cfg["I"], E, 2, g, u, d, 1, 1, 1.0, router_w=rw, max_rows=M)
+    x = W.activations(M, cfg["D"], M)
+    lg = np.zeros((M, E), np.float32)
+    for i in range(cfg["D"]):                                   # product and sum rounded separately, in order
+        lg += (x[:, i, None] * rw[None, :, i]).astype(np.float32)
+    a, b = lay(x), lay(x, lg)
+    for p, q in zip(a, b):
+        assert np.array_equal(p.view(np.uint32), q.view(np.uint32))
+    lay.free()
+    free_layer(be, (g, u, d, sh))
+
+
+@pytest.mark.parametrize("D", [64, 1024, 1028, 1030, 6146])     # D % 4 != 0: the form without bulk copies
+def test_pipe_router_widths(be, D):
+    import ctypes as C
+    E, K = 24, 3
+    rng = np.random.default_rng(D)
+    x, rw = rng.standard_normal(D).astype(np.float32), (rng.standard_normal((E, D)) / 16).astype(np.float32)
+    xd, rwd, rbd = (be.pipe_alloc(0, n * 4) for n in (D, E * D, E))
+    zero = np.zeros(E, np.float32)
+    for p, h in ((xd, x), (rwd, rw), (rbd, zero)):
+        assert be.pipe_upload(0, p, h.ctypes.data, h.nbytes)
+    idx, w, keff = np.zeros(K, np.int32), np.zeros(K, np.float32), np.zeros(1, np.int32)
+    assert be.pipe_router(0, xd, rwd, rbd, D, E, K, C.c_float(0.0), 0, C.c_float(1.0), idx.ctypes.data, w.ctypes.data, keff.ctypes.data)
+    lg = np.zeros(E, np.float32)
+    for i in range(D):
+        lg += (x[i] * rw[:, i]).astype(np.float32)
+    assert list(idx) == list(np.argsort(-lg, kind="stable")[:K]) and keff[0] == K
+    assert np.allclose(w, 1 / (1 + np.exp(-lg[idx].astype(np.float64))), rtol=1e-6)
+    for p in (xd, rwd, rbd):
+        be.pipe_free(0, p)
+
+
+@pytest.mark.parametrize("S,N", [(1, 1), (3, 7), (2, 8191), (1, 129280), (2, 33333)])
+def test_argmax_widths_and_ties(be, S, N):
+    x = np.random.default_rng(N).integers(0, max(2, N // 3), (S, N)).astype(np.float32)      # the largest value several times
+    xd, od = be.pipe_alloc(0, x.nbytes), be.pipe_alloc(0, S * 4)
+    out = np.zeros(S, np.int32)
+    assert be.pipe_upload(0, xd, x.ctypes.data, x.nbytes) and be.pipe_argmax(0, od, xd, S, N)
+    assert be.pipe_download(0, od, out.ctypes.data, out.nbytes)
+    assert np.array_equal(out, x.argmax(1))
+    be.pipe_free(0, xd)
+    be.pipe_free(0, od)
+
+
+@pytest.mark.parametrize("nbytes", [4, 65536, 65540, 1 << 20, (2 << 20) + 4, 11 * (1 << 20) + 12])
+def test_staged_transfers(be, nbytes):
+    a = np.random.default_rng(nbytes).integers(0, 1 << 32, nbytes // 4, dtype=np.uint32)
+    b = np.zeros_like(a)
+    p = be.pipe_alloc(0, nbytes)
+    assert be.pipe_upload(0, p, a.ctypes.data, nbytes) and be.pipe_download(0, p, b.ctypes.data, nbytes)
+    assert np.array_equal(a, b)
+    be.pipe_free(0, p)
