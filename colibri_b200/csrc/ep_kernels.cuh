@@ -155,7 +155,22 @@ __global__ void k_ep_combine(float *__restrict__ out, const float *y, const int 
     const int s = i / dq, d4 = i - (size_t)s * dq;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     const int ke = keff[s];
-    for (int kk = 0; kk < ke; kk++) {
+    int kk = 0;
+    for (; kk + 4 <= ke; kk += 4) {         // four rows requested before the first is added
+        float4 a[4];
+        float wgt[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            wgt[j] = wts[s * K + kk + j];
+            a[j] = reinterpret_cast<const float4 *>(y + (size_t)entry_of[s * K + kk + j] * D)[d4];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            acc.x = fmaf(wgt[j], a[j].x, acc.x); acc.y = fmaf(wgt[j], a[j].y, acc.y);
+            acc.z = fmaf(wgt[j], a[j].z, acc.z); acc.w = fmaf(wgt[j], a[j].w, acc.w);
+        }
+    }
+    for (; kk < ke; kk++) {
         const int pos = entry_of[s * K + kk];
         const float wgt = wts[s * K + kk];
         const float4 a = reinterpret_cast<const float4 *>(y + (size_t)pos * D)[d4];

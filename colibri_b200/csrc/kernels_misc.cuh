@@ -239,8 +239,26 @@ __global__ void k_combine(float *__restrict__ out, const float *part,
     if (i >= (size_t)M * dq) return;
     int s = i / dq, d4 = i - (size_t)s * dq;
     float4 acc = make_float4(0, 0, 0, 0);
-    int ke = keff[s];
-    for (int kk = 0; kk < ke; kk++) {
+    int ke = keff[s], kk = 0;
+    // one partial sum: four rows requested before the first is added (a row at a time, the two dependent loads of each
+    // were waited for in turn)
+    if (nkpart == 1) {
+        for (; kk + 4 <= ke; kk += 4) {
+            float4 y[4];
+            float wgt[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                wgt[j] = wts[s * K + kk + j];
+                y[j] = reinterpret_cast<const float4 *>(part + (size_t)pos_of[s * K + kk + j] * D)[d4];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                acc.x += wgt[j] * (0.f + y[j].x); acc.y += wgt[j] * (0.f + y[j].y);
+                acc.z += wgt[j] * (0.f + y[j].z); acc.w += wgt[j] * (0.f + y[j].w);
+            }
+        }
+    }
+    for (; kk < ke; kk++) {
         int pos = pos_of[s * K + kk];
         float wgt = wts[s * K + kk];
         float4 y = make_float4(0, 0, 0, 0);
