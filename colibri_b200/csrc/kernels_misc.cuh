@@ -616,7 +616,9 @@ __global__ void k_sum_slots(float *dst, const float *slots, int n, int D) {
 // pick): best = 0, then every i with x[i] > x[best] in ascending order, i.e. the first index
 // of the largest value, NaNs never winning; a NaN in x[0] keeps the answer at 0.
 // A row is shared by a cluster of ARGMAX_CLUSTER CTAs whose answers meet in the first one's shared memory: one CTA
-// per row took 35 us for 8 rows of 129280, waiting for its own loads.
+// per row took 35 us for 8 rows of 129280, waiting for its own loads. The first CTA's shared memory may be addressed
+// only once that CTA is known to run: every CTA arrives at the cluster barrier on entry and waits for it before its
+// answer leaves, with the row's loads in between.
 #define ARGMAX_CLUSTER 8
 __device__ __forceinline__ void argmax_take(float &bv, int &bi, float v, int i) {
     if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
@@ -624,6 +626,7 @@ __device__ __forceinline__ void argmax_take(float &bv, int &bi, float v, int i) 
 __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k_argmax_rows(int *__restrict__ out, const float *x,
                                                                                              int N) {
     pdl_enter();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int part = blockIdx.x % ARGMAX_CLUSTER, r = blockIdx.x / ARGMAX_CLUSTER, tid = threadIdx.x;
     const float *row = x + (size_t)r * N;
     __shared__ float sv[32];
@@ -646,6 +649,7 @@ __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k
     warp_best();
     if ((tid & 31) == 0) { sv[tid >> 5] = bv; si[tid >> 5] = bi; }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");         // every CTA of the cluster runs
     if (tid < 32) {
         bv = sv[tid]; bi = si[tid];
         warp_best();
@@ -656,6 +660,7 @@ __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(1024) k
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dv), "f"(bv) : "memory");
             asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(di), "r"(bi) : "memory");
         }
+        __syncwarp();
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (part == 0 && tid == 0) {
