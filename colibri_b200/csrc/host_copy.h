@@ -122,9 +122,9 @@ static void upload_ring_free(UploadRing *r) {
     }
     std::memset(r, 0, sizeof(*r));
 }
-// src (any host memory) -> dst (device) on `stream`. The source has been read when the call returns.
+// src (any host memory) -> dst (device) on `stream`. The source has been read when the call returns, small ones and
+// pinned ones included: cudaMemcpyAsync straight from a pinned source would return before the copy has run.
 static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
-    if (bytes <= (64u << 10)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);   // the driver's inline path
     for (size_t off = 0; off < bytes; off += UploadRing::PIECE) {
         const size_t n = bytes - off < UploadRing::PIECE ? bytes - off : UploadRing::PIECE;
         const int i = r->next;

@@ -1,0 +1,97 @@
+// Host transfers (csrc/host_copy.h) against a small stand-in for the CUDA runtime that moves data as late as the
+// real one may: a copy from or to pinned memory happens when its stream or event is waited for, a pageable source is read
+// before the call returns. Prints "ok" and returns 0, or says what failed. Usage: host_copy_check CHECK
+#include <cstddef>
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <functional>
+#include <map>
+#include <memory>
+#include <string>
+#include <vector>
+
+enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2 };
+enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+typedef struct Stream *cudaStream_t;
+typedef struct Event *cudaEvent_t;
+enum { cudaEventDisableTiming = 2 };
+
+struct Stream { std::deque<std::function<void()>> ops; uint64_t pushed = 0, done = 0; };
+struct Event { Stream *s = nullptr; uint64_t at = 0; };
+static std::map<char *, size_t> g_pinned;             // page-locked host ranges
+static int g_pin_budget = 1 << 30;                    // allocations of pinned memory that still succeed
+
+static bool pinned(const void *p) {
+    auto it = g_pinned.upper_bound((char *)p);
+    return it != g_pinned.begin() && (--it, (char *)p < it->first + it->second);
+}
+static void drain(Stream *s, uint64_t to) {
+    while (s->done < to) { s->ops.front()(); s->ops.pop_front(); s->done++; }
+}
+static cudaError_t cudaMallocHost(void **p, size_t n) {
+    if (g_pin_budget-- <= 0) return cudaErrorMemoryAllocation;
+    *p = std::malloc(n);
+    g_pinned[(char *)*p] = n;
+    return cudaSuccess;
+}
+static cudaError_t cudaFreeHost(void *p) { g_pinned.erase((char *)p); std::free(p); return cudaSuccess; }
+static cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = new Event(); return cudaSuccess; }
+static cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
+static cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { e->s = s; e->at = s->pushed; return cudaSuccess; }
+static cudaError_t cudaEventSynchronize(cudaEvent_t e) { if (e->s) drain(e->s, e->at); return cudaSuccess; }
+static cudaError_t cudaStreamSynchronize(cudaStream_t s) { drain(s, s->pushed); return cudaSuccess; }
+static cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind kind, cudaStream_t s) {
+    if (kind == cudaMemcpyHostToDevice && !pinned(src)) {
+        auto copy = std::make_shared<std::vector<char>>((const char *)src, (const char *)src + n);
+        s->ops.push_back([=] { std::memcpy(dst, copy->data(), n); });
+    } else {
+        s->ops.push_back([=] { std::memcpy(dst, src, n); });
+    }
+    s->pushed++;
+    if (kind == cudaMemcpyDeviceToHost && !pinned(dst)) drain(s, s->pushed);
+    return cudaSuccess;
+}
+
+#include "../colibri_b200/csrc/host_copy.h"
+
+#define REQUIRE(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); return 1; } } while (0)
+
+static std::vector<char> pattern(size_t n, unsigned seed) {
+    std::vector<char> v(n);
+    for (size_t i = 0; i < n; i++) { seed = seed * 1664525u + 1013904223u; v[i] = (char)(seed >> 24); }
+    return v;
+}
+static const size_t SIZES[] = {1, 4, 4096, 65536, 65537, 300000, (2u << 20), (2u << 20) + 5, (11u << 20) + 12};
+
+// The source of an upload, pinned or not, belongs to the caller again when the call returns.
+static int upload_sources() {
+    UploadRing ring = {};
+    Stream s;
+    for (size_t n : SIZES)
+        for (int pin = 0; pin < 2; pin++) {
+            const std::vector<char> want = pattern(n, (unsigned)n);
+            std::vector<char> dev(n, 0);
+            char *src;
+            if (pin) REQUIRE(cudaMallocHost((void **)&src, n) == cudaSuccess); else src = (char *)std::malloc(n);
+            std::memcpy(src, want.data(), n);
+            REQUIRE(upload_staged(&ring, dev.data(), src, n, &s) == cudaSuccess);
+            std::memset(src, 0x5A, n);                       // the caller reuses its buffer
+            cudaStreamSynchronize(&s);
+            REQUIRE(dev == want);
+            if (pin) cudaFreeHost(src); else std::free(src);
+        }
+    upload_ring_free(&ring);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    int rc = 2;
+    if (what == "upload_sources") rc = upload_sources();
+    if (rc == 2) std::printf("unknown check %s\n", what.c_str());
+    if (rc == 0) std::puts("ok");
+    return rc;
+}

@@ -69,3 +69,22 @@ def test_staged_transfers(be, nbytes):
     assert be.pipe_upload(0, p, a.ctypes.data, nbytes) and be.pipe_download(0, p, b.ctypes.data, nbytes)
     assert np.array_equal(a, b)
     be.pipe_free(0, p)
+
+
+@pytest.mark.parametrize("nbytes", [4096, 65536, 3 << 20])
+def test_upload_source_may_be_reused(be, nbytes):
+    """A pinned source overwritten right behind the call, while the stream is still busy with earlier work."""
+    import torch
+    want = torch.arange(nbytes // 4, dtype=torch.int32)
+    src = want.clone().pin_memory()
+    n = 1 << 28
+    busy, p = be.pipe_alloc(0, n * 4), be.pipe_alloc(0, nbytes)
+    got = np.zeros(nbytes // 4, np.int32)
+    for _ in range(8):                                          # about 4 ms of kernels before the copy's turn
+        assert be.pipe_add(0, busy, busy, n)
+    assert be.pipe_upload(0, p, src.data_ptr(), nbytes)
+    src.fill_(-1)
+    assert be.pipe_download(0, p, got.ctypes.data, nbytes)
+    assert np.array_equal(got, want.numpy())
+    be.pipe_free(0, busy)
+    be.pipe_free(0, p)

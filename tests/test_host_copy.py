@@ -1,0 +1,28 @@
+"""The host side of the transfers (csrc/host_copy.h), compiled with a stand-in for the CUDA runtime that reads
+and writes pinned memory as late as the real one may."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no host C++ compiler")
+    exe = str(tmp_path_factory.mktemp("host_copy") / "host_copy_check")
+    subprocess.check_call([gxx, "-std=c++17", "-O1", "-g", "-pthread", "-Wno-unused-function", "-o", exe,
+                           os.path.join(ROOT, "tests", "host_copy_check.cpp"), "-ldl"])
+
+    def run(what, **env):
+        r = subprocess.run([exe, what], env=dict(os.environ, **env), capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_upload_sources_are_the_callers_again(check):
+    check("upload_sources")
