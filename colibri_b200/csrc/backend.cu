@@ -1604,7 +1604,10 @@ extern "C" int coli_cuda_expert_group_resident_issue(ColiCudaTensor *const *gate
         !reserve(c, &c->misc, (size_t)(D + 64) * sizeof(float) + 4096)) return 0;
     float *partial_local = (float *)c->misc.p, *w_dev = partial_local + D;
     c->chain = false;
-    if (!cuda_ok(cudaMemcpyAsync(w_dev, weights, (size_t)count * sizeof(float), cudaMemcpyHostToDevice, c->stream), "resident group weights")) return 0;
+    // by way of the stack: a pageable source is captured before the call returns, the caller's own memory may be pinned
+    float w_host[64];
+    std::memcpy(w_host, weights, (size_t)count * sizeof(float));
+    if (!cuda_ok(cudaMemcpyAsync(w_dev, w_host, (size_t)count * sizeof(float), cudaMemcpyHostToDevice, c->stream), "resident group weights")) return 0;
     cudaError_t e = device == home_device
         ? cudaMemcpyAsync(c->x.p, x_src_dev, (size_t)D * sizeof(float), cudaMemcpyDeviceToDevice, c->stream)
         : cudaMemcpyPeerAsync(c->x.p, device, x_src_dev, home_device, (size_t)D * sizeof(float), c->stream);

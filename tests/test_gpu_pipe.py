@@ -80,3 +80,38 @@ def test_resident_group(be, oracle):
     for h in hs:
         for t in h:
             be.tensor_free(t)
+
+
+@pytest.mark.parametrize("fmt,gs,n", [(2, 0, 5), (1, 0, 5), (2, 0, 17)])     # one fused launch; raw experts; more than it takes
+def test_resident_group_weights_are_the_callers_again(be, oracle, fmt, gs, n):
+    """Pinned weights overwritten right behind the call, while the stream is still busy with earlier work."""
+    import torch
+    from colibri_b200.backend import Backend
+    D, I = 256, 128
+    experts = [W.expert_weights(D, I, fmt, gs, 170 + e) for e in range(n)]
+    hs = [[upload_qt(be, t) for t in e] for e in experts]
+    x = W.activations(1, D, 4)
+    wts = np.linspace(0.1, 0.9, n, dtype=np.float32)
+    src = torch.from_numpy(wts.copy()).pin_memory()
+    xd = dev(be, x)
+    slots, acc = be.pipe_alloc(0, D * 4), be.pipe_alloc(0, D * 4)
+    size = 1 << 28
+    busy = be.pipe_alloc(0, size * 4)
+    arr = lambda k: Backend.handle_array([h[k] for h in hs])
+    issue = lambda w: be.expert_group_resident_issue(arr(0), arr(1), arr(2), w, n, 0, xd, slots)
+    assert issue(wts.ctypes.data) and be.pipe_sync(0)             # (workspaces grow here, which waits for the stream)
+    for _ in range(8):
+        assert be.pipe_add(0, busy, busy, size)
+    assert issue(src.data_ptr())
+    src.fill_(1e6)
+    assert be.expert_group_resident_take(0, (C.c_int * 1)(0), 1, slots, acc, D)
+    got = back(be, acc, D)
+    want = np.zeros(D, np.float32)
+    for e, wgt in zip(experts, wts):
+        want += wgt * oracle.expert_mlp(x, *e)[0]
+    assert np.all(np.abs(got - want) <= 1e-3 * (np.abs(want) + 1e-3 * np.abs(want).max()))
+    for p in (xd, slots, acc, busy):
+        be.pipe_free(0, p)
+    for h in hs:
+        for t in h:
+            be.tensor_free(t)
