@@ -122,6 +122,7 @@ ADDITIVE_ABI = [
     ("coli_cuda_kernel_events", C.c_int, [C.c_int, _f32p, _i32p]),
     ("coli_cuda_stream", _vp, [C.c_int]),
     ("coli_cuda_kernel_status", C.c_int, [C.c_int]),
+    ("coli_cuda_expire_wait", C.c_int, [C.c_int]),
 ]
 
 

@@ -1466,7 +1466,8 @@ extern "C" int coli_cuda_pipe_copy_async(int device, void *dst, const void *src,
                                    stream ? static_cast<cudaStream_t>(stream) : c->stream), "pipe copy");
 }
 // Both run on the legacy stream, which waits for, and is waited for by, the backend's stream and every other
-// blocking stream of the device. An upload returns when the source has been read, a download when dst is filled.
+// blocking stream of the device. An upload returns when the source has been read, a download when dst is filled; a
+// download behind a kernel whose wait has expired leaves dst alone and returns 0, like every call that waits.
 extern "C" int coli_cuda_pipe_upload(int device, void *dst, const void *src, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
@@ -1475,7 +1476,9 @@ extern "C" int coli_cuda_pipe_upload(int device, void *dst, const void *src, siz
 extern "C" int coli_cuda_pipe_download(int device, const void *src, void *dst, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
-    return cuda_ok(download_staged(&c->up, dst, src, bytes, cudaStreamLegacy), "pipe download");
+    bool ready = true;
+    return cuda_ok(download_staged(&c->up, dst, src, bytes, cudaStreamLegacy, [c, &ready] { return ready = kernels_ok(c) != 0; }),
+                   "pipe download") && ready;
 }
 extern "C" int coli_cuda_pipe_rmsnorm_s(int device, float *y_dev, const float *x_dev, const float *w_dev,
                                         int S, int D, float eps, int xstride, int ystride) {
@@ -1549,7 +1552,13 @@ extern "C" int coli_cuda_pipe_peer_copy(int dst_dev, float *dst, int src_dev, co
 extern "C" int coli_cuda_pipe_sync(int device) {
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
-    return cuda_ok(cudaDeviceSynchronize(), "pipe sync");
+    return cuda_ok(cudaDeviceSynchronize(), "pipe sync") && kernels_ok(c);
+}
+extern "C" int coli_cuda_expire_wait(int device) {
+    DeviceCtx *c = find_ctx(device);
+    if (!select_ctx(c)) return 0;
+    k_expire_wait<<<1, 1, 0, c->stream>>>(c->status);
+    return cuda_ok(cudaGetLastError(), "expire wait");
 }
 
 static void launch_router(DeviceCtx *c, float *logits, const float *x, const float *w, int M, int D, int E) {
@@ -1577,7 +1586,7 @@ extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void 
     RouteRule rule{D, 0, E, Ksel, 1, norm_topk, routed_scale, topp};
     launch_router(c, logits, x_dev, (const float *)rw_dev, 1, D, E);
     launch_pdl(c, k_route_topk, 1, ROUTE_THREADS, route_smem(E), logits, (const float *)rb_dev, rule, 1, idx, w, keff);
-    if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !cuda_ok(cudaStreamSynchronize(c->stream), "pipe router sync")) return 0;
+    if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !check_status(c)) return 0;
     std::memcpy(idx_host, idx, (size_t)Ksel * 4);
     std::memcpy(w_host, w, (size_t)Ksel * 4);
     std::memcpy(keff_host, keff, 4);

@@ -65,6 +65,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     }
     return true;
 }
+// A wait that nothing ends but its limit, recorded like any other: what the callers do with an expired wait can be
+// tested with it (coli_cuda_expire_wait).
+__global__ void k_expire_wait(int *status) {
+    __shared__ __align__(8) unsigned long long bar;
+    mbar_init(smem_u32(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (!mbar_wait_bounded(smem_u32(&bar), 0)) kstat_set(status, KSTAT_MBAR_TIMEOUT);
+}
 // 1 in one lane of the (converged) warp: what it guards is issued with uniform operands.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;

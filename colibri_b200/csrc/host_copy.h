@@ -106,7 +106,7 @@ private:
     std::atomic<int> asleep_{0};
 };
 
-// Pinned pieces of one device's uploads, each with the event of the last copy out of it.
+// Pinned pieces of one device's transfers, each with the event of the last copy out of it or into it.
 struct UploadRing {
     static constexpr int N = 4;
     static constexpr size_t PIECE = 2u << 20;
@@ -143,8 +143,10 @@ static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size
 
 // src (device) -> dst (any host memory), after all work the stream waits for; done when the call returns. Pieces
 // of 1 MB leave the device while earlier ones are copied out of the pinned buffers (the driver's pageable
-// path moves 4 MB in 244 us, the bus in 84).
-static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+// path moves 4 MB in 244 us, the bus in 84). ready() is asked once, when the first piece is there (the kernels before
+// it are done then); if it says no, dst is left alone and nothing more is copied off the device.
+template <class Ready>
+static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream, Ready ready) {
     constexpr size_t STEP = 1u << 20;
     cudaError_t e;
     size_t out = 0;                             // pieces out: copied to dst
@@ -155,16 +157,18 @@ static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, si
             const int i = (first + (int)(in % UploadRing::N)) % UploadRing::N;
             if (!r->buf[i] && ((e = cudaMallocHost(reinterpret_cast<void **>(&r->buf[i]), UploadRing::PIECE)) != cudaSuccess ||
                                (e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming)) != cudaSuccess)) return e;
-            if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;      // an upload's copy out of it
+            if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;      // the copy before, out of it or into it
             const size_t n = bytes - in * STEP < STEP ? bytes - in * STEP : STEP;
             if ((e = cudaMemcpyAsync(r->buf[i], static_cast<const char *>(src) + in * STEP, n, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
                 (e = cudaEventRecord(r->ev[i], stream)) != cudaSuccess) return e;
-            r->busy[i] = false;
+            r->busy[i] = true;                  // until its event has been waited for, here or by the buffer's next user
             in++;
             continue;
         }
         const int i = (first + (int)(out % UploadRing::N)) % UploadRing::N;
         if ((e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;
+        r->busy[i] = false;
+        if (out == 0 && !ready()) return cudaSuccess;
         const size_t n = bytes - out * STEP < STEP ? bytes - out * STEP : STEP;
         CopyPool::get().copy(static_cast<char *>(dst) + out * STEP, r->buf[i], n);
         out++;

@@ -361,8 +361,13 @@ void *coli_cuda_stream(int device);
 
 /* Sticky error state of the device-side wait guards: 0 = none. Every bounded
  * wait in the kernels (mbarrier polls) records a code here instead of spinning
- * forever; the call that observed it returns 0. */
+ * forever; the next call that waits for the device (host-buffer calls, take,
+ * pipe_router, pipe_download, pipe_sync) returns 0 with its outputs untouched. */
 int coli_cuda_kernel_status(int device);
+
+/* Enqueues a kernel whose bounded wait (about 0.2 s) nothing ends, so that a caller's
+ * handling of an expired wait can be tested: the next call that waits returns 0. */
+int coli_cuda_expire_wait(int device);
 
 #ifdef __cplusplus
 }

@@ -87,10 +87,31 @@ static int upload_sources() {
     return 0;
 }
 
+// Downloads arrive whole; one whose kernels failed leaves the destination alone, and what it had under way into the
+// ring's buffers does not reach the transfer after it.
+static int downloads() {
+    UploadRing ring = {};
+    Stream s;
+    for (size_t n : SIZES)
+        for (int fine = 0; fine < 2; fine++) {
+            std::vector<char> dev = pattern(n, (unsigned)n + 1), dst(n, 0x11);
+            const std::vector<char> untouched = dst, want = pattern(n, (unsigned)n + 2);
+            REQUIRE(download_staged(&ring, dst.data(), dev.data(), n, &s, [&] { return fine != 0; }) == cudaSuccess);
+            REQUIRE(dst == (fine ? dev : untouched));
+            std::vector<char> up(n, 0);
+            REQUIRE(upload_staged(&ring, up.data(), want.data(), n, &s) == cudaSuccess);
+            cudaStreamSynchronize(&s);
+            REQUIRE(up == want);
+        }
+    upload_ring_free(&ring);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     int rc = 2;
     if (what == "upload_sources") rc = upload_sources();
+    if (what == "downloads") rc = downloads();
     if (rc == 2) std::printf("unknown check %s\n", what.c_str());
     if (rc == 0) std::puts("ok");
     return rc;

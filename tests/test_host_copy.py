@@ -26,3 +26,7 @@ def check(tmp_path_factory):
 
 def test_upload_sources_are_the_callers_again(check):
     check("upload_sources")
+
+
+def test_downloads_and_the_ring_behind_a_failed_one(check):
+    check("downloads")
