@@ -10,15 +10,20 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
-// Three helper threads, started on first use and kept until the process ends. One job at a time;
+// Helper threads, started on first use and kept until the process ends. One job at a time;
 // a caller that finds them busy copies alone, so any number of threads may copy at once.
 // A job is cut into pieces of 64 KB that the caller and whoever is awake take one after the other, so a copy never
 // waits for a sleeping helper (waking one takes about 50 us, as long as 1 MB takes to copy). Helpers look for
-// the next job for 200 us before they sleep: a call's result usually follows its input within that time.
+// the next job for 200 us before they sleep: a call's result usually follows its input within that time. So a program
+// that copies 256 KB or more at shorter intervals keeps them awake, on cores its own threads may want:
+// COLI_CUDA_COPY_THREADS=0 turns them off, 1 to 3 sets their number (read once). Without it there are three, or a quarter of the
+// host's hardware threads if that is less. One that the system does not grant is done without.
 class CopyPool {
 public:
     static CopyPool &get() {
@@ -26,7 +31,7 @@ public:
         return *p;
     }
     void copy(void *dst, const void *src, size_t bytes) {
-        if (bytes < MIN_SPLIT || bytes > MAX_JOB || !owner_.try_lock()) {
+        if (bytes < MIN_SPLIT || bytes > MAX_JOB || limit_ == 0 || !owner_.try_lock()) {
             if (bytes > MAX_JOB)
                 for (size_t off = 0; off < bytes; off += MAX_JOB)
                     copy(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, bytes - off < MAX_JOB ? bytes - off : MAX_JOB);
@@ -41,8 +46,11 @@ public:
         const uint64_t job = (++epoch_ << 32) | (n << 16);
         ticket_.store(job, std::memory_order_seq_cst);
         if (!started_) {
-            for (int i = 0; i < HELPERS; i++) std::thread([this] { work(); }).detach();
             started_ = true;
+            try {                               // (no exception may leave through the C entry points above)
+                for (int i = 0; i < limit_; i++) std::thread([this] { work(); }).detach();
+            } catch (const std::system_error &) {
+            }
         }
         if (asleep_.load(std::memory_order_seq_cst)) {
             { std::lock_guard<std::mutex> l(m_); }
@@ -55,6 +63,12 @@ public:
 
 private:
     static constexpr int HELPERS = 3;
+    static int helper_limit() {
+        const char *e = std::getenv("COLI_CUDA_COPY_THREADS");
+        const unsigned quarter = std::thread::hardware_concurrency() / 4;
+        const int n = e && *e ? std::atoi(e) : (int)quarter;
+        return n < 0 ? 0 : n > HELPERS ? HELPERS : n;
+    }
     static constexpr size_t MIN_SPLIT = 1 << 18, PIECE = 1 << 16, MAX_JOB = (size_t)1 << 30;
     static void pause() {
 #if defined(__x86_64__)
@@ -95,6 +109,7 @@ private:
             asleep_.fetch_sub(1, std::memory_order_seq_cst);
         }
     }
+    const int limit_ = helper_limit();
     std::mutex owner_, m_;
     std::condition_variable cv_;
     bool started_ = false;

@@ -8,7 +8,8 @@
  * Return convention (c/backend_cuda.h:70-80): 1 = done, 0 = refused or failed
  * with every output untouched (the engine then runs its CPU path); pointer
  * returns use NULL for failure. Host buffers are borrowed for the duration of
- * a call only.
+ * a call only. Copies of 256 KB and more are shared with up to three helper threads
+ * (COLI_CUDA_COPY_THREADS=0 to 3 in the environment sets how many).
  *
  * Part 2 declares the additive entry points of this backend (no counterpart in
  * the reference header): device-resident layer handles that run routing,

@@ -1,6 +1,12 @@
 // Host transfers (csrc/host_copy.h) against a small stand-in for the CUDA runtime that moves data as late as the
 // real one may: a copy from or to pinned memory happens when its stream or event is waited for, a pageable source is read
 // before the call returns. Prints "ok" and returns 0, or says what failed. Usage: host_copy_check CHECK
+#include <dlfcn.h>
+#include <dirent.h>
+#include <errno.h>
+#include <pthread.h>
+#include <unistd.h>
+
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
@@ -57,6 +63,20 @@ static cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMem
 
 #include "../colibri_b200/csrc/host_copy.h"
 
+static std::atomic<int> g_threads_left{1 << 30};      // threads that may still be created
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
+    if (g_threads_left.fetch_sub(1) <= 0) return EAGAIN;
+    static auto real = (int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *))dlsym(RTLD_NEXT, "pthread_create");
+    return real(t, a, f, arg);
+}
+static int threads() {                                 // of this process
+    int n = 0;
+    DIR *d = opendir("/proc/self/task");
+    while (dirent *e = readdir(d)) n += e->d_name[0] != '.';
+    closedir(d);
+    return n;
+}
+
 #define REQUIRE(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); return 1; } } while (0)
 
 static std::vector<char> pattern(size_t n, unsigned seed) {
@@ -107,11 +127,50 @@ static int downloads() {
     return 0;
 }
 
+static const size_t COPY_SIZES[] = {1, 65536, (1u << 18) - 1, 1u << 18, (1u << 18) + 1, (1u << 20) + 77, (9u << 20) + 3};
+
+// Copies are whole with as many helpers as asked for (argument), as the system grants, or none.
+static int helpers(int granted, int expected) {
+    g_threads_left = granted;
+    for (int rep = 0; rep < 3; rep++)
+        for (size_t n : COPY_SIZES) {
+            const std::vector<char> src = pattern(n, (unsigned)(n + rep));
+            std::vector<char> dst(n, 0);
+            CopyPool::get().copy(dst.data(), src.data(), n);
+            REQUIRE(dst == src);
+        }
+    REQUIRE(threads() == 1 + expected);
+    return 0;
+}
+
+// Several threads copy at once, each job whole and in its own buffer.
+static int many_callers() {
+    std::atomic<int> bad{0};
+    std::vector<std::thread> callers;
+    for (int c = 0; c < 6; c++)
+        callers.emplace_back([c, &bad] {
+            for (int rep = 0; rep < 60; rep++)
+                for (size_t n : COPY_SIZES) {
+                    if (n > (2u << 20) && rep % 10) continue;
+                    const std::vector<char> src = pattern(n, (unsigned)(n * 31 + c * 7 + rep));
+                    std::vector<char> dst(n, 0);
+                    CopyPool::get().copy(dst.data(), src.data(), n);
+                    if (dst != src) bad++;
+                    if (rep % 16 == 15) usleep(400);          // long enough for the helpers to fall asleep
+                }
+        });
+    for (auto &t : callers) t.join();
+    REQUIRE(bad == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     int rc = 2;
     if (what == "upload_sources") rc = upload_sources();
     if (what == "downloads") rc = downloads();
+    if (what == "helpers" && argc > 3) rc = helpers(std::atoi(argv[2]), std::atoi(argv[3]));
+    if (what == "many_callers") rc = many_callers();
     if (rc == 2) std::printf("unknown check %s\n", what.c_str());
     if (rc == 0) std::puts("ok");
     return rc;

@@ -18,8 +18,8 @@ def check(tmp_path_factory):
     subprocess.check_call([gxx, "-std=c++17", "-O1", "-g", "-pthread", "-Wno-unused-function", "-o", exe,
                            os.path.join(ROOT, "tests", "host_copy_check.cpp"), "-ldl"])
 
-    def run(what, **env):
-        r = subprocess.run([exe, what], env=dict(os.environ, **env), capture_output=True, text=True, timeout=120)
+    def run(*what, **env):
+        r = subprocess.run([exe, *what], env=dict(os.environ, **env), capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, r.stdout + r.stderr
     return run
 
@@ -30,3 +30,19 @@ def test_upload_sources_are_the_callers_again(check):
 
 def test_downloads_and_the_ring_behind_a_failed_one(check):
     check("downloads")
+
+
+@pytest.mark.parametrize("asked,granted,expected", [("3", 9, 3), ("1", 9, 1), ("0", 9, 0), ("7", 9, 3), ("-1", 9, 0),
+                                                    ("3", 0, 0), ("3", 1, 1)])
+def test_helper_threads_asked_for_and_granted(check, asked, granted, expected):
+    """Threads the system refuses are done without: no exception, no lock left behind."""
+    check("helpers", str(granted), str(expected), COLI_CUDA_COPY_THREADS=asked)
+
+
+def test_helper_threads_by_default(check):
+    check("helpers", "9", str(min(3, len(os.sched_getaffinity(0)) // 4)), COLI_CUDA_COPY_THREADS="")
+
+
+@pytest.mark.parametrize("asked", ["3", "0"])
+def test_several_threads_copy_at_once(check, asked):
+    check("many_callers", COLI_CUDA_COPY_THREADS=asked)
