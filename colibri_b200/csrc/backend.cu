@@ -47,9 +47,9 @@ struct DeviceCtx {
     Buf x, y, bq, bs, pg, pu, hq, hs, pd, segs1, segs2, ctl, gbuf, ubuf, misc;
     Buf pipe[27];
     Buf ep_ws, ep_x, ep_y;                    // expert-parallel layer: plan tables, permuted rows (streaming-kernel path)
-    float *host_x = nullptr, *host_y = nullptr;   // pinned rows of the grouped call (result valid until the next issue)
+    float *host_x = nullptr, *host_y = nullptr;   // pinned rows of the issued group: its alone from issue to the issue after its take
     size_t host_x_cap = 0, host_y_cap = 0;
-    float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the other host-buffer calls
+    float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the blocking host-buffer calls
     size_t io_x_cap = 0, io_y_cap = 0;
     bool chain = false;                       // the last thing this call put on the stream is a kernel
     UploadRing up = {};                       // pinned pieces of large uploads
@@ -1307,8 +1307,11 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
     DeviceCtx *c = find_ctx(device);
     if (!c || (async_issue && c->group_pending) || !select_ctx(c)) return 0;
     size_t xb = (size_t)total * D * sizeof(float);
+    // A blocking call may come between issue and take: the issued group's rows stay where no other call puts its own.
+    float **hx = async_issue ? &c->host_x : &c->io_x, **hy = async_issue ? &c->host_y : &c->io_y;
     if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, xb) ||
-        !reserve_pinned(&c->host_x, &c->host_x_cap, xb) || !reserve_pinned(&c->host_y, &c->host_y_cap, xb)) return 0;
+        !reserve_pinned(hx, async_issue ? &c->host_x_cap : &c->io_x_cap, xb) ||
+        !reserve_pinned(hy, async_issue ? &c->host_y_cap : &c->io_y_cap, xb)) return 0;
     const char *pe = std::getenv("COLI_CUDA_PROFILE");
     int profile = pe && std::atoi(pe);
     cudaEvent_t ev[4] = {};
@@ -1317,14 +1320,14 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         profile = 0; break;
     }
     if (profile) cudaEventRecord(ev[0], c->stream);
-    if (!cuda_ok(IoPieces::in(c->x.p, c->host_x, x, xb, c->stream), "expert group input upload")) return 0;
+    if (!cuda_ok(IoPieces::in(c->x.p, *hx, x, xb, c->stream), "expert group input upload")) return 0;
     if (profile) cudaEventRecord(ev[1], c->stream);
     timing_begin(c);
     if (!group_device(c, gates, ups, downs, rows, count, D, I, total, max_rows, all_packed,
                       (float *)c->y.p, (const float *)c->x.p, nullptr)) return 0;
     timing_end(c);
     if (profile) cudaEventRecord(ev[2], c->stream);
-    if (!cuda_ok(c->io.out_start(c->host_y, c->y.p, xb, c->stream), "expert group output download")) return 0;
+    if (!cuda_ok(c->io.out_start(*hy, c->y.p, xb, c->stream), "expert group output download")) return 0;
     if (profile) cudaEventRecord(ev[3], c->stream);
     if (async_issue) {
         c->group_pending = 1;
@@ -1332,7 +1335,7 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         if (profile) for (int i = 0; i < 4; i++) cudaEventDestroy(ev[i]);
         return 1;
     }
-    if (!c->io.out_finish(y, c->host_y, xb, [c] { return kernels_ok(c) != 0; })) return 0;
+    if (!c->io.out_finish(y, *hy, xb, [c] { return kernels_ok(c) != 0; })) return 0;
     if (profile && !cuda_ok(cudaStreamSynchronize(c->stream), "synchronize")) return 0;
     timing_collect(c);
     if (profile) {

@@ -123,3 +123,38 @@ def test_group_argument_checks(be):
     assert be.expert_group_take(0) is None                          # nothing pending
     be.tensor_free(ha)
     be.tensor_free(hb)
+
+
+@pytest.mark.parametrize("between", [3, 40])          # rows of the blocking call: fewer and more than the issued group's
+def test_blocking_group_between_issue_and_take(be, oracle, between):
+    """The issued group keeps its rows and its result while another group runs, and after the take until the next issue."""
+    import ctypes as C
+    from colibri_b200.backend import Backend
+    D, I = 256, 128
+    rng = np.random.default_rng(between)
+    ex = [[rand_qt(rng, I, D, 4, 32, half=True), rand_qt(rng, I, D, 4, 32, half=True), rand_qt(rng, D, I, 4, 32, half=True)]
+          for _ in range(2)]
+    hs = [[upload_qt(be, t) for t in e] for e in ex]
+    side = lambda k: [h[k] for h in hs]
+    x = rng.standard_normal((5, D)).astype(np.float32)
+    other = rng.standard_normal((between, D)).astype(np.float32)
+    ok, want = be.run_expert_group(side(0), side(1), side(2), [2, 3], x, D)
+    ok2, want2 = be.run_expert_group(side(0), side(1), side(2), [1, between - 1], other, D)
+    assert ok and ok2
+    n = 1 << 28
+    busy = be.pipe_alloc(0, n * 4)
+    for _ in range(4):                                # the issued rows are still on their way when the blocking call begins
+        assert be.pipe_add(0, busy, busy, n)
+    rows = np.array([2, 3], np.int32)
+    assert be.expert_group_issue(*[Backend.handle_array(side(k)) for k in range(3)], rows.ctypes.data_as(C.POINTER(C.c_int)), 2,
+                                 x.ctypes.data)
+    ok, got2 = be.run_expert_group(side(0), side(1), side(2), [1, between - 1], other, D)
+    p = be.expert_group_take(0)
+    got = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(5, D))
+    assert ok and np.array_equal(got2, want2) and np.array_equal(got, want)
+    be.run_expert_group(side(0), side(1), side(2), [1, between - 1], other, D)
+    assert np.array_equal(got, want)                  # valid until the next issue
+    be.pipe_free(0, busy)
+    for h in hs:
+        for t in h:
+            be.tensor_free(t)
