@@ -56,7 +56,7 @@ struct DeviceCtx {
     IoPieces io = {};                         // events of the pieces of a call's result
     uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
     uint32_t *check_host = nullptr;
-    int group_pending = 0;
+    int group_pending = 0;                    // a group is issued and not taken; -1: and a wait has expired since
     int *status = nullptr;                    // pinned host int the kernels store into (kstat_set): sticky kernel status
     unsigned int *dec_sync = nullptr;         // fused decode kernel: the grid barriers' arrival counter
     unsigned long long *exp_tab_dev = nullptr; // global-memory copy of the 2^(i/32) table
@@ -843,6 +843,7 @@ static int kernels_ok(DeviceCtx *c) {
         cudaMemsetAsync(c->dec_sync, 0, DEC_SYNC_WORDS * sizeof(unsigned int), c->stream);
         *reinterpret_cast<volatile int *>(c->status) = 0;
         c->sticky_status = v;
+        if (c->group_pending) c->group_pending = -1;      // it may have been that group's: its take reports it too
         return 0;
     }
     return 1;
@@ -1362,9 +1363,10 @@ extern "C" int coli_cuda_expert_group_issue(ColiCudaTensor *const *gates, ColiCu
 extern "C" const float *coli_cuda_expert_group_take(int device) {
     DeviceCtx *c = find_ctx(device);
     if (!c || !c->group_pending) return nullptr;
+    const bool expired = c->group_pending < 0;
     c->group_pending = 0;
     if (!select_ctx(c)) return nullptr;
-    if (!check_status(c)) return nullptr;
+    if (!check_status(c) || expired) return nullptr;
     timing_collect(c);
     return c->host_y;
 }

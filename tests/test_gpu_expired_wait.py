@@ -75,6 +75,12 @@ for name, (call, out) in cases.items():
     for o, w in zip(out, want):
         assert np.array_equal(o, w) and not np.all(o == 77), name
     assert be.kernel_status(0) == 1
+# seen by a blocking call between issue and take: the issued group may be the one it hit, so its take reports it too
+rows = np.array([1, 2], np.int32)
+issue = lambda: be.expert_group_issue(*[Backend.handle_array(side(k)[:2]) for k in range(3)],
+                                      rows.ctypes.data_as(C.POINTER(C.c_int)), 2, x.ctypes.data)
+assert be.expire_wait(0) and issue() and be.pipe_sync(0) == 0 and not be.expert_group_take(0)
+assert issue() and be.pipe_sync(0) == 1 and be.expert_group_take(0)
 be.shutdown()
 print("ok")
 """
