@@ -112,12 +112,22 @@ static int reserve(DeviceCtx *c, Buf *b, size_t bytes) {
     b->cap = want;
     return 1;
 }
-static int reserve_pinned(float **p, size_t *cap, size_t bytes) {
+// Pinned buffer for the rows of calls with host buffers, grow-only up to IO_PINNED_MAX, by a quarter more than asked
+// for: pinning 8 MB takes 8 ms and 32 MB 19, which a row count that rises step by step would pay at each step. -> 0: more
+// than that, or the system has none to give; the caller moves its rows through the ring of pieces instead.
+#define IO_PINNED_MAX ((size_t)32 << 20)
+static int reserve_pinned(DeviceCtx *c, float **p, size_t *cap, size_t bytes) {
     if (bytes <= *cap) return 1;
-    if (*p) cudaFreeHost(*p);
+    if (bytes > IO_PINNED_MAX) return 0;
+    if (*p) { cudaStreamSynchronize(c->stream); cudaFreeHost(*p); }
     *p = nullptr; *cap = 0;
-    if (!cuda_ok(cudaMallocHost((void **)p, bytes), "pinned allocation")) return 0;
-    *cap = bytes;
+    size_t want = bytes + bytes / 4 < IO_PINNED_MAX ? bytes + bytes / 4 : IO_PINNED_MAX;
+    if (cudaMallocHost((void **)p, want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        want = bytes;
+        if (!cuda_ok(cudaMallocHost((void **)p, want), "pinned allocation")) { *p = nullptr; return 0; }
+    }
+    *cap = want;
     return 1;
 }
 // Test hook of the reference (c/backend_cuda.cu:1340-1348): COLI_GPU_FAIL_AFTER=N
@@ -863,24 +873,36 @@ static int pull_rows(DeviceCtx *c, void *dst, const void *pinned, size_t bytes) 
     launch_pdl(c, k_pull, (n4 + 255) / 256, 256, 0, static_cast<float4 *>(dst), static_cast<const float4 *>(pinned), n4);
     return cuda_ok(cudaGetLastError(), "input upload");
 }
+// Rows to the device by way of a pinned buffer of their size, or of the ring where there is none.
+static int rows_in(DeviceCtx *c, void *dst, void *pinned, const void *src, size_t bytes) {
+    return cuda_ok(pinned ? IoPieces::in(dst, pinned, src, bytes, c->stream) : upload_staged(&c->up, dst, src, bytes, c->stream), "input upload");
+}
+// ... and back, once the kernels are known to have done well. rows_out_start only enqueues; the ring's part waits for rows_out_finish.
+static int rows_out_start(DeviceCtx *c, void *pinned, const void *src_dev, size_t bytes) {
+    return !pinned || cuda_ok(c->io.out_start(pinned, src_dev, bytes, c->stream), "output download");
+}
+static int rows_out_finish(DeviceCtx *c, void *dst, void *pinned, const void *src_dev, size_t bytes) {
+    if (pinned) return c->io.out_finish(dst, pinned, bytes, [c] { return kernels_ok(c) != 0; });
+    bool ready = true;
+    return cuda_ok(download_staged(&c->up, dst, src_dev, bytes, c->stream, [c, &ready] { return ready = kernels_ok(c) != 0; }),
+                   "output download") && ready;
+}
 // -> where the kernels find x, or NULL. read_once: the first kernel reads every element once (not every CTA all of them).
 static const float *io_in(DeviceCtx *c, const float *x, size_t bytes, bool read_once) {
-    if (!reserve_pinned(&c->io_x, &c->io_x_cap, bytes)) return nullptr;
-    if (read_once && bytes <= IO_DIRECT_BYTES) {
-        std::memcpy(c->io_x, x, bytes);
-        return c->io_x;
+    float *pinned = reserve_pinned(c, &c->io_x, &c->io_x_cap, bytes) ? c->io_x : nullptr;
+    if (pinned && read_once && bytes <= IO_DIRECT_BYTES) {
+        std::memcpy(pinned, x, bytes);
+        return pinned;
     }
     if (!reserve(c, &c->x, bytes)) return nullptr;
-    if (bytes <= IO_DIRECT_BYTES && bytes % 16 == 0) {
-        std::memcpy(c->io_x, x, bytes);
-        return pull_rows(c, c->x.p, c->io_x, bytes) ? (const float *)c->x.p : nullptr;
+    if (pinned && bytes <= IO_DIRECT_BYTES && bytes % 16 == 0) {
+        std::memcpy(pinned, x, bytes);
+        return pull_rows(c, c->x.p, pinned, bytes) ? (const float *)c->x.p : nullptr;
     }
-    if (!cuda_ok(IoPieces::in(c->x.p, c->io_x, x, bytes, c->stream), "input upload")) return nullptr;
-    return (const float *)c->x.p;
+    return rows_in(c, c->x.p, pinned, x, bytes) ? (const float *)c->x.p : nullptr;
 }
 static float *io_out(DeviceCtx *c, size_t bytes) {
-    if (!reserve_pinned(&c->io_y, &c->io_y_cap, bytes)) return nullptr;
-    if (bytes <= IO_DIRECT_BYTES) return c->io_y;
+    if (reserve_pinned(c, &c->io_y, &c->io_y_cap, bytes) && bytes <= IO_DIRECT_BYTES) return c->io_y;
     return reserve(c, &c->y, bytes) ? (float *)c->y.p : nullptr;
 }
 static int io_finish(DeviceCtx *c, float *y, const float *y_dev, size_t bytes) {
@@ -889,8 +911,8 @@ static int io_finish(DeviceCtx *c, float *y, const float *y_dev, size_t bytes) {
         std::memcpy(y, c->io_y, bytes);
         return 1;
     }
-    return cuda_ok(c->io.out_start(c->io_y, y_dev, bytes, c->stream), "output download") &&
-           c->io.out_finish(y, c->io_y, bytes, [c] { return kernels_ok(c) != 0; });
+    float *pinned = bytes <= c->io_y_cap ? c->io_y : nullptr;
+    return rows_out_start(c, pinned, y_dev, bytes) && rows_out_finish(c, y, pinned, y_dev, bytes);
 }
 
 extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *x, const void *weights,
@@ -1309,10 +1331,16 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
     if (!c || (async_issue && c->group_pending) || !select_ctx(c)) return 0;
     size_t xb = (size_t)total * D * sizeof(float);
     // A blocking call may come between issue and take: the issued group's rows stay where no other call puts its own.
-    float **hx = async_issue ? &c->host_x : &c->io_x, **hy = async_issue ? &c->host_y : &c->io_y;
-    if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, xb) ||
-        !reserve_pinned(hx, async_issue ? &c->host_x_cap : &c->io_x_cap, xb) ||
-        !reserve_pinned(hy, async_issue ? &c->host_y_cap : &c->io_y_cap, xb)) return 0;
+    // (The issued rows have to be pinned: up to 8, nothing waits for them here.)
+    if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, xb)) return 0;
+    float *hx, *hy;
+    if (async_issue) {
+        if (!reserve_pinned(c, &c->host_x, &c->host_x_cap, xb) || !reserve_pinned(c, &c->host_y, &c->host_y_cap, xb)) return 0;
+        hx = c->host_x; hy = c->host_y;
+    } else {
+        hx = reserve_pinned(c, &c->io_x, &c->io_x_cap, xb) ? c->io_x : nullptr;
+        hy = reserve_pinned(c, &c->io_y, &c->io_y_cap, xb) ? c->io_y : nullptr;
+    }
     const char *pe = std::getenv("COLI_CUDA_PROFILE");
     int profile = pe && std::atoi(pe);
     cudaEvent_t ev[4] = {};
@@ -1321,14 +1349,14 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         profile = 0; break;
     }
     if (profile) cudaEventRecord(ev[0], c->stream);
-    if (!cuda_ok(IoPieces::in(c->x.p, *hx, x, xb, c->stream), "expert group input upload")) return 0;
+    if (!rows_in(c, c->x.p, hx, x, xb)) return 0;
     if (profile) cudaEventRecord(ev[1], c->stream);
     timing_begin(c);
     if (!group_device(c, gates, ups, downs, rows, count, D, I, total, max_rows, all_packed,
                       (float *)c->y.p, (const float *)c->x.p, nullptr)) return 0;
     timing_end(c);
     if (profile) cudaEventRecord(ev[2], c->stream);
-    if (!cuda_ok(c->io.out_start(*hy, c->y.p, xb, c->stream), "expert group output download")) return 0;
+    if (!rows_out_start(c, hy, c->y.p, xb)) return 0;
     if (profile) cudaEventRecord(ev[3], c->stream);
     if (async_issue) {
         c->group_pending = 1;
@@ -1336,7 +1364,7 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
         if (profile) for (int i = 0; i < 4; i++) cudaEventDestroy(ev[i]);
         return 1;
     }
-    if (!c->io.out_finish(y, *hy, xb, [c] { return kernels_ok(c) != 0; })) return 0;
+    if (!rows_out_finish(c, y, hy, c->y.p, xb)) return 0;
     if (profile && !cuda_ok(cudaStreamSynchronize(c->stream), "synchronize")) return 0;
     timing_collect(c);
     if (profile) {
@@ -1584,17 +1612,23 @@ extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void 
     DeviceCtx *c = find_ctx(device);
     if (!x_dev || !rw_dev || !rb_dev || D < 1 || E < 1 || E > ROUTE_MAX_E || Ksel < 1 || Ksel > ROUTE_MAX_K ||
         Ksel > E || !idx_host || !w_host || !keff_host || !select_ctx(c)) return 0;
-    // the selection goes straight to pinned memory: idx [Ksel] | w [Ksel] | keff
-    if (!reserve(c, &c->misc, (size_t)E * 4) || !reserve_pinned(&c->io_y, &c->io_y_cap, (size_t)Ksel * 8 + 4)) return 0;
-    float *logits = (float *)c->misc.p, *w = c->io_y + Ksel;
-    int *idx = (int *)c->io_y, *keff = (int *)(w + Ksel);
+    // the selection goes straight to pinned memory where there is some: idx [Ksel] | w [Ksel] | keff
+    const size_t sel = (size_t)Ksel * 8 + 4;
+    if (!reserve(c, &c->misc, (size_t)E * 4 + sel)) return 0;
+    const bool pinned = reserve_pinned(c, &c->io_y, &c->io_y_cap, sel);
+    float *logits = (float *)c->misc.p;
+    int *idx = pinned ? (int *)c->io_y : (int *)(logits + E), *keff = idx + 2 * Ksel;
+    float *w = (float *)(idx + Ksel);
     RouteRule rule{D, 0, E, Ksel, 1, norm_topk, routed_scale, topp};
     launch_router(c, logits, x_dev, (const float *)rw_dev, 1, D, E);
     launch_pdl(c, k_route_topk, 1, ROUTE_THREADS, route_smem(E), logits, (const float *)rb_dev, rule, 1, idx, w, keff);
     if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !check_status(c)) return 0;
-    std::memcpy(idx_host, idx, (size_t)Ksel * 4);
-    std::memcpy(w_host, w, (size_t)Ksel * 4);
-    std::memcpy(keff_host, keff, 4);
+    int few[2 * ROUTE_MAX_K + 1];
+    if (!pinned && !rows_out_finish(c, few, nullptr, idx, sel)) return 0;
+    const int *got = pinned ? idx : few;
+    std::memcpy(idx_host, got, (size_t)Ksel * 4);
+    std::memcpy(w_host, got + Ksel, (size_t)Ksel * 4);
+    std::memcpy(keff_host, got + 2 * Ksel, 4);
     return 1;
 }
 

@@ -137,6 +137,16 @@ static void upload_ring_free(UploadRing *r) {
     }
     std::memset(r, 0, sizeof(*r));
 }
+// Buffer i of the ring, pinned on first use. Where the system has no pinned memory left the transfer goes without it, by
+// the driver's own staging: slower, not refused.
+static bool upload_ring_slot(UploadRing *r, int i) {
+    if (r->buf[i]) return true;
+    if (!r->ev[i] && cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming) != cudaSuccess) { r->ev[i] = nullptr; (void)cudaGetLastError(); return false; }
+    void *p = nullptr;
+    if (cudaMallocHost(&p, UploadRing::PIECE) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    r->buf[i] = static_cast<char *>(p);
+    return true;
+}
 // src (any host memory) -> dst (device) on `stream`. The source has been read when the call returns, small ones and
 // pinned ones included: cudaMemcpyAsync straight from a pinned source would return before the copy has run.
 static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
@@ -145,8 +155,10 @@ static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size
         const int i = r->next;
         r->next = (i + 1) % UploadRing::N;
         cudaError_t e;
-        if (!r->buf[i] && ((e = cudaMallocHost(reinterpret_cast<void **>(&r->buf[i]), UploadRing::PIECE)) != cudaSuccess ||
-                           (e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming)) != cudaSuccess)) return e;
+        if (!upload_ring_slot(r, i)) {
+            e = cudaMemcpyAsync(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, bytes - off, cudaMemcpyHostToDevice, stream);
+            return e != cudaSuccess ? e : cudaStreamSynchronize(stream);
+        }
         if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;
         CopyPool::get().copy(r->buf[i], static_cast<const char *>(src) + off, n);
         if ((e = cudaMemcpyAsync(static_cast<char *>(dst) + off, r->buf[i], n, cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
@@ -167,11 +179,17 @@ static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, si
     size_t out = 0;                             // pieces out: copied to dst
     const size_t np = (bytes + STEP - 1) / STEP;
     const int first = r->next;
+    for (size_t i = 0; i < np && i < (size_t)UploadRing::N; i++)
+        if (!upload_ring_slot(r, (first + (int)i) % UploadRing::N)) {
+            char few[16];                       // (a blocking copy: the kernels before it are done when it returns)
+            if ((e = cudaMemcpyAsync(few, src, bytes < sizeof(few) ? bytes : sizeof(few), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(stream)) != cudaSuccess || !ready()) return e;
+            if ((e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+            return cudaStreamSynchronize(stream);
+        }
     for (size_t in = 0; out < np;) {
         if (in < np && in - out < UploadRing::N) {
             const int i = (first + (int)(in % UploadRing::N)) % UploadRing::N;
-            if (!r->buf[i] && ((e = cudaMallocHost(reinterpret_cast<void **>(&r->buf[i]), UploadRing::PIECE)) != cudaSuccess ||
-                               (e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming)) != cudaSuccess)) return e;
             if (r->busy[i] && (e = cudaEventSynchronize(r->ev[i])) != cudaSuccess) return e;      // the copy before, out of it or into it
             const size_t n = bytes - in * STEP < STEP ? bytes - in * STEP : STEP;
             if ((e = cudaMemcpyAsync(r->buf[i], static_cast<const char *>(src) + in * STEP, n, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||

@@ -12,7 +12,7 @@ struct ColiCudaMoeLayer {
     LayerTables tab;
     // per-call buffers (device, grow-only)
     Buf x, out, logits, idx, w, keff, pos_of, uniq, scal, xq, xs, pg, pu, hq, hs, pd, seg1, seg2, ctl;
-    float *host_io;                          // pinned staging
+    float *host_io;                          // pinned staging of decode-sized calls
     size_t host_io_cap;
     // tensor handles (host arrays of E entries; shared: one each or NULL) for the paths that
     // build their work lists on the host
@@ -281,6 +281,7 @@ extern "C" int coli_cuda_moe_route_dev(ColiCudaMoeLayer *L, const float *x_dev, 
                      w_dev ? w_dev : (float *)L->w.p, keff_dev ? keff_dev : (int *)L->keff.p, 1, uniq_dev, nu_dev);
 }
 
+#define LAYER_PINNED_MAX ((size_t)1 << 20)
 extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float *x, const float *logits,
                                    int M, int *idx_out, float *w_out, int *keff_out) {
     if (fault_injected()) return 0;
@@ -291,35 +292,39 @@ extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float 
     const size_t xb = (size_t)M * r.D * sizeof(float), lb = logits ? (size_t)M * r.E * sizeof(float) : 0;
     const size_t rb = (size_t)M * r.K * 8 + (size_t)M * 4;
     if (!reserve(c, &L->x, xb + lb) || !reserve(c, &L->out, xb)) return 0;
-    // pinned staging: [x | logits | out | idx | w | keff]
-    size_t need = xb + lb + xb + rb;
-    if (need > L->host_io_cap) {
-        if (L->host_io) { cudaStreamSynchronize(c->stream); cudaFreeHost(L->host_io); L->host_io = nullptr; L->host_io_cap = 0; }
-        if (!cuda_ok(cudaMallocHost((void **)&L->host_io, need), "pinned allocation")) return 0;
-        L->host_io_cap = need;
+    // Pinned staging: [x | logits] and [out | idx | w | keff]. Decode-sized calls keep a buffer of the layer's own, larger
+    // ones share the device's two, so that a model of many layers does not pin its largest batch once per layer.
+    uint8_t *hp, *ho;
+    if (xb + lb + xb + rb <= LAYER_PINNED_MAX) {
+        hp = reserve_pinned(c, &L->host_io, &L->host_io_cap, xb + lb + xb + rb) ? reinterpret_cast<uint8_t *>(L->host_io) : nullptr;
+        ho = hp ? hp + xb + lb : nullptr;
+    } else {
+        hp = reserve_pinned(c, &c->io_x, &c->io_x_cap, xb + lb) ? reinterpret_cast<uint8_t *>(c->io_x) : nullptr;
+        ho = reserve_pinned(c, &c->io_y, &c->io_y_cap, xb + rb) ? reinterpret_cast<uint8_t *>(c->io_y) : nullptr;
     }
-    uint8_t *hp = reinterpret_cast<uint8_t *>(L->host_io);
-    if (xb + lb <= IO_DIRECT_BYTES && (xb + lb) % 16 == 0) {
+    if (hp && xb + lb <= IO_DIRECT_BYTES && (xb + lb) % 16 == 0) {
         std::memcpy(hp, x, xb);
         if (lb) std::memcpy(hp + xb, logits, lb);
         if (!pull_rows(c, L->x.p, hp, xb + lb)) return 0;
     } else {
-        if (lb) {
+        uint8_t *xd = static_cast<uint8_t *>(L->x.p);
+        if (lb && hp) {
             std::memcpy(hp + xb, logits, lb);
-            if (!cuda_ok(cudaMemcpyAsync(static_cast<uint8_t *>(L->x.p) + xb, hp + xb, lb, cudaMemcpyHostToDevice, c->stream), "layer input upload")) return 0;
+            if (!cuda_ok(cudaMemcpyAsync(xd + xb, hp + xb, lb, cudaMemcpyHostToDevice, c->stream), "layer input upload")) return 0;
+        } else if (lb && !rows_in(c, xd + xb, nullptr, logits, lb)) {
+            return 0;
         }
-        if (!cuda_ok(IoPieces::in(L->x.p, hp, x, xb, c->stream), "layer input upload")) return 0;
+        if (!rows_in(c, xd, hp, x, xb)) return 0;
     }
     const float *x_dev = (const float *)L->x.p;
     const float *lg_dev = lb ? reinterpret_cast<const float *>(static_cast<uint8_t *>(L->x.p) + xb) : nullptr;
-    uint8_t *ho = hp + xb + lb;
     const size_t kb = (size_t)M * r.K * 4;
     const int want_route = idx_out || w_out || keff_out;
     // Decode-sized calls: the kernel stores the result (and the routing) straight into the
     // pinned staging area, which the device addresses directly; a few KB of posted writes over
     // the bus cost less than the copy commands and their dependencies. Larger results are
     // copied by the DMA engines.
-    const int direct = M <= DEC_MAX_M && xb <= (64u << 10) && (xb + lb) % 16 == 0 && kb % 16 == 0;
+    const int direct = ho && M <= DEC_MAX_M && xb <= (64u << 10) && (xb + lb) % 16 == 0 && kb % 16 == 0;
     timing_begin(c);
     if (direct) {
         if (!layer_run(L, c, reinterpret_cast<float *>(ho), x_dev, lg_dev, M, reinterpret_cast<int *>(ho + xb),
@@ -330,20 +335,24 @@ extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float 
         if (!layer_run(L, c, (float *)L->out.p, x_dev, lg_dev, M, (int *)L->idx.p, (float *)L->w.p, (int *)L->keff.p,
                        0, nullptr, nullptr)) return 0;
         timing_end(c);
-        if (want_route) {
+        if (want_route && ho) {
             cudaMemcpyAsync(ho + xb, L->idx.p, kb, cudaMemcpyDeviceToHost, c->stream);
             cudaMemcpyAsync(ho + xb + kb, L->w.p, kb, cudaMemcpyDeviceToHost, c->stream);
             cudaMemcpyAsync(ho + xb + 2 * kb, L->keff.p, (size_t)M * 4, cudaMemcpyDeviceToHost, c->stream);
         }
-        if (!cuda_ok(c->io.out_start(ho, L->out.p, xb, c->stream), "layer output download")) return 0;
+        if (!rows_out_start(c, ho, L->out.p, xb)) return 0;
     }
     if (direct) {
         if (!check_status(c)) return 0;
         std::memcpy(out, ho, xb);
-    } else if (!c->io.out_finish(out, ho, xb, [c] { return kernels_ok(c) != 0; })) {
+    } else if (!rows_out_finish(c, out, ho, L->out.p, xb)) {
         return 0;
     }
     timing_collect(c);
+    if (want_route && !ho) {
+        return (!idx_out || rows_out_finish(c, idx_out, nullptr, L->idx.p, kb)) && (!w_out || rows_out_finish(c, w_out, nullptr, L->w.p, kb)) &&
+               (!keff_out || rows_out_finish(c, keff_out, nullptr, L->keff.p, (size_t)M * 4));
+    }
     if (want_route) {
         if (idx_out) std::memcpy(idx_out, ho + xb, kb);
         if (w_out) std::memcpy(w_out, ho + xb + kb, kb);

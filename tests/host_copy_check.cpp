@@ -43,6 +43,7 @@ static cudaError_t cudaMallocHost(void **p, size_t n) {
     g_pinned[(char *)*p] = n;
     return cudaSuccess;
 }
+static cudaError_t cudaGetLastError() { return cudaSuccess; }
 static cudaError_t cudaFreeHost(void *p) { g_pinned.erase((char *)p); std::free(p); return cudaSuccess; }
 static cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = new Event(); return cudaSuccess; }
 static cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
@@ -127,6 +128,28 @@ static int downloads() {
     return 0;
 }
 
+// With no or too little pinned memory transfers take another way and are as whole.
+static int no_pinned_memory() {
+    for (int budget = 0; budget < UploadRing::N; budget++) {
+        UploadRing ring = {};
+        Stream s;
+        g_pin_budget = budget;
+        for (size_t n : SIZES) {
+            const std::vector<char> want = pattern(n, (unsigned)n + budget);
+            std::vector<char> dev(n, 0), back(n, 0x11), src = want;
+            const std::vector<char> untouched = back;
+            REQUIRE(upload_staged(&ring, dev.data(), src.data(), n, &s) == cudaSuccess);
+            src.assign(n, 0x5A);
+            REQUIRE(download_staged(&ring, back.data(), dev.data(), n, &s, [] { return false; }) == cudaSuccess);
+            REQUIRE(back == untouched);
+            REQUIRE(download_staged(&ring, back.data(), dev.data(), n, &s, [] { return true; }) == cudaSuccess);
+            REQUIRE(dev == want && back == want);
+        }
+        upload_ring_free(&ring);
+    }
+    return 0;
+}
+
 static const size_t COPY_SIZES[] = {1, 65536, (1u << 18) - 1, 1u << 18, (1u << 18) + 1, (1u << 20) + 77, (9u << 20) + 3};
 
 // Copies are whole with as many helpers as asked for (argument), as the system grants, or none.
@@ -169,6 +192,7 @@ int main(int argc, char **argv) {
     int rc = 2;
     if (what == "upload_sources") rc = upload_sources();
     if (what == "downloads") rc = downloads();
+    if (what == "no_pinned_memory") rc = no_pinned_memory();
     if (what == "helpers" && argc > 3) rc = helpers(std::atoi(argv[2]), std::atoi(argv[3]));
     if (what == "many_callers") rc = many_callers();
     if (rc == 2) std::printf("unknown check %s\n", what.c_str());

@@ -46,3 +46,7 @@ def test_helper_threads_by_default(check):
 @pytest.mark.parametrize("asked", ["3", "0"])
 def test_several_threads_copy_at_once(check, asked):
     check("many_callers", COLI_CUDA_COPY_THREADS=asked)
+
+
+def test_transfers_without_pinned_memory(check):
+    check("no_pinned_memory")
