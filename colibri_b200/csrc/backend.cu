@@ -130,6 +130,13 @@ static int reserve_pinned(DeviceCtx *c, float **p, size_t *cap, size_t bytes) {
     *cap = want;
     return 1;
 }
+// Rows that kernels read or write 16 bytes at a time: a caller's pointer that does not lie on such a boundary is refused
+// here, on the GPU it would be a misaligned access.
+static int rows_aligned(const char *call, const void *x, const void *y = nullptr, uintptr_t to = 16) {
+    if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & (to - 1)) == 0) return 1;
+    std::fprintf(stderr, "[CUDA] %s: rows must start on %d-byte boundaries\n", call, (int)to);
+    return 0;
+}
 // Test hook of the reference (c/backend_cuda.cu:1340-1348): COLI_GPU_FAIL_AFTER=N
 // makes every compute entry point report failure after N successful calls.
 static int fault_injected() {
@@ -751,7 +758,8 @@ static void launch_rows(DeviceCtx *c, const ColiCudaTensor *t, float *y, const f
 // y_dev[S,O] = x_dev[S,I] @ W^T for a packed tensor, all on c->stream.
 static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {
     const int nkb = t->I / BLOCK_K;
-    if (S <= 8 && S * t->I <= ROWS_MAX_X && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0) {
+    if (!rows_aligned("linear", x_dev)) return 0;
+    if (S <= 8 && S * t->I <= ROWS_MAX_X) {
         switch (t->mode * 2 + (S > 4)) {
         case SC_ROW * 2: launch_rows<SC_ROW, 1>(c, t, y_dev, x_dev, S); break;
         case SC_ROW * 2 + 1: launch_rows<SC_ROW, 2>(c, t, y_dev, x_dev, S); break;
@@ -765,6 +773,7 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
         c->last_launches++;
         return cuda_ok(cudaGetLastError(), "linear launch");
     }
+    if (!rows_aligned("linear", y_dev)) return 0;
     const int nc = pick_nc(S), rpp = 4 * nc;
     const int npass = (S + rpp - 1) / rpp;
     const int nkpart = pick_nkpart(nkb, (long)npass * (t->O / TILE_ROWS), c->sms);
@@ -1237,8 +1246,7 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
                         ColiCudaTensor *const *downs, const int *rows, int count, int D, int I,
                         int total, int max_rows, int all_packed, float *y_dev, const float *x_dev,
                         const int *bcast_src /* optional: every row reads x row 0 */) {
-    if (all_packed && D % 128 == 0 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(y_dev) & 15) == 0 &&
-        group_tc_ok(gates, ups, downs, count, max_rows, total))
+    if (all_packed && D % 128 == 0 && I % 128 == 0 && group_tc_ok(gates, ups, downs, count, max_rows, total))
         return group_device_tc(c, gates, ups, downs, rows, count, D, I, total, y_dev, x_dev, bcast_src != nullptr);
     if (all_packed) {
         if (!bcast_src && rows) {
@@ -1709,6 +1717,7 @@ extern "C" int coli_cuda_expert_group_dev(ColiCudaTensor *const *gates, ColiCuda
     if (!group_shape_ok(g.data(), u.data(), d.data(), r.data(), (int)g.size(), &device, &D, &I, &total,
                         &max_rows, &all_packed, &any_packed)) return 0;
     if (!all_packed && any_packed) return 0;
+    if (all_packed && !rows_aligned("expert group", x_dev, y_dev)) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
     timing_begin(c);
@@ -1768,7 +1777,8 @@ extern "C" int coli_cuda_ep_plan_dev(int device, const float *x_dev, int m, int 
     DeviceCtx *c = find_ctx(device);
     const int nb = G * slots;
     if (!x_dev || !idx_dev || !keff_dev || !dest_dev || !slot_dev || !counts_dev || !entry_of_dev || !send_dev ||
-        !inexact_dev || m < 1 || K < 1 || K > 31 || E < 1 || G < 1 || slots < 1 || D < 4 || D % 4 || !select_ctx(c)) return 0;
+        !inexact_dev || m < 1 || K < 1 || K > 31 || E < 1 || G < 1 || slots < 1 || D < 4 || D % 4 || !rows_aligned("ep plan", x_dev) ||
+        !rows_aligned("ep plan", send_dev, nullptr, payload_bf16 ? 8 : 16) || !select_ctx(c)) return 0;
     if (!reserve(c, &c->ep_ws, ((size_t)nb + 1 + (size_t)m * K) * sizeof(int))) return 0;
     int *off = static_cast<int *>(c->ep_ws.p), *row_of = off + nb + 1;
     c->chain = false;
@@ -1818,15 +1828,18 @@ extern "C" int coli_cuda_ep_expert_group_dev(ColiCudaTensor *const *gates, ColiC
     if (!group_shape_ok(g.data(), u.data(), d.data(), rows.data(), (int)g.size(), &device, &D, &I, &total,
                         &max_rows, &all_packed, &any_packed)) return 0;
     if (!all_packed && any_packed) return 0;
+    // (raw experts may have D % 4 != 0, which the permuted copies do not take)
+    if (D % 4 || !rows_aligned("ep expert group", y_dev) || !rows_aligned("ep expert group", x_dev, nullptr, x_bf16 ? 4 : 8)) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
     timing_begin(c);
     int ok;
-    if (all_packed && D % 128 == 0 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(y_dev) & 15) == 0 &&
+    if (all_packed && D % 128 == 0 && I % 128 == 0 &&
         group_tc_ok(g.data(), u.data(), d.data(), (int)g.size(), max_rows, total)) {
         ok = group_device_tc(c, g.data(), u.data(), d.data(), rows.data(), (int)g.size(), D, I, total, y_dev, x_dev, 0,
                              rowmap.data(), x_bf16);
     } else {
+        if (!rows_aligned("ep expert group", x_dev, nullptr, x_bf16 ? 8 : 16)) return 0;
         if (!reserve(c, &c->ep_ws, ((size_t)n) * sizeof(int)) || !reserve(c, &c->ep_x, (size_t)n * D * sizeof(float)) ||
             !reserve(c, &c->ep_y, (size_t)n * D * sizeof(float))) return 0;
         int *map_dev = static_cast<int *>(c->ep_ws.p);
@@ -1892,7 +1905,7 @@ static unsigned char *g_noalloc_dev[64];   // device address of the array, per C
 
 extern "C" int coli_cuda_pipe_gemm_noalloc(ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {
     if (fault_injected()) return 0;
-    if (!t || !y_dev || !x_dev || S < 1) return 0;
+    if (!t || !y_dev || !x_dev || S < 1 || !rows_aligned("pipe_gemm_noalloc", x_dev, y_dev)) return 0;
     DeviceCtx *c = find_ctx(t->device);
     if (!select_ctx(c)) return 0;
     if (!t->packed) {

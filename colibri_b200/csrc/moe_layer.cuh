@@ -206,8 +206,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     }
     if (!route_only && g_fused_decode && M <= DEC_MAX_M && r.E <= DEC_MAX_E && r.K <= DEC_MAX_K &&
         L->mode_gu == L->mode_d && r.I <= DEC_MAX_I &&
-        M * r.K + 2 <= DEC_MAX_PASS && c->sms >= DEC_MAX_PASS && c->sms <= 256 &&
-        (reinterpret_cast<uintptr_t>(out_dev) & 15) == 0) {
+        M * r.K + 2 <= DEC_MAX_PASS && c->sms >= DEC_MAX_PASS && c->sms <= 256) {
         // one kernel for the whole layer (moe_decode.cuh)
         DecodeArgs a;
         std::memset(&a, 0, sizeof(a));
@@ -260,7 +259,7 @@ extern "C" int coli_cuda_moe_layer_dev(ColiCudaMoeLayer *L, float *out_dev, cons
                                        const float *logits_dev, int M, int *idx_dev, float *w_dev,
                                        int *keff_dev) {
     if (fault_injected()) return 0;
-    if (!L || !out_dev || !x_dev || M < 1 || M > L->max_rows) return 0;
+    if (!L || !out_dev || !x_dev || M < 1 || M > L->max_rows || !rows_aligned("moe_layer_dev", x_dev, out_dev)) return 0;
     DeviceCtx *c = find_ctx(L->device);
     if (!select_ctx(c) || !layer_route_bufs(L, c, M)) return 0;
     timing_begin(c);

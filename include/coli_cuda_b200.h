@@ -179,6 +179,10 @@ int coli_cuda_expert_group_resident_take(int home_device, const int *devices, in
 
 /* ===================== Part 2: additive entry points ===================== */
 
+/* Device rows (x_dev, y_dev, out_dev) of packed tensors and layers, here and in
+ * coli_cuda_pipe_gemm, start on 16-byte boundaries, as rows of whole allocations do;
+ * other pointers are refused (return 0). */
+
 /* No counterpart in the reference header. A layer handle binds already
  * uploaded expert tensors (E triples, plus an optional shared expert) and the
  * routing rule, so that one call runs the whole MoE layer on the device. */

@@ -88,3 +88,48 @@ def test_upload_source_may_be_reused(be, nbytes):
     assert np.array_equal(got, want.numpy())
     be.pipe_free(0, busy)
     be.pipe_free(0, p)
+
+
+def test_rows_off_their_boundary_are_refused(be):
+    """Device rows that kernels read or write 16 bytes at a time: a pointer between the boundaries is an answer of 0 with the
+    output left alone, where no kernel needs the boundary the call still runs."""
+    import ctypes as C
+    from colibri_b200.backend import Backend
+    from tests.util import upload_qt
+    D, I, E, K, M = 256, 128, 4, 2, 12
+    ex = [[upload_qt(be, t) for t in W.expert_weights(D, I, 4, 32, 60 + e)] for e in range(E)]
+    side = lambda k: Backend.handle_array([e[k] for e in ex])
+    lay = MoeLayer(be, D, I, E, K, [e[0] for e in ex], [e[1] for e in ex], [e[2] for e in ex], 0, 0, max_rows=M)
+    rows = np.array([3] * E, np.int32)
+    i32 = rows.ctypes.data_as(C.POINTER(C.c_int))
+    n = M * D * 4
+    x, y, lg = (be.pipe_alloc(0, n + 64) for _ in range(3))
+    a = np.random.default_rng(0).standard_normal(n // 4 + 16).astype(np.float32)
+    for p in (x, y, lg):
+        assert be.pipe_upload(0, p, a.ctypes.data, n + 64)
+    calls = {
+        "moe_layer_dev": lambda px, py, S: be.moe_layer_dev(lay.handle, py, px, lg + 4, S, None, None, None),
+        "expert_group_dev": lambda px, py, S: be.expert_group_dev(side(0), side(1), side(2), i32, E, py, px),
+        "ep_expert_group_dev": lambda px, py, S: be.ep_expert_group_dev(side(0), side(1), side(2), E, i32, 1, py, px, 0),
+        "pipe_gemm": lambda px, py, S: be.pipe_gemm(ex[0][0], py, px, S),
+        "pipe_gemm_noalloc": lambda px, py, S: be.pipe_gemm_noalloc(ex[0][0], py, px, S),
+    }
+    got = np.empty_like(a)
+    for name, call in calls.items():
+        for S in (2, M):
+            for dx, dy in ((4, 0), (0, 4), (8, 8), (12, 0)):
+                if name == "pipe_gemm" and S == 2 and dx == 0:
+                    continue
+                assert call(x + dx, y + dy, S) == 0, (name, S, dx, dy)
+    assert be.pipe_sync(0) and be.pipe_download(0, y, got.ctypes.data, n + 64) and np.array_equal(got, a)
+    for name, call in calls.items():
+        for S in (2, M):
+            assert call(x + 16, y + 32, S) and be.pipe_sync(0), name
+    assert be.pipe_gemm(ex[0][0], y + 4, x, 2) and be.pipe_sync(0)                 # few rows: results are stored one by one
+    assert be.kernel_status(0) == 0
+    lay.free()
+    for p in (x, y, lg):
+        be.pipe_free(0, p)
+    for e in ex:
+        for h in e:
+            be.tensor_free(h)
