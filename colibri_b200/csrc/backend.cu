@@ -1000,10 +1000,22 @@ static int g_tc_enabled = 1;
 extern "C" void coli_cuda_set_tensor_core(int enabled) { g_tc_enabled = enabled < 0 ? 0 : enabled > 2 ? 2 : enabled; }
 // The streaming kernel's cost grows with the rows (one set of MMAs per 4 rows and block of weights), the tensor-core
 // path's hardly does up to 30 rows per expert, but it starts higher, most of all where a weight takes two fp16
-// terms. Measured, streaming / tensor cores, at a mean of R rows per expert: per-row int4, OLMoE shape R = 2: 101 /
-// 105 us, 4: 129 / 109; MXFP4, DeepSeek-V3 shape R = 1: 841 / 940, 2: 1297 / 1200; grouped int4, OLMoE shape
-// R = 6: 154 / 160, 8: 167 / 161, 12: 255 / 166, DeepSeek-V3 shape R = 2: 1407 / 2390, 4: 2160 / 2797.
-static bool tc_pays(long rows, long experts, int mode) { return rows >= (mode == SC_H16 ? 7 : 2) * experts; }
+// terms (grouped int4), and that in either phase. So the line, as the mean of rows per expert, follows both phases' formats.
+// Measured, streaming / tensor cores in us, layers with random routing (M*K rows over E experts) at D x I 2048 x 1024 (E 64) |
+// 6144 x 2048 (E 64) | 7168 x 2048 (E 256 and a shared expert):
+//   per-row int4          mean 2: 95 / 91 | 275 / 299 | 1209 / 1244     3: 105 / 93 | 326 / 320 | 1538 / 1380
+//   MXFP4                 mean 2: 85 / 93 | 261 / 310 | 1232 / 1299     3: 93 / 95 | 318 / 321 | 1565 / 1447   4: 105 / 97 | 350 / 337 | 1670 / 1411
+//   grouped int4          mean 7: 152 / 148 | 576 / 640 | 2800 / 2858   8: 160 / 148 | 617 / 640 | 2961 / 2872   10: 183 / 150 | 717 / 641 | 3599 / 2903
+//   down grouped int4, gate and up per row    mean 4: 115 / 111 | 385 / 426     5: 140 / 113 | 496 / 429     (gate and up MXFP4: the same within 3 %)
+//   gate and up grouped int4, down per row    mean 5: 138 / 128 | 490 / 533     6: 152 / 128 | 544 / 535     (down MXFP4: the same within 3 %)
+// Smaller layers (1024 x 512) cross half a row to two rows earlier. Groups with unevenly spread rows cross where layers do
+// (2048 x 1024, 128 experts of 6144 x 2048: per-row 3: 95 / 74, 622 / 602; grouped 7: 129 / 127, 1253 / 1202); with the same
+// number of rows for every expert the line lies at the next pass width, 5 or 9 rows.
+static bool tc_pays(long rows, long experts, int mode_gu, int mode_d) {
+    const bool two_gu = mode_gu == SC_H16, two_d = mode_d == SC_H16;
+    const int halves = two_gu && two_d ? 16 : two_gu ? 11 : two_d ? 9 : mode_gu == SC_MX || mode_d == SC_MX ? 6 : 5;
+    return 2 * rows >= halves * experts;
+}
 
 template <int MODE, int PHASE>
 static void launch_tc_one(DeviceCtx *c, const TcArgs &a) {
@@ -1068,7 +1080,7 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
 static int group_tc_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                        ColiCudaTensor *const *downs, int count, int max_rows, int total) {
     if (!g_tc_enabled || max_rows < 2) return 0;
-    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode)) return 0;
+    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode, downs[0]->mode)) return 0;
     for (int e = 0; e < count; e++)
         if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok || gates[e]->mode != gates[0]->mode ||
             ups[e]->mode != gates[0]->mode || downs[e]->mode != downs[0]->mode) return 0;

@@ -341,8 +341,9 @@ void coli_cuda_set_fused_decode(int enabled);
  * tensor-core kernel when every tensor involved is int4 with per-row or fp16-exact
  * group scales, or MXFP4, and D and I are multiples of 128:
  *   1 (default)  when it pays, by the measured crossover with the streaming kernel: a mean
- *                of at least 7 rows per expert of the call for int4 with group scales (two
- *                fp16 terms per weight), 2 for MXFP4 and per-row int4; layer calls count M*K
+ *                of at least 8 rows per expert of the call for int4 with group scales (two
+ *                fp16 terms per weight; 5.5 when only gate and up have them, 4.5 when only
+ *                down has), 3 for MXFP4 and 2.5 for per-row int4; layer calls count M*K
  *                rows over E experts, from 9 rows (fewer are the fused kernel's)
  *   2            whenever the tensors and shapes allow it (tests)
  *   0            never: the streaming kernel takes every size (A/B testing)

@@ -61,3 +61,35 @@ def test_device_plan(be, E, K, M):
             be.tensor_free(t)
     assert np.array_equal(outs[0][1], outs[1][1])
     assert max_rel_err(outs[0][0], outs[1][0]) <= 1e-3 and be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("gu,dn,line", [((2, 0), (2, 0), 2.5), ((7, 0), (7, 0), 3), ((2, 0), (7, 0), 3), ((4, 32), (4, 32), 8),
+                                        ((2, 0), (4, 32), 4.5), ((7, 0), (4, 64), 4.5), ((4, 32), (2, 0), 5.5), ((4, 128), (7, 0), 5.5)])
+def test_rule_looks_at_both_phases(be, oracle, gu, dn, line):
+    """On both sides of the line between the streaming kernel (five launches) and the tensor cores (four), for gate and
+    up in one format and down in another."""
+    import ctypes as C
+    D, I, n = 256, 128, 4
+    rng = np.random.default_rng(int(line * 10) + gu[0])
+    ex = [(rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, D, I, *dn, half=True)) for _ in range(n)]
+    hs = [[upload_qt(be, t) for t in e] for e in ex]
+    be.set_timing(1)
+    try:
+        for total, want in ((int(line * n) - 1, 5), (int(line * n), 4)):
+            if total <= 8:                                                # (the fused kernel takes these when all formats agree)
+                be.set_fused_decode(0)
+            rows = [1, total - 4, 2, 1]
+            x = ((rng.random((total, D)) - 0.5) * 2).astype(np.float32)
+            ok, y = be.run_expert_group([h[0] for h in hs], [h[1] for h in hs], [h[2] for h in hs], rows, x, D)
+            ms, launches = C.c_float(), C.c_int()
+            assert ok and be.last_timing(0, C.byref(ms), C.byref(launches)) and launches.value == want, total
+            off = 0
+            for e, r in zip(ex, rows):
+                assert max_rel_err(y[off:off + r], oracle.expert_mlp(x[off:off + r], *e)) <= 1e-3
+                off += r
+    finally:
+        be.set_timing(0)
+        be.set_fused_decode(3)
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
