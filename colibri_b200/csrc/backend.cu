@@ -585,8 +585,6 @@ extern "C" int coli_cuda_tensor_update(ColiCudaTensor *t, const void *weights, c
 // ---------------------------------------------------------------------------
 // Streaming GEMV launch helpers
 // ---------------------------------------------------------------------------
-typedef void (*GemvKernel)(const GemvSeg *, const GemvCtl *, const __half *, const float *, int *);
-
 template <int MODE, int NC>
 static void launch_one(DeviceCtx *c, const GemvSeg *segs, const GemvCtl *ctl, const __half *bq,
                        const float *bs) {
@@ -791,7 +789,7 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
     const HostSegs *lists[1] = {&hs};
     if (!upload_segs(c, &sl, lists, 1, &c->segs2, S)) return 0;
     int nw = S * nkb;
-    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, S, t->I);
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, S, t->I);
     c->last_launches++;
     if (!run_segs(c, sl, 0, nc, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
     size_t n4 = (size_t)S * t->O / 4;
@@ -1167,7 +1165,7 @@ static int launch_decode(DeviceCtx *c, int mode, DecodeArgs &a, const DecPreset 
     if (!a.act_smem) {
         // x does not fit the kernel's shared memory: split it once here, the kernel reads the fragments
         if (!reserve(c, xq, (size_t)a.M * D * 2 * sizeof(__half)) || !reserve(c, xs, (size_t)a.M * nkb1 * sizeof(float))) return 0;
-        launch_pdl(c, k_prep_rows, (a.M * nkb1 * 32 + 255) / 256, 256, 0, (__half *)xq->p, (float *)xs->p, a.x, nullptr, a.M, D);
+        launch_pdl(c, k_prep_rows, (a.M * nkb1 * 32 + 255) / 256, 256, 0, (__half *)xq->p, (float *)xs->p, a.x, a.M, D);
         c->last_launches++;
     }
     a.xq = (const __half *)xq->p; a.xs = (const float *)xs->p;
@@ -1299,13 +1297,13 @@ static int group_device(DeviceCtx *c, ColiCudaTensor *const *gates, ColiCudaTens
         const HostSegs *lists[2] = {&h1, &h2};
         if (!upload_segs(c, &sl, lists, 2, &c->segs1, total)) return 0;
         int nw = nxrows * nkb1;
-        launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, nullptr, nxrows, D);
+        launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)c->bq.p, (float *)c->bs.p, x_dev, nxrows, D);
         c->last_launches++;
         if (!run_segs(c, sl, 0, nc, (const __half *)c->bq.p, (const float *)c->bs.p)) return 0;
         int nw2 = total * nkb2;
         launch_pdl(c, k_swiglu_prep, (nw2 * 32 + 255) / 256, 256, 0, 
             (__half *)c->hq.p, (float *)c->hs.p, (const float *)c->pg.p, (const float *)c->pu.p, nullptr,
-            total, I, nkp1, nullptr);
+            total, I, nkp1);
         c->last_launches++;
         if (!run_segs(c, sl, 1, nc, (const __half *)c->hq.p, (const float *)c->hs.p)) return 0;
         size_t n4 = (size_t)total * D / 4;
@@ -1969,7 +1967,7 @@ extern "C" int coli_cuda_pipe_gemm_noalloc(ColiCudaTensor *t, float *y_dev, cons
     if (!cuda_ok(cudaMemcpyAsync(seg_dev, &hs.seg, sizeof(GemvSeg), cudaMemcpyHostToDevice, c->stream), "noalloc segment") ||
         !cuda_ok(cudaMemcpyAsync(ctl_dev, &hc, sizeof(GemvCtl), cudaMemcpyHostToDevice, c->stream), "noalloc control")) return 0;
     const int nw = S * nkb;
-    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, bq_dev, bs_dev, x_dev, nullptr, S, t->I);
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, bq_dev, bs_dev, x_dev, S, t->I);
     switch (t->mode) {
     case SC_ROW: launch_mode<SC_ROW>(c, nc, seg_dev, ctl_dev, bq_dev, bs_dev); break;
     case SC_H16: launch_mode<SC_H16>(c, nc, seg_dev, ctl_dev, bq_dev, bs_dev); break;

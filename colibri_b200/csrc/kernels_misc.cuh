@@ -122,7 +122,6 @@ __global__ void k_repack_scales(uint8_t *__restrict__ pk, const void *__restrict
 // significant bits; lo may be subnormal, which tensor cores honour), and store
 // both in B-fragment order: halfs[((grp*2 + hl)*4 + t)*8 + i] for column
 // grp*32 + t*8 + i. The inverse scale goes to bscale[row*nkb + kb].
-// src_row: optional gather (row -> source row).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float block_scale_from_max(float m) {
     // m >= 0. Returns 2^(13 - floor(log2 m)), clamped; 1 for zero / non-finite.
@@ -161,15 +160,13 @@ __device__ __forceinline__ float warp_max(float m) {
 }
 
 __global__ void k_prep_rows(__half *__restrict__ bq, float *__restrict__ bscale,
-                            const float *x, const int *src_row, int nrows,
-                            int K) {
+                            const float *x, int nrows, int K) {
     pdl_enter();
     const int nkb = K / BLOCK_K;
     int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (wid >= nrows * nkb) return;
     int row = wid / nkb, kb = wid - row * nkb;
-    int srow = src_row ? src_row[row] : row;
-    float4 v = *reinterpret_cast<const float4 *>(x + (size_t)srow * K + kb * BLOCK_K + lane * 4);
+    float4 v = *reinterpret_cast<const float4 *>(x + (size_t)row * K + kb * BLOCK_K + lane * 4);
     float m = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     float s = block_scale_from_max(m);
     store_split4(bq + ((size_t)row * nkb + kb) * 256, lane, v, s);
@@ -182,8 +179,7 @@ __global__ void k_prep_rows(__half *__restrict__ bq, float *__restrict__ bscale,
 //   h = g/(1+exp(-g)) * u
 __global__ void k_swiglu_prep(__half *__restrict__ hq, float *__restrict__ hscale,
                               const float *pg, const float *pu,
-                              const int *npos_p, int npos_cap, int I, int nkpart,
-                              float *__restrict__ h_out) {
+                              const int *npos_p, int npos_cap, int I, int nkpart) {
     pdl_enter();
     const int npos = npos_p ? *npos_p : npos_cap;
     const int nkb = I / BLOCK_K;
@@ -203,7 +199,6 @@ __global__ void k_swiglu_prep(__half *__restrict__ hq, float *__restrict__ hscal
     h.y = (gsum.y / (1.0f + expf(-gsum.y))) * usum.y;
     h.z = (gsum.z / (1.0f + expf(-gsum.z))) * usum.z;
     h.w = (gsum.w / (1.0f + expf(-gsum.w))) * usum.w;
-    if (h_out) *reinterpret_cast<float4 *>(h_out + (size_t)pos * I + kb * BLOCK_K + lane * 4) = h;
     float m = warp_max(fmaxf(fmaxf(fabsf(h.x), fabsf(h.y)), fmaxf(fabsf(h.z), fabsf(h.w))));
     float s = block_scale_from_max(m);
     store_split4(hq + ((size_t)pos * nkb + kb) * 256, lane, h, s);
@@ -308,8 +303,9 @@ __global__ void k_combine_rows(float *__restrict__ out, const float *y,
 }
 
 // ---------------------------------------------------------------------------
-// Generic matmul for raw tensors (any fmt 0,1,2,3,4,7, any shape): one warp per
-// output row o and chunk of up to 8 input rows; lanes stride over columns,
+// Generic matmul, for what the row-major kernels leave: f32 rows that are not 16-byte aligned, int4 groups that are not
+// whole groups of 32 columns, and FP8 with a table other than E4M3's own whose rows are not 16-byte aligned. Any
+// shape: one warp per output row o and chunk of up to 8 input rows; lanes stride over columns,
 // products in f32, shuffle reduction. y[s*O+o].
 // ---------------------------------------------------------------------------
 __device__ float d_e4m3_lut[256];     // decode table of fmt 8, set by coli_cuda_fp8_set_lut
@@ -320,22 +316,9 @@ __device__ __forceinline__ float raw_weight(const void *w, const void *sc, int f
     if (fmt == 8)      // ng = 128-column blocks per row; one scale per 128x128 block
         return d_e4m3_lut[static_cast<const uint8_t *>(w)[(size_t)o * I + i]] *
                static_cast<const float *>(sc)[(size_t)(o >> 7) * ng + (i >> 7)];
-    if (fmt == 1)
-        return (float)static_cast<const int8_t *>(w)[(size_t)o * I + i] * static_cast<const float *>(sc)[o];
-    if (fmt == 3) {
-        uint8_t v = static_cast<const uint8_t *>(w)[(size_t)o * ((I + 3) / 4) + (i >> 2)];
-        return (float)(((v >> ((i & 3) * 2)) & 3) - 2) * static_cast<const float *>(sc)[o];
-    }
-    uint8_t v = static_cast<const uint8_t *>(w)[(size_t)o * ((I + 1) / 2) + (i >> 1)];
-    int n = (i & 1) ? (v >> 4) : (v & 15);
-    if (fmt == 2) return (float)(n - 8) * static_cast<const float *>(sc)[o];
-    if (fmt == 4) return (float)(n - 8) * static_cast<const float *>(sc)[(size_t)o * ng + i / gs];
-    // fmt 7
-    int mant = n & 1, ex = (n >> 1) & 3;
-    float mag = ex ? ldexpf(1.0f + 0.5f * (float)mant, ex - 1) : 0.5f * (float)mant;
-    if (n & 8) mag = -mag;
-    uint32_t sb = static_cast<const uint8_t *>(sc)[(size_t)o * ng + i / 32];
-    return mag * __uint_as_float(sb << 23);
+    const uint8_t v = static_cast<const uint8_t *>(w)[(size_t)o * ((I + 1) / 2) + (i >> 1)];      // fmt 4
+    const int n = (i & 1) ? (v >> 4) : (v & 15);
+    return (float)(n - 8) * static_cast<const float *>(sc)[(size_t)o * ng + i / gs];
 }
 
 __global__ void k_generic_matmul(float *__restrict__ y, const float *x, const void *w,

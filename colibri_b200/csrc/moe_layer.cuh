@@ -232,13 +232,13 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     c->last_launches++;
     if (route_only) return cuda_ok(cudaGetLastError(), "route launch");
     int nw = M * nkb1;
-    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)L->xq.p, (float *)L->xs.p, x_dev, nullptr, M, r.D);
+    launch_pdl(c, k_prep_rows, (nw * 32 + 255) / 256, 256, 0, (__half *)L->xq.p, (float *)L->xs.p, x_dev, M, r.D);
     c->last_launches++;
     launch_gemv(c, L->mode_gu, p.nc, bo.seg1, bo.ctl1, (const __half *)L->xq.p, (const float *)L->xs.p);
     long nw2 = (long)p.npos_cap * nkb2;
     launch_pdl(c, k_swiglu_prep, (unsigned)((nw2 * 32 + 255) / 256), 256, 0, 
         (__half *)L->hq.p, (float *)L->hs.p, (const float *)L->pg.p, (const float *)L->pu.p, scal + 1,
-        p.npos_cap, r.I, p.nkp1, nullptr);
+        p.npos_cap, r.I, p.nkp1);
     c->last_launches++;
     launch_gemv(c, L->mode_d, p.nc, bo.seg2, bo.ctl2, (const __half *)L->hq.p, (const float *)L->hs.p);
     size_t n4 = (size_t)M * r.D / 4;

@@ -66,3 +66,44 @@ def test_fp8_nan_byte_propagates(be):
     ok, y = be.run_matmul(box, np.ones((1, I), np.float32), w, s, 8, I, O)
     assert ok and y[0, 0] == 0 and np.isnan(y[0, 1]) and y[0, 2] == I and y[0, 3] == 0
     be.tensor_free(box[0])
+
+
+@pytest.mark.parametrize("I,O", [(256, 64), (272, 33), (1040, 160), (2048, 7), (130, 40), (77, 5)])     # 16-byte rows, and not
+def test_fp8_with_a_table_of_its_own(be, oracle, I, O):
+    """An engine may hand over another decode table than E4M3's; such tensors are multiplied without the conversion
+    instruction. Sums of I f32 terms in any order: 2e-6 of the sum of magnitudes."""
+    rng = np.random.default_rng(I + O)
+    table = (rng.standard_normal(256) * 3).astype(np.float32)
+    codes = rng.integers(0, 256, (O, I)).astype(np.uint8)
+    sc = (0.5 + rng.random((-(-O // 128), -(-I // 128)))).astype(np.float32)
+    scale = np.repeat(np.repeat(sc, 128, 0)[:O], 128, 1)[:, :I].astype(np.float64)
+    own, standard = table[codes].astype(np.float64) * scale, oracle.e4m3_table()
+    box = [None]
+    assert be.fp8_set_lut(table.ctypes.data)
+    try:
+        for S in (1, 7, 8, 9, 20):
+            x = rng.standard_normal((S, I)).astype(np.float32)
+            ok, y = be.run_matmul(box, x, codes, sc, 8, I, O)
+            assert ok
+            mag = np.abs(x).astype(np.float64) @ np.abs(own).T
+            assert np.all(np.abs(y - x.astype(np.float64) @ own.T) <= 2e-6 * mag + 1e-30), S
+    finally:
+        assert be.fp8_set_lut(standard.ctypes.data)
+    std = np.nan_to_num(standard)[codes].astype(np.float64) * scale        # (NaN codes: rows left out)
+    good = ~np.isnan(standard[codes]).any(1)
+    ok, y = be.run_matmul(box, x, None, None, 8, I, O)
+    mag = np.abs(x).astype(np.float64) @ np.abs(std).T
+    assert ok and np.all((np.abs(y - x.astype(np.float64) @ std.T) <= 2e-6 * mag + 1e-30)[:, good])
+    be.tensor_free(box[0])
+
+
+@pytest.mark.parametrize("I,O", [(77, 5), (130, 40), (1030, 9)])
+def test_f32_rows_off_their_boundary(be, I, O):
+    rng = np.random.default_rng(I)
+    w = rng.standard_normal((O, I)).astype(np.float32)
+    for S in (1, 8, 17):
+        box, x = [None], rng.standard_normal((S, I)).astype(np.float32)
+        ok, y = be.run_matmul(box, x, w, None, 0, I, O)
+        mag = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+        assert ok and np.all(np.abs(y - x.astype(np.float64) @ w.astype(np.float64).T) <= 2e-6 * mag + 1e-30)
+        be.tensor_free(box[0])
