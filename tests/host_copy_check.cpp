@@ -150,6 +150,30 @@ static int no_pinned_memory() {
     return 0;
 }
 
+// Rows of a blocking call: pieces of 512 KB, sixteen at most, whole both ways; a call whose kernels failed writes nothing.
+static int row_pieces() {
+    const size_t half = 512u << 10;
+    const struct { size_t bytes; uint64_t pieces; } cases[] = {{1, 1}, {half, 1}, {half + 1, 2}, {16 * half, 16}, {16 * half + 4, 16},
+                                                               {(40u << 20) + 12, 16}};
+    for (const auto &c : cases) {
+        IoPieces io = {};
+        Stream s;
+        const std::vector<char> want = pattern(c.bytes, (unsigned)c.bytes);
+        std::vector<char> src = want, dev(c.bytes, 0), dst(c.bytes, 0x11);
+        const std::vector<char> untouched = dst;
+        void *pin;
+        REQUIRE(cudaMallocHost(&pin, c.bytes) == cudaSuccess);
+        REQUIRE(IoPieces::in(dev.data(), pin, src.data(), c.bytes, &s) == cudaSuccess && s.pushed == c.pieces);
+        src.assign(c.bytes, 0x5A);
+        REQUIRE(io.out_start(pin, dev.data(), c.bytes, &s) == cudaSuccess && s.pushed == 2 * c.pieces);
+        REQUIRE(!io.out_finish(dst.data(), pin, c.bytes, [] { return false; }) && dst == untouched);
+        REQUIRE(io.out_finish(dst.data(), pin, c.bytes, [] { return true; }) && dst == want && dev == want);
+        io.free();
+        cudaFreeHost(pin);
+    }
+    return 0;
+}
+
 static const size_t COPY_SIZES[] = {1, 65536, (1u << 18) - 1, 1u << 18, (1u << 18) + 1, (1u << 20) + 77, (9u << 20) + 3};
 
 // Copies are whole with as many helpers as asked for (argument), as the system grants, or none.
@@ -192,6 +216,7 @@ int main(int argc, char **argv) {
     int rc = 2;
     if (what == "upload_sources") rc = upload_sources();
     if (what == "downloads") rc = downloads();
+    if (what == "row_pieces") rc = row_pieces();
     if (what == "no_pinned_memory") rc = no_pinned_memory();
     if (what == "helpers" && argc > 3) rc = helpers(std::atoi(argv[2]), std::atoi(argv[3]));
     if (what == "many_callers") rc = many_callers();

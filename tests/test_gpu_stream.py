@@ -14,8 +14,11 @@ pytestmark = pytest.mark.gpu
     (256, 128, [1, 4, 5, 8]),
     (256, 128, [8, 1, 9, 3, 1, 1, 2]),               # one expert above 8 rows: two passes
     (384, 256, [16, 17, 3, 32, 8, 33, 12]),          # every width in one launch
-    (4096, 128, [3, 9, 4]),                          # 256 KB of rows: one piece
-    (4096, 128, [5, 9, 3]),                          # and a ragged second one
+    (4096, 128, [3, 9, 4]),                          # host rows in one piece: up to 512 KB, 32 rows of 16 KB
+    (4096, 128, [5, 9, 3]),
+    (4096, 128, [20, 1, 11]),                        # exactly one
+    (4096, 128, [20, 1, 12]),                        # and a second one of a single row
+    (4096, 128, [400, 3, 197]),                      # 9.8 MB: sixteen pieces above 512 KB
 ])
 def test_uneven_group(be, oracle, fmt, gs, half, D, I, rows):
     rng = np.random.default_rng(D + sum(rows) + fmt)
@@ -36,7 +39,8 @@ def test_uneven_group(be, oracle, fmt, gs, half, D, I, rows):
             be.tensor_free(t)
 
 
-@pytest.mark.parametrize("S", [1, 17, 130, 300])     # pulled by a kernel; pieces of 256 KB; 16 larger pieces
+# 16 KB of x a row: pulled by a kernel; one piece; five and ten pieces of 512 KB; sixteen larger ones (above 8 MB)
+@pytest.mark.parametrize("S", [1, 17, 130, 300, 512, 513, 600])
 def test_matmul_rows_in_pieces(be, S):
     I, O = 4096, 4128
     rng = np.random.default_rng(S)

@@ -50,3 +50,7 @@ def test_several_threads_copy_at_once(check, asked):
 
 def test_transfers_without_pinned_memory(check):
     check("no_pinned_memory")
+
+
+def test_rows_of_a_blocking_call_in_pieces(check):
+    check("row_pieces")
