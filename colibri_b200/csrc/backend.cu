@@ -1521,12 +1521,12 @@ extern "C" int coli_cuda_pipe_copy_async(int device, void *dst, const void *src,
 // download behind a kernel whose wait has expired leaves dst alone and returns 0, like every call that waits.
 extern "C" int coli_cuda_pipe_upload(int device, void *dst, const void *src, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
-    if (!select_ctx(c)) return 0;
+    if ((bytes && (!dst || !src)) || !select_ctx(c)) return 0;       // (the host reads src here, the runtime does not look at it first)
     return cuda_ok(upload_staged(&c->up, dst, src, bytes, cudaStreamLegacy), "pipe upload");
 }
 extern "C" int coli_cuda_pipe_download(int device, const void *src, void *dst, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
-    if (!select_ctx(c)) return 0;
+    if ((bytes && (!dst || !src)) || !select_ctx(c)) return 0;
     bool ready = true;
     return cuda_ok(download_staged(&c->up, dst, src, bytes, cudaStreamLegacy, [c, &ready] { return ready = kernels_ok(c) != 0; }),
                    "pipe download") && ready;

@@ -71,6 +71,15 @@ def test_staged_transfers(be, nbytes):
     be.pipe_free(0, p)
 
 
+@pytest.mark.parametrize("nbytes", [4, 100000])
+def test_transfers_without_an_end_are_refused(be, nbytes):
+    p, a = be.pipe_alloc(0, nbytes), np.ones(nbytes // 4, np.float32)
+    assert be.pipe_upload(0, p, None, nbytes) == 0 and be.pipe_upload(0, None, a.ctypes.data, nbytes) == 0
+    assert be.pipe_download(0, p, None, nbytes) == 0 and be.pipe_download(0, None, a.ctypes.data, nbytes) == 0
+    assert be.pipe_upload(0, None, None, 0) == 1 and be.pipe_download(0, None, None, 0) == 1 and np.all(a == 1)
+    be.pipe_free(0, p)
+
+
 @pytest.mark.parametrize("nbytes", [4096, 65536, 3 << 20])
 def test_upload_source_may_be_reused(be, nbytes):
     """A pinned source overwritten right behind the call, while the stream is still busy with earlier work."""
