@@ -11,8 +11,9 @@
 // 16-byte loads; column 2r of an MMA is row r's hi part, 2r+1 its lo part. Weight and activation scales are
 // applied in f32 once per block (grouped formats: per 32 columns).
 // Why: the scalar kernel before it decoded every weight to f32 and multiplied it with 8 rows by
-// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows. This one is
-// bound by HBM / L2 (50 MB there).
+// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows. This one takes
+// 32, 50 MB at 1.6 TB/s: bound by the latency of its loads (a warp multiplies a block with nothing of the next one requested), and
+// 256 CTAs leave some of 148 SMs with two and some with one.
 // Rows need no alignment: without 16-byte rows, words come from two aligned loads and a funnel shift (raw
 // tensors carry 16 spare bytes at the end); columns beyond I are masked.
 #pragma once

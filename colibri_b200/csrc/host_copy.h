@@ -24,6 +24,8 @@
 // that copies 256 KB or more at shorter intervals keeps them awake, on cores its own threads may want:
 // COLI_CUDA_COPY_THREADS=0 turns them off, 1 to 3 sets their number (read once). Without it there are three, or a quarter of the
 // host's hardware threads if that is less. One that the system does not grant is done without.
+// Measured, three helpers / none: a group of 1.5 MB each way back to back 320 / 408 us, in calls 5 ms apart (helpers asleep) 405 to
+// 434 / 416; uploads of 25 MB (one expert) 1150 / 2010, apart 1170 / 2170.
 class CopyPool {
 public:
     static CopyPool &get() {

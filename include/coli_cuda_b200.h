@@ -163,7 +163,8 @@ int coli_cuda_pipe_copy2d(int device, float *dst, int dpitch, const float *src, 
 int coli_cuda_pipe_peer_copy(int dst_dev, float *dst, int src_dev, const float *src, size_t bytes);
 int coli_cuda_pipe_sync(int device);
 /* One decode row routed on the device: sigmoid scores, bias-augmented top-K by
- * strict '>' (lowest index wins), optional top-p, norm, scale; E<=4096, Ksel<=64. */
+ * strict '>' (lowest index wins), optional top-p, norm, scale; Ksel <= 64 and, here,
+ * E <= 1024 (the reference takes 4096): more is refused. */
 int coli_cuda_pipe_router(int device, const float *x_dev, const void *rw_dev, const void *rb_dev,
                           int D, int E, int Ksel, float topp, int norm_topk, float routed_scale,
                           int *idx_host, float *w_host, int *keff_host);
