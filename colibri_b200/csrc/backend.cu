@@ -52,7 +52,6 @@ struct DeviceCtx {
     float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the blocking host-buffer calls
     size_t io_x_cap = 0, io_y_cap = 0;
     bool chain = false;                       // the last thing this call put on the stream is a kernel
-    UploadRing up = {};                       // pinned pieces of large uploads
     IoPieces io = {};                         // events of the pieces of a call's result
     uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
     uint32_t *check_host = nullptr;
@@ -73,6 +72,8 @@ struct DeviceCtx {
 };
 
 static DeviceCtx g_ctx[COLI_CUDA_MAX_DEVICES];
+static UploadRing g_ring[COLI_CUDA_MAX_DEVICES];     // pinned pieces of the device's transfers
+static UploadRing *ring_of(const DeviceCtx *c) { return &g_ring[c - g_ctx]; }
 static int g_nctx = 0;
 static std::mutex g_mu;
 static int g_timing = 0;
@@ -279,7 +280,7 @@ extern "C" void coli_cuda_shutdown(void) {
         if (c->dec_sync) cudaFree(c->dec_sync);
         if (c->check) cudaFree(c->check);
         if (c->check_host) cudaFreeHost(c->check_host);
-        upload_ring_free(&c->up);
+        upload_ring_free(ring_of(c));
         c->io.free();
         if (c->exp_tab_dev) cudaFree(c->exp_tab_dev);
         if (c->ev0) cudaEventDestroy(c->ev0);
@@ -446,21 +447,21 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
             if (sbytes && !cuda_ok(cudaMalloc(&t->raw_s, sbytes), "scale allocation")) return 0;
             t->physical_bytes = wbytes + sbytes;
         }
-        if (!cuda_ok(upload_staged(&c->up, t->raw_w, weights, wbytes, c->stream), "tensor upload")) return 0;
-        if (sbytes && !cuda_ok(upload_staged(&c->up, t->raw_s, scales, sbytes, c->stream), "scale upload")) return 0;
+        if (!cuda_ok(upload_staged(ring_of(c), t->raw_w, weights, wbytes, c->stream), "tensor upload")) return 0;
+        if (sbytes && !cuda_ok(upload_staged(ring_of(c), t->raw_s, scales, sbytes, c->stream), "scale upload")) return 0;
         return cuda_ok(cudaStreamSynchronize(c->stream), "tensor upload sync");
     }
     if (!reserve(c, &c->stage_w, wbytes) || (sbytes && !reserve(c, &c->stage_s, sbytes))) return 0;
     // Scales first: what the storage class depends on is found on the device while the codes travel.
     // Nothing of an existing tensor is overwritten before its new scales have been accepted.
-    if (!cuda_ok(upload_staged(&c->up, c->stage_s.p, scales, sbytes, c->stream), "scale upload")) return 0;
+    if (!cuda_ok(upload_staged(ring_of(c), c->stage_s.p, scales, sbytes, c->stream), "scale upload")) return 0;
     if (t->fmt == 4) {
         cudaMemsetAsync(c->check, 0, 4 * sizeof(uint32_t), c->stream);
         k_check_scales<<<(unsigned)((scount + 1023) / 1024), 256, 0, c->stream>>>(c->check, static_cast<const float *>(c->stage_s.p), scount);
         cudaMemcpyAsync(c->check_host, c->check, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
         cudaEventRecord(c->ev_done, c->stream);
     }
-    if (!cuda_ok(upload_staged(&c->up, c->stage_w.p, weights, wbytes, c->stream), "tensor upload")) return 0;
+    if (!cuda_ok(upload_staged(ring_of(c), c->stage_w.p, weights, wbytes, c->stream), "tensor upload")) return 0;
     if (t->fmt == 7) {
         cudaMemsetAsync(c->check, 0, 4 * sizeof(uint32_t), c->stream);
         k_check_mx<<<(unsigned)((scount + 255) / 256), 256, 0, c->stream>>>(c->check, static_cast<const uint8_t *>(c->stage_w.p),
@@ -882,7 +883,7 @@ static int pull_rows(DeviceCtx *c, void *dst, const void *pinned, size_t bytes) 
 }
 // Rows to the device by way of a pinned buffer of their size, or of the ring where there is none.
 static int rows_in(DeviceCtx *c, void *dst, void *pinned, const void *src, size_t bytes) {
-    return cuda_ok(pinned ? IoPieces::in(dst, pinned, src, bytes, c->stream) : upload_staged(&c->up, dst, src, bytes, c->stream), "input upload");
+    return cuda_ok(pinned ? IoPieces::in(dst, pinned, src, bytes, c->stream) : upload_staged(ring_of(c), dst, src, bytes, c->stream), "input upload");
 }
 // ... and back, once the kernels are known to have done well. rows_out_start only enqueues; the ring's part waits for rows_out_finish.
 static int rows_out_start(DeviceCtx *c, void *pinned, const void *src_dev, size_t bytes) {
@@ -891,7 +892,7 @@ static int rows_out_start(DeviceCtx *c, void *pinned, const void *src_dev, size_
 static int rows_out_finish(DeviceCtx *c, void *dst, void *pinned, const void *src_dev, size_t bytes) {
     if (pinned) return c->io.out_finish(dst, pinned, bytes, [c] { return kernels_ok(c) != 0; });
     bool ready = true;
-    return cuda_ok(download_staged(&c->up, dst, src_dev, bytes, c->stream, [c, &ready] { return ready = kernels_ok(c) != 0; }),
+    return cuda_ok(download_staged(ring_of(c), dst, src_dev, bytes, c->stream, [c, &ready] { return ready = kernels_ok(c) != 0; }),
                    "output download") && ready;
 }
 // -> where the kernels find x, or NULL. read_once: the first kernel reads every element once (not every CTA all of them).
@@ -1522,13 +1523,13 @@ extern "C" int coli_cuda_pipe_copy_async(int device, void *dst, const void *src,
 extern "C" int coli_cuda_pipe_upload(int device, void *dst, const void *src, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if ((bytes && (!dst || !src)) || !select_ctx(c)) return 0;       // (the host reads src here, the runtime does not look at it first)
-    return cuda_ok(upload_staged(&c->up, dst, src, bytes, cudaStreamLegacy), "pipe upload");
+    return cuda_ok(upload_staged(ring_of(c), dst, src, bytes, cudaStreamLegacy), "pipe upload");
 }
 extern "C" int coli_cuda_pipe_download(int device, const void *src, void *dst, size_t bytes) {
     DeviceCtx *c = find_ctx(device);
     if ((bytes && (!dst || !src)) || !select_ctx(c)) return 0;
     bool ready = true;
-    return cuda_ok(download_staged(&c->up, dst, src, bytes, cudaStreamLegacy, [c, &ready] { return ready = kernels_ok(c) != 0; }),
+    return cuda_ok(download_staged(ring_of(c), dst, src, bytes, cudaStreamLegacy, [c, &ready] { return ready = kernels_ok(c) != 0; }),
                    "pipe download") && ready;
 }
 extern "C" int coli_cuda_pipe_rmsnorm_s(int device, float *y_dev, const float *x_dev, const float *w_dev,

@@ -123,21 +123,24 @@ private:
     std::atomic<int> asleep_{0};
 };
 
-// Pinned pieces of one device's transfers, each with the event of the last copy out of it or into it.
+// Pinned pieces of one device's transfers, each with the event of the last copy out of it or into it. A transfer holds the
+// ring from its first piece to its last: a thread that brings experts in and one that runs the model may share a device.
 struct UploadRing {
     static constexpr int N = 4;
     static constexpr size_t PIECE = 2u << 20;
-    char *buf[N];
-    cudaEvent_t ev[N];
-    bool busy[N];
-    int next;
+    char *buf[N] = {};
+    cudaEvent_t ev[N] = {};
+    bool busy[N] = {};
+    int next = 0;
+    std::mutex mu;
 };
 static void upload_ring_free(UploadRing *r) {
     for (int i = 0; i < UploadRing::N; i++) {
         if (r->ev[i]) cudaEventDestroy(r->ev[i]);
         if (r->buf[i]) cudaFreeHost(r->buf[i]);
+        r->ev[i] = nullptr; r->buf[i] = nullptr; r->busy[i] = false;
     }
-    std::memset(r, 0, sizeof(*r));
+    r->next = 0;
 }
 // Buffer i of the ring, pinned on first use. Where the system has no pinned memory left the transfer goes without it, by
 // the driver's own staging: slower, not refused.
@@ -152,6 +155,7 @@ static bool upload_ring_slot(UploadRing *r, int i) {
 // src (any host memory) -> dst (device) on `stream`. The source has been read when the call returns, small ones and
 // pinned ones included: cudaMemcpyAsync straight from a pinned source would return before the copy has run.
 static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    std::lock_guard<std::mutex> hold(r->mu);
     for (size_t off = 0; off < bytes; off += UploadRing::PIECE) {
         const size_t n = bytes - off < UploadRing::PIECE ? bytes - off : UploadRing::PIECE;
         const int i = r->next;
@@ -177,6 +181,7 @@ static cudaError_t upload_staged(UploadRing *r, void *dst, const void *src, size
 template <class Ready>
 static cudaError_t download_staged(UploadRing *r, void *dst, const void *src, size_t bytes, cudaStream_t stream, Ready ready) {
     constexpr size_t STEP = 1u << 20;
+    std::lock_guard<std::mutex> hold(r->mu);
     cudaError_t e;
     size_t out = 0;                             // pieces out: copied to dst
     const size_t np = (bytes + STEP - 1) / STEP;

@@ -16,6 +16,7 @@
 #include <functional>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -30,27 +31,33 @@ struct Event { Stream *s = nullptr; uint64_t at = 0; };
 static std::map<char *, size_t> g_pinned;             // page-locked host ranges
 static int g_pin_budget = 1 << 30;                    // allocations of pinned memory that still succeed
 
+static std::recursive_mutex g_rt;                    // the runtime may be entered by several threads
+#define RT std::lock_guard<std::recursive_mutex> rt(g_rt)
 static bool pinned(const void *p) {
+    RT;
     auto it = g_pinned.upper_bound((char *)p);
     return it != g_pinned.begin() && (--it, (char *)p < it->first + it->second);
 }
 static void drain(Stream *s, uint64_t to) {
+    RT;
     while (s->done < to) { s->ops.front()(); s->ops.pop_front(); s->done++; }
 }
 static cudaError_t cudaMallocHost(void **p, size_t n) {
+    RT;
     if (g_pin_budget-- <= 0) return cudaErrorMemoryAllocation;
     *p = std::malloc(n);
     g_pinned[(char *)*p] = n;
     return cudaSuccess;
 }
 static cudaError_t cudaGetLastError() { return cudaSuccess; }
-static cudaError_t cudaFreeHost(void *p) { g_pinned.erase((char *)p); std::free(p); return cudaSuccess; }
+static cudaError_t cudaFreeHost(void *p) { RT; g_pinned.erase((char *)p); std::free(p); return cudaSuccess; }
 static cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = new Event(); return cudaSuccess; }
 static cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
-static cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { e->s = s; e->at = s->pushed; return cudaSuccess; }
-static cudaError_t cudaEventSynchronize(cudaEvent_t e) { if (e->s) drain(e->s, e->at); return cudaSuccess; }
+static cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { RT; e->s = s; e->at = s->pushed; return cudaSuccess; }
+static cudaError_t cudaEventSynchronize(cudaEvent_t e) { RT; if (e->s) drain(e->s, e->at); return cudaSuccess; }
 static cudaError_t cudaStreamSynchronize(cudaStream_t s) { drain(s, s->pushed); return cudaSuccess; }
 static cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind kind, cudaStream_t s) {
+    RT;
     if (kind == cudaMemcpyHostToDevice && !pinned(src)) {
         auto copy = std::make_shared<std::vector<char>>((const char *)src, (const char *)src + n);
         s->ops.push_back([=] { std::memcpy(dst, copy->data(), n); });
@@ -89,7 +96,7 @@ static const size_t SIZES[] = {1, 4, 4096, 65536, 65537, 300000, (2u << 20), (2u
 
 // The source of an upload, pinned or not, belongs to the caller again when the call returns.
 static int upload_sources() {
-    UploadRing ring = {};
+    UploadRing ring;
     Stream s;
     for (size_t n : SIZES)
         for (int pin = 0; pin < 2; pin++) {
@@ -111,7 +118,7 @@ static int upload_sources() {
 // Downloads arrive whole; one whose kernels failed leaves the destination alone, and what it had under way into the
 // ring's buffers does not reach the transfer after it.
 static int downloads() {
-    UploadRing ring = {};
+    UploadRing ring;
     Stream s;
     for (size_t n : SIZES)
         for (int fine = 0; fine < 2; fine++) {
@@ -131,7 +138,7 @@ static int downloads() {
 // With no or too little pinned memory transfers take another way and are as whole.
 static int no_pinned_memory() {
     for (int budget = 0; budget < UploadRing::N; budget++) {
-        UploadRing ring = {};
+        UploadRing ring;
         Stream s;
         g_pin_budget = budget;
         for (size_t n : SIZES) {
@@ -171,6 +178,32 @@ static int row_pieces() {
         io.free();
         cudaFreeHost(pin);
     }
+    return 0;
+}
+
+// One ring, several threads with streams of their own: nobody's pieces reach another's transfer.
+static int ring_of_several_threads() {
+    UploadRing ring;
+    std::atomic<int> bad{0};
+    std::vector<Stream> streams(4);                   // (the ring's events remember them)
+    std::vector<std::thread> users;
+    for (int c = 0; c < 4; c++)
+        users.emplace_back([&ring, &bad, &streams, c] {
+            Stream &s = streams[c];
+            for (int rep = 0; rep < 40; rep++) {
+                const size_t n = SIZES[(rep + c) % 9];
+                const std::vector<char> want = pattern(n, (unsigned)(n + 17 * c + rep));
+                std::vector<char> dev(n, 0), back(n, 0), src = want;
+                if (upload_staged(&ring, dev.data(), src.data(), n, &s) != cudaSuccess) bad++;
+                src.assign(n, 0x5A);
+                if (download_staged(&ring, back.data(), dev.data(), n, &s, [] { return true; }) != cudaSuccess) bad++;
+                cudaStreamSynchronize(&s);
+                if (dev != want || back != want) bad++;
+            }
+        });
+    for (auto &t : users) t.join();
+    upload_ring_free(&ring);
+    REQUIRE(bad == 0);
     return 0;
 }
 
@@ -216,6 +249,7 @@ int main(int argc, char **argv) {
     int rc = 2;
     if (what == "upload_sources") rc = upload_sources();
     if (what == "downloads") rc = downloads();
+    if (what == "ring_of_several_threads") rc = ring_of_several_threads();
     if (what == "row_pieces") rc = row_pieces();
     if (what == "no_pinned_memory") rc = no_pinned_memory();
     if (what == "helpers" && argc > 3) rc = helpers(std::atoi(argv[2]), std::atoi(argv[3]));

@@ -54,3 +54,7 @@ def test_transfers_without_pinned_memory(check):
 
 def test_rows_of_a_blocking_call_in_pieces(check):
     check("row_pieces")
+
+
+def test_ring_of_several_threads(check):
+    check("ring_of_several_threads")
