@@ -74,6 +74,10 @@ struct DeviceCtx {
 static DeviceCtx g_ctx[COLI_CUDA_MAX_DEVICES];
 static UploadRing g_ring[COLI_CUDA_MAX_DEVICES];     // pinned pieces of the device's transfers
 static UploadRing *ring_of(const DeviceCtx *c) { return &g_ring[c - g_ctx]; }
+// Held by a blocking call from its rows' way in to its result's way out: io_x and io_y are the device's, and layer calls of
+// two threads, or one beside a projection, may meet there.
+static std::mutex g_io_mu[COLI_CUDA_MAX_DEVICES];
+static std::mutex &io_mutex(const DeviceCtx *c) { return g_io_mu[c - g_ctx]; }
 static int g_nctx = 0;
 static std::mutex g_mu;
 static int g_timing = 0;
@@ -933,6 +937,7 @@ extern "C" int coli_cuda_matmul(ColiCudaTensor **tensor, float *y, const float *
     ColiCudaTensor *t = *tensor;
     DeviceCtx *c = find_ctx(t->device);
     if (!select_ctx(c)) return 0;
+    std::lock_guard<std::mutex> hold(io_mutex(c));
     size_t xb = (size_t)S * I * sizeof(float), yb = (size_t)S * O * sizeof(float);
     const float *xd = io_in(c, x, xb, t->packed ? S > 8 : t->fmt != 0);
     float *yd = io_out(c, yb);
@@ -1351,6 +1356,8 @@ static int group_host(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
     size_t xb = (size_t)total * D * sizeof(float);
     // A blocking call may come between issue and take: the issued group's rows stay where no other call puts its own.
     // (The issued rows have to be pinned: up to 8, nothing waits for them here.)
+    std::unique_lock<std::mutex> hold(io_mutex(c), std::defer_lock);
+    if (!async_issue) hold.lock();
     if (!reserve(c, &c->x, xb) || !reserve(c, &c->y, xb)) return 0;
     float *hx, *hy;
     if (async_issue) {
@@ -1428,6 +1435,7 @@ extern "C" int coli_cuda_expert_mlp(ColiCudaTensor *gate, ColiCudaTensor *up, Co
     if (!all_packed && any_packed) return 0;
     DeviceCtx *c = find_ctx(device);
     if (!select_ctx(c)) return 0;
+    std::lock_guard<std::mutex> hold(io_mutex(c));
     size_t xb = (size_t)S * D * sizeof(float);
     const float *xd = io_in(c, x, xb, all_packed && S > DEC_MAX_M);
     float *yd = io_out(c, xb);
@@ -1633,6 +1641,7 @@ extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void 
         Ksel > E || !idx_host || !w_host || !keff_host || !select_ctx(c)) return 0;
     // the selection goes straight to pinned memory where there is some: idx [Ksel] | w [Ksel] | keff
     const size_t sel = (size_t)Ksel * 8 + 4;
+    std::lock_guard<std::mutex> hold(io_mutex(c));
     if (!reserve(c, &c->misc, (size_t)E * 4 + sel)) return 0;
     const bool pinned = reserve_pinned(c, &c->io_y, &c->io_y_cap, sel);
     float *logits = (float *)c->misc.p;

@@ -291,13 +291,16 @@ extern "C" int coli_cuda_moe_layer(ColiCudaMoeLayer *L, float *out, const float 
     const size_t xb = (size_t)M * r.D * sizeof(float), lb = logits ? (size_t)M * r.E * sizeof(float) : 0;
     const size_t rb = (size_t)M * r.K * 8 + (size_t)M * 4;
     if (!reserve(c, &L->x, xb + lb) || !reserve(c, &L->out, xb)) return 0;
-    // Pinned staging: [x | logits] and [out | idx | w | keff]. Decode-sized calls keep a buffer of the layer's own, larger
-    // ones share the device's two, so that a model of many layers does not pin its largest batch once per layer.
+    // Pinned staging: [x | logits] and [out | idx | w | keff]. Decode-sized calls keep a buffer of the layer's own (8 rows of
+    // 7168 take 0.5 MB), larger ones share the device's two, so that a model of many layers does not pin its largest batch
+    // once per layer.
     uint8_t *hp, *ho;
+    std::unique_lock<std::mutex> hold(io_mutex(c), std::defer_lock);
     if (xb + lb + xb + rb <= LAYER_PINNED_MAX) {
         hp = reserve_pinned(c, &L->host_io, &L->host_io_cap, xb + lb + xb + rb) ? reinterpret_cast<uint8_t *>(L->host_io) : nullptr;
         ho = hp ? hp + xb + lb : nullptr;
     } else {
+        hold.lock();
         hp = reserve_pinned(c, &c->io_x, &c->io_x_cap, xb + lb) ? reinterpret_cast<uint8_t *>(c->io_x) : nullptr;
         ho = reserve_pinned(c, &c->io_y, &c->io_y_cap, xb + rb) ? reinterpret_cast<uint8_t *>(c->io_y) : nullptr;
     }

@@ -107,3 +107,37 @@ def test_without_pinned_memory(tmp_path):
     src.write_text(SHIM)
     subprocess.check_call(["gcc", "-D_GNU_SOURCE", "-shared", "-fPIC", "-o", str(lib), str(src), "-ldl"])
     run([1, 7, 40, 300, 3000], LD_PRELOAD=str(lib))
+
+
+def test_layers_of_two_threads(be):
+    """Host-buffer calls of two layers at once, larger than a layer's own staging: each gets its own rows."""
+    import threading
+    import numpy as np
+    from colibri_b200 import workloads as W
+    from colibri_b200.backend import MoeLayer
+    from tests.util import upload_qt
+    D, I, E, K, M = 4096, 128, 96, 1, 48                     # 0.5 rows an expert: the streaming kernel, with the layer's own workspaces
+    ex = [[upload_qt(be, t) for t in W.expert_weights(D, I, 4, 32, 5 + e)] for e in range(8)]
+    side = lambda k: [ex[e % 8][k] for e in range(E)]
+    lays = [MoeLayer(be, D, I, E, K, side(0), side(1), side(2), 0, 0, max_rows=M) for _ in range(2)]
+    rng = np.random.default_rng(0)
+    xs = [rng.standard_normal((M, D)).astype(np.float32) for _ in range(2)]
+    lgs = [rng.standard_normal((M, E)).astype(np.float32) for _ in range(2)]
+    want = [lay(x, lg)[0] for lay, x, lg in zip(lays, xs, lgs)]
+    bad = []
+
+    def work(i):
+        for _ in range(150):
+            if not np.array_equal(lays[i](xs[i], lgs[i])[0], want[i]):
+                bad.append(i)
+    t = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for a in t:
+        a.start()
+    for a in t:
+        a.join()
+    assert not bad and be.kernel_status(0) == 0
+    for lay in lays:
+        lay.free()
+    for e in ex:
+        for h in e:
+            be.tensor_free(h)
