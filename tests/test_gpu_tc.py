@@ -1,10 +1,10 @@
-"""Tensor-core path of the expert group (experts with more than 32 rows: prefill
+"""Tensor-core path of the expert group (prefill
 and batched decode, c/colibri.c:4819-4839 called with S > 1) against the CPU
 oracle and against the streaming kernel on the same inputs.
 
 Bars: max relative error 1e-3 against the oracle (FP32 accumulate on both
 sides); the two GPU kernels agree to the same bar. Row counts sit on both sides
-of the 16-row padding and the 128-row pass size; the kernel's status word must
+of the 16-row padding and of one, two and four passes of 64 rows; the kernel's status word must
 stay clear (no wait guard expired)."""
 import numpy as np
 import pytest
