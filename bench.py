@@ -329,6 +329,11 @@ def run_reference_arm(args):
     cfg = W.CONFIGS[args.workload.split("_")[0]]
     restore_omp_threads()
     cpu = CpuExperts()
+    if cpu.kind != "reference":
+        # the oracle's restatement is this repository's own code: its times are not the reference's
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU kernels are not built (oracle/_ref: its sources "
+                          "were absent at build time)"}), flush=True)
+        return
     L, M = args.layers, args.M
     xs, lgs, biases = host_inputs(cfg, L, M)
     layers_host = host_layers_for(cpu.oracle, cfg, L, lgs, biases)
