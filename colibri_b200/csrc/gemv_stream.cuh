@@ -74,6 +74,9 @@ __global__ void k_expire_wait(int *status) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (!mbar_wait_bounded(smem_u32(&bar), 0)) kstat_set(status, KSTAT_MBAR_TIMEOUT);
 }
+__device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 // 1 in one lane of the (converged) warp: what it guards is issued with uniform operands.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;

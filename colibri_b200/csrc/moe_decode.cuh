@@ -175,9 +175,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 // Grid barrier on one counter. Every barrier adds exactly 256 to it (CTA 0 adds what the
 // others leave), so between launches it is a multiple of 256, also across the wrap of the

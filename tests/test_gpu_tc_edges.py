@@ -93,3 +93,27 @@ def test_rule_looks_at_both_phases(be, oracle, gu, dn, line):
         for h in hs:
             for t in h:
                 be.tensor_free(t)
+
+
+@pytest.mark.parametrize("fmt,gs", [(4, 32), (2, 0), (7, 0)])
+@pytest.mark.parametrize("nrows", [3, 37, 64])
+def test_task_end_over_the_gate_range(be, oracle, fmt, gs, nrows):
+    """The SwiGLU's division away from ordinary gates: denominators from 1 to overflow, gates that are zero or tiny. Row by
+    row against the oracle (f32 on both sides: 1e-3 with the row's own noise floor)."""
+    D, I = 640, 256
+    rng = np.random.default_rng(fmt + nrows)
+    ex = (rand_qt(rng, I, D, fmt, gs, half=True), rand_qt(rng, I, D, fmt, gs, half=True), rand_qt(rng, D, I, fmt, gs, half=True))
+    scale = np.array([1, 40, 1e3, 1e6, 0, 1e-9, 1e-12], np.float32)[np.arange(nrows) % 7]
+    x = (((rng.random((nrows, D)) - 0.5) * 2) * scale[:, None]).astype(np.float32)
+    hs = [upload_qt(be, t) for t in ex]
+    try:
+        be.set_tensor_core(2)
+        ok, y = be.run_expert_group(hs[:1], hs[1:2], hs[2:], [nrows], x, D)
+    finally:
+        be.set_tensor_core(1)
+        for t in hs:
+            be.tensor_free(t)
+    assert ok and be.kernel_status(0) == 0
+    want = oracle.expert_mlp(x, *ex)
+    for s in range(nrows):
+        assert np.all(np.isfinite(y[s])) and max_rel_err(y[s], want[s]) <= 1e-3, (s, float(scale[s]))
