@@ -257,6 +257,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         set_smem(k_expert_gemm_tc<SC_H16, 1>, tc_smem_total(SC_H16)); set_smem(k_expert_gemm_tc<SC_H16, 2>, tc_smem_total(SC_H16));
         set_smem(k_expert_gemm_tc<SC_MX, 1>, tc_smem_total(SC_MX)); set_smem(k_expert_gemm_tc<SC_MX, 2>, tc_smem_total(SC_MX));
         set_smem(k_tc_plan, 33 * ROUTE_MAX_E * (int)sizeof(int));
+        set_smem(k_route_build, ROUTE_BUILD_INTS * ROUTE_MAX_E * (int)sizeof(int));
         if (!cuda_ok(cudaGetLastError(), "kernel attributes")) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
     }
     g_nctx = count;

@@ -227,7 +227,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     bo.pos_of = (int *)L->pos_of.p; bo.uniq = uniq_dev ? uniq_dev : (int *)L->uniq.p;
     bo.nu = nu_dev ? nu_dev : scal; bo.npos = scal + 1; bo.shared_pos0 = scal + 2;
     bo.partG = (float *)L->pg.p; bo.partU = (float *)L->pu.p; bo.partD = (float *)L->pd.p;
-    launch_pdl(c, k_route_build, 1, 1024, (size_t)5 * r.E * sizeof(int), idx_dev, keff_dev, M, r, L->tab, bo, p.rpp,
+    launch_pdl(c, k_route_build, 1, 1024, (size_t)ROUTE_BUILD_INTS * r.E * sizeof(int), idx_dev, keff_dev, M, r, L->tab, bo, p.rpp,
                                                                       p.nkp1, p.nkp2, p.seg_cap);
     c->last_launches++;
     if (route_only) return cuda_ok(cudaGetLastError(), "route launch");

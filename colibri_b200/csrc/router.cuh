@@ -153,127 +153,132 @@ struct BuildOut {
     float *partG, *partU, *partD;
 };
 
-// One CTA. Builds the union, the packed row order (expert-major in union
-// order, rows of an expert in ascending token order) and the segment lists.
-__global__ void k_route_build(const int *idx, const int *keff, int M,
-                              RouteRule rule, LayerTables tab, BuildOut out, int rpp, int nkpart1,
-                              int nkpart2, int seg_cap) {
+// One CTA of 1024 threads. Builds the union (first-appearance order), the packed row order (expert-major in union
+// order, entries of an expert in ascending order) and the segment lists. A warp walks a contiguous slice of the entries; ranks
+// come from match masks and per-warp counts, so no atomics decide an order. Bound by latency, a few dependent round trips:
+// 512 entries of 256 experts in 13 us, where a warp per expert that searched all rows for it, and one thread that summed
+// up the union, took 47. Dynamic shared memory: ROUTE_BUILD_INTS * E ints.
+#define ROUTE_BUILD_INTS 37
+__global__ void __launch_bounds__(1024) k_route_build(const int *idx, const int *keff, int M, RouteRule rule, LayerTables tab,
+                                                      BuildOut out, int rpp, int nkpart1, int nkpart2, int seg_cap) {
     pdl_enter();
     extern __shared__ int sm_build[];
     const int E = rule.E, K = rule.K, D = rule.D, I = rule.I;
-    int *first = sm_build, *cnt = first + E, *base = cnt + E, *uniq = base + E, *passbase = uniq + E;
-    __shared__ int s_nu, s_npass;
-    const int tid = threadIdx.x, nth = blockDim.x;
-    for (int e = tid; e < E; e += nth) { first[e] = 0x7fffffff; cnt[e] = 0; }
-    if (tid == 0) s_nu = 0;
+    int *hist = sm_build, *first = hist + 32 * E, *cnt = first + E, *base = cnt + E, *uniq = base + E, *passbase = uniq + E;
+    __shared__ int s_a[32], s_b[32], s_c[32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n = M * K, slice = ((n + 31) / 32 + 31) & ~31, i0 = warp * slice, i1 = min(n, i0 + slice);
+    for (int e = tid; e < 32 * E; e += 1024) hist[e] = 0;
+    if (tid < E) first[tid] = 0x7fffffff;
     __syncthreads();
-    for (int i = tid; i < M * K; i += nth) {
-        int s = i / K, kk = i - s * K;
-        if (kk < keff[s]) {
-            int e = idx[i];
-            atomicMin(&first[e], i);
-            atomicAdd(&cnt[e], 1);
+    auto entry = [&](int i) { const int s = i / K; return i < i1 && i - s * K < keff[s] ? idx[i] : -1; };
+    // exclusive sums over the CTA's threads of two values, and the totals
+    auto scan = [&](int &a, int &b, int &ta, int &tb) {
+        int pa = a, pb = b;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, pa, d), y = __shfl_up_sync(0xffffffffu, pb, d);
+            if (lane >= d) { pa += x; pb += y; }
         }
+        if (lane == 31) { s_a[warp] = pa; s_b[warp] = pb; }
+        __syncthreads();
+        int wa = s_a[lane], wb = s_b[lane];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, wa, d), y = __shfl_up_sync(0xffffffffu, wb, d);
+            if (lane >= d) { wa += x; wb += y; }
+        }
+        ta = __shfl_sync(0xffffffffu, wa, 31); tb = __shfl_sync(0xffffffffu, wb, 31);
+        a = pa - a + __shfl_sync(0xffffffffu, wa, warp) - s_a[warp];
+        b = pb - b + __shfl_sync(0xffffffffu, wb, warp) - s_b[warp];
+    };
+    int *mine = hist + warp * E;
+    for (int b = i0; b < i1; b += 32) {
+        const int e = entry(b + lane);
+        const unsigned m = __match_any_sync(0xffffffffu, e);
+        if (e >= 0 && lane == __ffs(m) - 1) {
+            if (mine[e] == 0) atomicMin(&first[e], b + lane);
+            mine[e] += __popc(m);
+        }
+        __syncwarp();
     }
     __syncthreads();
-    for (int e = tid; e < E; e += nth) {
-        if (cnt[e] > 0) {
-            int rank = 0;
-            for (int o = 0; o < E; o++) rank += (cnt[o] > 0 && first[o] < first[e]);
-            uniq[rank] = e;
-            atomicAdd(&s_nu, 1);
-        }
+    // union: entry i opens an expert iff it is that expert's first; its place is the number of such entries before it
+    int opens = 0;
+    for (int b = i0; b < i1; b += 32) {
+        const int e = entry(b + lane);
+        opens += __popc(__ballot_sync(0xffffffffu, e >= 0 && first[e >= 0 ? e : 0] == b + lane));
+    }
+    if (lane == 0) s_c[warp] = opens;
+    if (tid < E) {
+        int c = 0;
+        for (int w = 0; w < 32; w++) { const int h = hist[w * E + tid]; hist[w * E + tid] = c; c += h; }
+        cnt[tid] = c;
     }
     __syncthreads();
-    const int nu = s_nu;
-    if (tid == 0) {
-        int pos = 0, np = 0;
-        for (int j = 0; j < nu; j++) {
-            int e = uniq[j];
-            base[e] = pos; passbase[e] = np;
-            pos += cnt[e];
-            np += (cnt[e] + rpp - 1) / rpp;
-        }
-        int shared_pos0 = pos;
-        int np_routed = np;
-        if (tab.sh_gate_pk) { pos += M; np += (M + rpp - 1) / rpp; }
-        if (np > seg_cap) np = seg_cap;   // capacity is sized for the worst case; never exceeded
-        s_npass = np;
-        *out.npos = pos; *out.shared_pos0 = shared_pos0; *out.nu = nu;
-        out.ctl1->nseg = 2 * np; out.ctl1->ntask = 2 * np * (I / TILE_ROWS) * nkpart1; out.ctl1->npos = pos;
-        out.ctl1->tasks_per_seg = (I / TILE_ROWS) * nkpart1;
-        out.ctl2->nseg = np; out.ctl2->ntask = np * (D / TILE_ROWS) * nkpart2; out.ctl2->npos = pos;
-        out.ctl2->tasks_per_seg = (D / TILE_ROWS) * nkpart2;
-        // shared expert segments
-        if (tab.sh_gate_pk) {
-            for (int p = 0; p < (M + rpp - 1) / rpp && np_routed + p < seg_cap; p++) {
-                int sidx = np_routed + p;
-                int r0 = p * rpp, nr = min(rpp, M - r0);
-                GemvSeg *sg_ = &out.seg1[2 * sidx], *su_ = &out.seg1[2 * sidx + 1], *sd_ = &out.seg2[sidx];
-                sg_->w = tab.sh_gate_pk; sg_->rowscale = tab.sh_gate_rs; sg_->out = out.partG;
-                su_->w = tab.sh_up_pk; su_->rowscale = tab.sh_up_rs; su_->out = out.partU;
-                sd_->w = tab.sh_down_pk; sd_->rowscale = tab.sh_down_rs; sd_->out = out.partD;
-                for (int r = 0; r < nr; r++) {
-                    sg_->rowid[r] = r0 + r; su_->rowid[r] = r0 + r; sd_->rowid[r] = shared_pos0 + r0 + r;
-                }
-                sg_->nrows = su_->nrows = sd_->nrows = nr;
-                sg_->pos0 = su_->pos0 = sd_->pos0 = shared_pos0 + r0;
-            }
-        }
+    int at = 0;
+    for (int w = 0; w < 32; w++) { const int o = s_c[w]; at += w < warp ? o : 0; }
+    for (int b = i0; b < i1; b += 32) {
+        const int e = entry(b + lane);
+        const bool op = e >= 0 && first[e] == b + lane;
+        const unsigned m = __ballot_sync(0xffffffffu, op);
+        if (op) uniq[at + __popc(m & ((1u << lane) - 1u))] = e;
+        at += __popc(m);
     }
-    for (int j = tid; j < nu; j += nth) out.uniq[j] = uniq[j];
+    int nu = 0;
+    for (int w = 0; w < 32; w++) nu += s_c[w];
     __syncthreads();
-    // row lists: one warp per union expert
-    const int warp = tid >> 5, lane = tid & 31, nwarps = nth >> 5;
-    for (int j = warp; j < nu; j += nwarps) {
-        int e = uniq[j];
-        int run = 0;
-        for (int s0 = 0; s0 < M; s0 += 32) {
-            int s = s0 + lane, hit = -1;
-            if (s < M) {
-                int ke = keff[s];
-                for (int kk = 0; kk < ke; kk++) if (idx[s * K + kk] == e) { hit = kk; break; }
-            }
-            unsigned mask = __ballot_sync(0xffffffffu, hit >= 0);
-            if (hit >= 0) {
-                int r = run + __popc(mask & ((1u << lane) - 1));
-                int pos = base[e] + r;
-                out.pos_of[s * K + hit] = pos;
-                int sidx = passbase[e] + r / rpp;
-                if (sidx < seg_cap) {
-                    out.seg1[2 * sidx].rowid[r % rpp] = s;
-                    out.seg1[2 * sidx + 1].rowid[r % rpp] = s;
-                    out.seg2[sidx].rowid[r % rpp] = pos;
-                }
-            }
-            run += __popc(mask);
-        }
-        // per-pass constants of this expert
-        int npass = (cnt[e] + rpp - 1) / rpp;
-        for (int p = lane; p < npass; p += 32) {
-            int sidx = passbase[e] + p;
-            if (sidx >= seg_cap) continue;
-            int nr = min(rpp, cnt[e] - p * rpp);
-            GemvSeg *sg_ = &out.seg1[2 * sidx], *su_ = &out.seg1[2 * sidx + 1], *sd_ = &out.seg2[sidx];
-            sg_->w = tab.gate_pk[e]; sg_->rowscale = tab.gate_rs ? tab.gate_rs[e] : nullptr; sg_->out = out.partG;
-            su_->w = tab.up_pk[e]; su_->rowscale = tab.up_rs ? tab.up_rs[e] : nullptr; su_->out = out.partU;
-            sd_->w = tab.down_pk[e]; sd_->rowscale = tab.down_rs ? tab.down_rs[e] : nullptr; sd_->out = out.partD;
-            sg_->nrows = su_->nrows = sd_->nrows = nr;
-            sg_->pos0 = su_->pos0 = sd_->pos0 = base[e] + p * rpp;
-        }
-    }
-    __syncthreads();
-    // shape constants and task offsets of every segment
-    const int np = s_npass;
+    // packed rows and passes before expert number tid of the union
+    const int e = tid < nu ? uniq[tid] : 0, c = tid < nu ? cnt[e] : 0, np = (c + rpp - 1) / rpp;
+    int pos = c, pass = np, npos, npass;
+    scan(pos, pass, npos, npass);
+    if (tid < nu) { base[e] = pos; passbase[e] = pass; out.uniq[tid] = e; }
+    const int nsh = tab.sh_gate_pk ? (M + rpp - 1) / rpp : 0;
+    const int nseg = min(npass + nsh, seg_cap);      // capacity is sized for the worst case; never exceeded
     const int t1 = (I / TILE_ROWS) * nkpart1, t2 = (D / TILE_ROWS) * nkpart2;
-    for (int i = tid; i < 2 * np; i += nth) {
-        GemvSeg *sgm = &out.seg1[i];
-        sgm->O = I; sgm->ntiles = I / TILE_ROWS; sgm->nkb = D / BLOCK_K;
-        sgm->nkpart = nkpart1; sgm->kb_per_part = (D / BLOCK_K) / nkpart1; sgm->task0 = i * t1;
+    if (tid == 0) {
+        const int all = npos + (nsh ? M : 0);
+        *out.npos = all; *out.shared_pos0 = npos; *out.nu = nu;
+        out.ctl1->nseg = 2 * nseg; out.ctl1->ntask = 2 * nseg * t1; out.ctl1->npos = all; out.ctl1->tasks_per_seg = t1;
+        out.ctl2->nseg = nseg; out.ctl2->ntask = nseg * t2; out.ctl2->npos = all; out.ctl2->tasks_per_seg = t2;
     }
-    for (int i = tid; i < np; i += nth) {
-        GemvSeg *sgm = &out.seg2[i];
-        sgm->O = D; sgm->ntiles = D / TILE_ROWS; sgm->nkb = I / BLOCK_K;
-        sgm->nkpart = nkpart2; sgm->kb_per_part = (I / BLOCK_K) / nkpart2; sgm->task0 = i * t2;
+    auto put = [&](int si, int which, const uint8_t *w, const float *rs, int nrows, int pos0) {
+        GemvSeg *sg = which == 2 ? &out.seg2[si] : &out.seg1[2 * si + which];
+        const int O = which == 2 ? D : I, nkb = (which == 2 ? I : D) / BLOCK_K, nkpart = which == 2 ? nkpart2 : nkpart1;
+        sg->w = w; sg->rowscale = rs; sg->out = which == 0 ? out.partG : which == 1 ? out.partU : out.partD;
+        sg->nrows = nrows; sg->pos0 = pos0;
+        sg->O = O; sg->ntiles = O / TILE_ROWS; sg->nkb = nkb; sg->nkpart = nkpart; sg->kb_per_part = nkb / nkpart;
+        sg->task0 = which == 2 ? si * t2 : (2 * si + which) * t1;
+    };
+    if (tid < nu) {
+        const uint8_t *wg = tab.gate_pk[e], *wu = tab.up_pk[e], *wd = tab.down_pk[e];
+        const float *rg = tab.gate_rs ? tab.gate_rs[e] : nullptr, *ru = tab.up_rs ? tab.up_rs[e] : nullptr, *rd = tab.down_rs ? tab.down_rs[e] : nullptr;
+        for (int p = 0; p < np && pass + p < nseg; p++) {
+            const int nr = min(rpp, c - p * rpp), p0 = pos + p * rpp;
+            put(pass + p, 0, wg, rg, nr, p0); put(pass + p, 1, wu, ru, nr, p0); put(pass + p, 2, wd, rd, nr, p0);
+        }
+    }
+    for (int p = tid; p < nsh && npass + p < nseg; p += 1024) {
+        const int si = npass + p, r0 = p * rpp, nr = min(rpp, M - r0);
+        put(si, 0, tab.sh_gate_pk, tab.sh_gate_rs, nr, npos + r0);
+        put(si, 1, tab.sh_up_pk, tab.sh_up_rs, nr, npos + r0);
+        put(si, 2, tab.sh_down_pk, tab.sh_down_rs, nr, npos + r0);
+    }
+    for (int s = tid; s < (nsh ? M : 0); s += 1024) {
+        const int si = npass + s / rpp, r = s % rpp;
+        if (si < nseg) { out.seg1[2 * si].rowid[r] = s; out.seg1[2 * si + 1].rowid[r] = s; out.seg2[si].rowid[r] = npos + s; }
+    }
+    __syncthreads();
+    for (int b = i0; b < i1; b += 32) {
+        const int i = b + lane, s = i / K, e = entry(i);
+        const unsigned m = __match_any_sync(0xffffffffu, e);
+        if (e >= 0) {
+            const int r = mine[e] + __popc(m & ((1u << lane) - 1u)), si = passbase[e] + r / rpp, q = r % rpp;
+            out.pos_of[i] = base[e] + r;
+            if (si < nseg) { out.seg1[2 * si].rowid[q] = s; out.seg1[2 * si + 1].rowid[q] = s; out.seg2[si].rowid[q] = base[e] + r; }
+        }
+        __syncwarp();
+        if (e >= 0 && lane == __ffs(m) - 1) mine[e] += __popc(m);
+        __syncwarp();
     }
 }

@@ -117,3 +117,28 @@ def test_task_end_over_the_gate_range(be, oracle, fmt, gs, nrows):
     want = oracle.expert_mlp(x, *ex)
     for s in range(nrows):
         assert np.all(np.isfinite(y[s])) and max_rel_err(y[s], want[s]) <= 1e-3, (s, float(scale[s]))
+
+
+@pytest.mark.parametrize("E,K,M,topp", [(300, 8, 40, 0.0), (300, 8, 40, 0.6), (1, 1, 33, 0.0), (64, 16, 130, 0.4), (1000, 2, 700, 0.0)])
+def test_segment_lists_of_the_streaming_path(be, E, K, M, topp):
+    """The streaming path's lists (union, rows of an expert, passes) against the tensor-core plan, which is built by other code:
+    more experts than warps, dead entries behind a top-p cut, one expert with all rows, more passes than experts."""
+    cfg = dict(D=128, I=128, E=E, K=K, gating=1, norm_topk=1, shared=True, fmt=7, gs=0)
+    L = W.HostLayerWeights(cfg, 3)
+    up = lambda t: upload_qt(be, t)
+    g, u, d = ([up(t) for t in side] for side in (L.gate, L.up, L.down))
+    sh = tuple(up(t) for t in L.shared)
+    lay = MoeLayer(be, 128, 128, E, K, g, u, d, 1, 1, 2.5, topp, router_bias=L.router_bias, shared=sh, max_rows=M)
+    x, lg = W.activations(M, 128, 1), W.router_logits(M, E, 2, zipf=1.1 if E > 1 else 0.0)
+    outs = []
+    try:
+        for mode in (2, 0):
+            be.set_tensor_core(mode)
+            outs.append(lay(x, lg))
+    finally:
+        be.set_tensor_core(1)
+        lay.free()
+        for t in g + u + d + list(sh):
+            be.tensor_free(t)
+    assert np.array_equal(outs[0][1], outs[1][1]) and np.array_equal(outs[0][3], outs[1][3])
+    assert max_rel_err(outs[0][0], outs[1][0]) <= 1e-3 and be.kernel_status(0) == 0
