@@ -129,7 +129,7 @@ struct DecShared {
     int pos_of[DEC_MAX_M * DEC_MAX_K];
     int keff[DEC_MAX_M];
     DecPass pass[DEC_MAX_PASS];
-    int nu, npass, npos, shared_pos0, failed;
+    int npass, npos, shared_pos0, failed;
     float rowtmp[2 * DEC_MAX_M];
     int rowflag[DEC_MAX_M];
     unsigned long long exp_tab[32];
@@ -474,11 +474,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     // routing scratch inside the partial-sum buffers (dead before the first partial sum is written)
     float *score = reinterpret_cast<float *>(part);                     // [M*E]  (<= 8 KB)
     float *choice = reinterpret_cast<float *>(part + 8192);             // [M*E]
-    int *t_first = reinterpret_cast<int *>(part + 16384);               // [E] each
-    int *t_cnt = t_first + DEC_MAX_E, *t_base = t_cnt + DEC_MAX_E, *t_passbase = t_base + DEC_MAX_E;
-    int *t_uniq = t_passbase + DEC_MAX_E;
-    const uint8_t **ptab = reinterpret_cast<const uint8_t **>(part + 16384 + 5 * DEC_MAX_E * 4);   // [3*E]
-    unsigned long long *wtab = reinterpret_cast<unsigned long long *>(part + 16384 + 5 * DEC_MAX_E * 4 + 3 * DEC_MAX_E * 8) + warp * 32;
+    int *t_e = reinterpret_cast<int *>(part + 16384);                   // [M*K] an entry's expert, or -1
+    int *t_info = t_e + DEC_MAX_M * DEC_MAX_K;                          // [M*K] first entry of its expert | entries << 16 | of these before it << 24
+    const uint8_t **ptab = reinterpret_cast<const uint8_t **>(t_info + DEC_MAX_M * DEC_MAX_K);     // [3*E]
+    unsigned long long *wtab = reinterpret_cast<unsigned long long *>(ptab + 3 * DEC_MAX_E) + warp * 32;
 
     // Programmatic dependent launch (when the host asked for it): let the next kernel of the
     // stream be scheduled onto SMs as this grid's CTAs leave them, and wait here until the
@@ -551,13 +550,11 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     }
     if (tid < 32) sh->zeros[tid] = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
-        sh->failed = 0; sh->nu = 0;
+        sh->failed = 0;
         // one more barrier, behind the warps' own: the SwiGLU activations arriving for the down phase
         mbar_init(smem_u32(smem) + ring_bytes + DEC_WARPS * DEC_BARS_PER_WARP * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-#pragma unroll 1
-    for (int e = tid; e < E; e += blockDim.x) { t_first[e] = 0x7fffffff; t_cnt[e] = 0; }
     wtab[lane] = tab_v;          // this warp's own copy of the table (no CTA-wide wait before the routing)
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
@@ -737,7 +734,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
                 ps.wg = a.tab.sh_gate_pk; ps.wu = a.tab.sh_up_pk; ps.wd = a.tab.sh_down_pk;
                 npass++; spos++;
             }
-            sh->npass = npass; sh->npos = spos; sh->nu = K;
+            sh->npass = npass; sh->npos = spos;
         }
         __syncthreads();
         if (!PRESET && !fast1) route_tail();
@@ -766,7 +763,9 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         if (tid < ke) {
             sh->pos_of[tid] = tid;
             DecPass &ps = sh->pass[tid];
-            ps.e = sh->idx[tid]; ps.rowid[0] = 0; ps.nrows = 1; ps.pos0 = tid;
+            const int e = sh->idx[tid];
+            ps.e = e; ps.rowid[0] = 0; ps.nrows = 1; ps.pos0 = tid;
+            ps.wg = ptab[e]; ps.wu = ptab[E + e]; ps.wd = ptab[2 * E + e];
         }
         if (tid == 0) {
             int npass = ke, spos = ke;
@@ -774,89 +773,85 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
             if (a.tab.sh_gate_pk) {
                 DecPass &ps = sh->pass[npass];
                 ps.e = -1; ps.pos0 = spos; ps.nrows = 1; ps.rowid[0] = 0;
+                ps.wg = a.tab.sh_gate_pk; ps.wu = a.tab.sh_up_pk; ps.wd = a.tab.sh_down_pk;
                 npass++; spos++;
             }
-            sh->npass = npass; sh->npos = spos; sh->nu = ke;
+            sh->npass = npass; sh->npos = spos;
         }
         __syncthreads();
     } else {
+// Eight neighbouring lanes share an entry and compare it with an eighth of the others each. An expert's first entry
+        // stands for its place in the union (first-appearance order): packed rows and passes before it are those of the
+        // experts with an earlier first entry. Two barriers; searching entry by entry with one barrier per table took 6 us at four
+        // rows, this takes 2.
+        const int n = M * K, oct = tid & 7;
+        const int i0 = tid >> 3, step = (DEC_WARPS * 32) / 8;
+        auto live = [&](int i) { const int s = i / K; return i - s * K < sh->keff[s]; };
 #pragma unroll 1
-        for (int i = tid; i < M * K; i += blockDim.x) {
-            int s = i / K, kk = i - s * K;
-            if (kk < sh->keff[s]) { int e = sh->idx[i]; atomicMin(&t_first[e], i); atomicAdd(&t_cnt[e], 1); }
-        }
-        __syncthreads();
-        // union in first-appearance order: entry i opens a new expert iff it is that
-        // expert's first entry; its rank is the number of such entries before it
-#pragma unroll 1
-        for (int i = tid; i < M * K; i += blockDim.x) {
-            int s = i / K, kk = i - s * K;
-            sh->pos_of[i] = (kk < sh->keff[s] && t_first[sh->idx[i]] == i) ? 1 : 0;
-        }
+        for (int q = tid; q < n; q += DEC_WARPS * 32) t_e[q] = live(q) ? sh->idx[q] : -1;
         __syncthreads();
 #pragma unroll 1
-        for (int i = tid; i < M * K; i += blockDim.x) {
-            if (sh->pos_of[i]) {
-                int rank = 0;
-#pragma unroll 1
-                for (int q = 0; q < i; q++) rank += sh->pos_of[q];
-                t_uniq[rank] = sh->idx[i];
-                atomicAdd(&sh->nu, 1);
+        for (int i = i0; i < ((n + 3) & ~3); i += step) {          // (whole warps: four entries each)
+            const int e = i < n ? t_e[i] : -1;
+            int cnt = 0, before = 0, f = DEC_MAX_M * DEC_MAX_K;
+#pragma unroll 2
+            for (int q = oct; q < n; q += 8)
+                if (t_e[q] == e) { cnt++; before += q < i; f = min(f, q); }
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) {
+                cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+                before += __shfl_xor_sync(0xffffffffu, before, off);
+                f = min(f, __shfl_xor_sync(0xffffffffu, f, off));
             }
+            if (oct == 0 && i < n) t_info[i] = e < 0 ? 0xffff : f | (cnt << 16) | (before << 24);
         }
         __syncthreads();
-        const int nu = sh->nu;
 #pragma unroll 1
-        for (int j = tid; j < nu; j += blockDim.x) {
-            int pos = 0, np = 0;
-#pragma unroll 1
-            for (int q = 0; q < j; q++) { int c = t_cnt[t_uniq[q]]; pos += c; np += (c + 3) >> 2; }
-            int e = t_uniq[j];
-            t_base[e] = pos; t_passbase[e] = np;
-            if (j == nu - 1) {
-                int c = t_cnt[e];
-                int spos = pos + c, npass = np + ((c + 3) >> 2);
-                sh->shared_pos0 = spos;
-                if (a.tab.sh_gate_pk) {
-#pragma unroll 1
-                    for (int p = 0; p < (M + 3) / 4; p++) {
-                        DecPass &ps = sh->pass[npass + p];
-                        ps.e = -1; ps.pos0 = spos + 4 * p; ps.nrows = min(4, M - 4 * p);
-#pragma unroll 1
-                        for (int q = 0; q < ps.nrows; q++) ps.rowid[q] = 4 * p + q;
-                    }
-                    npass += (M + 3) / 4; spos += M;
-                }
-                sh->npass = npass; sh->npos = spos;
+        for (int i = i0; i < ((n + 3) & ~3); i += step) {
+            const int me = i < n ? t_info[i] : 0xffff, f = me & 0xffff;
+            int rows = 0, np = 0;                                   // packed rows and passes of the experts before
+#pragma unroll 2
+            for (int q = oct; q < n; q += 8) {
+                const int o = t_info[q], fo = o & 0xffff;
+                if (fo < f) { rows++; np += fo == q ? (((o >> 16) & 255) + 3) >> 2 : 0; }
             }
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int i = tid; i < M * K; i += blockDim.x) {
-            int s = i / K, kk = i - s * K;
-            if (kk < sh->keff[s]) {
-                int e = sh->idx[i], rr = 0;
-#pragma unroll 1
-                for (int s2 = 0; s2 < s; s2++)
-#pragma unroll 1
-                    for (int k2 = 0; k2 < sh->keff[s2]; k2++) rr += (sh->idx[s2 * K + k2] == e);
-#pragma unroll 1
-                for (int k2 = 0; k2 < kk; k2++) rr += (sh->idx[s * K + k2] == e);
-                int pos = t_base[e] + rr;
-                sh->pos_of[i] = pos;
-                DecPass &ps = sh->pass[t_passbase[e] + (rr >> 2)];
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) {
+                rows += __shfl_xor_sync(0xffffffffu, rows, off);
+                np += __shfl_xor_sync(0xffffffffu, np, off);
+            }
+            if (oct == 0 && f != 0xffff) {
+                const int e = t_e[i], cnt = (me >> 16) & 255, rr = (unsigned)me >> 24, s = i / K;
+                sh->pos_of[i] = rows + rr;
+                DecPass &ps = sh->pass[np + (rr >> 2)];
                 ps.rowid[rr & 3] = s;
-                if ((rr & 3) == 0) { ps.e = e; ps.pos0 = pos; ps.nrows = min(4, t_cnt[e] - (rr & ~3)); }
+                if ((rr & 3) == 0) {
+                    ps.e = e; ps.pos0 = rows + rr; ps.nrows = min(4, cnt - rr);
+                    ps.wg = ptab[e]; ps.wu = ptab[E + e]; ps.wd = ptab[2 * E + e];
+                }
             }
         }
-        __syncthreads();
-    }
-    if (!PRESET && !fast1) {
+        // totals: entry n stands behind them all; then the shared expert's passes
+        if (warp == DEC_WARPS - 1) {
+            int rows = 0, np = 0;
 #pragma unroll 1
-        for (int p = tid; p < sh->npass; p += blockDim.x) {
-            DecPass &ps = sh->pass[p];
-            if (ps.e >= 0) { ps.wg = ptab[ps.e]; ps.wu = ptab[E + ps.e]; ps.wd = ptab[2 * E + ps.e]; }
-            else { ps.wg = a.tab.sh_gate_pk; ps.wu = a.tab.sh_up_pk; ps.wd = a.tab.sh_down_pk; }
+            for (int q = lane; q < n; q += 32) {
+                const int o = t_info[q], fo = o & 0xffff;
+                if (fo != 0xffff) { rows++; np += fo == q ? (((o >> 16) & 255) + 3) >> 2 : 0; }
+            }
+            rows = __reduce_add_sync(0xffffffffu, rows); np = __reduce_add_sync(0xffffffffu, np);
+            const bool shared = a.tab.sh_gate_pk != nullptr;
+            if (lane == 0) {
+                sh->shared_pos0 = rows;
+                sh->npos = rows + (shared ? M : 0); sh->npass = np + (shared ? (M + 3) / 4 : 0);
+            }
+            if (shared && lane < (M + 3) / 4) {
+                DecPass &ps = sh->pass[np + lane];
+                ps.e = -1; ps.pos0 = rows + 4 * lane; ps.nrows = min(4, M - 4 * lane);
+#pragma unroll
+                for (int q = 0; q < 4; q++) ps.rowid[q] = 4 * lane + q;
+                ps.wg = a.tab.sh_gate_pk; ps.wu = a.tab.sh_up_pk; ps.wd = a.tab.sh_down_pk;
+            }
         }
         __syncthreads();
     }
