@@ -2,6 +2,8 @@
 and the 64-row pass, contractions that fill a partial sum of four 128-column blocks and ones that
 end inside it, rows with and without fp16 lo terms in one pass, and a layer whose plan is made on
 the device. CPU oracle, max relative error 1e-3."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -142,3 +144,35 @@ def test_segment_lists_of_the_streaming_path(be, E, K, M, topp):
             be.tensor_free(t)
     assert np.array_equal(outs[0][1], outs[1][1]) and np.array_equal(outs[0][3], outs[1][3])
     assert max_rel_err(outs[0][0], outs[1][0]) <= 1e-3 and be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("fmt,gs", [(7, 0)])
+def test_repeated_calls_agree(be, fmt, gs):
+    """The same call again and again while every stage of the kernel's rings is in turn the slowest one (passes of 1 to 64 rows):
+    bit for bit the same rows. A slot that is filled again before its last word was read shows here as a few
+    wrong features of one pass, in one call of thirty."""
+    import torch
+    D, I, n = 6144, 2048, 256
+    rng = np.random.default_rng(fmt)
+    ex = [(rand_qt(rng, I, D, fmt, gs, half=True), rand_qt(rng, I, D, fmt, gs, half=True), rand_qt(rng, D, I, fmt, gs, half=True))
+          for _ in range(2)]
+    lg = W.router_logits(2048, n, 5, zipf=1.1)                     # rows per expert: from 1800 down to one
+    rows = np.maximum(1, np.bincount(np.argsort(-lg, axis=1)[:, :8].ravel(), minlength=n)).astype(np.int32)
+    x = torch.randn((int(rows.sum()), D), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").bfloat16().float()
+    ys = [torch.empty_like(x) for _ in range(2)]
+    hs = [[upload_qt(be, t) for t in ex[e % 2]] for e in range(n)]
+    side = [be.handle_array([h[m] for h in hs]) for m in range(3)]
+    run = lambda y: be.expert_group_dev(*side, rows.ctypes.data_as(C.POINTER(C.c_int)), n, y.data_ptr(), x.data_ptr())
+    try:
+        be.set_tensor_core(2)
+        ok, bad = run(ys[0]), 0
+        for _ in range(80):
+            ok = run(ys[1]) and ok
+            assert be.kernel_status(0) == 0
+            bad += not torch.equal(*ys)
+    finally:
+        be.set_tensor_core(1)
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
+    assert ok and be.kernel_status(0) == 0 and bad == 0
