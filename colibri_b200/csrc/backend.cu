@@ -811,9 +811,11 @@ static void launch_dense(DeviceCtx *c, const ColiCudaTensor *t, float *y, int S,
     const uint8_t *w = static_cast<const uint8_t *>(t->raw_w);
     const size_t rb = row_bytes(t->fmt, t->I);
     const int gs = t->gs > 0 ? t->gs : t->I;
-    if (nc == 1) launch_pdl(c, k_dense_mma<FMT, 1, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
-    else if (nc == 2) launch_pdl(c, k_dense_mma<FMT, 2, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
-    else launch_pdl(c, k_dense_mma<FMT, 4, AL16>, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng);
+    auto go = [&](auto kern) { launch_pdl(c, kern, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng); };
+    if (nc == 1) go(k_dense_mma<FMT, 1, AL16, 2>);
+    else if (nc == 2) go(k_dense_mma<FMT, 2, AL16, 2>);
+    else if ((int)(grid.x * grid.y) > c->sms) go(k_dense_mma<FMT, 4, AL16, 2>);
+    else go(k_dense_mma<FMT, 4, AL16, 1>);
 }
 
 static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {

@@ -11,11 +11,17 @@
 // 16-byte loads; column 2r of an MMA is row r's hi part, 2r+1 its lo part. Weight and activation scales are
 // applied in f32 once per block (grouped formats: per 32 columns).
 // Why: the scalar kernel before it decoded every weight to f32 and multiplied it with 8 rows by
-// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows. This one takes
-// 32, 50 MB at 1.6 TB/s: bound by the latency of its loads (a warp multiplies a block with nothing of the next one requested), and
-// 256 CTAs leave some of 148 SMs with two and some with one.
-// Rows need no alignment: without 16-byte rows, words come from two aligned loads and a funnel shift (raw
-// tensors carry 16 spare bytes at the end); columns beyond I are masked.
+// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows, 24 so (50 MB at 2.1 TB/s). Bound by the
+// latency of its loads (a warp multiplies a block with nothing of the next one requested), and 256 CTAs leave some of 148 SMs with
+// two and some with one.
+// CTAS: CTAs that share an SM. More than 8 rows want 140 to 180 registers a thread, and with one CTA per SM a second wave
+// runs behind the first; so when there are more CTAs than SMs the registers are capped for two (and spill a little: 1 % slower where
+// there are fewer CTAs than SMs, so not there). Call times with that and with the activations' fragments requested before the decoding, before / after, 12 rows of
+// 6144 x 8192: FP8 43 / 33, 2-bit 67 / 42, of 6150 x 8200: grouped int4 116 / 73, MXFP4 90 / 62, per-row int4 102 / 57. Requesting
+// half a block or a block ahead was slower for rows on 16 bytes (FP8 33 / 38), for the registers it takes.
+// Rows need no alignment: without 16-byte rows, words come from aligned loads and funnel shifts, a run of 16 bytes from five (FP8, 6150
+// columns: 12 rows 132 / 50 us, one row 67 / 34, with a pair of loads for every word 72 and 67); raw
+// tensors carry 16 spare bytes at the end; columns beyond I are masked.
 #pragma once
 #include "common.cuh"
 #include "gemv_stream.cuh"
@@ -91,8 +97,8 @@ __device__ __forceinline__ void dense_i2x16(uint32_t q, uint32_t (&v)[8]) {     
     for (int j = 0; j < 8; j++) v[j] = h2_as_u32(__hsub2(u32_as_h2(((q >> (2 * j)) & 0x00030003u) | c_magic_1024), k1026));
 }
 
-template <int FMT, int NC, bool AL16>
-__global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restrict__ y, const __half *bq,
+template <int FMT, int NC, bool AL16, int CTAS>
+__global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__restrict__ y, const __half *bq,
                                                                 const float *bscale, const uint8_t *__restrict__ w,
                                                                 const void *sc, int S, int I, int O, size_t rowb,
                                                                 int gs, int ng) {
@@ -151,8 +157,18 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
                         const uint4 u = k < I ? __ldcs(reinterpret_cast<const uint4 *>(wr[j] + k)) : make_uint4(0, 0, 0, 0);
                         q[j][c * 4] = u.x; q[j][c * 4 + 1] = u.y; q[j][c * 4 + 2] = u.z; q[j][c * 4 + 3] = u.w;
                     } else {
+                        // 16 bytes that start anywhere: five aligned words, of which none starts behind the row
+                        const uintptr_t at = reinterpret_cast<uintptr_t>(wr[j]) + k, end = reinterpret_cast<uintptr_t>(wr[j]) + I;
+                        const uint32_t *pa = reinterpret_cast<const uint32_t *>(at & ~(uintptr_t)3);
+                        uint32_t r[5];
 #pragma unroll
-                        for (int i = 0; i < 4; i++) q[j][c * 4 + i] = word(j, k + i * 4);
+                        for (int i = 0; i < 5; i++) r[i] = reinterpret_cast<uintptr_t>(pa + i) < end ? __ldg(pa + i) : 0;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const int left = I - k - i * 4;        // bytes of the row in this word
+                            q[j][c * 4 + i] = __funnelshift_r(r[i], r[i + 1], (int)(at & 3) * 8) &
+                                              (left >= 4 ? 0xFFFFFFFFu : left <= 0 ? 0u : 0xFFFFFFFFu >> (32 - 8 * left));
+                        }
                     }
                 }
             } else if (FMT == 3) {
@@ -176,6 +192,12 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
         if (RUN16) {
 #pragma unroll
             for (int c = 0; c < 2; c++) {
+                uint4 b[NC][2];                                // all sets' fragments are requested together, before the decoding
+#pragma unroll
+                for (int cs = 0; cs < NC; cs++) {
+                    b[cs][0] = ldg128(bp[cs] + (size_t)kb * 256 + c * 128);
+                    b[cs][1] = ldg128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
+                }
                 uint32_t v[4][8];                              // by row: the run's 16 columns as 8 pairs
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
@@ -190,7 +212,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b0 = ldg128(bp[cs] + (size_t)kb * 256 + c * 128), b1 = ldg128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
+                    const uint4 b0 = b[cs][0], b1 = b[cs][1];
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         mma_f16(bacc[cs][m], v[2 * m][0], v[2 * m + 1][0], v[2 * m][1], v[2 * m + 1][1], b0.x, b0.y);
@@ -208,6 +230,9 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
         } else {
 #pragma unroll
             for (int c = 0; c < 4; c++) {
+                uint4 bf[NC];
+#pragma unroll
+                for (int cs = 0; cs < NC; cs++) bf[cs] = ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
                 uint32_t v[4][4];
                 float sw[4] = {1.f, 1.f, 1.f, 1.f};
                 const int k = k0 + c * 32;
@@ -219,7 +244,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) k_dense_mma(float *__restric
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b = ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
+                    const uint4 b = bf[cs];
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         float acc[4] = {0.f, 0.f, 0.f, 0.f};

@@ -33,3 +33,44 @@ def test_formats_and_shapes(be, fmt, gs, I, O):
         mag = np.abs(x).astype(np.float64) @ np.abs(w).T
         assert np.all(np.abs(y - x.astype(np.float64) @ w.T) <= 2e-6 * mag + 1e-30), (S, fmt)
     assert be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("fmt", [1, 8])
+@pytest.mark.parametrize("I", [1, 3, 15, 17, 63, 66, 127, 250])
+def test_runs_of_bytes_that_start_anywhere(be, fmt, I):
+    """Byte rows of odd lengths: every start of a row within a word, runs of 16 that end inside one, and a last row that ends with
+    the tensor. Same bound as above."""
+    rng = np.random.default_rng(fmt * 1000 + I)
+    t = quantize((rng.standard_normal((37, I)) * 0.02).astype(np.float32), fmt, 0)
+    w = t.dequant().astype(np.float64)
+    for S in (1, 8, 9):
+        x = rng.standard_normal((S, I)).astype(np.float32)
+        box = [None]
+        ok, y = be.run_matmul(box, x, t.w, t.s, fmt, I, 37, gs=0)
+        assert ok
+        be.tensor_free(box[0])
+        mag = np.abs(x).astype(np.float64) @ np.abs(w).T
+        assert np.all(np.abs(y - x.astype(np.float64) @ w.T) <= 2e-6 * mag + 1e-30), S
+    assert be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("fmt,gs,I", [(1, 0, 272), (1, 0, 130), (2, 0, 130), (3, 0, 272), (4, 64, 192), (7, 0, 160), (8, 0, 272), (8, 0, 130)])
+def test_more_tiles_than_sms(be, fmt, gs, I):
+    """More than 8 rows over 151 tiles of 32 outputs: the instance for two CTAs per SM. Same bound as above."""
+    O, S = 4805, 11
+    rng = np.random.default_rng(fmt * 1000 + I)
+    if fmt == 3:
+        codes, sc = rng.integers(0, 4, (O, I)), rng.random(O).astype(np.float32)
+        packed = sum(codes[:, j::4] << (2 * j) for j in range(4)).astype(np.uint8)
+        t, w = QTensor(packed, sc, 3, I, O), (codes - 2.0) * sc[:, None].astype(np.float64)
+    else:
+        t = quantize((rng.standard_normal((O, I)) * 0.02).astype(np.float32), fmt, gs)
+        w = t.dequant().astype(np.float64)
+    x = rng.standard_normal((S, I)).astype(np.float32)
+    box = [None]
+    ok, y = be.run_matmul(box, x, t.w, t.s, fmt, I, O, gs=gs)
+    assert ok
+    be.tensor_free(box[0])
+    mag = np.abs(x).astype(np.float64) @ np.abs(w).T
+    assert np.all(np.abs(y - x.astype(np.float64) @ w.T) <= 2e-6 * mag + 1e-30)
+    assert be.kernel_status(0) == 0
