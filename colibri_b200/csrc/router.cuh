@@ -30,9 +30,10 @@ __device__ __forceinline__ float expf_host_exact(float x) { return coli_expf_exa
 // because an SM takes in about 50 B per cycle and 64 weight rows at once were slower than their chains.
 // A stage of the ring is 256 columns of the CTA's weight rows and of its x row(s) (row stride 260 floats:
 // rows start 16-byte aligned and the 128-bit reads of 8 threads walking different rows do not collide).
-// The products of 64 columns are formed while the additions of the 64 before run: the loads and
-// multiplications fill the chain's gaps. Measured at 256 outputs of 6144 terms: 89 us with 64 outputs
-// per CTA, products before additions and CTA barriers between tiles of 64; 39 us with 16 outputs, the barriers left.
+// The additions run beside the products of the next 16 columns and the loads of those behind them. Measured (cold) at 256
+// outputs of 6144 terms: 89 us with 64 outputs per CTA, products before additions and CTA barriers between tiles of 64; 30 us with 16
+// outputs and copies ahead of the chains, the products of 64 columns formed from loads that the chain waited for; 24 so (2048 outputs of
+// 7168: 35 -> 28). Six cycles an addition, where its latency is four.
 // Two forms: k_router_logits, one copy warp with bulk copies of 256 columns per row and an mbarrier per stage
 // (rows that start 16-byte aligned), and k_router_logits_any, plain loads, for the rest.
 #define ROUTER_STAGES 6
@@ -73,48 +74,52 @@ __global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(flo
         return;
     }
     const int row = tid & (OUT - 1);                    // (lanes beyond OUT repeat a row)
+    // Steps of 16 columns in three stages: while the products of one are added, those of the next are formed and the operands
+    // of the one behind it are on their way, so the chain of additions waits for nothing. (A zero operand, or
+    // a sum that starts with +0, changes no bit of it.)
     float a = 0.f;
-    float4 p[16];                                       // products of the 64 columns before
+    float4 w0[4], x0[4], w1[4], x1[4], p0[4], p1[4];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 16; q++) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < 4; q++) w1[q] = x1[q] = p0[q] = zero;
+    auto load = [](float4 (&w)[4], float4 (&xv)[4], const float4 *wt, const float4 *xt) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) { w[q] = wt[q]; xv[q] = xt[q]; }
+    };
+    auto mul = [](float4 (&p)[4], const float4 (&w)[4], const float4 (&xv)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            p[q] = make_float4(__fmul_rn(xv[q].x, w[q].x), __fmul_rn(xv[q].y, w[q].y), __fmul_rn(xv[q].z, w[q].z), __fmul_rn(xv[q].w, w[q].w));
+    };
+    auto add = [&](const float4 (&p)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
+            a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
+        }
+    };
     bool ok = true;
     for (int t = 0; t < ntile; t++) {
         const int st = t % NS, width = min(TILE, D - t * TILE);
         if (!mbar_wait_bounded(smem_u32(s_full + st), (t / NS) & 1)) ok = false;
         const float4 *wt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2) * OUT + row) * LD);
         const float4 *xt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2 + 1) * OUT + (one_x ? 0 : row)) * LD);
-        for (int c = 0; c < width; c += 64, wt += 16, xt += 16) {
-            const int n4 = min(16, (width - c) >> 2);
-            // (the first round adds the zeros p starts with: the engine's sum starts from zero too)
-            if (n4 == 16) {
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const float4 wv = wt[q], xv = xt[q], old = p[q];
-                    p[q] = make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w));
-                    a = __fadd_rn(a, old.x); a = __fadd_rn(a, old.y);
-                    a = __fadd_rn(a, old.z); a = __fadd_rn(a, old.w);
-                }
-            } else {                                    // the ragged end: nothing stays pending
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
-                    a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
-                    p[q] = make_float4(-0.f, -0.f, -0.f, -0.f);
-                }
-                for (int q = 0; q < n4; q++) {
-                    const float4 wv = wt[q], xv = xt[q];
-                    a = __fadd_rn(a, __fmul_rn(xv.x, wv.x)); a = __fadd_rn(a, __fmul_rn(xv.y, wv.y));
-                    a = __fadd_rn(a, __fmul_rn(xv.z, wv.z)); a = __fadd_rn(a, __fmul_rn(xv.w, wv.w));
-                }
+#pragma unroll 1
+        for (int c = width >> 5; c > 0; c--, wt += 8, xt += 8) {
+            load(w0, x0, wt, xt); mul(p1, w1, x1); add(p0);
+            load(w1, x1, wt + 4, xt + 4); mul(p0, w0, x0); add(p1);
+        }
+        if (width < TILE || t == ntile - 1) {           // the end: what is under way, then up to 28 columns one by one
+            mul(p1, w1, x1); add(p0); add(p1);
+            for (int q = (width & 31) >> 2; q > 0; q--, wt++, xt++) {
+                const float4 wv = *wt, xv = *xt;
+                a = __fadd_rn(a, __fmul_rn(xv.x, wv.x)); a = __fadd_rn(a, __fmul_rn(xv.y, wv.y));
+                a = __fadd_rn(a, __fmul_rn(xv.z, wv.z)); a = __fadd_rn(a, __fmul_rn(xv.w, wv.w));
             }
         }
+        // the tile before has been multiplied: its last operands were in the first products of this one
         __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(s_empty + st)) : "memory");
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-        a = __fadd_rn(a, p[q].x); a = __fadd_rn(a, p[q].y);
-        a = __fadd_rn(a, p[q].z); a = __fadd_rn(a, p[q].w);
+        if (t > 0 && lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(s_empty + (t - 1) % NS)) : "memory");
     }
     if (tid < nrow) logits[i0 + tid] = a;
     if (!ok && lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
