@@ -1652,7 +1652,7 @@ extern "C" int coli_cuda_pipe_router(int device, const float *x_dev, const void 
     float *w = (float *)(idx + Ksel);
     RouteRule rule{D, 0, E, Ksel, 1, norm_topk, routed_scale, topp};
     launch_router(c, logits, x_dev, (const float *)rw_dev, 1, D, E);
-    launch_pdl(c, k_route_topk, 1, ROUTE_THREADS, route_smem(E), logits, (const float *)rb_dev, rule, 1, idx, w, keff);
+    launch_pdl(c, k_route_topk, route_grid(1), ROUTE_THREADS, route_smem(E), logits, (const float *)rb_dev, rule, 1, idx, w, keff);
     if (!cuda_ok(cudaGetLastError(), "pipe router launch") || !check_status(c)) return 0;
     int few[2 * ROUTE_MAX_K + 1];
     if (!pinned && !rows_out_finish(c, few, nullptr, idx, sel)) return 0;

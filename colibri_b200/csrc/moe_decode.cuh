@@ -1210,30 +1210,101 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     }
 }
 
-// Stand-alone routing kernel of the multi-kernel path: one CTA per row (one warp per row took 49 us for
-// 2048 rows of 256 scores), E <= 1024, K <= 64; the same routing function as the fused kernel. Dynamic shared
-// memory: 2 * E floats.
-#define ROUTE_THREADS 128
+// Stand-alone routing kernel of the multi-kernel path: a warp per row, E <= 1024, K <= 64. Scores as in the fused kernel (the
+// softmax denominator is the engine's serial sum), then the engine's K passes of "largest untaken by strict '>', lowest index
+// wins ties" as they are: a pass is E / 32 comparisons a lane and two warp reductions, on the value as an ordered integer
+// (a zero of either sign is the same value) and on the index. Bound by the latency of these passes. Ranking every
+// candidate against all others with a CTA per row took 44 us for 2048 rows of 256 scores and 14 for one row, this 13 for either
+// (cold). Dynamic shared memory: route_smem(E).
+#define ROUTE_WARPS 4
+#define ROUTE_THREADS (ROUTE_WARPS * 32)
+__host__ __device__ inline int route_row_floats(int E) { return 2 * ((E + 3) & ~3) + 2 * ROUTE_MAX_K; }
+static inline size_t route_smem(int E) { return (size_t)ROUTE_WARPS * route_row_floats(E) * sizeof(float); }
+static inline unsigned route_grid(int M) { return (unsigned)((M + ROUTE_WARPS - 1) / ROUTE_WARPS); }
 __global__ void __launch_bounds__(ROUTE_THREADS) k_route_topk(const float *logits, const float *bias,
                                                               RouteRule rule, int M, int *__restrict__ idx_out,
                                                               float *__restrict__ w_out, int *__restrict__ keff_out) {
-    pdl_enter();
     extern __shared__ __align__(16) float sm_route[];
     __shared__ unsigned long long s_tab[32];
-    __shared__ RouteRule s_rule;
-    __shared__ float s_tmp[2 * DEC_MAX_M], s_wk[ROUTE_MAX_K];
-    __shared__ int s_flag[DEC_MAX_M], s_idx[ROUTE_MAX_K], s_keff[1];
-    const int s = blockIdx.x, tid = threadIdx.x, E = rule.E, K = rule.K;
-    if (tid < 32) s_tab[tid] = c_exp2_tab[tid];
-    if (tid == 0) s_rule = rule;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.x * ROUTE_WARPS + warp, E = rule.E, K = rule.K;
+    if (threadIdx.x < 32) s_tab[lane] = c_exp2_tab[lane];
     __syncthreads();
-    // E rounded up to 4: the second array starts 16-byte aligned too
-    route_rows_cta(logits + (size_t)s * E, bias, s_rule, 1, sm_route, sm_route + ((E + 3) & ~3), s_tmp, s_flag, s_idx, s_wk, s_keff,
-                   reinterpret_cast<const uint64_t *>(s_tab));
-    for (int kk = tid; kk < K; kk += ROUTE_THREADS) {
-        idx_out[(size_t)s * K + kk] = s_idx[kk];
-        w_out[(size_t)s * K + kk] = s_wk[kk];
+    pdl_enter();
+    if (s >= M) return;
+    float *sc = sm_route + (size_t)warp * route_row_floats(E), *ch = sc + ((E + 3) & ~3), *w = ch + ((E + 3) & ~3);
+    int *ix = reinterpret_cast<int *>(w + ROUTE_MAX_K);
+    const uint64_t *tab = reinterpret_cast<const uint64_t *>(s_tab);
+    const float *z = logits + (size_t)s * E;
+    if (rule.gating == 0) {
+        float m = -1e30f;
+        for (int e = lane; e < E; e += 32) { const float v = z[e]; ch[e] = v; if (v > m) m = v; }
+#pragma unroll
+        for (int off = 16; off; off >>= 1) { const float o = __shfl_xor_sync(0xffffffffu, m, off); if (o > m) m = o; }
+#pragma unroll 4
+        for (int e = lane; e < E; e += 32) sc[e] = coli_expf_exact(__fsub_rn(ch[e], m), tab);
+        __syncwarp();
+        float tot = 0.f;             // the engine's serial ascending sum, by every lane
+        int e = 0;
+#pragma unroll 4
+        for (; e + 4 <= E; e += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(sc + e);
+            tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, v.x), v.y), v.z), v.w);
+        }
+        for (; e < E; e++) tot = __fadd_rn(tot, sc[e]);
+        __syncwarp();
+        for (e = lane; e < E; e += 32) { const float p = __fdiv_rn(sc[e], tot); sc[e] = p; ch[e] = p; }
+    } else {
+#pragma unroll 4
+        for (int e = lane; e < E; e += 32) {
+            const float sg = __fdiv_rn(1.f, __fadd_rn(1.f, coli_expf_exact(-z[e], tab)));
+            sc[e] = sg;
+            ch[e] = bias ? __fadd_rn(sg, bias[e]) : sg;
+        }
     }
-    if (tid == 0) keff_out[s] = s_keff[0];
+    for (int kk = 0; kk < K; kk++) {
+        int best = -1;
+        float bv = -1e30f;
+#pragma unroll 8
+        for (int e = lane; e < E; e += 32) { const float c = ch[e]; if (c > bv) { bv = c; best = e; } }       // (own elements only)
+        const uint32_t u = __float_as_uint(__fadd_rn(bv, 0.f)), key = best < 0 ? 0u : u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+        best = (int)__reduce_min_sync(0xffffffffu, best >= 0 && key == top ? (uint32_t)best : 0x7fffffffu);
+        if (best == 0x7fffffff) best = kk < E ? kk : 0;
+        if ((best & 31) == lane) { ix[kk] = best; w[kk] = sc[best]; ch[best] = __uint_as_float(0x7fc00000u); }
+    }
+    __syncwarp();
+    int Ke = K;
+    if (rule.gating == 1 && rule.topp > 0.f && rule.topp < 1.f) {
+        if (lane == 0) {
+            for (int a = 1; a < K; a++) {
+                int ii = ix[a]; float ww = w[a]; int b = a - 1;
+                while (b >= 0 && w[b] < ww) { w[b + 1] = w[b]; ix[b + 1] = ix[b]; b--; }
+                w[b + 1] = ww; ix[b + 1] = ii;
+            }
+            float tot = 1e-20f;
+            for (int kk = 0; kk < K; kk++) tot = __fadd_rn(tot, w[kk]);
+            float cum = 0.f;
+            for (int kk = 0; kk < K; kk++) {
+                cum = __fadd_rn(cum, w[kk]);
+                if (cum >= __fmul_rn(rule.topp, tot)) { Ke = kk + 1; break; }
+            }
+        }
+        Ke = __shfl_sync(0xffffffffu, Ke, 0);
+        __syncwarp();
+    }
+    float sm = 0.f;                  // by every lane, like the sum above
+    if (rule.norm_topk) {
+        for (int kk = 0; kk < Ke; kk++) sm = __fadd_rn(sm, w[kk]);
+        if (rule.gating == 1) sm = __fadd_rn(sm, 1e-20f);
+    }
+    for (int kk = lane; kk < K; kk += 32) {
+        float v = w[kk];
+        if (kk < Ke) {
+            if (rule.norm_topk) v = __fdiv_rn(v, sm);
+            if (rule.gating == 1) v = __fmul_rn(v, rule.routed_scale);
+        }
+        idx_out[(size_t)s * K + kk] = ix[kk];
+        w_out[(size_t)s * K + kk] = v;
+    }
+    if (lane == 0) keff_out[s] = Ke;
 }
-static inline size_t route_smem(int E) { return (size_t)2 * ((E + 3) & ~3) * sizeof(float); }

@@ -216,7 +216,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
         a.M = M;
         return launch_decode(c, L->mode_gu, a, nullptr, p.npos_cap, &L->xq, &L->xs, &L->hq, &L->hs, &L->pd);
     }
-    launch_pdl(c, k_route_topk, M, ROUTE_THREADS, route_smem(r.E), lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
+    launch_pdl(c, k_route_topk, route_grid(M), ROUTE_THREADS, route_smem(r.E), lg, L->router_bias, r, M, idx_dev, w_dev, keff_dev);
     c->last_launches++;
     if (use_tc)
         return layer_run_tc(L, c, out_dev, x_dev, M, idx_dev, w_dev, keff_dev);
@@ -373,7 +373,7 @@ extern "C" int coli_cuda_route_topk_dev(int device, const float *logits_dev, con
     if (!logits_dev || !idx_dev || !w_dev || !keff_dev || M < 1 || E < 1 || E > ROUTE_MAX_E || K < 1 ||
         K > ROUTE_MAX_K || K > E || !select_ctx(c)) return 0;
     RouteRule r{0, 0, E, K, gating, norm_topk, routed_scale, topp};
-    launch_pdl(c, k_route_topk, M, ROUTE_THREADS, route_smem(E), logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
+    launch_pdl(c, k_route_topk, route_grid(M), ROUTE_THREADS, route_smem(E), logits_dev, bias_dev, r, M, idx_dev, w_dev, keff_dev);
     c->last_launches++;
     return cuda_ok(cudaGetLastError(), "route launch");
 }

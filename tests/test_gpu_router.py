@@ -160,3 +160,46 @@ def test_expert_counts_that_are_not_multiples_of_four(be, oracle, E, K, M, gatin
     assert be.kernel_status(0) == 0
     lay.free()
     free_layer(be, (g, u, d, sh))
+
+
+@pytest.mark.parametrize("E,K", [(1, 1), (31, 31), (64, 8), (256, 8), (257, 16), (1000, 64), (1024, 1)])
+@pytest.mark.parametrize("gating,topp", [(0, 0.0), (1, 0.0), (1, 0.5)])
+def test_selection_passes_at_their_limits(be, oracle, E, K, gating, topp):
+    """The stand-alone routing kernel on rows that decide by the rule itself: ties across lanes, zeros of both signs, NaN and
+    infinities, every candidate below the starting value. Indices and weights are those of the oracle, bit for bit."""
+    rng = np.random.default_rng(E * 10 + K)
+    lg = rng.standard_normal((11, E), dtype=np.float32)
+    lg[1] = 0.25
+    lg[2] = np.round(lg[2])
+    lg[3, ::2] = np.nan
+    lg[4] = np.nan
+    lg[5, : E // 2] = -np.inf
+    lg[6, E // 2] = np.inf
+    lg[7] = -1e30 if gating == 0 else 200.0
+    bias = (rng.standard_normal(E) * 0.05).astype(np.float32)
+    bias[: E // 3] = -np.float32(1.0) / (np.float32(1.0) + np.exp(np.float32(-0.25)))      # sums of zero where the score is that
+    M = len(lg)
+    bufs = {}
+    for name, a in (("lg", lg), ("bias", bias), ("idx", np.zeros((M, K), np.int32)), ("w", np.zeros((M, K), np.float32)),
+                    ("keff", np.zeros(M, np.int32))):
+        bufs[name] = (be.pipe_alloc(0, max(a.nbytes, 16)), a)
+        assert be.pipe_upload(0, bufs[name][0], a.ctypes.data, a.nbytes)
+    p = lambda n: bufs[n][0]
+    assert be.route_topk_dev(0, p("lg"), p("bias") if gating else None, M, E, K, gating, 1, 2.5, topp, p("idx"), p("w"), p("keff"))
+    for n in ("idx", "w", "keff"):
+        assert be.pipe_download(0, p(n), bufs[n][1].ctypes.data, bufs[n][1].nbytes)
+        be.pipe_free(0, p(n))
+    idx, w, keff = (bufs[n][1] for n in ("idx", "w", "keff"))
+    if gating:
+        oi, ow, ok_, _ = oracle.route_sigmoid(lg, bias, K, topp, True, 2.5)
+    else:
+        oi, ow, _ = oracle.route_softmax(lg, K, True)
+        ok_ = np.full(M, K, np.int32)
+    assert np.array_equal(keff, ok_)
+    for s in range(M):
+        k = keff[s]
+        assert np.array_equal(idx[s, :k], oi[s, :k]), s
+        same = w[s, :k].view(np.uint32) == ow[s, :k].view(np.uint32)
+        assert np.all(same | (np.isnan(w[s, :k]) & np.isnan(ow[s, :k]))), s
+    be.pipe_free(0, p("lg"))
+    be.pipe_free(0, p("bias"))
