@@ -55,7 +55,7 @@ sys.path.insert(0, ROOT)
 from colibri_b200 import workloads as W  # noqa: E402
 from colibri_b200.quant import QTensor  # noqa: E402
 
-TC_MEAN_ROWS = {4: 8, 2: 2.5, 7: 3}    # the backend's rule for layer calls of more than 8 rows: mean rows per expert by format
+TC_MEAN_ROWS = {4: 8, 2: 3, 7: 4}    # the backend's rule for layer calls of more than 8 rows and experts of a million weights a matrix and more: mean rows per expert by format
 ROUTED_SCALE = 2.5    # sigmoid-gated configurations (GLM / DeepSeek-V3 style)
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the fused decode kernel (one ncu
 # capture of configuration 2 at M=1); other workloads have no capture and report null

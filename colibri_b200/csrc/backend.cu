@@ -1005,23 +1005,32 @@ static int group_shape_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
 // 0: never; 1: when it pays (tc_pays); 2: whenever the tensors and shapes allow it (tests).
 static int g_tc_enabled = 1;
 extern "C" void coli_cuda_set_tensor_core(int enabled) { g_tc_enabled = enabled < 0 ? 0 : enabled > 2 ? 2 : enabled; }
-// The streaming kernel's cost grows with the rows (one set of MMAs per 4 rows and block of weights), the tensor-core
-// path's hardly does up to 30 rows per expert, but it starts higher, most of all where a weight takes two fp16
-// terms (grouped int4), and that in either phase. So the line, as the mean of rows per expert, follows both phases' formats.
-// Measured, streaming / tensor cores in us, layers with random routing (M*K rows over E experts) at D x I 2048 x 1024 (E 64) |
-// 6144 x 2048 (E 64) | 7168 x 2048 (E 256 and a shared expert):
-//   per-row int4          mean 2: 95 / 91 | 275 / 299 | 1209 / 1244     3: 105 / 93 | 326 / 320 | 1538 / 1380
-//   MXFP4                 mean 2: 85 / 93 | 261 / 310 | 1232 / 1299     3: 93 / 95 | 318 / 321 | 1565 / 1447   4: 105 / 97 | 350 / 337 | 1670 / 1411
-//   grouped int4          mean 7: 152 / 148 | 576 / 640 | 2800 / 2858   8: 160 / 148 | 617 / 640 | 2961 / 2872   10: 183 / 150 | 717 / 641 | 3599 / 2903
-//   down grouped int4, gate and up per row    mean 4: 115 / 111 | 385 / 426     5: 140 / 113 | 496 / 429     (gate and up MXFP4: the same within 3 %)
-//   gate and up grouped int4, down per row    mean 5: 138 / 128 | 490 / 533     6: 152 / 128 | 544 / 535     (down MXFP4: the same within 3 %)
-// Smaller layers (1024 x 512) cross half a row to two rows earlier. Groups with unevenly spread rows cross where layers do
-// (2048 x 1024, 128 experts of 6144 x 2048: per-row 3: 95 / 74, 622 / 602; grouped 7: 129 / 127, 1253 / 1202); with the same
-// number of rows for every expert the line lies at the next pass width, 5 or 9 rows.
-static bool tc_pays(long rows, long experts, int mode_gu, int mode_d) {
+// The streaming kernel's cost grows with the rows (one set of MMAs per 4 rows and block of weights, and a wider pass for all from a
+// mean of 4 in layers), the tensor-core path's hardly does up to 30 rows per expert, but it starts higher, most of all where a
+// weight takes two fp16 terms (grouped int4), and that in either phase. So the line, as the mean of rows per expert, follows both phases'
+// formats. Measured, streaming / tensor cores in us, layers with random routing (M*K rows over E experts) at D x I
+// 2048 x 1024 (E 64) | 6144 x 2048 (E 64) | 7168 x 2048 (E 256 and a shared expert):
+//   per-row int4          mean 2.5: 80 / 82 | 261 / 275 | 1128 / 1121     3: 84 / 82 | 279 / 281 | 1341 / 1307     4: 89 / 83 | 310 / 296 | 1522 / 1352
+//   MXFP4                 mean 3: 80 / 83 | 268 / 286 | 1306 / 1353     4: 85 / 83 | 299 / 306 | 1440 / 1383
+//   grouped int4          mean 4: 92 / 109 | 334 / 452 | 1557 / 2093     4.5: 112 / 110 | 431 / 452 | 2029 / 1943     5: 118 / 109 | 455 / 452 | 2236 / 2002
+//   down grouped int4, gate and up per row    mean 4: 90 / 92 | 320 / 347 | 1530 / 1592     4.5: 112 / 92 | 420 / 347 | 2055 / 1463
+//   gate and up grouped int4, down per row    mean 4: 92 / 101 | 328 / 402 | 1525 / 1882     4.5: 113 / 101 | 430 / 401 | 2024 / 1722
+// Layers of less than TC_SMALL weights a matrix are short of launches rather than of work and cross later (1024 x 512, E 64: per
+// row 4: 46 / 50, 4.5: 55 / 50; grouped 5: 56 / 57, 6: 61 / 58).
+// Groups of experts with unevenly spread rows widen single passes instead of all (24 experts, 2048 x 1024 | 6144 x 2048): per-row 2.5:
+// 42 / 42 | 118 / 137, 3: 43 / 42 | 144 / 138; MXFP4 3: 42 / 43 | 140 / 139, 4: 42 / 44 | 150 / 140; grouped 5: 48 / 56 | 174 / 211, 6: 63 / 56 |
+// 232 / 209; down grouped 5: 47 / 50 | 161 / 162, 6: 61 / 49 | 220 / 159; gate and up grouped 5: 48 / 52 | 164 / 186, 6: 63 / 52 | 225 / 191. Small
+// ones take the same 22 us on either side of their line (256 x 128).
+// Grouped int4 has its line above where the times cross. Its products fill the accumulator, which truncates: against 64 bits an
+// expert of 2048 x 1024 is off by 2.9e-6 on the tensor cores and by 1.5e-7 in the streaming kernel (per-row int4 2.2e-7 | 1.3e-7, MXFP4
+// 2.6e-7 | 1.1e-7: few bits a product, most sums exact). A call is not taken there for less than a good part of its time.
+#define TC_SMALL (1L << 20)
+static bool tc_pays(long rows, long experts, int mode_gu, int mode_d, bool layer, long weights) {
     const bool two_gu = mode_gu == SC_H16, two_d = mode_d == SC_H16;
-    const int halves = two_gu && two_d ? 16 : two_gu ? 11 : two_d ? 9 : mode_gu == SC_MX || mode_d == SC_MX ? 6 : 5;
-    return 2 * rows >= halves * experts;
+    const int kind = two_gu && two_d ? 2 : two_gu ? 4 : two_d ? 3 : mode_gu == SC_MX || mode_d == SC_MX ? 1 : 0;
+    // half rows: per-row int4, MXFP4, grouped int4, only down grouped, only gate and up grouped
+    static const int halves[2][2][5] = {{{5, 6, 16, 9, 11}, {6, 7, 16, 11, 12}}, {{9, 9, 16, 9, 11}, {6, 8, 16, 9, 11}}};
+    return 2 * rows >= (long)halves[layer][weights >= TC_SMALL][kind] * experts;
 }
 
 template <int MODE, int PHASE>
@@ -1087,7 +1096,7 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
 static int group_tc_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                        ColiCudaTensor *const *downs, int count, int max_rows, int total) {
     if (!g_tc_enabled || max_rows < 2) return 0;
-    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode, downs[0]->mode)) return 0;
+    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode, downs[0]->mode, false, (long)gates[0]->I * gates[0]->O)) return 0;
     for (int e = 0; e < count; e++)
         if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok || gates[e]->mode != gates[0]->mode ||
             ups[e]->mode != gates[0]->mode || downs[e]->mode != downs[0]->mode) return 0;

@@ -175,7 +175,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     const LayerPlan p = layer_plan(L, c, M);
     const int nkb1 = r.D / BLOCK_K, nkb2 = r.I / BLOCK_K;
     bool use_tc = !route_only && !uniq_dev && L->tc_ok && M >= TC_LAYER_MIN_ROWS &&
-                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, L->mode_gu, L->mode_d)));
+                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, L->mode_gu, L->mode_d, true, (long)r.D * r.I)));
     if (use_tc) {
         // coli_cuda_tensor_update may have refreshed a tensor with scales the tensor-core
         // path cannot carry exactly since the layer was created: look again (E flags)

@@ -344,8 +344,10 @@ void coli_cuda_set_fused_decode(int enabled);
  *   1 (default)  when it pays, by the measured crossover with the streaming kernel: a mean
  *                of at least 8 rows per expert of the call for int4 with group scales (two
  *                fp16 terms per weight; 5.5 when only gate and up have them, 4.5 when only
- *                down has), 3 for MXFP4 and 2.5 for per-row int4; layer calls count M*K
- *                rows over E experts, from 9 rows (fewer are the fused kernel's)
+ *                down has), 4 for MXFP4 and 3 for per-row int4; layer calls count M*K
+ *                rows over E experts, from 9 rows (fewer are the fused kernel's). Groups take
+ *                6, 5.5, 3.5 and 3 in place of the last four; below a million weights a
+ *                matrix layers take 4.5 for the last two, groups 5.5, 4.5, 3 and 2.5
  *   2            whenever the tensors and shapes allow it (tests)
  *   0            never: the streaming kernel takes every size (A/B testing)
  * No counterpart in the reference. */

@@ -176,3 +176,60 @@ def test_repeated_calls_agree(be, fmt, gs):
             for t in h:
                 be.tensor_free(t)
     assert ok and be.kernel_status(0) == 0 and bad == 0
+
+
+@pytest.mark.parametrize("gu,dn,D,I,line", [((2, 0), (2, 0), 1024, 1024, 3), ((7, 0), (7, 0), 1024, 1024, 4), ((4, 32), (4, 32), 1024, 1024, 8),
+                                             ((2, 0), (4, 64), 1024, 1024, 4.5), ((4, 32), (7, 0), 1024, 1024, 5.5), ((4, 32), (4, 32), 512, 256, 8),
+                                             ((7, 0), (7, 0), 512, 256, 4.5)])
+def test_rule_of_layers(be, gu, dn, D, I, line):
+    """Layer calls on both sides of their line: the default is bit for bit the streaming kernel's result below it and the
+    tensor cores' from it on (the two add in different orders, so their results differ in some bits), and the two agree to 1e-3."""
+    E, K = 16, 4
+    rng = np.random.default_rng(int(line * 10) + D)
+    ex = [(rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, D, I, *dn, half=True)) for _ in range(E)]
+    hs = [[upload_qt(be, t) for t in e] for e in ex]
+    at = int(line * E / K)
+    lay = MoeLayer(be, D, I, E, K, *([h[m] for h in hs] for m in range(3)), 0, 0, max_rows=at)
+    try:
+        for M, tc in ((at - 1, False), (at, True)):
+            be.set_fused_decode(0)
+            x, lg = rng.standard_normal((M, D), dtype=np.float32), W.router_logits(M, E, 2)
+            out = {}
+            for mode in (0, 2, 1):
+                be.set_tensor_core(mode)
+                out[mode] = lay(x, lg)[0].copy()
+            assert max_rel_err(out[0], out[2]) <= 1e-3 and be.kernel_status(0) == 0
+            if M >= 9:                                                 # (fewer rows never take the tensor cores)
+                assert not np.array_equal(out[0], out[2])
+                assert np.array_equal(out[1], out[2] if tc else out[0]), (M, tc)
+    finally:
+        be.set_tensor_core(1)
+        be.set_fused_decode(3)
+        lay.free()
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
+
+
+@pytest.mark.parametrize("gu,dn,line", [((2, 0), (2, 0), 3), ((7, 0), (7, 0), 3.5), ((4, 32), (4, 32), 8), ((2, 0), (4, 32), 5.5), ((4, 32), (2, 0), 6)])
+def test_rule_of_larger_groups(be, gu, dn, line):
+    """The line of grouped calls for experts of a million weights and more, by the number of launches (five below, four from it on)."""
+    D, I, n = 1024, 1024, 4
+    rng = np.random.default_rng(int(line * 10) + gu[0])
+    ex = (rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, D, I, *dn, half=True))
+    hs = [[upload_qt(be, t) for t in ex] for _ in range(n)]
+    be.set_timing(1)
+    be.set_fused_decode(0)
+    try:
+        for total, want in ((int(line * n) - 1, 5), (int(line * n), 4)):
+            x = rng.standard_normal((total, D), dtype=np.float32)
+            ok, y = be.run_expert_group(*([h[m] for h in hs] for m in range(3)), [1, total - 4, 2, 1], x, D)
+            ms, launches = C.c_float(), C.c_int()
+            assert ok and be.last_timing(0, C.byref(ms), C.byref(launches)) and launches.value == want, total
+    finally:
+        be.set_timing(0)
+        be.set_fused_decode(3)
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
+    assert be.kernel_status(0) == 0
