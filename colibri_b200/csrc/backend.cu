@@ -210,6 +210,19 @@ static void setup_decode() {
     set_smem(k_gemv_rows<MODE, 1>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096); set_smem(k_gemv_rows<MODE, 2>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096);
 }
 
+// The grouped GEMM's warps share out the registers of its launch: their number must be what the split was made for.
+template <int MODE, int PHASE>
+static int setup_tc_phase() {
+    set_smem(k_expert_gemm_tc<MODE, PHASE>, tc_smem_total(MODE));
+    cudaFuncAttributes fa{};
+    if (!cuda_ok(cudaFuncGetAttributes(&fa, k_expert_gemm_tc<MODE, PHASE>), "kernel attributes")) return 0;
+    if ((fa.numRegs + 7) / 8 * 8 == TC_REGS_LAUNCH) return 1;
+    std::fprintf(stderr, "[CUDA] grouped GEMM built with %d registers a thread, %d needed\n", fa.numRegs, TC_REGS_LAUNCH);
+    return 0;
+}
+template <int MODE>
+static int setup_tc() { return setup_tc_phase<MODE, 1>() && setup_tc_phase<MODE, 2>(); }
+
 extern "C" int coli_cuda_init(const int *devices, int count) {
     if (!devices || count < 1 || count > COLI_CUDA_MAX_DEVICES) return 0;
     if (g_nctx) coli_cuda_shutdown();
@@ -253,9 +266,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         set_smem(k_router_logits<16, 256>, router_smem(16, 256)); set_smem(k_router_logits<64, 64>, router_smem(64, 64));
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         setup_decode<SC_ROW>(); setup_decode<SC_H16>(); setup_decode<SC_F32>(); setup_decode<SC_MX>();
-        set_smem(k_expert_gemm_tc<SC_ROW, 1>, tc_smem_total(SC_ROW)); set_smem(k_expert_gemm_tc<SC_ROW, 2>, tc_smem_total(SC_ROW));
-        set_smem(k_expert_gemm_tc<SC_H16, 1>, tc_smem_total(SC_H16)); set_smem(k_expert_gemm_tc<SC_H16, 2>, tc_smem_total(SC_H16));
-        set_smem(k_expert_gemm_tc<SC_MX, 1>, tc_smem_total(SC_MX)); set_smem(k_expert_gemm_tc<SC_MX, 2>, tc_smem_total(SC_MX));
+        if (!setup_tc<SC_ROW>() || !setup_tc<SC_H16>() || !setup_tc<SC_MX>()) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
         set_smem(k_tc_plan, 33 * ROUTE_MAX_E * (int)sizeof(int));
         set_smem(k_route_build, ROUTE_BUILD_INTS * ROUTE_MAX_E * (int)sizeof(int));
         if (!cuda_ok(cudaGetLastError(), "kernel attributes")) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
