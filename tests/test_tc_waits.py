@@ -69,3 +69,17 @@ def test_decode_warps_leave_when_a_wait_has_expired():
     assert len(loops) == 2 and all("!gone" in loop for loop in loops), loops
     flush = role[role.index(loops[1]):]
     assert re.search(r"gone = __any_sync\(0xffffffffu, dead\);", flush)
+
+
+def test_copies_and_mmas_in_flight_are_waited_for_whoever_gave_up():
+    """What a role has started is waited for by that role, not only when it gave up itself: the roles that would have
+    waited for it may have."""
+    text = re.sub(r"//[^\n]*", "", open(SOURCE).read())
+    kernel = text[text.index("k_expert_gemm_tc(TcArgs a)"):]
+    drains = [m.start() for m in re.finditer(r"mbar_wait_bounded\(", kernel)]
+    assert len(drains) == 3                                  # MMAs; weight copies; activation copies
+    for at in drains:
+        before = kernel[:at]
+        head = before[before.rindex("while (ct.task < ntask"):]
+        tail = head[max(head.rfind("if (dead) break;"), head.rfind("umma_commit(bar_acc_full")):]
+        assert "if (dead)" not in tail.replace("if (dead) break;", ""), tail
