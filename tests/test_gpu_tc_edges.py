@@ -146,7 +146,7 @@ def test_segment_lists_of_the_streaming_path(be, E, K, M, topp):
     assert max_rel_err(outs[0][0], outs[1][0]) <= 1e-3 and be.kernel_status(0) == 0
 
 
-@pytest.mark.parametrize("fmt,gs", [(7, 0)])
+@pytest.mark.parametrize("fmt,gs", [(7, 0), (4, 32), (2, 0)])
 def test_repeated_calls_agree(be, fmt, gs):
     """The same call again and again while every stage of the kernel's rings is in turn the slowest one (passes of 1 to 64 rows):
     bit for bit the same rows. A slot that is filled again before its last word was read shows here as a few

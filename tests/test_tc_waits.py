@@ -83,3 +83,15 @@ def test_copies_and_mmas_in_flight_are_waited_for_whoever_gave_up():
         head = before[before.rindex("while (ct.task < ntask"):]
         tail = head[max(head.rfind("if (dead) break;"), head.rfind("umma_commit(bar_acc_full")):]
         assert "if (dead)" not in tail.replace("if (dead) break;", ""), tail
+
+
+def test_a_raw_slot_is_given_back_behind_completed_stores():
+    """The arrival that lets the next copy into a raw slot comes behind the wait for the tensor-memory stores, which need every
+    word read from the slot, and behind a barrier of the warp, whose other lanes read from it too."""
+    text = re.sub(r"//[^\n]*", "", open(SOURCE).read())
+    role = text[text.index("if (warp >= TC_DEC_WARP0) {"):text.index("} else if (warp >= TC_EPI_WARP0) {")]
+    arrive = [m.start() for m in re.finditer(r"mbar_arrive\([^;]*TC_BAR_RAW_EMPTY", role)]
+    assert len(arrive) == 1
+    stored = role.rindex("tmem_st_frag16(")
+    waited = role.index("tcgen05.wait::st", stored)
+    assert waited < role.index("__syncwarp()", waited) < arrive[0]
