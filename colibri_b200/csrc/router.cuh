@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(flo
     if (tid >= CW * 32) {
         // copies: row j of the weights, or of x
         const int rows = nrow + (one_x ? 1 : nrow);
-        for (int t = 0; t < ntile; t++) {
+        int t = 0;
+        for (; t < ntile; t++) {
             const int st = t % NS, width = min(TILE, D - t * TILE);
             const uint32_t bar = smem_u32(s_full + st);
             if (t >= NS && !mbar_wait_bounded(smem_u32(s_empty + st), (t / NS + 1) & 1)) break;
@@ -71,6 +72,8 @@ __global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(flo
                 bulk_g2s(smem_u32(rt + ((size_t)(st * 2 + is_x) * OUT + r) * LD), src, width * 4, bar);
             }
         }
+        // copies in flight land before the shared memory goes away (bounded): chains that gave up no longer wait for them
+        for (int i = max(0, t - NS); i < t; i++) mbar_wait_bounded(smem_u32(s_full + i % NS), (i / NS) & 1);
         return;
     }
     const int row = tid & (OUT - 1);                    // (lanes beyond OUT repeat a row)
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(OUT <= 32 ? 64 : OUT + 32) k_router_logits(flo
     bool ok = true;
     for (int t = 0; t < ntile; t++) {
         const int st = t % NS, width = min(TILE, D - t * TILE);
-        if (!mbar_wait_bounded(smem_u32(s_full + st), (t / NS) & 1)) ok = false;
+        if (ok && !mbar_wait_bounded(smem_u32(s_full + st), (t / NS) & 1)) ok = false;      // (one expired wait, not one a tile)
         const float4 *wt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2) * OUT + row) * LD);
         const float4 *xt = reinterpret_cast<const float4 *>(rt + ((size_t)(st * 2 + 1) * OUT + (one_x ? 0 : row)) * LD);
 #pragma unroll 1

@@ -1,5 +1,5 @@
-"""What the grouped GEMM's roles do when a wait has run out, checked without a GPU: the wait functions of
-csrc/gemm_tc.cuh are compiled for the host with a barrier that never completes."""
+"""What kernels do when a wait has run out, checked without a GPU: the wait functions of csrc/gemm_tc.cuh are compiled for
+the host with a barrier that never completes, and the order of waits is read off the sources."""
 import os
 import re
 import shutil
@@ -95,3 +95,13 @@ def test_a_raw_slot_is_given_back_behind_completed_stores():
     stored = role.rindex("tmem_st_frag16(")
     waited = role.index("tcgen05.wait::st", stored)
     assert waited < role.index("__syncwarp()", waited) < arrive[0]
+
+
+def test_router_waits_once_for_copies_that_do_not_come():
+    """The chains of the router kernel wait for no tile after one that did not come (a wait per tile would add up to the limit times
+    the tiles), and the copy warp, whose copies they then do not wait for, does so itself before it leaves."""
+    text = open(os.path.join(ROOT, "colibri_b200", "csrc", "router.cuh")).read()
+    kernel = re.sub(r"//[^\n]*", "", text[text.index("k_router_logits("):text.index("__global__ void k_router_logits_any")])
+    copies, chains = kernel[:kernel.index("return;")], kernel[kernel.index("return;"):]
+    assert re.search(r"for \(int i = max\(0, t - NS\); i < t; i\+\+\) mbar_wait_bounded\(smem_u32\(s_full \+ i % NS\), \(i / NS\) & 1\);\s*$", copies)
+    assert re.findall(r"if \(([^\n]*?)!mbar_wait_bounded", chains) == ["ok && "]
