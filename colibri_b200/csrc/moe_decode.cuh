@@ -401,7 +401,7 @@ struct WarpRing {
     int pi, ci;               // slot the next copy goes to / the next wait looks at
     int nst, sb;
     uint32_t par;             // parity the consumer waits with, flips when it wraps
-    bool ok;                  // false once a wait has expired: later waits are skipped
+    bool ok;                  // false once a wait has expired: later waits are skipped, no copy is started any more
     __device__ __forceinline__ void start(uint32_t r, uint32_t b, int n, int bytes) {
         ring = r; bars = b; nst = n; sb = bytes; issued = consumed = pi = ci = 0; par = 0;
     }
@@ -422,10 +422,15 @@ __device__ __forceinline__ void dec_issue_one(WarpRing &wr, DecIt &it, const Dec
     dec_it_next<CH>(it, ph, sh);
 }
 
-// Waits for the oldest outstanding chunk of the ring; returns its shared-memory address.
-__device__ __forceinline__ uint32_t dec_wait_chunk(WarpRing &wr) {
-    if (wr.ok && !mbar_wait_bounded(wr.bars + wr.ci * 8, wr.par)) wr.ok = false;
+// Waits for the oldest outstanding chunk of the ring; returns its shared-memory address. When the wait expires the stream
+// ends: a later copy would go to a slot, and be counted on a barrier, that still has one in flight.
+__device__ __forceinline__ uint32_t dec_wait_chunk(WarpRing &wr, DecIt &it) {
+    if (wr.ok && !mbar_wait_bounded(wr.bars + wr.ci * 8, wr.par)) { wr.ok = false; it.live = 0; }
     return wr.ring + wr.ci * wr.sb;
+}
+// Behind an expired wait: the last copy of every slot has landed, or the limit has passed once more for it.
+__device__ __forceinline__ void dec_drain(const WarpRing &wr) {
+    for (int i = max(0, wr.issued - wr.nst); i < wr.issued; i++) mbar_wait_bounded(wr.bars + i % wr.nst * 8, (i / wr.nst) & 1);
 }
 // after the chunk has been read: its slot is free again
 __device__ __forceinline__ void dec_release_chunk(WarpRing &wr) {
@@ -940,7 +945,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                     for (int grp = 0; grp < 4; grp++)
                         bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                    const uint32_t st = dec_wait_chunk(wr);
+                    const uint32_t st = dec_wait_chunk(wr, it);
                     float bacc[1][2][4];
                     block_mma<MODE, 1>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc);
 #pragma unroll
@@ -991,8 +996,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     // Every gate/up block of this warp has landed and been read, so nothing is in flight: the
     // down stream starts now, ahead of the barrier (its weights do not depend on the other
     // CTAs). For the local combine the ring becomes six slots of half a chunk.
+    if (!wr.ok) dec_drain(wr);
     wr.start(wr.ring, wr.bars + nst * 8, a.local2 ? 2 * nst : nst, a.local2 ? CH / 2 : CH);
     dec_it_start<CH>(it, ph2, sh);
+    if (!wr.ok) it.live = 0;
 #pragma unroll 1
     for (int s = 0; s < wr.nst; s++) dec_issue_one<CH>(wr, it, ph2, sh, el);
     DEC_PROBE(a, 4);   // gate/up consumed (the ring already holds the first down blocks)
@@ -1041,7 +1048,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         }
     }
     // every thread observes the completion itself, which also makes the copied bytes visible to it
-    if (nslot > 0 && !mbar_wait_bounded(hbar, 0)) wr.ok = false;
+    if (nslot > 0 && !mbar_wait_bounded(hbar, 0)) { wr.ok = false; it.live = 0; }
     DEC_PROBE(a, 6);
     if (a.local2) {
         // ---- down with a local combine: this CTA's 16 output rows over every pass ------------
@@ -1070,7 +1077,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                     for (int grp = 0; grp < 4; grp++)
                         bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                    const uint32_t st = dec_wait_chunk(wr);
+                    const uint32_t st = dec_wait_chunk(wr, it);
                     if (tid == 0 && p == ph2.gidx && kb == ph2.wl) DEC_PROBE_T(a, 11);   // first down block has landed
                     float bacc[1][2][4];
                     block_mma<MODE, 1, true, 1>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc, ixg);
@@ -1144,7 +1151,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
 #pragma unroll
                 for (int grp = 0; grp < 4; grp++)
                     bpre[grp] = *reinterpret_cast<const uint4 *>(bptr + kb * bstr + grp * 64);
-                const uint32_t st = dec_wait_chunk(wr);
+                const uint32_t st = dec_wait_chunk(wr, it);
                 float bacc[1][2][4];
                 block_mma<MODE, 1, true>(st, lane, g, [&](int grp, int) { return bpre[grp]; }, bacc, ixg);
 #pragma unroll
@@ -1203,11 +1210,9 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
     __syncthreads();
     if (sh->failed) {
         if (tid == 0) kstat_set(a.status, sh->failed == 2 ? KSTAT_MBAR_TIMEOUT : KSTAT_GRID_TIMEOUT);
-        // drain copies still in flight before the shared memory goes away (bounded)
-        for (int i = wr.consumed; i < wr.issued; i++) {
-            if (!mbar_wait_bounded(wr.bars + wr.ci * 8, wr.par)) break;
-            if (++wr.ci == wr.nst) { wr.ci = 0; wr.par ^= 1; }
-        }
+        // copies still in flight land before the shared memory goes away (bounded)
+        dec_drain(wr);
+        if (nslot > 0) mbar_wait_bounded(hbar, 0);
     }
 }
 

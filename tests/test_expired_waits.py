@@ -105,3 +105,101 @@ def test_router_waits_once_for_copies_that_do_not_come():
     copies, chains = kernel[:kernel.index("return;")], kernel[kernel.index("return;"):]
     assert re.search(r"for \(int i = max\(0, t - NS\); i < t; i\+\+\) mbar_wait_bounded\(smem_u32\(s_full \+ i % NS\), \(i / NS\) & 1\);\s*$", copies)
     assert re.findall(r"if \(([^\n]*?)!mbar_wait_bounded", chains) == ["ok && "]
+
+
+RING = r"""
+#include <algorithm>
+#include <cstdint>
+#include <cstdio>
+#include <map>
+#include <vector>
+using std::max;
+#define __device__
+#define __forceinline__ inline
+struct DecPass { const uint8_t *wg, *wu, *wd; };
+struct DecShared { DecPass pass[4]; };
+static int dec_div(int n, unsigned long long m) { return n / (int)m; }
+// barriers of one arrival each, by address: copies pending in the present phase, phases ended
+struct Bar { int arrived = 0, pending = 0; unsigned phase = 0; };
+static std::map<uint32_t, Bar> bars;
+static std::map<uint32_t, int> slot;                    // copies in flight into a ring address
+static std::vector<std::pair<uint32_t, uint32_t>> flight;
+static int faults = 0, late = 1 << 30, copies = 0, landed_behind = 0;
+static void land(size_t k) {
+    slot[flight[k].first]--;
+    Bar &b = bars[flight[k].second];
+    if (--b.pending == 0 && b.arrived == 1) { b.arrived = 0; b.phase++; }
+    flight.erase(flight.begin() + k);
+}
+static void mbar_expect_tx(uint32_t bar, uint32_t) { if (bars[bar].arrived++) { std::puts("a second arrival in one phase"); faults++; } }
+static void bulk_g2s(uint32_t dst, const void *, uint32_t, uint32_t bar) {
+    if (slot[dst]++) { std::puts("a copy into a slot with one in flight"); faults++; }
+    bars[bar].pending++; copies++;
+    flight.push_back({dst, bar});
+}
+static bool ended(uint32_t bar, uint32_t parity) { return (bars[bar].phase & 1) != parity; }
+static bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
+    if (ended(bar, parity)) return true;
+    for (size_t k = 0; k < flight.size(); k++)
+        if (flight[k].second == bar) {
+            if (late-- == 0) return false;              // this one is later than the limit; the next wait finds it landed
+            land(k);
+            return ended(bar, parity);
+        }
+    return false;
+}
+@FUNCTIONS@
+int main() {
+    const int CH = 64;
+    DecShared sh{};
+    for (int first = 0; first < 40; first++) {          // which wait expires
+        bars.clear(); slot.clear(); flight.clear();
+        late = first; copies = 0;
+        DecPhase ph{};
+        ph.which = 1; ph.nt = 1; ph.nkb = 8; ph.wpk = 1; ph.ng = 1; ph.mg_nt = 1; ph.u1 = 2; ph.cnt = 8; ph.npass = 2;
+        WarpRing wr; DecIt it;
+        wr.ok = true;
+        wr.start(4096, 0, 3, CH);
+        for (int phase = 0; phase < 2; phase++) {
+            if (phase) {
+                if (!wr.ok) dec_drain(wr);
+                wr.start(wr.ring, 1024, 6, CH / 2);
+                ph.which = 2;
+            }
+            dec_it_start<CH>(it, ph, &sh);
+            if (!wr.ok) it.live = 0;
+            for (int s = 0; s < wr.nst; s++) dec_issue_one<CH>(wr, it, ph, &sh, 1);
+            for (int b = 0; b < (phase ? 16 : 32); b++) {
+                const bool was = wr.ok;
+                const int before = copies;
+                dec_wait_chunk@ARGS@;
+                dec_release_chunk(wr);
+                dec_issue_one<CH>(wr, it, ph, &sh, 1);
+                if (!was && copies != before) { std::puts("a copy started behind an expired wait"); faults++; }
+            }
+        }
+        if (!wr.ok) dec_drain(wr);
+        if (!flight.empty()) { std::printf("wait %d expired: %zu copies in flight at the end\n", first, flight.size()); faults++; }
+        if (faults) return 1;
+    }
+    std::puts("ok");
+}
+"""
+
+
+def test_the_fused_kernels_stream_ends_with_an_expired_wait(tmp_path):
+    """The weight ring of the fused decode kernel (csrc/moe_decode.cuh) over both phases, with one wait after the other expiring:
+    no copy goes to a slot, or is counted on a barrier, that has one in flight, and none is in flight at the end."""
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no host C++ compiler")
+    text = open(os.path.join(ROOT, "colibri_b200", "csrc", "moe_decode.cuh")).read()
+    code = text[text.index("struct DecPhase {"):text.index("// This CTA's contiguous share")]
+    (tmp_path / "ring.cpp").write_text(RING.replace("@FUNCTIONS@", code).replace("@ARGS@", "(wr, it)"))
+    exe = str(tmp_path / "ring")
+    subprocess.check_call([gxx, "-std=c++17", "-O1", "-o", exe, str(tmp_path / "ring.cpp")])
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
+    assert re.search(r"if \(!wr\.ok\) dec_drain\(wr\);\s*wr\.start\([^;]*;\s*dec_it_start<CH>\(it, ph2, sh\);\s*if \(!wr\.ok\) it\.live = 0;", text)
+    assert re.search(r"if \(nslot > 0 && !mbar_wait_bounded\(hbar, 0\)\) \{ wr\.ok = false; it\.live = 0; \}", text)
+    assert re.search(r"dec_drain\(wr\);\s*if \(nslot > 0\) mbar_wait_bounded\(hbar, 0\);", text)
