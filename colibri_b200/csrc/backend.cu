@@ -815,17 +815,46 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
     return cuda_ok(cudaGetLastError(), "linear launch");
 }
 
+// CTAs that share an SM at up to four rows. A wave takes a CTA's loads one behind the other, so what counts is how many
+// waves there are: the fewest CTAs an SM that need the fewest, between LO and HI. More of them leave a thread fewer
+// registers (128, 80, 64 at 2, 3, 4), that is fewer words ahead: 8-bit formats spill at 64, and FP8, which gains most from them, at 80.
+// One row, us at two / three / four an SM by O (columns in parentheses):
+//   grouped int4 (6150)  8200: 56 / 58 / 58    9480: 77 / 58 / 58    12296: 101 / 60 / 60    18440: 103 / 109 / 67    32776: 194 / 159 / 118
+//   MXFP4 (6150)         8200: 42 / 44 / 44    9480: 52 / 44 / 46    12296: 75 / 46 / 46     18440: 75 / 81 / 50      32776: 140 / 118 / 89
+//   per-row int4 (6150)  9480: 42 / 42 / 42    14216: 54 / 54 / 44   18440: 75 / 77 / 48     21320: 77 / 77 / 79      32776: 110 / 110 / 83
+//   2-bit (6144)         9504: 30 / 30 / 30    14208: 32 / 32 / 32   18432: 50 / 50 / 34     21312: 50 / 52 / 50      32768: 71 / 71 / 56
+//   int8 (6144)          9472: 22 / 22 / 24    9504: 26 / 22 / 26    12288: 30 / 24 / 28     18432: 32 / 34 / 34      32768: 50 / 46 / 52
+//   FP8 (6144)           9472: 19 / 22 / 26    9504: 24 / 22 / 26    12288: 26 / 26 / 28     18432: 28 / 36 / 38      32768: 44 / 52 / 54
+// (2-bit and per-row int4 take 72 to 80 registers however many they may: two and three are one.)
+template <int FMT> struct DenseCtas {
+    static constexpr int LO = FMT == 2 || FMT == 3 ? 3 : 2, HI = FMT == 8 ? 2 : FMT == 1 ? 3 : 4;
+};
+static int dense_ctas(int lo, int hi, long ctas, int sms) {
+    int best = lo;
+    for (int k = lo + 1; k <= hi; k++)
+        if ((ctas + (long)k * sms - 1) / ((long)k * sms) < (ctas + (long)best * sms - 1) / ((long)best * sms)) best = k;
+    return best;
+}
 template <int FMT, bool AL16>
 static void launch_dense(DeviceCtx *c, const ColiCudaTensor *t, float *y, int S, const __half *bq, const float *bs) {
     const int nc = S <= 4 ? 1 : S <= 8 ? 2 : 4;
     const dim3 grid((unsigned)((t->O + 31) / 32), (unsigned)((S + 4 * nc - 1) / (4 * nc)));
+    const long ctas = (long)grid.x * grid.y;
     const uint8_t *w = static_cast<const uint8_t *>(t->raw_w);
     const size_t rb = row_bytes(t->fmt, t->I);
     const int gs = t->gs > 0 ? t->gs : t->I;
     auto go = [&](auto kern) { launch_pdl(c, kern, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng); };
-    if (nc == 1) go(k_dense_mma<FMT, 1, AL16, 2>);
-    else if (nc == 2) go(k_dense_mma<FMT, 2, AL16, 2>);
-    else if ((int)(grid.x * grid.y) > c->sms) go(k_dense_mma<FMT, 4, AL16, 2>);
+    // More than 8 rows, 8-bit rows on 16 bytes: three waves of one CTA an SM against one of two and a rest (12 rows of 6144 x 9504 |
+    // 12288 | 14208: int8 42 / 44 | 46 / 44 | 48 / 52, FP8 36 / 38 | 38 / 42 | 40 / 44 us; at two and four waves two an SM are as fast or faster)
+    const bool three = ctas > 2L * c->sms && ctas <= 3L * c->sms;
+    if (nc == 1) {
+        constexpr int LO = DenseCtas<FMT>::LO, HI = DenseCtas<FMT>::HI;
+        const int k = dense_ctas(LO, HI, ctas, c->sms);
+        if (k == LO) go(k_dense_mma<FMT, 1, AL16, LO>);
+        else if (k == HI) go(k_dense_mma<FMT, 1, AL16, HI>);
+        else go(k_dense_mma<FMT, 1, AL16, (LO + HI) / 2>);
+    } else if (nc == 2) go(k_dense_mma<FMT, 2, AL16, 2>);
+    else if (ctas > c->sms && !(AL16 && three)) go(k_dense_mma<FMT, 4, AL16, 2>);
     else go(k_dense_mma<FMT, 4, AL16, 1>);
 }
 

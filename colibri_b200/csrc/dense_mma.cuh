@@ -11,12 +11,13 @@
 // 16-byte loads; column 2r of an MMA is row r's hi part, 2r+1 its lo part. Weight and activation scales are
 // applied in f32 once per block (grouped formats: per 32 columns).
 // Why: the scalar kernel before it decoded every weight to f32 and multiplied it with 8 rows by
-// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows, 24 so (50 MB at 2.1 TB/s). Bound by the
+// FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows, 22 so (50 MB at 2.3 TB/s). Bound by the
 // latency of its loads (a warp multiplies a block with nothing of the next one requested), and 256 CTAs leave some of 148 SMs with
 // two and some with one.
-// CTAS: CTAs that share an SM. More than 8 rows want 140 to 180 registers a thread, and with one CTA per SM a second wave
-// runs behind the first; so when there are more CTAs than SMs the registers are capped for two (and spill a little: 1 % slower where
-// there are fewer CTAs than SMs, so not there). Call times with that and with the activations' fragments requested before the decoding, before / after, 12 rows of
+// CTAS: CTAs that share an SM; the registers of a thread are capped to that. More than 8 rows want 190 to 245 of them, and with one CTA
+// per SM a second wave runs behind the first; so when there are more CTAs than SMs the cap is for two (and spills a little: 1 % slower
+// where there are fewer CTAs than SMs, so not there). Up to four rows take two to four by format and number of CTAs (launch_dense, with the
+// figures). Call times with a cap and with the activations' fragments requested before the decoding, before / after, 12 rows of
 // 6144 x 8192: FP8 43 / 33, 2-bit 67 / 42, of 6150 x 8200: grouped int4 116 / 73, MXFP4 90 / 62, per-row int4 102 / 57. Requesting
 // half a block or a block ahead was slower for rows on 16 bytes (FP8 33 / 38), for the registers it takes.
 // Rows need no alignment: without 16-byte rows, words come from aligned loads and funnel shifts, a run of 16 bytes from five (FP8, 6150

@@ -74,3 +74,26 @@ def test_more_tiles_than_sms(be, fmt, gs, I):
     mag = np.abs(x).astype(np.float64) @ np.abs(w).T
     assert np.all(np.abs(y - x.astype(np.float64) @ w.T) <= 2e-6 * mag + 1e-30)
     assert be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("fmt,gs,I", [(1, 0, 272), (1, 0, 130), (2, 0, 130), (3, 0, 272), (4, 64, 192), (7, 0, 160), (8, 0, 272), (8, 0, 130)])
+@pytest.mark.parametrize("O,S", [(9601, 4), (14500, 3), (21000, 1), (9601, 9), (14500, 9)])
+def test_ctas_that_share_an_sm(be, fmt, gs, I, O, S):
+    """Few rows over more tiles than two CTAs per SM hold (three, four, and two waves), and more than 8 rows where three waves of one
+    are taken. Same bound as above."""
+    rng = np.random.default_rng(fmt * 1000 + I + S)
+    if fmt == 3:
+        codes, sc = rng.integers(0, 4, (O, I)), rng.random(O).astype(np.float32)
+        packed = sum(codes[:, j::4] << (2 * j) for j in range(4)).astype(np.uint8)
+        t, w = QTensor(packed, sc, 3, I, O), (codes - 2.0) * sc[:, None].astype(np.float64)
+    else:
+        t = quantize((rng.standard_normal((O, I)) * 0.02).astype(np.float32), fmt, gs)
+        w = t.dequant().astype(np.float64)
+    x = rng.standard_normal((S, I)).astype(np.float32)
+    box = [None]
+    ok, y = be.run_matmul(box, x, t.w, t.s, fmt, I, O, gs=gs)
+    assert ok
+    be.tensor_free(box[0])
+    mag = np.abs(x).astype(np.float64) @ np.abs(w).T
+    assert np.all(np.abs(y - x.astype(np.float64) @ w.T) <= 2e-6 * mag + 1e-30)
+    assert be.kernel_status(0) == 0
