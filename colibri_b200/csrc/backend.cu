@@ -51,6 +51,7 @@ struct DeviceCtx {
     size_t host_x_cap = 0, host_y_cap = 0;
     float *io_x = nullptr, *io_y = nullptr;       // pinned rows of the blocking host-buffer calls
     size_t io_x_cap = 0, io_y_cap = 0;
+    bool tc = false;                          // the grouped GEMM was built as its register split needs it
     bool chain = false;                       // the last thing this call put on the stream is a kernel
     IoPieces io = {};                         // events of the pieces of a call's result
     uint32_t *check = nullptr;                // scale facts of an upload: 4 words on the device, then pinned
@@ -210,14 +211,15 @@ static void setup_decode() {
     set_smem(k_gemv_rows<MODE, 1>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096); set_smem(k_gemv_rows<MODE, 2>, rows_smem(MODE, 1, ROWS_MAX_X) + 4096);
 }
 
-// The grouped GEMM's warps share out the registers of its launch: their number must be what the split was made for.
+// The grouped GEMM's warps share out the registers of its launch: their number must be what the split was made for. Where it is not,
+// no tensor qualifies for that kernel and the streaming one takes its calls.
 template <int MODE, int PHASE>
 static int setup_tc_phase() {
     set_smem(k_expert_gemm_tc<MODE, PHASE>, tc_smem_total(MODE));
     cudaFuncAttributes fa{};
     if (!cuda_ok(cudaFuncGetAttributes(&fa, k_expert_gemm_tc<MODE, PHASE>), "kernel attributes")) return 0;
     if ((fa.numRegs + 7) / 8 * 8 == TC_REGS_LAUNCH) return 1;
-    std::fprintf(stderr, "[CUDA] grouped GEMM built with %d registers a thread, %d needed\n", fa.numRegs, TC_REGS_LAUNCH);
+    std::fprintf(stderr, "[CUDA] grouped GEMM built with %d registers a thread, %d needed: not used\n", fa.numRegs, TC_REGS_LAUNCH);
     return 0;
 }
 template <int MODE>
@@ -266,7 +268,7 @@ extern "C" int coli_cuda_init(const int *devices, int count) {
         set_smem(k_router_logits<16, 256>, router_smem(16, 256)); set_smem(k_router_logits<64, 64>, router_smem(64, 64));
         set_smem(k_dense_gemv<0>, DENSE_GEMV_SMEM); set_smem(k_dense_gemv<8>, DENSE_GEMV_SMEM);
         setup_decode<SC_ROW>(); setup_decode<SC_H16>(); setup_decode<SC_F32>(); setup_decode<SC_MX>();
-        if (!setup_tc<SC_ROW>() || !setup_tc<SC_H16>() || !setup_tc<SC_MX>()) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
+        c->tc = setup_tc<SC_ROW>() && setup_tc<SC_H16>() && setup_tc<SC_MX>();
         set_smem(k_tc_plan, 33 * ROUTE_MAX_E * (int)sizeof(int));
         set_smem(k_route_build, ROUTE_BUILD_INTS * ROUTE_MAX_E * (int)sizeof(int));
         if (!cuda_ok(cudaGetLastError(), "kernel attributes")) { g_nctx = i + 1; coli_cuda_shutdown(); return 0; }
@@ -415,9 +417,9 @@ extern "C" int coli_cuda_kernel_status(int device) {
 //           lie within 2^-12 of the largest so that the hi/lo split keeps its low bits
 //   SC_MX   2^(e - 127 + shift) must be an fp16 power of two <= 2^13 for every group that holds a
 //           non-zero code: shift = 140 - e_max, spread e_max - e <= TC_MX_SPREAD (down to 2^-11)
-static void tensor_tc_params(ColiCudaTensor *t, const uint32_t *f) {
+static void tensor_tc_params(const DeviceCtx *c, ColiCudaTensor *t, const uint32_t *f) {
     t->tc_ok = 0; t->tc_shift = 0;
-    if (!t->packed || (t->O % 128) || (t->I % 128)) return;
+    if (!c->tc || !t->packed || (t->O % 128) || (t->I % 128)) return;
     if (t->mode == SC_ROW) { t->tc_ok = 1; return; }
     if (t->mode == SC_H16) {
         float smax, smin;
@@ -493,7 +495,7 @@ static int tensor_fill(DeviceCtx *c, ColiCudaTensor *t, const void *weights, con
     } else if (t->fmt == 4 && mode == SC_H16 && c->check_host[0]) {
         return 0;   // the refreshed scales no longer fit the storage chosen at upload
     }
-    tensor_tc_params(t, c->check_host);
+    tensor_tc_params(c, t, c->check_host);
     const int ch = chunk_bytes_of(mode);
     const size_t nblk = (size_t)(t->O / TILE_ROWS) * (t->I / BLOCK_K);
     const size_t pkbytes = nblk * ch;
