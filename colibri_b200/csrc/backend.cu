@@ -1135,10 +1135,11 @@ static int tc_ffn(DeviceCtx *c, int mode_gu, int mode_d, const TcList &l, const 
     return cuda_ok(cudaGetLastError(), "tensor-core gemm launch");
 }
 
+// whatever: also where it does not pay
 static int group_tc_ok(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
-                       ColiCudaTensor *const *downs, int count, int max_rows, int total) {
+                       ColiCudaTensor *const *downs, int count, int max_rows, int total, bool whatever = false) {
     if (!g_tc_enabled || max_rows < 2) return 0;
-    if (g_tc_enabled == 1 && !tc_pays(total, count, gates[0]->mode, downs[0]->mode, false, (long)gates[0]->I * gates[0]->O)) return 0;
+    if (g_tc_enabled == 1 && !whatever && !tc_pays(total, count, gates[0]->mode, downs[0]->mode, false, (long)gates[0]->I * gates[0]->O)) return 0;
     for (int e = 0; e < count; e++)
         if (!gates[e]->tc_ok || !ups[e]->tc_ok || !downs[e]->tc_ok || gates[e]->mode != gates[0]->mode ||
             ups[e]->mode != gates[0]->mode || downs[e]->mode != downs[0]->mode) return 0;
@@ -1908,8 +1909,10 @@ extern "C" int coli_cuda_ep_expert_group_dev(ColiCudaTensor *const *gates, ColiC
     if (!select_ctx(c)) return 0;
     timing_begin(c);
     int ok;
+    // rows that start off the boundaries of the other path's loads: the tensor cores' preparation reads them, at any mean
+    const bool odd = (reinterpret_cast<uintptr_t>(x_dev) & (x_bf16 ? 7 : 15)) != 0;
     if (all_packed && D % 128 == 0 && I % 128 == 0 &&
-        group_tc_ok(g.data(), u.data(), d.data(), (int)g.size(), max_rows, total)) {
+        group_tc_ok(g.data(), u.data(), d.data(), (int)g.size(), max_rows, total, odd)) {
         ok = group_device_tc(c, g.data(), u.data(), d.data(), rows.data(), (int)g.size(), D, I, total, y_dev, x_dev, 0,
                              rowmap.data(), x_bf16);
     } else {

@@ -142,3 +142,40 @@ def test_rows_off_their_boundary_are_refused(be):
     for e in ex:
         for h in e:
             be.tensor_free(h)
+
+
+@pytest.mark.parametrize("fmt,gs", [(2, 0), (7, 0), (4, 32)])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_ep_rows_between_boundaries(be, fmt, gs, bf16):
+    """Received rows that start on 8 bytes (bf16: 4) but not on 16 (8): taken whatever the mean of rows per expert, the line
+    between the two kernels only says which one is faster. Bit for bit the tensor cores' result of the same rows on a boundary."""
+    import ctypes as C
+    from colibri_b200.backend import Backend
+    from tests.util import upload_qt
+    D, I, E = 256, 128, 4
+    ex = [[upload_qt(be, t) for t in W.expert_weights(D, I, fmt, gs, 60 + e)] for e in range(E)]
+    side = [Backend.handle_array([e[k] for e in ex]) for k in range(3)]
+    for counts in ([2, 1, 1, 1], [3, 2, 2, 3], [9, 8, 8, 9]):
+        rows = np.array(counts, np.int32)
+        n = int(rows.sum())
+        x = W.bf16_round(np.random.default_rng(n).standard_normal((n, D)).astype(np.float32))
+        raw = (x.view(np.uint32) >> 16).astype(np.uint16) if bf16 else x
+        xd, yd = be.pipe_alloc(0, raw.nbytes + 16), be.pipe_alloc(0, x.nbytes)
+        out = []
+        try:
+            for off, mode in ((0, 2), (4 if bf16 else 8, 1)):
+                be.set_tensor_core(mode)
+                assert be.pipe_upload(0, xd + off, raw.ctypes.data, raw.nbytes)
+                assert be.ep_expert_group_dev(*side, E, rows.ctypes.data_as(C.POINTER(C.c_int)), 1, yd, xd + off, bf16), (counts, off)
+                y = np.empty((n, D), np.float32)
+                assert be.pipe_download(0, yd, y.ctypes.data, y.nbytes)
+                out.append(y)
+        finally:
+            be.set_tensor_core(1)
+            be.pipe_free(0, xd)
+            be.pipe_free(0, yd)
+        assert np.array_equal(*out) and np.any(out[0]), counts
+    assert be.kernel_status(0) == 0
+    for e in ex:
+        for h in e:
+            be.tensor_free(h)
