@@ -1057,22 +1057,33 @@ extern "C" void coli_cuda_set_tensor_core(int enabled) { g_tc_enabled = enabled 
 //   grouped int4          mean 4: 92 / 109 | 334 / 452 | 1557 / 2093     4.5: 112 / 110 | 431 / 452 | 2029 / 1943     5: 118 / 109 | 455 / 452 | 2236 / 2002
 //   down grouped int4, gate and up per row    mean 4: 90 / 92 | 320 / 347 | 1530 / 1592     4.5: 112 / 92 | 420 / 347 | 2055 / 1463
 //   gate and up grouped int4, down per row    mean 4: 92 / 101 | 328 / 402 | 1525 / 1882     4.5: 113 / 101 | 430 / 401 | 2024 / 1722
-// Layers of less than TC_SMALL weights a matrix are short of launches rather than of work and cross later (1024 x 512, E 64: per
-// row 4: 46 / 50, 4.5: 55 / 50; grouped 5: 56 / 57, 6: 61 / 58).
+// Layers of less than TC_LARGE weights a matrix are short of launches rather than of work and cross later, at a mean of 4.5 where streaming
+// passes widen (1024 x 512, E 64: per row 4: 43 / 47, 4.5: 52 / 46; MXFP4 43 / 47, 50 / 47; down grouped 45 / 49, 53 / 50; gate and up grouped 5: 55 / 53;
+// 1024 x 768: per row 53 / 55, 65 / 55; gate and up grouped 4.5: 65 / 65). A little above it the lines of large layers come early, by 2 to 10 %
+// (per-row 3, MXFP4 4: 1024 x 1024 58 / 60, 58 / 61; 1152 x 1024 62 / 68, 62 / 68; 1280 x 1024 70 / 70, 72 / 71; 1536 x 768 67 / 65, 68 / 69); grouped int4 at 8 does not
+// (1024 x 512 63 / 56; 512 x 256 40 / 41).
 // Groups of experts with unevenly spread rows widen single passes instead of all (24 experts, 2048 x 1024 | 6144 x 2048): per-row 2.5:
 // 42 / 42 | 118 / 137, 3: 43 / 42 | 144 / 138; MXFP4 3: 42 / 43 | 140 / 139, 4: 42 / 44 | 150 / 140; grouped 5: 48 / 56 | 174 / 211, 6: 63 / 56 |
-// 232 / 209; down grouped 5: 47 / 50 | 161 / 162, 6: 61 / 49 | 220 / 159; gate and up grouped 5: 48 / 52 | 164 / 186, 6: 63 / 52 | 225 / 191. Small
-// ones take the same 22 us on either side of their line (256 x 128).
+// 232 / 209; down grouped 5: 47 / 50 | 161 / 162, 6: 61 / 49 | 220 / 159; gate and up grouped 5: 48 / 52 | 164 / 186, 6: 63 / 52 | 225 / 191.
+// Below TC_LARGE the lines lie where those passes widen, at 6, whatever the format (per row | MXFP4 | down grouped | gate and up grouped, at 5.5 and 6:
+// 1024 x 512 26 / 28, 32 / 28 | 25 / 28, 31 / 28 | 26 / 29, 32 / 29 | 26 / 31, 32 / 31; 768 x 384 24 / 25, 27 / 25 | 23 / 25, 26 / 25 | 24 / 26, 27 / 26 | 24 / 26, 27 / 26;
+// 1152 x 768 32 / 33, 40 / 32 | 31 / 33, 38 / 32 | 32 / 35, 40 / 34 | 32 / 37, 39 / 36), above it they come early up to 1.5 million weights (1280 x 1024: per row 3:
+// 33 / 35, 4.5: 36 / 36; MXFP4 3.5: 32 / 36, 5: 36 / 36; 1536 x 1024 37 / 36 and 36 / 36 at the lines). Below TC_TINY both sides take the same 22 to 23 us,
+// from a mean of 2 to 8 (256 x 128, 512 x 256).
 // Grouped int4 has its line above where the times cross. Its products fill the accumulator, which truncates: against 64 bits an
 // expert of 2048 x 1024 is off by 2.9e-6 on the tensor cores and by 1.5e-7 in the streaming kernel (per-row int4 2.2e-7 | 1.3e-7, MXFP4
-// 2.6e-7 | 1.1e-7: few bits a product, most sums exact). A call is not taken there for less than a good part of its time.
-#define TC_SMALL (1L << 20)
+// 2.6e-7 | 1.1e-7: few bits a product, most sums exact). A call is not taken there for less than a good part of its time; the
+// same goes for gate and up or down alone.
+#define TC_LARGE (1L << 20)
+#define TC_TINY (1L << 17)
 static bool tc_pays(long rows, long experts, int mode_gu, int mode_d, bool layer, long weights) {
     const bool two_gu = mode_gu == SC_H16, two_d = mode_d == SC_H16;
     const int kind = two_gu && two_d ? 2 : two_gu ? 4 : two_d ? 3 : mode_gu == SC_MX || mode_d == SC_MX ? 1 : 0;
     // half rows: per-row int4, MXFP4, grouped int4, only down grouped, only gate and up grouped
-    static const int halves[2][2][5] = {{{5, 6, 16, 9, 11}, {6, 7, 16, 11, 12}}, {{9, 9, 16, 9, 11}, {6, 8, 16, 9, 11}}};
-    return 2 * rows >= (long)halves[layer][weights >= TC_SMALL][kind] * experts;
+    static const int layers[3][5] = {{9, 9, 16, 9, 11}, {9, 9, 16, 9, 11}, {6, 8, 16, 9, 11}};
+    static const int groups[3][5] = {{5, 6, 16, 9, 11}, {12, 12, 16, 12, 12}, {6, 7, 16, 11, 12}};
+    const int size = weights >= TC_LARGE ? 2 : weights >= TC_TINY ? 1 : 0;
+    return 2 * rows >= (long)(layer ? layers : groups)[size][kind] * experts;
 }
 
 template <int MODE, int PHASE>

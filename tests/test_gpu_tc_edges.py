@@ -233,3 +233,28 @@ def test_rule_of_larger_groups(be, gu, dn, line):
             for t in h:
                 be.tensor_free(t)
     assert be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("gu,dn,line", [((2, 0), (2, 0), 6), ((7, 0), (7, 0), 6), ((4, 32), (4, 32), 8), ((2, 0), (4, 32), 6), ((4, 32), (2, 0), 6)])
+@pytest.mark.parametrize("D,I", [(512, 256), (1024, 512), (1024, 896)])
+def test_rule_of_small_groups(be, gu, dn, line, D, I):
+    """The line of grouped calls for experts of 2^17 weights up to a million, by the number of launches (five below, four from it on)."""
+    n = 4
+    rng = np.random.default_rng(D + I + gu[0])
+    ex = (rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, I, D, *gu, half=True), rand_qt(rng, D, I, *dn, half=True))
+    hs = [[upload_qt(be, t) for t in ex] for _ in range(n)]
+    be.set_timing(1)
+    be.set_fused_decode(0)
+    try:
+        for total, want in ((line * n - 1, 5), (line * n, 4)):
+            x = rng.standard_normal((total, D), dtype=np.float32)
+            ok, y = be.run_expert_group(*([h[m] for h in hs] for m in range(3)), [1, total - 4, 2, 1], x, D)
+            ms, launches = C.c_float(), C.c_int()
+            assert ok and be.last_timing(0, C.byref(ms), C.byref(launches)) and launches.value == want, total
+    finally:
+        be.set_timing(0)
+        be.set_fused_decode(3)
+        for h in hs:
+            for t in h:
+                be.tensor_free(t)
+    assert be.kernel_status(0) == 0
