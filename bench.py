@@ -55,7 +55,6 @@ sys.path.insert(0, ROOT)
 from colibri_b200 import workloads as W  # noqa: E402
 from colibri_b200.quant import QTensor  # noqa: E402
 
-TC_MEAN_ROWS = {4: 8, 2: 3, 7: 4}    # the backend's rule for layer calls of more than 8 rows and experts of a million weights a matrix and more: mean rows per expert by format
 ROUTED_SCALE = 2.5    # sigmoid-gated configurations (GLM / DeepSeek-V3 style)
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the fused decode kernel (one ncu
 # capture of configuration 2 at M=1); other workloads have no capture and report null
@@ -793,6 +792,7 @@ def run_gpu_arm(args):
             torch.cuda.synchronize()
             e2e_blocks.append((time.perf_counter() - t0) * 1e3)
 
+    uses_tc = bool(be.moe_layer_tensor_core(layers[0].handle, M))
     for lay in layers:
         lay.free()
     for hg, hu, hd, sh in handles:
@@ -826,7 +826,6 @@ def run_gpu_arm(args):
         e2e_med = float(np.median(e2e_b))
         e2e = all_bytes * steps / (e2e_med * 1e-3) / 1e9
         fused = M <= 8
-        uses_tc = M > 8 and (args.tc == 2 or (args.tc == 1 and M * K >= TC_MEAN_ROWS.get(fmt, 1 << 30) * E))
         if fused:
             # one launch per layer call: the kernel's share of the timed step (launch gaps included)
             launch_us = ms_med / steps / L * 1e3

@@ -117,6 +117,7 @@ ADDITIVE_ABI = [
     ("coli_cuda_set_timing", None, [C.c_int]),
     ("coli_cuda_set_fused_decode", None, [C.c_int]),
     ("coli_cuda_set_tensor_core", None, [C.c_int]),
+    ("coli_cuda_moe_layer_tensor_core", C.c_int, [_vp, C.c_int]),
     ("coli_cuda_launch_total", C.c_ulonglong, [C.c_int]),
     ("coli_cuda_set_kernel_events", None, [C.c_int]),
     ("coli_cuda_kernel_events", C.c_int, [C.c_int, _f32p, _i32p]),

@@ -166,6 +166,18 @@ static int layer_run_tc(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const
     return cuda_ok(cudaGetLastError(), "layer launch");
 }
 
+// Does a call of M rows run on the tensor cores?
+static bool layer_takes_tc(const ColiCudaMoeLayer *L, int M) {
+    const RouteRule &r = L->rule;
+    bool ok = L->tc_ok && M >= TC_LAYER_MIN_ROWS &&
+              (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, L->mode_gu, L->mode_d, true, (long)r.D * r.I)));
+    // coli_cuda_tensor_update may have refreshed a tensor with scales the tensor-core
+    // path cannot carry exactly since the layer was created: look again (E flags)
+    for (int e = 0; e < r.E && ok; e++) ok = L->h_gates[e]->tc_ok && L->h_ups[e]->tc_ok && L->h_downs[e]->tc_ok;
+    if (ok && L->has_shared) ok = L->h_shared[0]->tc_ok && L->h_shared[1]->tc_ok && L->h_shared[2]->tc_ok;
+    return ok;
+}
+
 // Everything on c->stream with device buffers. idx/w/keff must be device
 // buffers of the layer or the caller ([M,K], [M,K], [M]).
 static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const float *x_dev,
@@ -174,15 +186,7 @@ static int layer_run(ColiCudaMoeLayer *L, DeviceCtx *c, float *out_dev, const fl
     const RouteRule &r = L->rule;
     const LayerPlan p = layer_plan(L, c, M);
     const int nkb1 = r.D / BLOCK_K, nkb2 = r.I / BLOCK_K;
-    bool use_tc = !route_only && !uniq_dev && L->tc_ok && M >= TC_LAYER_MIN_ROWS &&
-                  (g_tc_enabled == 2 || (g_tc_enabled == 1 && tc_pays((long)M * r.K, r.E, L->mode_gu, L->mode_d, true, (long)r.D * r.I)));
-    if (use_tc) {
-        // coli_cuda_tensor_update may have refreshed a tensor with scales the tensor-core
-        // path cannot carry exactly since the layer was created: look again (E flags)
-        for (int e = 0; e < r.E && use_tc; e++)
-            use_tc = L->h_gates[e]->tc_ok && L->h_ups[e]->tc_ok && L->h_downs[e]->tc_ok;
-        if (use_tc && L->has_shared) use_tc = L->h_shared[0]->tc_ok && L->h_shared[1]->tc_ok && L->h_shared[2]->tc_ok;
-    }
+    const bool use_tc = !route_only && !uniq_dev && layer_takes_tc(L, M);
     if (!reserve(c, &L->logits, (size_t)M * r.E * sizeof(float)) ||
         !reserve(c, &L->pos_of, (size_t)M * r.K * sizeof(int)) ||
         !reserve(c, &L->uniq, (size_t)r.E * sizeof(int)) || !reserve(c, &L->scal, 64) ||
@@ -253,6 +257,10 @@ static int layer_route_bufs(ColiCudaMoeLayer *L, DeviceCtx *c, int M) {
     return reserve(c, &L->idx, (size_t)M * L->rule.K * sizeof(int)) &&
            reserve(c, &L->w, (size_t)M * L->rule.K * sizeof(float)) &&
            reserve(c, &L->keff, (size_t)M * sizeof(int));
+}
+
+extern "C" int coli_cuda_moe_layer_tensor_core(const ColiCudaMoeLayer *L, int M) {
+    return L && M >= 1 && M <= L->max_rows && layer_takes_tc(L, M);
 }
 
 extern "C" int coli_cuda_moe_layer_dev(ColiCudaMoeLayer *L, float *out_dev, const float *x_dev,

@@ -341,17 +341,16 @@ void coli_cuda_set_fused_decode(int enabled);
 /* Expert groups and layer calls with many rows per expert run on the tcgen05
  * tensor-core kernel when every tensor involved is int4 with per-row or fp16-exact
  * group scales, or MXFP4, and D and I are multiples of 128:
- *   1 (default)  when it pays, by the measured crossover with the streaming kernel: a mean
- *                of at least 8 rows per expert of the call for int4 with group scales (two
- *                fp16 terms per weight; 5.5 when only gate and up have them, 4.5 when only
- *                down has), 4 for MXFP4 and 3 for per-row int4; layer calls count M*K
- *                rows over E experts, from 9 rows (fewer are the fused kernel's). Groups take
- *                6, 5.5, 3.5 and 3 in place of the last four; below a million weights a
- *                matrix layers take 4.5 for the last two, groups 5.5, 4.5, 3 and 2.5
+ *   1 (default)  when it pays: from a mean of rows per expert that was measured by format, size
+ *                and kind of call (tc_pays in csrc/backend.cu has the lines and their figures;
+ *                2.5 to 8). Groups count their rows over their experts, layer calls M*K rows
+ *                over E experts, from 9 rows (fewer are the fused kernel's)
  *   2            whenever the tensors and shapes allow it (tests)
  *   0            never: the streaming kernel takes every size (A/B testing)
  * No counterpart in the reference. */
 void coli_cuda_set_tensor_core(int enabled);
+/* 1 when a call of M rows of this layer takes that kernel, with the setting as it is. */
+int coli_cuda_moe_layer_tensor_core(const ColiCudaMoeLayer *layer, int M);
 
 /* Kernels this backend has launched on `device` since coli_cuda_init (every compute
  * entry point counts its own launches). No counterpart in the reference. */

@@ -258,3 +258,30 @@ def test_rule_of_small_groups(be, gu, dn, line, D, I):
             for t in h:
                 be.tensor_free(t)
     assert be.kernel_status(0) == 0
+
+
+@pytest.mark.parametrize("fmt,gs,line", [(2, 0, 3), (7, 0, 4), (4, 32, 8)])
+def test_a_layer_says_which_kernel_it_takes(be, fmt, gs, line):
+    """coli_cuda_moe_layer_tensor_core against the results of the call itself, around the line and by the setting."""
+    D, I, E, K = 1024, 1024, 16, 4
+    rng = np.random.default_rng(fmt)
+    ex = [upload_qt(be, rand_qt(rng, *s, fmt, gs, half=True)) for s in ((I, D), (I, D), (D, I))]
+    at = line * E // K
+    lay = MoeLayer(be, D, I, E, K, *([h] * E for h in ex), 0, 0, max_rows=at)
+    takes = lambda m: be.moe_layer_tensor_core(lay.handle, m)
+    try:
+        for M in (at - 1, at):
+            x, lg = rng.standard_normal((M, D), dtype=np.float32), W.router_logits(M, E, 2)
+            out, says = {}, {}
+            for mode in (0, 2, 1):
+                be.set_tensor_core(mode)
+                out[mode], says[mode] = lay(x, lg)[0].copy(), takes(M)
+            assert (says[0], says[2], says[1]) == (0, 1, int(M == at))
+            assert np.array_equal(out[1], out[2 if says[1] else 0]) and not np.array_equal(out[0], out[2])
+        assert (takes(8), takes(0), takes(at + 1), be.moe_layer_tensor_core(None, 9)) == (0, 0, 0, 0)
+    finally:
+        be.set_tensor_core(1)
+        lay.free()
+        for h in ex:
+            be.tensor_free(h)
+    assert be.kernel_status(0) == 0
