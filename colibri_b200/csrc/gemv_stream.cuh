@@ -443,7 +443,7 @@ k_gemv_stream(const GemvSeg *segs, const GemvCtl *ctl,
         if (lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
         // drain whatever is still in flight before leaving (bounded)
         for (int i = consumed; i < issued; i++) {
-            if (!mbar_wait_bounded(bars + ci * 8, par)) break;
+            mbar_wait_bounded(bars + ci * 8, par);          // (one that does not come says nothing of those behind it)
             if (++ci == NST) { ci = 0; par ^= 1; }
         }
     }
