@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) k_gemv_rows(float *__restrict
     uint32_t par = 0;
     bool ok = true;
     for (int kb = warp; kb < nkb; kb += ROWS_WARPS) {
-        if (ok && !mbar_wait_bounded(bars + s * 8, par)) ok = false;
+        // (behind an expired wait one try a block)
+        if (!mbar_try_wait(bars + s * 8, par) && !(ok && mbar_wait_bounded(bars + s * 8, par))) ok = false;
         float bacc[NC][2][4];
         block_mma<MODE, NC, false, 1>(ring + s * HS, lane, g,
                                       [&](int grp, int cs) { return *reinterpret_cast<const uint4 *>(bp[cs] + (size_t)kb * 256 + grp * 64); },
@@ -93,12 +94,6 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) k_gemv_rows(float *__restrict
         }
         if (++s == ROWS_NST) { s = 0; par ^= 1; }
     }
-    if (!ok && lane == 0) {
-        kstat_set(status, KSTAT_MBAR_TIMEOUT);
-        // copies in flight land before the shared memory goes away (bounded): the last one of every stage
-        const int n = (issued - warp) / ROWS_WARPS;
-        for (int i = max(0, n - ROWS_NST); i < n; i++) mbar_wait_bounded(bars + i % ROWS_NST * 8, (i / ROWS_NST) & 1);
-    }
 #pragma unroll
     for (int cs = 0; cs < NC; cs++) part[(warp * 2 + cs) * 32 + lane] = make_float2(R[cs][0] + R[cs][1], R[cs][2] + R[cs][3]);
     __syncthreads();
@@ -111,5 +106,12 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) k_gemv_rows(float *__restrict
         for (int k = 0; k < ROWS_WARPS; k++) a += p[k * 2 * 32 * 2];
         if (MODE == SC_ROW) a *= rowscale[blockIdx.x * 16 + o];
         y[(size_t)r * O + blockIdx.x * 16 + o] = a;
+    }
+    if (!ok && lane == 0) {                             // (last, out of the way of the ordinary end)
+        kstat_set(status, KSTAT_MBAR_TIMEOUT);
+        // copies in flight land before the shared memory goes away (bounded): the last one of every stage
+        const int n = (issued - warp) / ROWS_WARPS;
+#pragma unroll 1
+        for (int i = max(0, n - ROWS_NST); i < n; i++) mbar_wait_bounded(bars + i % ROWS_NST * 8, (i / ROWS_NST) & 1);
     }
 }

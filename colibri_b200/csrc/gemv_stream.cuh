@@ -441,9 +441,9 @@ k_gemv_stream(const GemvSeg *segs, const GemvCtl *ctl,
     }
     if (!ok) {
         if (lane == 0) kstat_set(status, KSTAT_MBAR_TIMEOUT);
-        // drain whatever is still in flight before leaving (bounded)
+        // drain whatever is still in flight before leaving (bounded; one that does not come says nothing of those behind it)
         for (int i = consumed; i < issued; i++) {
-            mbar_wait_bounded(bars + ci * 8, par);          // (one that does not come says nothing of those behind it)
+            if (!mbar_wait_bounded(bars + ci * 8, par)) kstat_set(status, KSTAT_MBAR_TIMEOUT);
             if (++ci == NST) { ci = 0; par ^= 1; }
         }
     }

@@ -205,13 +205,13 @@ def test_the_fused_kernels_stream_ends_with_an_expired_wait(tmp_path):
     assert re.search(r"dec_drain\(wr\);\s*if \(nslot > 0\) mbar_wait_bounded\(hbar, 0\);", text)
 
 
-@pytest.mark.parametrize("name,drain", [
-    ("gemv_rows.cuh", r"for \(int i = max\(0, n - ROWS_NST\); i < n; i\+\+\) mbar_wait_bounded\(bars \+ i % ROWS_NST \* 8, \(i / ROWS_NST\) & 1\);"),
-    ("gemv_stream.cuh", r"for \(int i = consumed; i < issued; i\+\+\) \{\s*mbar_wait_bounded\(bars \+ ci \* 8, par\);")], ids=["rows", "stream"])
-def test_streaming_kernels_wait_for_every_copy_in_flight(name, drain):
-    """Behind an expired wait no block is waited for any more, and before the kernel ends every copy in flight is, also those
-    behind one that does not come."""
+@pytest.mark.parametrize("name,wait,drain", [
+    ("gemv_rows.cuh", r"if \(!mbar_try_wait\(bars \+ s \* 8, par\) && !\(ok && mbar_wait_bounded\(bars \+ s \* 8, par\)\)\) ok = false;",
+     r"for \(int i = max\(0, n - ROWS_NST\); i < n; i\+\+\) mbar_wait_bounded\(bars \+ i % ROWS_NST \* 8, \(i / ROWS_NST\) & 1\);"),
+    ("gemv_stream.cuh", r"if \(!mbar_wait_bounded\([^;]*return false;",
+     r"for \(int i = consumed; i < issued; i\+\+\) \{\s*if \(!mbar_wait_bounded\(bars \+ ci \* 8, par\)\) kstat_set\(status, KSTAT_MBAR_TIMEOUT\);")], ids=["rows", "stream"])
+def test_streaming_kernels_wait_for_every_copy_in_flight(name, wait, drain):
+    """Behind an expired wait no block is waited for any more (one try each at most), and before the kernel ends every copy in
+    flight is, also those behind one that does not come."""
     text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "colibri_b200", "csrc", name)).read())
-    assert len(re.findall(drain, text)) == 1
-    wait = r"if \(ok && !mbar_wait_bounded" if name == "gemv_rows.cuh" else r"if \(!mbar_wait_bounded\([^;]*return false;"
-    assert len(re.findall(wait, text)) == 1
+    assert len(re.findall(drain, text)) == 1 and len(re.findall(wait, text)) == 1
