@@ -827,9 +827,14 @@ static int linear_packed(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, co
 //   2-bit (6144)         9504: 30 / 30 / 30    14208: 32 / 32 / 32   18432: 50 / 50 / 34     21312: 50 / 52 / 50      32768: 71 / 71 / 56
 //   int8 (6144)          9472: 22 / 22 / 24    9504: 26 / 22 / 26    12288: 30 / 24 / 28     18432: 32 / 34 / 34      32768: 50 / 46 / 52
 //   FP8 (6144)           9472: 19 / 22 / 26    9504: 24 / 22 / 26    12288: 26 / 26 / 28     18432: 28 / 36 / 38      32768: 44 / 52 / 54
-// (2-bit and per-row int4 take 72 to 80 registers however many they may: two and three are one.)
-template <int FMT> struct DenseCtas {
-    static constexpr int LO = FMT == 2 || FMT == 3 ? 3 : 2, HI = FMT == 8 ? 2 : FMT == 1 ? 3 : 4;
+// (2-bit and per-row int4 take 72 to 80 registers however many they may: two and three are one. 2-bit in more tiles than two an SM hold
+// takes what the compiler chooses, 63: one row of 12288 20 / 19, 18432 27 / 25 us, capped for three and four / so. int8 off 16-byte
+// rows has two: of 6150 x 32768 65, three 71.)
+// Five to eight rows: capped for two an SM (128 registers) where that beats the 100 to 120 that the compiler takes: capped / not, 6144 x 8192
+// FP8 16.6 / 18.6, 6150 x 12288 int8 36 / 43, 6150 x 4736 per-row int4 26 / 29; 6150 x 8192 MXFP4 34 / 31, 6150 x 2048 grouped int4 41 / 39, 6144 x 18432
+// 2-bit 42 / 39, 6144 x 32768 int8 51 / 50.
+template <int FMT, bool AL16> struct DenseCtas {
+    static constexpr int LO = FMT == 2 ? 3 : 2, HI = FMT == 8 || (FMT == 1 && !AL16) ? 2 : FMT == 1 ? 3 : 4;
 };
 static int dense_ctas(int lo, int hi, long ctas, int sms) {
     int best = lo;
@@ -846,18 +851,20 @@ static void launch_dense(DeviceCtx *c, const ColiCudaTensor *t, float *y, int S,
     const size_t rb = row_bytes(t->fmt, t->I);
     const int gs = t->gs > 0 ? t->gs : t->I;
     auto go = [&](auto kern) { launch_pdl(c, kern, grid, DENSE_WARPS * 32, 0, y, bq, bs, w, t->raw_s, S, t->I, t->O, rb, gs, t->ng); };
-    // More than 8 rows, 8-bit rows on 16 bytes: three waves of one CTA an SM against one of two and a rest (12 rows of 6144 x 9504 |
+    // More than 8 rows, one CTA an SM: int8 runs faster in the 178 registers of the compiler's choice than in the 211 it may take (16 rows of
+    // 6144 x 4736 17.4 / 18.6). 8-bit rows on 16 bytes: three waves of one CTA an SM against one of two and a rest (12 rows of 6144 x 9504 |
     // 12288 | 14208: int8 42 / 44 | 46 / 44 | 48 / 52, FP8 36 / 38 | 38 / 42 | 40 / 44 us; at two and four waves two an SM are as fast or faster)
     const bool three = ctas > 2L * c->sms && ctas <= 3L * c->sms;
     if (nc == 1) {
-        constexpr int LO = DenseCtas<FMT>::LO, HI = DenseCtas<FMT>::HI;
+        constexpr int LO = DenseCtas<FMT, AL16>::LO, HI = DenseCtas<FMT, AL16>::HI;
         const int k = dense_ctas(LO, HI, ctas, c->sms);
-        if (k == LO) go(k_dense_mma<FMT, 1, AL16, LO>);
+        if (k == LO) go(k_dense_mma<FMT, 1, AL16, FMT == 3 ? 3 : LO>);
+        else if (FMT == 3) go(k_dense_mma<FMT, 1, AL16, 0>);
         else if (k == HI) go(k_dense_mma<FMT, 1, AL16, HI>);
         else go(k_dense_mma<FMT, 1, AL16, (LO + HI) / 2>);
-    } else if (nc == 2) go(k_dense_mma<FMT, 2, AL16, 2>);
+    } else if (nc == 2) go(k_dense_mma<FMT, 2, AL16, FMT == 2 || FMT == 8 || (FMT == 1 && !AL16) ? 2 : 0>);
     else if (ctas > c->sms && !(AL16 && three)) go(k_dense_mma<FMT, 4, AL16, 2>);
-    else go(k_dense_mma<FMT, 4, AL16, 1>);
+    else go(k_dense_mma<FMT, 4, AL16, FMT == 1 ? 0 : 1>);
 }
 
 static int linear_raw(DeviceCtx *c, const ColiCudaTensor *t, float *y_dev, const float *x_dev, int S) {

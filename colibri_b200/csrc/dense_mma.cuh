@@ -14,11 +14,13 @@
 // FFMA, through a 256-entry shared-memory table for FP8: 163 us at 6144 x 8192 FP8 and 12 rows, 22 so (50 MB at 2.3 TB/s). Bound by the
 // latency of its loads (a warp multiplies a block with nothing of the next one requested), and 256 CTAs leave some of 148 SMs with
 // two and some with one.
-// CTAS: CTAs that share an SM; the registers of a thread are capped to that. More than 8 rows want 190 to 245 of them, and with one CTA
-// per SM a second wave runs behind the first; so when there are more CTAs than SMs the cap is for two (and spills a little: 1 % slower
-// where there are fewer CTAs than SMs, so not there). Up to four rows take two to four by format and number of CTAs (launch_dense, with the
-// figures). Call times with a cap and with the activations' fragments requested before the decoding, before / after, 12 rows of
-// 6144 x 8192: FP8 43 / 33, 2-bit 67 / 42, of 6150 x 8200: grouped int4 116 / 73, MXFP4 90 / 62, per-row int4 102 / 57. Requesting
+// CTAS: CTAs that share an SM; the registers of a thread are capped to that (0: the compiler's own choice). More than 8 rows take
+// 180 to 245 of them, and with one CTA per SM a second wave runs behind the first; so when there are more CTAs than SMs the cap is for
+// two (and spills a little: 1 % slower where there are fewer CTAs than SMs, so not there). Fewer rows take two to four by format and
+// number of CTAs (launch_dense, with the figures). AHEAD: the activations' fragments are requested together before the decoding, except under
+// that cap at more than 8 rows, where they cost more spills than they save waiting (ahead / not, 48 rows of 6144 x 8192: int8 68 / 57, FP8 56 / 53;
+// of 6150 x 8192: MXFP4 128 / 119, per-row int4 114 / 109). Call times before both / with both, 12 rows of 6144 x 8192: FP8 43 / 33, 2-bit 67 /
+// 42, of 6150 x 8200: grouped int4 116 / 71, MXFP4 90 / 61, per-row int4 102 / 57. Requesting
 // half a block or a block ahead was slower for rows on 16 bytes (FP8 33 / 38), for the registers it takes.
 // Rows need no alignment: without 16-byte rows, words come from aligned loads and funnel shifts, a run of 16 bytes from five (FP8, 6150
 // columns: 12 rows 132 / 50 us, one row 67 / 34, with a pair of loads for every word 72 and 67); raw
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__r
                                                                 int gs, int ng) {
     pdl_enter();
     constexpr bool RUN16 = dense_run16(FMT);
+    constexpr bool AHEAD = NC < 4 || CTAS == 1;         // all sets' fragments are requested together, before the decoding
     constexpr int VPW = (FMT == 1 || FMT == 8) ? 4 : FMT == 3 ? 16 : 8;      // values per 32-bit word
     __shared__ float2 s_part[DENSE_WARPS][NC][2][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -193,9 +196,9 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__r
         if (RUN16) {
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                uint4 b[NC][2];                                // all sets' fragments are requested together, before the decoding
+                uint4 b[NC][2];
 #pragma unroll
-                for (int cs = 0; cs < NC; cs++) {
+                for (int cs = 0; AHEAD && cs < NC; cs++) {
                     b[cs][0] = ldg128(bp[cs] + (size_t)kb * 256 + c * 128);
                     b[cs][1] = ldg128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
                 }
@@ -213,7 +216,8 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__r
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b0 = b[cs][0], b1 = b[cs][1];
+                    const uint4 b0 = AHEAD ? b[cs][0] : ldg128(bp[cs] + (size_t)kb * 256 + c * 128);
+                    const uint4 b1 = AHEAD ? b[cs][1] : ldg128(bp[cs] + (size_t)kb * 256 + c * 128 + 8);
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         mma_f16(bacc[cs][m], v[2 * m][0], v[2 * m + 1][0], v[2 * m][1], v[2 * m + 1][1], b0.x, b0.y);
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__r
             for (int c = 0; c < 4; c++) {
                 uint4 bf[NC];
 #pragma unroll
-                for (int cs = 0; cs < NC; cs++) bf[cs] = ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
+                for (int cs = 0; AHEAD && cs < NC; cs++) bf[cs] = ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
                 uint32_t v[4][4];
                 float sw[4] = {1.f, 1.f, 1.f, 1.f};
                 const int k = k0 + c * 32;
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, CTAS) k_dense_mma(float *__r
                 }
 #pragma unroll
                 for (int cs = 0; cs < NC; cs++) {
-                    const uint4 b = bf[cs];
+                    const uint4 b = AHEAD ? bf[cs] : ldg128(bp[cs] + (size_t)kb * 256 + c * 64);
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         float acc[4] = {0.f, 0.f, 0.f, 0.f};
