@@ -162,23 +162,9 @@ def test_expert_counts_that_are_not_multiples_of_four(be, oracle, E, K, M, gatin
     free_layer(be, (g, u, d, sh))
 
 
-@pytest.mark.parametrize("E,K", [(1, 1), (31, 31), (64, 8), (256, 8), (257, 16), (1000, 64), (1024, 1)])
-@pytest.mark.parametrize("gating,topp", [(0, 0.0), (1, 0.0), (1, 0.5)])
-def test_selection_passes_at_their_limits(be, oracle, E, K, gating, topp):
-    """The stand-alone routing kernel on rows that decide by the rule itself: ties across lanes, zeros of both signs, NaN and
-    infinities, every candidate below the starting value. Indices and weights are those of the oracle, bit for bit."""
-    rng = np.random.default_rng(E * 10 + K)
-    lg = rng.standard_normal((11, E), dtype=np.float32)
-    lg[1] = 0.25
-    lg[2] = np.round(lg[2])
-    lg[3, ::2] = np.nan
-    lg[4] = np.nan
-    lg[5, : E // 2] = -np.inf
-    lg[6, E // 2] = np.inf
-    lg[7] = -1e30 if gating == 0 else 200.0
-    bias = (rng.standard_normal(E) * 0.05).astype(np.float32)
-    bias[: E // 3] = -np.float32(1.0) / (np.float32(1.0) + np.exp(np.float32(-0.25)))      # sums of zero where the score is that
-    M = len(lg)
+def selection_is_the_oracles(be, oracle, lg, bias, K, gating, topp):
+    """coli_cuda_route_topk_dev on these rows: indices, weights and effective K of the oracle, bit for bit."""
+    M, E = lg.shape
     bufs = {}
     for name, a in (("lg", lg), ("bias", bias), ("idx", np.zeros((M, K), np.int32)), ("w", np.zeros((M, K), np.float32)),
                     ("keff", np.zeros(M, np.int32))):
@@ -203,3 +189,44 @@ def test_selection_passes_at_their_limits(be, oracle, E, K, gating, topp):
         assert np.all(same | (np.isnan(w[s, :k]) & np.isnan(ow[s, :k]))), s
     be.pipe_free(0, p("lg"))
     be.pipe_free(0, p("bias"))
+    return idx
+
+
+@pytest.mark.parametrize("E,K", [(1, 1), (31, 31), (64, 8), (256, 8), (257, 16), (1000, 64), (1024, 1)])
+@pytest.mark.parametrize("gating,topp", [(0, 0.0), (1, 0.0), (1, 0.5)])
+def test_selection_passes_at_their_limits(be, oracle, E, K, gating, topp):
+    """The stand-alone routing kernel on rows that decide by the rule itself: ties across lanes, sums of zero, NaN and
+    infinities, equal scores (saturated, or all underflowed but one sum)."""
+    rng = np.random.default_rng(E * 10 + K)
+    lg = rng.standard_normal((11, E), dtype=np.float32)
+    lg[1] = 0.25
+    lg[2] = np.round(lg[2])
+    lg[3, ::2] = np.nan
+    lg[4] = np.nan
+    lg[5, : E // 2] = -np.inf
+    lg[6, E // 2] = np.inf
+    lg[7] = -1e30 if gating == 0 else 200.0
+    bias = (rng.standard_normal(E) * 0.05).astype(np.float32)
+    bias[: E // 3] = -np.float32(1.0) / (np.float32(1.0) + np.exp(np.float32(-0.25)))      # sums of zero where the score is that
+    selection_is_the_oracles(be, oracle, lg, bias, K, gating, topp)
+
+
+@pytest.mark.parametrize("E,K", [(31, 31), (64, 8), (257, 16), (1000, 64)])
+@pytest.mark.parametrize("kind", ["some", "none", "equal", "ties"])
+@pytest.mark.parametrize("topp", [0.0, 0.5])
+def test_selection_among_negative_candidates(be, oracle, E, K, kind, topp):
+    """Biases that push candidates below zero and below the starting value of the search (-1e30): fewer than K candidates left, none
+    (entry kk is expert kk then), all equal at -1e20 (scores vanish in the sum), and negative ties across lanes."""
+    rng = np.random.default_rng(E + K)
+    lg = rng.standard_normal((5, E), dtype=np.float32)
+    bias = np.where(np.arange(E) % 2, -np.inf, -2e30).astype(np.float32)
+    if kind == "some":
+        bias[rng.permutation(E)[:K // 2]] = [-3e5, -0.5, 0.25, -1e29][E % 4]
+    elif kind == "equal":
+        bias[:] = -1e20
+    elif kind == "ties":
+        bias = -np.float32(2.0) ** rng.integers(10, 16, E).astype(np.float32)
+        lg = np.round(lg)
+    idx = selection_is_the_oracles(be, oracle, lg, bias, K, 1, topp)
+    if topp == 0.0 and kind in ("none", "equal"):
+        assert np.array_equal(idx, np.tile(np.arange(K, dtype=np.int32), (len(lg), 1)))
