@@ -1048,7 +1048,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         }
     }
     // every thread observes the completion itself, which also makes the copied bytes visible to it
-    if (nslot > 0 && !mbar_wait_bounded(hbar, 0)) { wr.ok = false; it.live = 0; }
+    if (nslot > 0 && !mbar_wait_bounded(hbar, 0)) {
+        wr.ok = false; it.live = 0;
+        mbar_wait_bounded(hbar, 0);      // (once more, as for every copy behind an expired wait; here and not at the end, where it cost 1 %)
+    }
     DEC_PROBE(a, 6);
     if (a.local2) {
         // ---- down with a local combine: this CTA's 16 output rows over every pass ------------
@@ -1212,7 +1215,6 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         if (tid == 0) kstat_set(a.status, sh->failed == 2 ? KSTAT_MBAR_TIMEOUT : KSTAT_GRID_TIMEOUT);
         // copies still in flight land before the shared memory goes away (bounded)
         dec_drain(wr);
-        if (nslot > 0) mbar_wait_bounded(hbar, 0);
     }
 }
 
