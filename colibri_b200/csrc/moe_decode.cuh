@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 1) k_moe_decode(DecodeArgs a, 
         }
         __syncthreads();
     } else {
-// Eight neighbouring lanes share an entry and compare it with an eighth of the others each. An expert's first entry
+        // Eight neighbouring lanes share an entry and compare it with an eighth of the others each. An expert's first entry
         // stands for its place in the union (first-appearance order): packed rows and passes before it are those of the
         // experts with an earlier first entry. Two barriers; searching entry by entry with one barrier per table took 6 us at four
         // rows, this takes 2.
